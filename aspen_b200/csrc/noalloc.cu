@@ -1,23 +1,23 @@
-// aspen_b200_matmul_noalloc: one matmul layer run as a tile graph by the persistent scheduler
-// kernel, for callers that must not allocate.
+// aspen_b200_matmul_noalloc: one matmul layer for callers that must not allocate.
 //
 // Who cannot allocate: plug-ins that are handed a fixed memory budget by their host framework (a
 // serving runtime that pre-sizes every pool at start-up and treats a later cudaMalloc as a bug), and
 // latency-critical loops where the implicit device synchronisation of cudaMalloc / cudaFree is not
 // acceptable.  The regular API builds a device image per nasm (arena, descriptors, counters, queue)
-// with cudaMalloc; this entry point keeps everything the scheduler needs besides the caller's own
-// input / weight / output buffers in one file-scope device array of fixed size.
+// with cudaMalloc; a single layer has no dependencies between its tiles, so this entry point is one kernel
+// launch over the output blocks that needs no memory besides the caller's own buffers, and one wait.
 //
-// Consequences of the fixed array, all documented in the header too:
-//   * sizes are limited (NOALLOC_MAX_TILES output tiles of 128 x 128); larger calls are rejected;
-//   * every call on a device uses the same array: it keeps the previous call's contents, so the
-//     set-up kernel rewrites all of it that a run reads (counters and queue start from zero again);
-//     two calls that overlap on the GPU (different streams, or different host threads) race;
-//   * the first call on a device looks the array's address up (cudaGetSymbolAddress) -- make that
-//     call before any stream capture;
-//   * every call ends by reading the scheduler's status back and synchronising its stream.
+//   * n_cols <= 8 (a few tokens): the layer reads its weights once and does next to nothing else, so a warp takes one
+//     weight row, its lanes stride over k with wide loads, and the dot products with all columns end in a
+//     warp reduction -- every SM pulls weights at once, which no 32-row block shape achieves here.
+//     The line lies at 8: with 16 columns the 32 x 32 blocks below are faster (19.9 against 23.6 us at k = 768, m = 3072).
+//   * larger: the fp32 FMA blocks of gemm_ffma.cuh, shape by `pick_shape`.
+// B200, wall time of a call, launch and wait included (before: the tile queue of the scheduler kernel, set up by a kernel of
+// its own, scalar FMAs from global memory):  1 x 768 x 768 97 -> 14 us, 333 x 770 x 1000 2447 -> 42 us,
+// 4096 x 768 x 3072 4650 -> 470 us (columns x k x rows).
 #include "internal.h"
-#include "scheduler.cuh"
+#include "tiles_simt.cuh"
+#include "gemm_ffma.cuh"
 
 #include <cuda_runtime.h>
 #include <algorithm>
@@ -27,76 +27,158 @@ namespace {
 constexpr unsigned NOALLOC_MAX_TILES = ASPEN_B200_NOALLOC_MAX_TILES;
 constexpr unsigned NOALLOC_TILE = 128;
 
-struct NoAllocScratch {
-    CtrlDev ctrl;
-    StatusHost status;
-    NasmDev nasm;
-    LayerDev layer;
-    unsigned layer_done, layer_tiles, layers_completed, completed;
-    unsigned queue[NOALLOC_MAX_TILES];
-    unsigned dep[NOALLOC_MAX_TILES];
-    TileDev tiles[NOALLOC_MAX_TILES];
-};
-
-// The scratch memory itself.  In host code this name is only a handle for cudaGetSymbolAddress, never
-// a pointer a kernel could use.
-static __device__ __align__(256) unsigned char g_noalloc_scratch[sizeof(NoAllocScratch)];
-
-struct NoAllocArgs {
+struct Args {
     const float *x, *w, *bias;
     float *out;
     unsigned n_cols, k, m;
     int act;
-    unsigned long long stall_ns, pipe_ns;
+    bool vec_out;             // rows of out start on 16-byte boundaries
 };
 
-// Rebuilds the whole image in the scratch array: descriptors, zeroed counters, a queue that already
-// holds every tile (a single layer has no dependencies between its tiles).
-__global__ void noalloc_setup(NoAllocScratch *s, NoAllocArgs a) {
-    const unsigned tiles_h = (a.m + NOALLOC_TILE - 1) / NOALLOC_TILE, tiles_w = (a.n_cols + NOALLOC_TILE - 1) / NOALLOC_TILE;
-    const unsigned n = tiles_h * tiles_w;
-    const unsigned stride = gridDim.x * blockDim.x, t0 = blockIdx.x * blockDim.x + threadIdx.x;
-    for (unsigned t = t0; t < n; t += stride) {
-        TileDev T;
-        T.layer = 0;
-        T.pos_h = (t % tiles_h) * NOALLOC_TILE;
-        T.pos_w = (t / tiles_h) * NOALLOC_TILE;
-        T.tile_h = min(NOALLOC_TILE, a.m - T.pos_h);
-        T.tile_w = min(NOALLOC_TILE, a.n_cols - T.pos_w);
-        T.child_off = 0; T.child_cnt = 0; T.need = 0; T.flags = 0;
-        s->tiles[t] = T;
-        s->queue[t] = t + 1u;
-        s->dep[t] = 0u;
+// VEC consecutive values of a row in one load (16, 8 or 4 bytes, whatever every row's alignment allows); zeros outside.
+template <int VEC>
+struct Rows {
+    const float *base;
+    unsigned rows, k;
+    __device__ __forceinline__ float4 operator()(unsigned row, unsigned k0) const {
+        float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (row >= rows) return v;
+        const float *p = base + (size_t)row * k + k0;
+        if (VEC == 4) {
+            if (k0 < k) v = __ldg(reinterpret_cast<const float4 *>(p));
+        } else if (VEC == 2) {
+            if (k0 < k) { const float2 a = __ldg(reinterpret_cast<const float2 *>(p)); v.x = a.x; v.y = a.y; }
+            if (k0 + 2u < k) { const float2 a = __ldg(reinterpret_cast<const float2 *>(p + 2)); v.z = a.x; v.w = a.y; }
+        } else {
+            if (k0 < k) v.x = __ldg(p);
+            if (k0 + 1u < k) v.y = __ldg(p + 1);
+            if (k0 + 2u < k) v.z = __ldg(p + 2);
+            if (k0 + 3u < k) v.w = __ldg(p + 3);
+        }
+        return v;
     }
-    if (t0 != 0) return;
-    LayerDev L;
-    memset(&L, 0, sizeof L);
-    L.type = MATMUL_LAYER; L.act = a.act;
-    L.out = a.out; L.ldc = a.m; L.H = a.m; L.W = a.n_cols;
-    L.in0 = a.x; L.ld0 = a.k; L.H0 = a.k;
-    L.weight = a.w; L.bias = a.bias;
-    L.K = a.k; L.Kpad = a.k; L.rows = a.m;
-    L.wmap = -1; L.amap = -1; L.resmap = -1; L.bw = 128;
-    L.a_vec4 = (a.k % 4 == 0) && ((reinterpret_cast<uintptr_t>(a.x) | reinterpret_cast<uintptr_t>(a.w)) % 16 == 0);
-    s->layer = L;
-    NasmDev G;
-    memset(&G, 0, sizeof G);
-    G.layers = &s->layer; G.tiles = s->tiles; G.children = s->dep; G.dep = s->dep; G.dep_init = s->dep;
-    G.layer_done = &s->layer_done; G.layer_tiles = &s->layer_tiles; G.init_ready = s->queue;
-    G.layers_completed = &s->layers_completed; G.completed = &s->completed;
-    G.n_tiles = n; G.n_layers = 1; G.n_init = n;
-    s->nasm = G;
-    s->layer_done = 0; s->layer_tiles = n; s->layers_completed = 0; s->completed = 0;
-    s->status.status = 0; s->status.info0 = 0; s->status.info1 = 0; s->status.tiles_done = 0;
-    CtrlDev c;
-    memset(&c, 0, sizeof c);
-    c.head = 0; c.tail = n; c.done = 0; c.total = n; c.cap = n; c.n_nasm = 1;
-    c.stall_ns = a.stall_ns; c.pipe_ns = a.pipe_ns;
-    s->ctrl = c;
+};
+
+struct Finish {
+    const Args &a;
+    unsigned m0, n0;
+    __device__ __forceinline__ void operator()(unsigned mi, unsigned ni, const float *v) const {
+        const unsigned m = m0 + mi, n = n0 + ni;
+        if (n >= a.n_cols || m >= a.m) return;
+        float r[4];
+        #pragma unroll
+        for (unsigned j = 0; j < 4; j++) r[j] = activate(v[j] + (a.bias && m + j < a.m ? __ldg(a.bias + m + j) : 0.f), a.act);
+        float *o = a.out + (size_t)n * a.m + m;
+        if (a.vec_out && m + 4u <= a.m) *reinterpret_cast<float4 *>(o) = make_float4(r[0], r[1], r[2], r[3]);
+        else
+            #pragma unroll
+            for (unsigned j = 0; j < 4; j++) if (m + j < a.m) o[j] = r[j];
+    }
+};
+
+// Block operand: VEC-wide asynchronous copies of a row's values.
+template <int VEC, int NR>
+struct Stage {
+    const float *base;
+    unsigned rows, k;
+    const float *p[NR];
+    bool ok[NR];
+    unsigned k0;
+    __device__ __forceinline__ Stage(const float *b, unsigned r, unsigned kk) : base(b), rows(r), k(kk), k0(0) {}
+    __device__ __forceinline__ void row(int i, unsigned r) { ok[i] = r < rows; p[i] = base + (size_t)(ok[i] ? r : 0u) * k; }
+    __device__ __forceinline__ void at(unsigned kk) { k0 = kk; }
+    __device__ __forceinline__ void copy(unsigned dst, int i) const {
+        #pragma unroll
+        for (unsigned e = 0; e < 4; e += VEC) {
+            const bool in = ok[i] && k0 + e < k;
+            fmablk::copy_async<VEC * 4>(dst + e * 4u, in ? p[i] + k0 + e : base, in);
+        }
+    }
+};
+
+struct BlockBarrier { __device__ __forceinline__ void operator()() const { __syncthreads(); } };
+
+template <typename S, int VEC>
+__global__ void __launch_bounds__(fmablk::THREADS, 2) matmul_blocks(const Args a) {
+    extern __shared__ __align__(128) unsigned char smem[];
+    const unsigned m0 = blockIdx.x * S::BM, n0 = blockIdx.y * S::BN;
+    Stage<VEC, S::RW> lw(a.w + (size_t)m0 * a.k, a.m - m0, a.k);
+    Stage<VEC, S::RX> lx(a.x + (size_t)n0 * a.k, a.n_cols - n0, a.k);
+    Finish fin{a, m0, n0};
+    fmablk::block<S>(smem, threadIdx.x, a.k, lw, lx, BlockBarrier(), fin);
 }
 
-NoAllocScratch *g_scratch_ptr[16] = {};
-size_t g_smem_bytes = sizeof(tc::Shared) + 1024;
+// One weight row per warp, N columns (the last ones may be missing).
+template <int N, int VEC>
+__global__ void __launch_bounds__(fmablk::THREADS) matmul_rows(const Args a) {
+    const unsigned m = blockIdx.x * (fmablk::THREADS / 32) + threadIdx.x / 32, lane = threadIdx.x % 32;
+    if (m >= a.m) return;
+    const Rows<VEC> w{a.w, a.m, a.k}, x{a.x, a.n_cols, a.k};
+    float acc[N];
+    #pragma unroll
+    for (int n = 0; n < N; n++) acc[n] = 0.f;
+    constexpr unsigned STEP = 128;
+    constexpr int U = N == 1 ? 8 : N <= 4 ? 4 : 2;                         // weight pieces in flight per lane
+    for (unsigned k0 = lane * 4u; k0 < a.k; k0 += U * STEP) {
+        float4 wv[U];
+        #pragma unroll
+        for (int u = 0; u < U; u++) wv[u] = w(m, k0 + u * STEP);
+        #pragma unroll
+        for (int u = 0; u < U; u++)
+            #pragma unroll
+            for (int n = 0; n < N; n++) {
+                const float4 xv = x(n, k0 + u * STEP);
+                acc[n] = fmaf(wv[u].x, xv.x, acc[n]); acc[n] = fmaf(wv[u].y, xv.y, acc[n]);
+                acc[n] = fmaf(wv[u].z, xv.z, acc[n]); acc[n] = fmaf(wv[u].w, xv.w, acc[n]);
+            }
+    }
+    float mine = 0.f;
+    #pragma unroll
+    for (int n = 0; n < N; n++) {
+        #pragma unroll
+        for (int o = 16; o > 0; o >>= 1) acc[n] += __shfl_xor_sync(0xffffffffu, acc[n], o);
+        if ((int)lane == n) mine = acc[n];
+    }
+    if (lane < N && lane < a.n_cols) a.out[(size_t)lane * a.m + m] = activate(mine + (a.bias ? __ldg(a.bias + m) : 0.f), a.act);
+}
+
+// Shape with the shortest longest SM: blocks are dealt whole, so an SM runs ceil(blocks / SMs) of them, each
+// BM * BN * k FMAs at the shape's share of the FMA rate (one block of k = 3072 alone on its SM: 190, 96 and 30 us).
+unsigned pick_shape(unsigned n_cols, unsigned m, unsigned sms) {
+    static const struct { unsigned bm, bn; float rate; } shapes[] = {{128, 64, 0.80f}, {64, 64, 0.80f}, {32, 32, 0.65f}};
+    unsigned best = 0;
+    float best_cost = 0.f;
+    for (unsigned i = 0; i < 3; i++) {
+        const unsigned bm = shapes[i].bm, bn = shapes[i].bn;
+        const unsigned long long blocks = (unsigned long long)((m + bm - 1) / bm) * ((n_cols + bn - 1) / bn);
+        const float cost = (float)((blocks + sms - 1) / sms) * (float)(bm * bn) / shapes[i].rate;
+        if (i == 0 || cost < best_cost) { best = i; best_cost = cost; }
+    }
+    return best;
+}
+
+template <typename S, int VEC>
+void launch_blocks(const Args &a, cudaStream_t stream) {
+    // the attribute is per device; asking for it on every call costs a fraction of the launch
+    cudaFuncSetAttribute(matmul_blocks<S, VEC>, cudaFuncAttributeMaxDynamicSharedMemorySize, S::SMEM_BYTES);
+    matmul_blocks<S, VEC><<<dim3((a.m + S::BM - 1) / S::BM, (a.n_cols + S::BN - 1) / S::BN), fmablk::THREADS, S::SMEM_BYTES, stream>>>(a);
+}
+
+template <int VEC>
+void launch(const Args &a, unsigned sms, cudaStream_t stream) {
+    if (a.n_cols <= 8) {
+        const unsigned grid = (a.m + fmablk::THREADS / 32 - 1) / (fmablk::THREADS / 32);
+        if (a.n_cols == 1) matmul_rows<1, VEC><<<grid, fmablk::THREADS, 0, stream>>>(a);
+        else if (a.n_cols == 2) matmul_rows<2, VEC><<<grid, fmablk::THREADS, 0, stream>>>(a);
+        else if (a.n_cols <= 4) matmul_rows<4, VEC><<<grid, fmablk::THREADS, 0, stream>>>(a);
+        else matmul_rows<8, VEC><<<grid, fmablk::THREADS, 0, stream>>>(a);
+        return;
+    }
+    const unsigned shape = pick_shape(a.n_cols, a.m, sms);
+    if (shape == 0) launch_blocks<fmablk::Large, VEC>(a, stream);
+    else if (shape == 1) launch_blocks<fmablk::Medium, VEC>(a, stream);
+    else launch_blocks<fmablk::Small, VEC>(a, stream);
+}
 
 }  // namespace
 
@@ -110,37 +192,23 @@ extern "C" int aspen_b200_matmul_noalloc(const float *x_dev, const float *w_dev,
     // 64-bit: m or n_cols close to 2^32 must not wrap into a small tile count
     const unsigned long long tiles = (((unsigned long long)m + NOALLOC_TILE - 1) / NOALLOC_TILE) * (((unsigned long long)n_cols + NOALLOC_TILE - 1) / NOALLOC_TILE);
     if (tiles > NOALLOC_MAX_TILES) {
-        ASPEN_ERR("aspen_b200_matmul_noalloc: %u x %u outputs need %llu tiles of 128 x 128; the fixed scratch array holds %u. "
+        ASPEN_ERR("aspen_b200_matmul_noalloc: %u x %u outputs need %llu tiles of 128 x 128; the limit is %u. "
                   "Use the regular API (it allocates) for larger layers.\n", m, n_cols, tiles, NOALLOC_MAX_TILES);
         return -2;
     }
-    int dev = 0;
+    int dev = 0, sms = 0;
     cudaError_t err = cudaGetDevice(&dev);
-    if (err != cudaSuccess || dev < 0 || dev >= 16) { ASPEN_ERR("aspen_b200_matmul_noalloc: no current CUDA device (%s)\n", cudaGetErrorString(err)); return -3; }
-    if (!g_scratch_ptr[dev]) {
-        // once per device, with that device current: the device address behind the symbol
-        void *p = nullptr;
-        err = cudaGetSymbolAddress(&p, g_noalloc_scratch);
-        if (err != cudaSuccess || !p) { ASPEN_ERR("aspen_b200_matmul_noalloc: cudaGetSymbolAddress failed: %s\n", cudaGetErrorString(err)); return -3; }
-        g_scratch_ptr[dev] = static_cast<NoAllocScratch *>(p);
-    }
-    NoAllocScratch *s = g_scratch_ptr[dev];
-    int sms = 0;
-    err = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    if (err != cudaSuccess || sms <= 0) { ASPEN_ERR("aspen_b200_matmul_noalloc: cannot query the device (%s)\n", cudaGetErrorString(err)); return -3; }
+    if (err == cudaSuccess) err = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    if (err != cudaSuccess || sms <= 0) { ASPEN_ERR("aspen_b200_matmul_noalloc: no current CUDA device (%s)\n", cudaGetErrorString(err)); return -3; }
     cudaStream_t stream = static_cast<cudaStream_t>(cuda_stream);
-    NoAllocArgs a{x_dev, w_dev, bias_dev, out_dev, n_cols, k, m, activation, 2000000000ull, 1000000000ull};
-    noalloc_setup<<<(unsigned)((tiles + 255) / 256), 256, 0, stream>>>(s, a);
-    const unsigned ctas = (unsigned)std::min<unsigned long long>(tiles, (unsigned long long)sms);
-    sched::scheduler_kernel<false><<<ctas, sched::SCHED_THREADS, g_smem_bytes, stream>>>(&s->nasm, &s->ctrl, s->queue, &s->status, nullptr);
+    const Args a{x_dev, w_dev, bias_dev, out_dev, n_cols, k, m, activation, m % 4 == 0 && reinterpret_cast<uintptr_t>(out_dev) % 16 == 0};
+    const uintptr_t align = reinterpret_cast<uintptr_t>(x_dev) | reinterpret_cast<uintptr_t>(w_dev);
+    if (k % 4 == 0 && align % 16 == 0) launch<4>(a, (unsigned)sms, stream);
+    else if (k % 2 == 0 && align % 8 == 0) launch<2>(a, (unsigned)sms, stream);
+    else launch<1>(a, (unsigned)sms, stream);
     err = cudaGetLastError();
     if (err != cudaSuccess) { ASPEN_ERR("aspen_b200_matmul_noalloc: launch failed: %s\n", cudaGetErrorString(err)); return -3; }
-    // synchronous: the status word lives in the scratch array and the next call overwrites it
-    unsigned status[2] = {0, 0};
-    err = cudaMemcpyAsync(&status[0], const_cast<const unsigned *>(&s->status.status), sizeof(unsigned), cudaMemcpyDeviceToHost, stream);
-    if (err == cudaSuccess) err = cudaMemcpyAsync(&status[1], &s->completed, sizeof(unsigned), cudaMemcpyDeviceToHost, stream);
-    if (err == cudaSuccess) err = cudaStreamSynchronize(stream);
+    err = cudaStreamSynchronize(stream);
     if (err != cudaSuccess) { ASPEN_ERR("aspen_b200_matmul_noalloc: %s\n", cudaGetErrorString(err)); return -3; }
-    if (status[0] != 0 || status[1] != 1) { ASPEN_ERR("aspen_b200_matmul_noalloc: scheduler status %u, completed %u\n", status[0], status[1]); return -4; }
     return 0;
 }
