@@ -18,7 +18,6 @@
 namespace fmablk {
 
 constexpr unsigned THREADS = 256;
-constexpr int STAGES = 3;
 
 __device__ __forceinline__ void fma2(unsigned long long &d, unsigned long long a, unsigned long long b) {
     asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(d) : "l"(a), "l"(b));
@@ -35,9 +34,9 @@ __device__ __forceinline__ void copy_async(unsigned dst, const void *src, bool o
     else asm volatile("cp.async.ca.shared.global [%0], [%1], %2, %3;" ::"r"(dst), "l"(src), "n"(BYTES), "r"(ok ? (unsigned)BYTES : 0u) : "memory");
 }
 
-template <int BM_, int BN_, int TM_, int TN_, int KS_>
+template <int BM_, int BN_, int TM_, int TN_, int KS_, int STAGES_ = 3>
 struct Shape {
-    static constexpr int BM = BM_, BN = BN_, TM = TM_, TN = TN_, KS = KS_;
+    static constexpr int BM = BM_, BN = BN_, TM = TM_, TN = TN_, KS = KS_, STAGES = STAGES_;
     static constexpr int KT = KS * 32;                                // k values per step
     static constexpr int STAGE_BYTES = (BM + BN) * 128 * KS;          // [slice][W rows, X rows][32 k]
     static constexpr int RED_BYTES = KS > 1 ? KS * BN * (BM + 4) * 4 : 0;
@@ -49,6 +48,7 @@ struct Shape {
 typedef Shape<128, 64, 8, 4, 1> Large;
 typedef Shape<64, 64, 8, 4, 2> Medium;
 typedef Shape<32, 32, 4, 4, 4> Small;
+typedef Shape<64, 32, 4, 2, 1, 2> Tight;      // 24 KB of staging, beside the tensor-core ring
 
 // Loader (one per operand):  void row(int i, unsigned r): row r of the block is this thread's i-th row;
 //     void at(unsigned k): the pieces that follow start at k;  void copy(unsigned dst, int i): stage 4 values of row i.
@@ -71,7 +71,7 @@ __device__ __forceinline__ void block(unsigned char *smem, unsigned tid, unsigne
         if (step < steps) {
             #pragma unroll
             for (int s = 0; s < S::KS; s++) {
-                const unsigned slice = base + (step % STAGES) * S::STAGE_BYTES + s * (S::BM + S::BN) * 128;
+                const unsigned slice = base + (step % S::STAGES) * S::STAGE_BYTES + s * (S::BM + S::BN) * 128;
                 const unsigned k = step * S::KT + s * 32u + piece * 4u;
                 loadw.at(k);
                 #pragma unroll
@@ -96,18 +96,18 @@ __device__ __forceinline__ void block(unsigned char *smem, unsigned tid, unsigne
         #pragma unroll
         for (int j = 0; j < S::TN; j++) acc[i][j] = 0ull;
     #pragma unroll
-    for (int s = 0; s < STAGES - 1; s++) stage(s);
+    for (int s = 0; s < S::STAGES - 1; s++) stage(s);
     for (unsigned step = 0; step < steps; step++) {
-        asm volatile("cp.async.wait_group %0;" ::"n"(STAGES - 2) : "memory");
+        asm volatile("cp.async.wait_group %0;" ::"n"(S::STAGES - 2) : "memory");
         bar();                                        // everybody's copies of this step have landed, the oldest stage is free
-        stage(step + STAGES - 1);
-        const unsigned char *w = smem + (step % STAGES) * S::STAGE_BYTES + group * (S::BM + S::BN) * 128 + ty * 512;
-        const unsigned char *x = smem + (step % STAGES) * S::STAGE_BYTES + group * (S::BM + S::BN) * 128 + S::BM * 128 + tx * 512;
+        stage(step + S::STAGES - 1);
+        const unsigned char *w = smem + (step % S::STAGES) * S::STAGE_BYTES + group * (S::BM + S::BN) * 128 + ty * 512;
+        const unsigned char *x = smem + (step % S::STAGES) * S::STAGE_BYTES + group * (S::BM + S::BN) * 128 + S::BM * 128 + tx * (S::TN * 128);
         #pragma unroll
         for (unsigned c = 0; c < 8; c++) {            // 4 values of k at a time
             ulonglong2 b[S::TN];
             #pragma unroll
-            for (int j = 0; j < S::TN; j++) b[j] = *reinterpret_cast<const ulonglong2 *>(x + j * 128 + ((c ^ (tx & 7u)) << 4));
+            for (int j = 0; j < S::TN; j++) b[j] = *reinterpret_cast<const ulonglong2 *>(x + j * 128 + ((c ^ ((tx * S::TN / 4u) & 7u)) << 4));
             #pragma unroll
             for (int i = 0; i < S::TM; i++) {
                 const ulonglong2 a = *reinterpret_cast<const ulonglong2 *>(w + (i / 4) * (S::BM * 64) + (i % 4) * 128 + ((c ^ (ty & 7u)) << 4));
@@ -122,7 +122,7 @@ __device__ __forceinline__ void block(unsigned char *smem, unsigned tid, unsigne
             #pragma unroll
             for (int i = 0; i < S::TM; i += 4) {
                 const float v[4] = {pair_sum(acc[i][j]), pair_sum(acc[i + 1][j]), pair_sum(acc[i + 2][j]), pair_sum(acc[i + 3][j])};
-                out(4u * ty + (i / 4) * (S::BM / 2), 4u * tx + j, v);
+                out(4u * ty + (i / 4) * (S::BM / 2), S::TN * tx + j, v);
             }
         bar();
     } else {
@@ -134,7 +134,7 @@ __device__ __forceinline__ void block(unsigned char *smem, unsigned tid, unsigne
         for (int j = 0; j < S::TN; j++)
             #pragma unroll
             for (int i = 0; i < S::TM; i += 4)
-                *reinterpret_cast<float4 *>(red + (group * S::BN + 4u * tx + j) * P + 4u * ty + (i / 4) * (S::BM / 2)) =
+                *reinterpret_cast<float4 *>(red + (group * S::BN + S::TN * tx + j) * P + 4u * ty + (i / 4) * (S::BM / 2)) =
                     make_float4(pair_sum(acc[i][j]), pair_sum(acc[i + 1][j]), pair_sum(acc[i + 2][j]), pair_sum(acc[i + 3][j]));
         bar();
         #pragma unroll

@@ -75,26 +75,14 @@ extern "C" int aspen_b200_dnn_set_embedding(aspen_dnn_t *dnn, const float *token
 extern "C" void aspen_b200_rpool_add_nasm_tokens(rpool_t *rpool, nasm_t *nasm, const int *token_ids) {
     if (!rpool || !nasm || !token_ids) { ASPEN_ERR("ERROR: aspen_b200_rpool_add_nasm_tokens: NULL argument.\n"); return; }
     if (!rpool->engine) { ASPEN_ERR("ERROR: aspen_b200_rpool_add_nasm_tokens: attach the rpool to a dse group first (the gather runs on its device).\n"); return; }
-    if (engine_in_service(rpool->engine)) {
-        if (!nasm->has_graph) { ASPEN_ERR("ERROR: aspen_b200_rpool_add_nasm_tokens: nasm has no dependency graph.\n"); return; }
-        if (nasm->rpool && nasm->rpool != rpool) { ASPEN_ERR("ERROR: aspen_b200_rpool_add_nasm_tokens: nasm already belongs to another rpool.\n"); return; }
-        bool present = false;
-        for (nasm_t *n : rpool->nasms) present |= n == nasm;
-        if (!present) rpool->nasms.push_back(nasm);
-        nasm->rpool = rpool;
-        nasm->completed.store(0);
-        if (engine_service_tokens(rpool->engine, nasm, token_ids) != 0) ASPEN_ERR("ERROR: aspen_b200_rpool_add_nasm_tokens: device upload failed.\n");
-        return;
-    }
-    // the graph joins the pool exactly as with a raw input (image built on first use); layer 0 is then filled from the ids
-    if (!nasm->dev || nasm->rpool != rpool) {
-        rpool_add_nasm_raw_input(rpool, nasm, nullptr);
-        if (!nasm->dev) return;
-    } else {
-        nasm->completed.store(0);
-        if (engine_rearm(rpool->engine, nasm) != 0) return;
-    }
-    if (engine_set_tokens(nasm, token_ids) != 0) ASPEN_ERR("ERROR: aspen_b200_rpool_add_nasm_tokens: device gather failed.\n");
+    if (!nasm->has_graph) { ASPEN_ERR("ERROR: aspen_b200_rpool_add_nasm_tokens: nasm has no dependency graph.\n"); return; }
+    if (nasm->rpool && nasm->rpool != rpool) { ASPEN_ERR("ERROR: aspen_b200_rpool_add_nasm_tokens: nasm already belongs to another rpool.\n"); return; }
+    bool present = false;
+    for (nasm_t *n : rpool->nasms) present |= n == nasm;
+    if (!present) rpool->nasms.push_back(nasm);
+    nasm->rpool = rpool;
+    nasm->completed.store(0);
+    if (engine_attach_tokens(rpool->engine, nasm, token_ids) != 0) ASPEN_ERR("ERROR: aspen_b200_rpool_add_nasm_tokens: device upload failed.\n");
 }
 
 extern "C" void rpool_add_nasm(rpool_t *rpool, nasm_t *nasm, char *input_filename) {

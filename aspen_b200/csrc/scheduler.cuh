@@ -1,25 +1,42 @@
 // Persistent device-side dataflow scheduler: the B200 counterpart of the reference's DSE worker
 // loop (dse_schedule, ref src/dse.c:20-108) and ready pool (ref src/rpool.c:390-685).
 //
-// One CTA per SM stays resident for a whole run.  Its control warp
+// One CTA per SM stays resident for a whole launch.  Its scheduler warp
 //   pops a ready tile      (rpool_fetch_ninsts)     ticket = atomicAdd(head); wait for queue[ticket]
 //   lets the CTA run it    (switch on layer type, ref src/dse.c:39-79)
-//   accounts completion    (layer counter -> layers-completed counter -> completed flag, ref src/dse.c:80-106)
 //   updates the children   (update_children_but_prioritize_dse_target, ref src/dse.c:363-401):
 //                          atomicAdd on each child's dependency counter; a child whose last parent
 //                          this was becomes ready; the first such child is kept as this CTA's next
-//                          tile (depth first, no queue round trip), the others are pushed.
+//                          tile (depth first, no queue round trip), the others are pushed
+//   accounts completion    one counter per graph; its last tile ends the graph's pass (ref src/dse.c:80-106)
 // There is no kernel boundary and no barrier between layers: a tile fires as soon as its own
 // parent tiles are complete.
 //
-// The queue is a ticket ring: every tile is pushed at most once per run (per pass in service mode,
-// where the ring holds a fixed number of passes and the kernel is launched again when they are used
-// up), so it never wraps; slot value = global tile id + 1, 0 = not yet filled.  A popper that holds a
-// ticket whose slot is still empty waits -- bounded: when no tile anywhere completes for
+// Passes.  The host asks for pass number p of a graph by writing p to the graph's SVC_TARGET word.  An idle scheduler
+// warp that finds an idle graph with target != started claims it (CAS on SVC_IDLE) and pushes its layer-0 tiles; those
+// prepare the input, everything else follows from the dependency counters.  The warp that retires the last tile of a
+// pass writes the pass number to the graph's mapped host word and marks the graph idle.
+//   A launch per run (dse_group_run by default): the passes owed are written before the launch, and the kernel leaves when
+//   none is left.
+//   Service mode: the kernel stays resident while the host keeps asking (the counterpart of the reference's DSE threads,
+//   which run from dse_group_run to dse_group_stop and serve whatever rpool_add_nasm brings, ref src/dse.c:20-108,
+//   215-232).  It leaves -- without error -- when no pass is running or asked for and the host has asked it to
+//   stop, when nothing has run for idle_ns, or when the queue of this launch is used up; the host launches it
+//   again if work is left.
+// The counters are never reset between the passes of a launch: a pass only starts when the previous one of its graph is
+// complete, so a child is ready whenever its counter reaches a multiple of the count it waits for.
+//
+// The queue is a ticket ring with room for a fixed number of passes, so it never wraps; 0 = slot not yet filled.  A popper
+// that holds a ticket whose slot is still empty waits -- bounded: when no tile anywhere completes for
 // `stall_ns` it records ASPEN_B200_ERR_STALL, raises the abort flag and every CTA leaves.
 //
-// Memory ordering: tile data is written by the worker threads; bar.sync orders it before the
-// control warp's fence.acq_rel.gpu + relaxed atomicAdd on the child counter (release).  The CTA
+// Latency.  From the last store of a tile to the first load of the tile it makes ready lie the scheduler's round trips to
+// L2 (about 0.4 us each): fence, child counters, fence, and -- through the queue -- tail, slot, the popper's poll, the
+// descriptors.  What can be known earlier is fetched earlier: a tile's child list while the tile runs; queue entries and
+// child lists name the layer and the graph, so that a tile's descriptor and its layer's are read side by side.
+//
+// Memory ordering: tile data is written by the worker threads; their mbarrier arrivals order it before the
+// scheduler warp's fence.acq_rel.gpu + relaxed atomicAdd on the child counter (release).  The CTA
 // whose increment completes the count fences again after the atomic (acquiring every earlier
 // parent's data through the counter's RMW chain) before it publishes or keeps the child.
 #pragma once
@@ -29,6 +46,10 @@ namespace sched {
 
 constexpr unsigned PROF_LAYERS = 256;
 constexpr unsigned PROF_SLOTS = 2 + 2 * PROF_LAYERS + 2;
+
+// A ready tile: low word = local tile id + 1 (0: none), high word = graph << 16 | layer.
+typedef unsigned long long Entry;
+__device__ __forceinline__ Entry make_entry(unsigned tile, unsigned g, unsigned layer) { return (Entry)(tile + 1u) | ((Entry)((g << 16) | layer) << 32); }
 
 __device__ __forceinline__ unsigned long long global_ns() {
     unsigned long long t;
@@ -40,39 +61,47 @@ __device__ __forceinline__ unsigned ld_acquire(const unsigned *p) {
     asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
     return v;
 }
+__device__ __forceinline__ Entry ld_acquire(const Entry *p) {
+    Entry v;
+    asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
+    return v;
+}
+__device__ __forceinline__ void st_release(Entry *p, Entry v) { asm volatile("st.release.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory"); }
 __device__ __forceinline__ unsigned ld_relaxed(const unsigned *p) {
     unsigned v;
     asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
     return v;
 }
+__device__ __forceinline__ unsigned ld_acquire_sys(const unsigned *p) {
+    unsigned v;
+    asm volatile("ld.acquire.sys.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+    return v;
+}
 
-// Child update of a completed tile; called by the whole (converged) scheduler warp.  `children` holds
-// (child tile, count the child waits for) pairs so one load feeds both the atomic and the test.
-// Returns the global id of a child this CTA should run next (only when want_keep), or ASPEN_TILE_NONE.
-// SERVICE: the counters are never reset between the passes of a graph; a pass only starts when the previous one is complete,
-// so a child is ready whenever its counter reaches a multiple of the count it waits for.
-template <bool SERVICE>
-static __device__ unsigned complete_children(const NasmDev &G, unsigned child_off, unsigned child_cnt, CtrlDev *ctrl, unsigned *queue, bool want_keep) {
+// Child update of a completed tile; called by the whole (converged) scheduler warp.  An edge is (child tile, layer << 16 |
+// count the child waits for); `e` holds this lane's first edge, fetched while the tile ran.
+// Returns a child this CTA should run next (only when want_keep), or 0.
+static __device__ __forceinline__ Entry complete_children(const NasmDev &G, unsigned g, uint2 e, unsigned child_off, unsigned child_cnt, CtrlDev *ctrl, Entry *queue, bool want_keep) {
     const unsigned lane = threadIdx.x & 31u;
-    const uint2 *edges = reinterpret_cast<const uint2 *>(G.children);
+    const uint2 *edges = reinterpret_cast<const uint2 *>(G.children) + child_off;
+    unsigned *dep = G.dep;
     __threadfence();                                     // release: this tile's output
-    unsigned next = ASPEN_TILE_NONE;
+    Entry next = 0;
     for (unsigned base = 0; base < child_cnt; base += 32u) {
         const unsigned idx = base + lane;
-        unsigned child = ASPEN_TILE_NONE;
         bool ready = false;
         if (idx < child_cnt) {
-            const uint2 e = edges[child_off + idx];
-            child = e.x;
-            const unsigned now = atomicAdd(&G.dep[child], 1u) + 1u;
-            ready = SERVICE ? (now % e.y == 0u) : (now == e.y);
+            if (base) e = edges[idx];
+            const unsigned now = atomicAdd(&dep[e.x], 1u) + 1u;
+            ready = now % (e.y & 0xffffu) == 0u;
         }
         unsigned mask = __ballot_sync(0xffffffffu, ready);
         if (mask == 0u) continue;
         __threadfence();                                 // acquire the other parents' outputs (through the counters), then publish
-        if (want_keep && next == ASPEN_TILE_NONE) {
+        const Entry mine = make_entry(e.x, g, e.y >> 16);
+        if (want_keep && next == 0) {
             const unsigned first = __ffs(mask) - 1u;
-            next = __shfl_sync(0xffffffffu, child, first) + G.tile_base;
+            next = __shfl_sync(0xffffffffu, mine, first);
             mask &= ~(1u << first);
             if (lane == first) ready = false;
         }
@@ -83,50 +112,17 @@ static __device__ unsigned complete_children(const NasmDev &G, unsigned child_of
             pos = __shfl_sync(0xffffffffu, pos, 0);
             if (ready) {
                 const unsigned rank = __popc(mask & ((1u << lane) - 1u));
-                if (pos + rank < ctrl->cap)
-                    asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(&queue[pos + rank]), "r"(child + G.tile_base + 1u) : "memory");
+                if (pos + rank < ctrl->cap) st_release(&queue[pos + rank], mine);
             }
         }
     }
     return next;
 }
 
-// Completion accounting (ref src/dse.c:80-106): layer counter -> layers-completed counter -> the
-// graph's completed flag; run-wide tile count.  Not on the path of the next tile: done after it is posted.
-static __device__ void complete_accounting(const NasmDev &G, unsigned layer, CtrlDev *ctrl, StatusHost *status) {
-    if ((threadIdx.x & 31u) != 0u) return;
-    unsigned d = atomicAdd(&G.layer_done[layer], 1u);
-    unsigned t = atomicAdd(&ctrl->done, 1u);
-    if (d + 1u == G.layer_tiles[layer]) {
-        unsigned l = atomicAdd(G.layers_completed, 1u);
-        if (l + 1u == G.n_layers) {
-            __threadfence_system();
-            *G.completed = 1u;                           // mapped host flag: the nasm is complete
-        }
-    }
-    if (((t + 1u) & 1023u) == 0u || t + 1u == ctrl->total) status->tiles_done = t + 1u;
-}
-
-// ---- service mode ------------------------------------------------------------------------------
-// The kernel stays resident while the host keeps asking for passes of the graphs it was launched with (the counterpart
-// of the reference's DSE threads, which run from dse_group_run to dse_group_stop and serve whatever rpool_add_nasm
-// brings, ref src/dse.c:20-108, 215-232).  The host asks for pass number p of a graph by writing p to the graph's
-// SVC_TARGET word (a 4-byte copy that follows the input upload on the transfer stream).  An idle scheduler warp that
-// finds an idle graph with target != started claims it (CAS on SVC_IDLE) and pushes its layer-0 tiles; those tiles
-// prepare the input, everything else follows from the dependency counters.  The warp that retires the last tile of a
-// pass writes the pass number to the graph's mapped host word and marks the graph idle.  The kernel leaves -- without
-// error -- when no pass is running or asked for and the host has asked it to stop, when nothing has run for idle_ns,
-// or when the queue of this launch is used up; the host launches it again if work is left.
-__device__ __forceinline__ unsigned ld_acquire_sys(const unsigned *p) {
-    unsigned v;
-    asm volatile("ld.acquire.sys.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
-    return v;
-}
-
 // Looks at every graph; starts the next pass where one is asked for.  Whole (converged) warp.
 // Returns bit 0: some graph has a pass in progress, bit 1: a pass is asked for but this launch's queue has no room left,
 // bit 2: this warp started a pass.
-static __device__ unsigned svc_scan(const NasmDev *nasms, unsigned n_nasm, CtrlDev *ctrl, unsigned *queue) {
+static __device__ unsigned svc_scan(const NasmDev *nasms, unsigned n_nasm, CtrlDev *ctrl, Entry *queue) {
     const unsigned lane = threadIdx.x & 31u;
     unsigned st = 0;
     for (unsigned g = 0; g < n_nasm; g++) {
@@ -134,13 +130,16 @@ static __device__ unsigned svc_scan(const NasmDev *nasms, unsigned n_nasm, CtrlD
         unsigned go = 0;
         if (lane == 0) {
             if (ld_acquire(&G.svc[SVC_IDLE]) == 0u) go = 1u;
-            else if (ld_acquire_sys(&G.svc[SVC_TARGET]) != ld_relaxed(&G.svc[SVC_STARTED])) {
+            else if (ld_acquire_sys(&G.svc[SVC_TARGET]) == ld_acquire(&G.svc[SVC_STARTED])) {
+                // nothing asked for -- or another warp has claimed the pass between the two reads
+                go = ld_acquire(&G.svc[SVC_IDLE]) == 0u ? 1u : 0u;
+            } else {
                 if (ld_relaxed(&ctrl->tail) + ctrl->total > ctrl->cap) go = 2u;
                 else if (atomicCAS(&G.svc[SVC_IDLE], 1u, 0u) == 1u) {
                     // only the holder of the claim changes SVC_STARTED: look again now that it is ours
                     const unsigned started = ld_relaxed(&G.svc[SVC_STARTED]);
                     if (ld_acquire_sys(&G.svc[SVC_TARGET]) != started) {
-                        asm volatile("st.relaxed.gpu.global.u32 [%0], %1;" ::"l"(&G.svc[SVC_STARTED]), "r"(started + 1u) : "memory");
+                        asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(&G.svc[SVC_STARTED]), "r"(started + 1u) : "memory");
                         atomicAdd(&ctrl->busy, 1u);
                         go = 4u;
                     } else asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(&G.svc[SVC_IDLE]), "r"(1u) : "memory");
@@ -154,127 +153,94 @@ static __device__ unsigned svc_scan(const NasmDev *nasms, unsigned n_nasm, CtrlD
             if (lane == 0) pos = atomicAdd(&ctrl->tail, G.n_input);
             pos = __shfl_sync(0xffffffffu, pos, 0);
             for (unsigned i = lane; i < G.n_input; i += 32u)
-                if (pos + i < ctrl->cap)
-                    asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(&queue[pos + i]), "r"(i + G.tile_base + 1u) : "memory");
+                if (pos + i < ctrl->cap) st_release(&queue[pos + i], make_entry(i, g, 0));
         }
     }
     return st;
 }
 
-// Completion accounting in service mode: one counter per graph; every n_exec-th completion ends a pass.
-static __device__ void svc_account(const NasmDev *nasms, unsigned n_nasm, unsigned g, CtrlDev *ctrl, unsigned *queue) {
+// `t` tiles of graph g have completed since the launch: every n_exec-th completion ends a pass.  Whole warp.
+static __device__ void end_of_pass(const NasmDev *nasms, unsigned n_nasm, unsigned g, unsigned t, CtrlDev *ctrl, Entry *queue) {
     const NasmDev &G = nasms[g];
-    const unsigned lane = threadIdx.x & 31u;
-    unsigned t = 0;
-    if (lane == 0) { atomicAdd(&ctrl->done, 1u); t = atomicAdd(&G.svc[SVC_COUNT], 1u) + 1u; }
-    t = __shfl_sync(0xffffffffu, t, 0);
-    if (t % G.n_exec != 0u) return;
-    if (lane == 0) {
+    if ((threadIdx.x & 31u) == 0) {
         __threadfence_system();
-        *G.completed = G.svc_base + t / G.n_exec;          // mapped host word: number of the pass that is complete
+        *G.completed = ld_relaxed(&G.svc[SVC_BASE]) + t / G.n_exec;          // mapped host word: number of the pass that is complete
         __threadfence_system();
         atomicSub(&ctrl->busy, 1u);
         asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(&G.svc[SVC_IDLE]), "r"(1u) : "memory");
     }
     __syncwarp();
-    svc_scan(nasms, n_nasm, ctrl, queue);                  // the next pass of this graph may already be asked for
+    // the next pass of this graph may already be asked for; with nothing left and the host's request to stop, everybody leaves
+    if (svc_scan(nasms, n_nasm, ctrl, queue) == 0u && (threadIdx.x & 31u) == 0u && ld_relaxed(&ctrl->svc_stop) != 0u) atomicExch(&ctrl->svc_close, 1u);
 }
 
-// Arms a service launch: empty queue, zero counters, every graph idle at the pass count the host has seen complete.
-static __global__ void svc_arm_kernel(NasmDev *nasms, CtrlDev *ctrl, unsigned *queue, unsigned cap, unsigned total, unsigned long long stall_ns,
-                               unsigned long long pipe_ns, unsigned long long idle_ns, unsigned svc_stop, unsigned svc_ahead) {
+// Arms a launch: empty queue, zero counters, every graph idle at the pass count the host has seen complete.  The pass numbers
+// travel as arguments (a launch of the same graphs then needs no copy); more than ARM_GRAPHS graphs take several launches,
+// the first of which (g0 = 0) also resets the queue and the control words.
+constexpr unsigned ARM_GRAPHS = 32;
+struct ArmArgs {
+    unsigned g0, n, n_nasm, cap, total, svc_stop, ahead;
+    unsigned long long stall_ns, pipe_ns, idle_ns;
+    unsigned base[ARM_GRAPHS], target[ARM_GRAPHS];
+};
+static __global__ void arm_kernel(const NasmDev *nasms, CtrlDev *ctrl, Entry *queue, const ArmArgs a) {
     const unsigned stride = gridDim.x * blockDim.x, t0 = blockIdx.x * blockDim.x + threadIdx.x;
-    const unsigned n_nasm = ctrl->n_nasm;
-    for (unsigned i = t0; i < cap; i += stride) queue[i] = 0u;
-    for (unsigned g = 0; g < n_nasm; g++) {
-        const NasmDev G = nasms[g];
-        for (unsigned i = t0; i < G.n_tiles; i += stride) G.dep[i] = 0u;
-        if (t0 == 0) { G.svc[SVC_STARTED] = G.svc_base; G.svc[SVC_IDLE] = 1u; G.svc[SVC_COUNT] = 0u; }
+    if (a.g0 == 0)
+        for (unsigned i = t0; i < a.cap; i += stride) queue[i] = 0u;
+    for (unsigned g = 0; g < a.n; g++) {
+        const NasmDev &G = nasms[a.g0 + g];
+        unsigned *dep = G.dep;
+        for (unsigned i = t0, n = G.n_tiles; i < n; i += stride) dep[i] = 0u;
+        if (t0 == 0) {
+            G.svc[SVC_STARTED] = G.svc[SVC_BASE] = a.base[g];
+            G.svc[SVC_TARGET] = a.target[g];
+            G.svc[SVC_IDLE] = 1u; G.svc[SVC_COUNT] = 0u;
+        }
     }
-    if (t0 == 0) {
-        ctrl->head = 0u; ctrl->tail = 0u; ctrl->done = 0u; ctrl->total = total; ctrl->cap = cap;
-        ctrl->abort = 0u; ctrl->stop = 0u; ctrl->stall_ns = stall_ns; ctrl->pipe_ns = pipe_ns;
-        ctrl->svc_stop = svc_stop; ctrl->svc_close = 0u; ctrl->busy = 0u; ctrl->idle_ns = idle_ns; ctrl->svc_ahead = svc_ahead;
-    }
-}
-
-// Resets the counters of every graph in the run and seeds the queue with the tiles that only
-// depend on input tiles (push_first_layer_to_rpool, ref src/dse.c:443-470).
-static __global__ void arm_kernel(NasmDev *nasms, CtrlDev *ctrl, unsigned *queue, unsigned total, unsigned n_init_total,
-                           unsigned n_input_total, unsigned long long stall_ns, unsigned long long pipe_ns, unsigned ahead) {
-    const unsigned stride = gridDim.x * blockDim.x, t0 = blockIdx.x * blockDim.x + threadIdx.x;
-    const unsigned n_nasm = ctrl->n_nasm;
-    for (unsigned i = t0; i < total; i += stride) queue[i] = 0u;
-    __threadfence();
-    for (unsigned g = 0; g < n_nasm; g++) {
-        const NasmDev G = nasms[g];
-        for (unsigned i = t0; i < G.n_tiles; i += stride) G.dep[i] = G.dep_init[i];
-        for (unsigned i = t0; i < G.n_layers; i += stride) G.layer_done[i] = G.layer_done_init[i];
-        if (t0 == 0) { *G.layers_completed = G.layers_done_init; *G.completed = 0u; }
-    }
-    if (t0 == 0) {
-        ctrl->head = 0u; ctrl->tail = n_init_total; ctrl->done = n_input_total; ctrl->total = total; ctrl->cap = total;
-        ctrl->abort = 0u; ctrl->stop = 0u; ctrl->stall_ns = stall_ns; ctrl->pipe_ns = pipe_ns; ctrl->svc_ahead = ahead;
-    }
-}
-// Second step of arming (after every slot was cleared): write the initial ready tiles.
-static __global__ void seed_kernel(NasmDev *nasms, CtrlDev *ctrl, unsigned *queue) {
-    const unsigned stride = gridDim.x * blockDim.x, t0 = blockIdx.x * blockDim.x + threadIdx.x;
-    for (unsigned g = 0; g < ctrl->n_nasm; g++) {
-        const NasmDev G = nasms[g];
-        for (unsigned i = t0; i < G.n_init; i += stride) queue[G.queue_base + i] = G.init_ready[i] + G.tile_base + 1u;
+    if (t0 == 0 && a.g0 == 0) {
+        ctrl->head = 0u; ctrl->tail = 0u; ctrl->done = 0u; ctrl->total = a.total; ctrl->cap = a.cap; ctrl->n_nasm = a.n_nasm;
+        ctrl->abort = 0u; ctrl->stop = 0u; ctrl->stall_ns = a.stall_ns; ctrl->pipe_ns = a.pipe_ns;
+        ctrl->svc_stop = a.svc_stop; ctrl->svc_close = 0u; ctrl->busy = 0u; ctrl->idle_ns = a.idle_ns; ctrl->ahead = a.ahead;
     }
 }
 
-template <bool TENSOR_CORES, bool ATTENTION, bool SERVICE>
-__device__ __forceinline__ void run_tile(const LayerDev &L, const TileDev &T, const NasmDev &G, unsigned char *stage_mem, tc::Shared *sh,
-                                         tc::PipeState &ps, CtrlDev *ctrl, StatusHost *status) {
-    const unsigned tid = threadIdx.x;
+// A tile that runs on the worker warps alone; `wt`: worker thread 0 .. tc::NW-1, `scratch`: the shared memory of fp32 blocks.
+template <bool TENSOR_CORES>
+static __device__ __noinline__ void worker_tile(const tc::Slot &sl, unsigned wt, unsigned char *scratch) {
+    const LayerDev &L = sl.layer;
+    const TileDev &T = sl.tile;
     switch (L.type) {
-        case CONV_LAYER: case FC_LAYER: case MATMUL_LAYER: case K_ATTENTION_LAYER: case V_ATTENTION_LAYER:
-            if (TENSOR_CORES && ATTENTION && L.att_fused) {
-                tc::AttnArgs a;
-                a.seq = L.seq; a.hd = L.hd; a.heads = L.heads; a.masked = L.masked; a.ldc = L.ldc; a.round_out = L.round_out;
-                a.att_p_ld = L.att_p_ld; a.att_p_round = L.att_p_round; a.out = L.out; a.att_p_out = L.att_p_out;
-                a.qmap = (const unsigned char *)G.wmaps + (size_t)L.att_qmap * 128;
-                a.kmap = (const unsigned char *)G.wmaps + (size_t)L.att_kmap * 128;
-                a.vmap = (const unsigned char *)G.wmaps + (size_t)L.wmap * 128;
-                tc::AttnPipe ap;
-                ap.att_tiles = ps.att_tiles; ap.att_groups = ps.att_groups; ap.dead = ps.dead;
-                ps.dead = tc::tile_attention(a, T, stage_mem, sh, ap, ctrl, status);
-                ps.att_tiles++;
-                ps.att_groups += tc::attention_groups(L.seq, L.masked, T);
-            } else if (TENSOR_CORES) tc::tile_gemm(L, T, G, stage_mem, sh, ps, ctrl, status);
-            else if (tid < tc::NW) tile_gemm_ffma(L, T, tid, tc::NW);
-            break;
-        case RESIDUAL_LAYER: if (tid < tc::NW) tile_residual(L, T, tid, tc::NW); break;
-        case MAXPOOL_LAYER: if (tid < tc::NW) tile_pool<true>(L, T, tid, tc::NW); break;
-        case AVGPOOL_LAYER: if (tid < tc::NW) tile_pool<false>(L, T, tid, tc::NW); break;
-        case LAYERNORM_LAYER: if (tid < tc::NW) tile_layernorm(L, T, tid, tc::NW); break;
-        case SOFTMAX_LAYER: if (tid < tc::NW) tile_softmax(L, T, tid, tc::NW); break;
-        case YOLO_LAYER: if (tid < tc::NW) tile_yolo(L, T, tid, tc::NW); break;
-        case APPEND_LAYER: if (tid < tc::NW) tile_append(L, T, tid, tc::NW); break;
-        case INPUT_LAYER: if (SERVICE && tid < tc::NW) tile_input(G.input, L, T, tid, tc::NW); break;
+        case CONV_LAYER: case FC_LAYER: case MATMUL_LAYER: case K_ATTENTION_LAYER: case V_ATTENTION_LAYER: tile_gemm_ffma<!TENSOR_CORES>(L, T, wt, tc::NW, scratch); break;
+        case RESIDUAL_LAYER: tile_residual(L, T, wt, tc::NW); break;
+        case MAXPOOL_LAYER: tile_pool<true>(L, T, wt, tc::NW); break;
+        case AVGPOOL_LAYER: tile_pool<false>(L, T, wt, tc::NW); break;
+        case LAYERNORM_LAYER: tile_layernorm(L, T, wt, tc::NW); break;
+        case SOFTMAX_LAYER: tile_softmax(L, T, wt, tc::NW); break;
+        case YOLO_LAYER: tile_yolo(L, T, wt, tc::NW); break;
+        case APPEND_LAYER: tile_append(L, T, wt, tc::NW); break;
+        case INPUT_LAYER: tile_input(*sl.input, L, T, wt, tc::NW); break;
         default: break;
     }
 }
 
 // ---- the persistent kernel -------------------------------------------------------------------
-// Threads 0 .. tc::NTHREADS-1 are the EXECUTORS (worker warps, TMA thread, MMA thread): they run one tile
-// after the other out of a two-slot mailbox in shared memory.  The last warp is the SCHEDULER: when
-// the executors finish a tile it updates the children first (the first child that became ready is
-// posted straight back to the executors), and does the completion accounting and the queue
-// traffic while the executors already run the next tile.
-//   mailbox[k], k = sequence number & 1:  scheduler writes the tile id, arrives on posted[k];
-//   executors wait posted[k], run the tile, every executor thread arrives on finished[k];
-//   the scheduler waits finished[k] (so all stores of the tile are ordered before its gpu-scope
-//   fence and the counter updates), retires the tile and may then reuse slot k.
-constexpr unsigned SCHED_THREADS = tc::NTHREADS + 32u;
+// The SCHEDULER warp hands tiles to the other roles (tiles_tc.cuh) through SLOTS slots in shared memory; slot k = sequence
+// number % SLOTS.  It copies the tile's descriptor and its layer's into the slot and arrives on posted[k]; every role takes
+// the slots in order, at its own pace, and arrives on finished[k] when it is done with the slot (the worker warps: when all
+// stores of the tile are made).  The scheduler then updates the children (a first child that became ready is kept as this
+// CTA's next tile), does the completion accounting, and may use the slot again.
+// The fp32 kernel has no producers: its scheduler is warp 0, its workers follow, and nobody shares the registers.
+template <bool TENSOR_CORES> __host__ __device__ constexpr unsigned threads() { return TENSOR_CORES ? tc::THREADS : 32u + tc::NW; }
+// dynamic shared memory: operand ring and transposing buffers (tensor cores), or the staging of the fp32 blocks
+constexpr unsigned FFMA_BYTES = 96u * 1024u;
+template <bool TENSOR_CORES> __host__ __device__ constexpr unsigned work_bytes() { return TENSOR_CORES ? tc::RING_BYTES + tc::EPI_BYTES : FFMA_BYTES; }
 
-// Executors' wait for the next tile.  The scheduler always posts an exit marker eventually (end of
+// A role's wait for the next tile.  The scheduler always posts an exit marker eventually (end of
 // run, stop, stall, abort); the time bound only guards against that logic failing.
 __device__ __forceinline__ bool wait_posted(unsigned long long *bar, unsigned parity, CtrlDev *ctrl, StatusHost *status) {
-    if (tc::mbar_try_wait(bar, parity)) return true;
+    #pragma unroll 1
+    for (unsigned spin = 0; spin < 1024u; spin++)
+        if (tc::mbar_try_wait(bar, parity)) return true;
     const unsigned long long t0 = global_ns(), budget = 2ull * ctrl->stall_ns + 4ull * ctrl->pipe_ns + 1000000000ull;
     for (unsigned spin = 1;; spin++) {
         if (tc::mbar_try_wait(bar, parity)) return true;
@@ -290,70 +256,86 @@ __device__ __forceinline__ bool wait_posted(unsigned long long *bar, unsigned pa
     return false;
 }
 
-template <bool SERVICE>
-static __device__ void scheduler_warp(const NasmDev *nasms, unsigned n_nasm, CtrlDev *ctrl, unsigned *queue, StatusHost *status,
-                               tc::Shared *sh, unsigned long long *my_prof) {
-    const unsigned lane = threadIdx.x & 31u;
-    unsigned issued = 0, retired = 0;          // tiles posted to / retired from the mailbox
-    unsigned fl_nasm[2] = {0, 0}, fl_off[2] = {0, 0}, fl_cnt[2] = {0, 0}, fl_layer[2] = {0, 0};   // tiles in flight
-    unsigned acct_nasm = 0, acct_layer = ASPEN_TILE_NONE;   // completion accounting still to do
-    unsigned next = ASPEN_TILE_NONE;           // a ready tile waiting for a free slot
-    unsigned kept = ASPEN_TILE_NONE;           // a child made ready by a tile this CTA completed
-    unsigned ticket = ASPEN_TILE_NONE;         // a queue position we hold and wait on
-    bool closed = false;                        // no further tiles will be issued (end of run, stop, abort)
+// Fills a slot with a ready tile and hands it to the roles (whole warp).  The tile's and the layer's descriptors are independent
+// loads; both and the graph's addresses are constant while the kernel runs.
+static __device__ __forceinline__ void post(tc::Slot &sl, unsigned long long &posted, const NasmDev *nasms, Entry entry) {
+    const unsigned lane = threadIdx.x & 31u, g = (unsigned)(entry >> 48), layer = (unsigned)(entry >> 32) & 0xffffu, tile = (unsigned)entry - 1u;
+    const NasmDev &G = nasms[g];
+    constexpr unsigned LW = sizeof(LayerDev) / 4, TW = sizeof(TileDev) / 4;
+    static_assert(sizeof(LayerDev) % 4 == 0 && LW <= 96 && TW <= 32, "copied in words");
+    const unsigned *lsrc = reinterpret_cast<const unsigned *>(G.layers + layer), *tsrc = reinterpret_cast<const unsigned *>(G.tiles + tile);
+    unsigned lw[3] = {}, tw = 0;
+    #pragma unroll
+    for (unsigned i = 0; i < 3; i++) if (i * 32u + lane < LW) lw[i] = __ldg(lsrc + i * 32u + lane);
+    if (lane < TW) tw = __ldg(tsrc + lane);
+    #pragma unroll
+    for (unsigned i = 0; i < 3; i++) if (i * 32u + lane < LW) reinterpret_cast<unsigned *>(&sl.layer)[i * 32u + lane] = lw[i];
+    if (lane < TW) reinterpret_cast<unsigned *>(&sl.tile)[lane] = tw;
+    if (lane == 0) { sl.live = 1u; sl.nasm = g; sl.maps = (const unsigned char *)G.wmaps; sl.input = &G.input; }
+    __syncwarp();
+    if (lane == 0) tc::mbar_arrive(&posted);
+}
+
+static __device__ __noinline__ void scheduler_warp(const NasmDev *nasms, CtrlDev *ctrl, Entry *queue, StatusHost *status, tc::Shared *sh, unsigned long long *my_prof) {
+    const unsigned lane = threadIdx.x & 31u, n_nasm = ctrl->n_nasm;
+    unsigned issued = 0, retired = 0;           // tiles posted to / retired from the slots: at most two apart
+    uint2 edge0 = make_uint2(0u, 1u), edge1 = edge0;   // this lane's first child edge of the tiles in the slots (by parity)
+    unsigned acct_nasm = 0;                     // completion accounting still to do
+    bool acct = false;
+    Entry kept = 0;                             // a child made ready by a tile this CTA completed
+    unsigned ticket = ASPEN_TILE_NONE;          // a queue position we hold and wait on
+    bool closed = false;                        // no further tiles will be issued (end of run, stop)
     bool no_tickets = false;                    // the queue has no unowned position left; kept children still run
-    const unsigned total = ctrl->total, cap = ctrl->cap;
+    const unsigned cap = ctrl->cap, ahead = ctrl->ahead;
+    const unsigned *watch = lane == 1u ? &ctrl->abort : lane == 2u ? &ctrl->stop : lane == 3u ? &ctrl->svc_close : &ctrl->done;
     unsigned last_done = 0;
     unsigned long long t_progress = __shfl_sync(0xffffffffu, global_ns(), 0), t_mark = t_progress;
     const unsigned long long window = ctrl->stall_ns;
-    unsigned idle_spins = SERVICE ? 30u : 0u, turn = 0, flags = 0, done = 0, ahead_turn = 0;
-    const unsigned ahead = ctrl->svc_ahead;   // service: the first idle turns already look for a pass to start
+    unsigned idle_spins = 30u, turn = 0, flags = 0, done = 0, ahead_turn = 0;   // the first idle turns already look for a pass to start
     while (true) {
         bool progressed = false;
-        // control state is read by lane 0 and broadcast so the warp never diverges on it
-        // (global loads cost an L2 round trip each: while tiles are in flight they are sampled every 8th turn)
-        if (issued == retired || (turn++ & 7u) == 0u) {
-            unsigned f = 0, d = 0;
-            if (lane == 0) {
-                f = (ld_relaxed(&ctrl->abort) != 0u ? 1u : 0u) | (ld_relaxed(&ctrl->stop) != 0u ? 2u : 0u);
-                if (SERVICE && ld_relaxed(&ctrl->svc_close) != 0u) f |= 4u;
-                d = ld_relaxed(&ctrl->done);
-            }
-            flags = __shfl_sync(0xffffffffu, f, 0);
-            done = __shfl_sync(0xffffffffu, d, 0);
+        // Control words (lanes 1 - 4) and the slot we wait on (lane 0) are read together: one L2 round trip a turn.  With a tile
+        // in work the control words are sampled every 8th turn.
+        unsigned word = 0;
+        Entry slot = 0;
+        const bool sample = issued == retired || (turn++ & 7u) == 0u;
+        if (sample && lane >= 1u && lane <= 4u) word = ld_relaxed(watch);
+        if (ticket != ASPEN_TILE_NONE && lane == 0u) slot = ld_acquire(&queue[ticket]);
+        if (sample) {
+            flags = __ballot_sync(0xffffffffu, lane >= 1u && lane <= 3u && word != 0u);
+            done = __shfl_sync(0xffffffffu, word, 4);
+            if (flags & 2u) break;               // aborted: roles leave their tiles unfinished, nothing more will be retired
+            if (flags) closed = true;
         }
-        const bool halt = flags != 0u;
-        // 1. retire the oldest tile in flight once every executor thread has finished it
+        // 1. retire the oldest tile in flight once every role has finished it
         if (issued > retired) {
-            const unsigned k = retired & 1u;
-            unsigned ok = lane == 0 ? (unsigned)tc::mbar_test_wait(&sh->finished[k], (retired >> 1) & 1u) : 0u;
+            const unsigned k = retired % tc::SLOTS;
+            unsigned ok = lane == 0 ? (unsigned)tc::mbar_test_wait(&sh->finished[k], (retired / tc::SLOTS) & 1u) : 0u;
             ok = __shfl_sync(0xffffffffu, ok, 0);
             if (ok) {
                 if (my_prof && lane == 0) t_mark = global_ns();
-                if (!(flags & 1u)) {
-                    unsigned child = complete_children<SERVICE>(nasms[fl_nasm[k]], fl_off[k], fl_cnt[k], ctrl, queue, kept == ASPEN_TILE_NONE);
-                    if (child != ASPEN_TILE_NONE) kept = child;
-                    acct_nasm = fl_nasm[k]; acct_layer = fl_layer[k];
-                }
+                const tc::Slot &sl = sh->slots[k];
+                const unsigned g = sl.nasm;
+                const Entry child = complete_children(nasms[g], g, (retired & 1u) ? edge1 : edge0, sl.tile.child_off, sl.tile.child_cnt, ctrl, queue, kept == 0);
+                if (child) kept = child;
                 if (my_prof && lane == 0) my_prof[1] += global_ns() - t_mark;
+                acct_nasm = g;
+                acct = true;
                 retired++;
                 progressed = true;
             }
         }
         // 2. find the next tile
-        if (halt) closed = true;
-        if (!closed && next == ASPEN_TILE_NONE) {
-            if (kept != ASPEN_TILE_NONE) { next = kept; kept = ASPEN_TILE_NONE; progressed = true; }
-            else {
-                // Only an idle CTA queues up for the next ready tile.  Claiming one while still busy was
-                // measured to cost 40 % of throughput: the claimed tile waits in this CTA's mailbox while
-                // other SMs that could have started it at once sit idle.
-                bool take = ticket == ASPEN_TILE_NONE && !no_tickets && issued == retired;
-                if (ahead != 0u && !take && ticket == ASPEN_TILE_NONE && !no_tickets && issued - retired == 1u && (ahead_turn++ & 15u) == 0u) {
-                    // Busy with one tile, nothing lined up.  With several requests in the kernel the queue usually holds ready
-                    // tiles that no idle CTA is waiting for: taking one now lets the executors go from this tile straight to
-                    // the next while the completion (child counters, queue pushes) runs beside them.  Only with a backlog: a
-                    // ticket held for a tile that is not there yet would keep that tile from an idle SM.
+        Entry next = 0;
+        if (!closed && issued - retired < 2u) {
+            if (kept) { next = kept; kept = 0; }
+            else if (!no_tickets) {
+                // An idle CTA queues up for the next ready tile.  A busy one (one tile in work) lines up a second only when at
+                // least `ahead` ready tiles wait unclaimed: its operands then stream in under the first one's epilogue, and
+                // the completion of the first runs beside the second.  A ticket held for a tile that is not there yet would
+                // keep that tile from an idle SM.
+                bool take = ticket == ASPEN_TILE_NONE && issued == retired;
+                if (ahead != 0u && !take && ticket == ASPEN_TILE_NONE && (ahead_turn++ & 7u) == 0u) {
                     int backlog = 0;
                     if (lane == 0) backlog = (int)(ld_relaxed(&ctrl->tail) - ld_relaxed(&ctrl->head));
                     take = __shfl_sync(0xffffffffu, backlog, 0) >= (int)ahead;
@@ -363,46 +345,35 @@ static __device__ void scheduler_warp(const NasmDev *nasms, unsigned n_nasm, Ctr
                     ticket = __shfl_sync(0xffffffffu, t, 0);
                     if (ticket >= cap) { ticket = ASPEN_TILE_NONE; no_tickets = true; }   // every tile that can be pushed has an owner
                 }
-                if (ticket != ASPEN_TILE_NONE) {
-                    unsigned v = lane == 0 ? ld_acquire(&queue[ticket]) : 0u;
-                    v = __shfl_sync(0xffffffffu, v, 0);
-                    if (v != 0u) { next = v - 1u; ticket = ASPEN_TILE_NONE; progressed = true; }
+                else if (ticket != ASPEN_TILE_NONE) {
+                    next = __shfl_sync(0xffffffffu, slot, 0);
+                    if (next) ticket = ASPEN_TILE_NONE;
                 }
             }
         }
-        // 3. post it when a mailbox slot is free
-        if (next != ASPEN_TILE_NONE && issued - retired < 2u) {
-            unsigned g = 0;
-            while (g + 1u < n_nasm && next >= nasms[g + 1u].tile_base) g++;
-            const TileDev T = nasms[g].tiles[next - nasms[g].tile_base];
-            if (T.flags & TILE_WRITTEN_BY_PARENTS) {
-                // nothing to execute: the tiles it waited for wrote its values; it completes right here
-                if (!(flags & 1u)) {
-                    unsigned child = complete_children<SERVICE>(nasms[g], T.child_off, T.child_cnt, ctrl, queue, kept == ASPEN_TILE_NONE);
-                    if (child != ASPEN_TILE_NONE) kept = child;
-                    if (SERVICE) svc_account(nasms, n_nasm, g, ctrl, queue);
-                    else complete_accounting(nasms[g], T.layer, ctrl, status);
-                }
-            } else {
-                const unsigned k = issued & 1u;
-                if (lane == 0) { sh->tile_desc[k] = T; sh->tile_nasm[k] = g; sh->mailbox[k] = next; tc::mbar_arrive(&sh->posted[k]); }
-                // remember what retiring this tile will need (loaded now, off the critical path)
-                fl_nasm[k] = g; fl_off[k] = T.child_off; fl_cnt[k] = T.child_cnt; fl_layer[k] = T.layer;
-                issued++;
-            }
-            next = ASPEN_TILE_NONE;
+        // 3. post it: one tile in work, one behind it
+        if (next) {
+            const unsigned k = issued % tc::SLOTS;
+            post(sh->slots[k], sh->posted[k], nasms, next);
+            const tc::Slot &sl = sh->slots[k];
+            uint2 e = make_uint2(0u, 1u);
+            if (lane < sl.tile.child_cnt) e = __ldg(reinterpret_cast<const uint2 *>(nasms[sl.nasm].children) + sl.tile.child_off + lane);
+            if (issued & 1u) edge1 = e; else edge0 = e;
+            issued++;
             progressed = true;
         }
-        if (acct_layer != ASPEN_TILE_NONE) {
-            if (SERVICE) svc_account(nasms, n_nasm, acct_nasm, ctrl, queue);
-            else complete_accounting(nasms[acct_nasm], acct_layer, ctrl, status);
-            acct_layer = ASPEN_TILE_NONE;
+        // 4. completion accounting, behind everything that another tile may be waiting for
+        if (acct) {
+            unsigned t = 0;
+            if (lane == 0) { atomicAdd(&ctrl->done, 1u); t = atomicAdd(&nasms[acct_nasm].svc[SVC_COUNT], 1u) + 1u; }
+            t = __shfl_sync(0xffffffffu, t, 0);
+            if (t % nasms[acct_nasm].n_exec == 0u) end_of_pass(nasms, n_nasm, acct_nasm, t, ctrl, queue);
+            acct = false;
         }
-        // 4. end of run / stall detection
-        if (!SERVICE && done >= total) closed = true;
+        // 5. end of launch / stall detection
         if (issued == retired) {
-            if (closed && (next == ASPEN_TILE_NONE || halt)) break;
-            if (no_tickets && next == ASPEN_TILE_NONE && kept == ASPEN_TILE_NONE && ticket == ASPEN_TILE_NONE) break;   // can never get work again
+            if (closed) break;
+            if (no_tickets && kept == 0) break;   // can never get work again
         }
         if (progressed || done != last_done) {
             unsigned long long now = lane == 0 ? global_ns() : 0ull;
@@ -413,7 +384,7 @@ static __device__ void scheduler_warp(const NasmDev *nasms, unsigned n_nasm, Ctr
             unsigned long long now = lane == 0 ? global_ns() : 0ull;
             now = __shfl_sync(0xffffffffu, now, 0);
             unsigned svc = 1u;
-            if (SERVICE && issued == retired && !closed) {
+            if (issued == retired && !closed) {
                 // an idle CTA looks for passes to start, and decides when the kernel has nothing left to wait for
                 svc = svc_scan(nasms, n_nasm, ctrl, queue);
                 if (svc & 4u) t_progress = now;
@@ -437,74 +408,108 @@ static __device__ void scheduler_warp(const NasmDev *nasms, unsigned n_nasm, Ctr
             }
             if (my_prof && lane == 0 && issued == retired) my_prof[0] += 1ull;   // idle polls with nothing in flight
         }
-        __nanosleep(issued == retired ? 100u : 20u);
+        __nanosleep(20u);
     }
-    if (lane == 0) { sh->mailbox[issued & 1u] = ASPEN_TILE_NONE; tc::mbar_arrive(&sh->posted[issued & 1u]); }
+    if (lane == 0) { sh->slots[issued % tc::SLOTS].live = 0u; tc::mbar_arrive(&sh->posted[issued % tc::SLOTS]); }
 }
 
-// ATTENTION: the instantiation that contains the fused attention tile.  It is a kernel of its own because the mere presence
-// of that code changes the register allocation of the contraction tile's main loop (measured: the whole kernel 40 % slower);
-// graphs without a fused attention layer run the instantiation without it.
-// SERVICE: the kernel serves pass after pass of its graphs until the host stops it (see "service mode" above).
-template <bool TENSOR_CORES, bool ATTENTION = false, bool SERVICE = false>
-__global__ void __launch_bounds__(SCHED_THREADS, 1)
-scheduler_kernel(const NasmDev *nasms, CtrlDev *ctrl, unsigned *queue, StatusHost *status, unsigned long long *prof) {
-    extern __shared__ unsigned char smem_raw[];
-    // stage buffers need 1024-byte alignment for the 128-byte swizzle
-    unsigned char *stage_mem = reinterpret_cast<unsigned char *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023u) & ~(uintptr_t)1023u);
-    tc::Shared *sh = reinterpret_cast<tc::Shared *>(stage_mem + (TENSOR_CORES ? tc::STAGES * tc::STAGE_BYTES + tc::EPI_BYTES + tc::RES_BYTES : 0u));
-    const unsigned tid = threadIdx.x, warp = tid >> 5;
-    const unsigned ctrl_warp = tc::NW >> 5;
-    tc::PipeState ps;
+// The loops of the one-thread roles, all their state inside: a reference to it would put it into local memory.
+template <unsigned ROLE>
+static __device__ __forceinline__ void single_thread_role(unsigned char *smem, tc::Shared *sh, CtrlDev *ctrl, StatusHost *status) {
+    const unsigned ring = tc::smem_u32(smem);
+    tc::Ring r;
+    unsigned half = 0, acc_uses = 0;
+    for (unsigned seq = 0;; seq++) {
+        const unsigned k = seq % tc::SLOTS;
+        if (!wait_posted(&sh->posted[k], (seq / tc::SLOTS) & 1u, ctrl, status)) break;
+        const tc::Slot &sl = sh->slots[k];
+        if (!sl.live) break;
+        if (sl.layer.tc) {
+            bool ok;
+            if (ROLE == tc::WARP_A) ok = tc::produce_a(sl, ring, r, sh, ctrl, status);
+            else if (ROLE == tc::WARP_B) ok = tc::produce_b(sl, ring, r, sh, ctrl, status);
+            else ok = tc::issue_mma(sl, ring, r, half, acc_uses, sh, ctrl, status);
+            if (!ok) break;
+        }
+        tc::mbar_arrive(&sh->finished[k]);
+    }
+    if (*(volatile unsigned *)&ctrl->abort) {
+        // copies and MMAs of this CTA may still be in flight; they take microseconds
+        const unsigned long long t0 = global_ns();
+        while (global_ns() - t0 < 2000000ull) __nanosleep(1000);
+    }
+}
+
+// Registers move from the first warpgroup to the two of workers: 128 x 104 + 256 x 200 = 384 x 168, what the launch holds.
+constexpr int ROLE_REGISTERS = 104, WORKER_REGISTERS = 200;
+static_assert(128 * ROLE_REGISTERS + 256 * WORKER_REGISTERS <= 384 * 168, "register split");
+
+template <bool TENSOR_CORES>
+__global__ void __launch_bounds__(threads<TENSOR_CORES>(), 1)
+scheduler_kernel(const NasmDev *nasms, CtrlDev *ctrl, Entry *queue, StatusHost *status, unsigned long long *prof) {
+    extern __shared__ __align__(1024) unsigned char smem[];      // stages need 1024-byte alignment for the 128-byte swizzle
+    tc::Shared *sh = reinterpret_cast<tc::Shared *>(smem + work_bytes<TENSOR_CORES>());
+    const unsigned tid = threadIdx.x, warp = tid >> 5, lane = tid & 31u;
+    constexpr unsigned sched_warp = TENSOR_CORES ? tc::WARP_SCHED : 0u, first_worker = TENSOR_CORES ? tc::WARP_WORK : 1u;
 
     if (tid == 0) {
-        for (int s = 0; s < tc::STAGES; s++) { tc::mbar_init(&sh->full[s], tc::NW); tc::mbar_init(&sh->empty[s], 1u); tc::mbar_init(&sh->landed[s], 1u); }
-        tc::mbar_init(&sh->accum, 1u);
-        for (unsigned w = 0; w < tc::NW / 32u; w++) tc::mbar_init(&sh->res_full[w], 1u);
-        tc::mbar_init(&sh->att_q, 1u); tc::mbar_init(&sh->att_k, 1u); tc::mbar_init(&sh->att_v, 1u);
-        tc::mbar_init(&sh->att_s, 1u); tc::mbar_init(&sh->att_p, tc::NW); tc::mbar_init(&sh->att_o, 1u);
-        for (int k = 0; k < 2; k++) { tc::mbar_init(&sh->posted[k], 1u); tc::mbar_init(&sh->finished[k], tc::NTHREADS); }
+        for (unsigned s = 0; s < tc::MAX_STAGES; s++) { tc::mbar_init(&sh->full[s], 2u); tc::mbar_init(&sh->empty[s], 1u); }
+        for (unsigned h = 0; h < 2; h++) { tc::mbar_init(&sh->acc_full[h], 1u); tc::mbar_init(&sh->acc_empty[h], tc::NW / 32u); }
+        for (unsigned k = 0; k < tc::SLOTS; k++) { tc::mbar_init(&sh->posted[k], 1u); tc::mbar_init(&sh->finished[k], tc::NW / 32u + (TENSOR_CORES ? 3u : 0u)); }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         tc::fence_proxy_async_smem();
     }
     if (TENSOR_CORES) {
-        if (warp == ctrl_warp + 1u) tc::tmem_alloc(&sh->tmem_base, tc::TMEM_COLS);
+        if (warp == tc::WARP_MMA) tc::tmem_alloc(&sh->tmem_base, tc::TMEM_COLS);
         tc::tc_fence_before();
     }
     __syncthreads();
     if (TENSOR_CORES) tc::tc_fence_after();
 
-    const unsigned n_nasm = ctrl->n_nasm;
     // Optional time accounting per CTA: [0] scheduler idle polls, [1] completion + child update (ns),
-    // [2 + layer] ns the executors spent on tiles of that layer (index modulo PROF_LAYERS),
-    // [2 + PROF_LAYERS + layer] tile counts, [PROF_SLOTS - 1] ns the executors waited for a tile.
+    // [2 + layer] ns the workers spent on tiles of that layer (index modulo PROF_LAYERS),
+    // [2 + PROF_LAYERS + layer] tile counts, [PROF_SLOTS - 1] ns the workers waited for a tile.
     unsigned long long *my_prof = prof ? prof + (size_t)blockIdx.x * PROF_SLOTS : nullptr;
 
-    if (warp == (SCHED_THREADS >> 5) - 1u) {
-        scheduler_warp<SERVICE>(nasms, n_nasm, ctrl, queue, status, sh, my_prof);
-    } else {
+    // The first four warps need few registers, the workers many: a spill costs an L2 round trip here, because the ring leaves
+    // almost no L1 (with 168 registers for everybody the epilogue of a 256 x 128 block took 12 us instead of 6).
+    if (TENSOR_CORES) {
+        if (warp >= first_worker) asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(WORKER_REGISTERS));
+        else asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(ROLE_REGISTERS));
+    }
+    if (warp == sched_warp) {
+        scheduler_warp(nasms, ctrl, queue, status, sh, my_prof);
+    } else if (warp >= first_worker) {
+        const unsigned wt = tid - first_worker * 32u;
+        unsigned half = 0, acc_uses = 0;
         unsigned long long t_mark = my_prof ? global_ns() : 0ull;
         for (unsigned seq = 0;; seq++) {
-            const unsigned k = seq & 1u;
-            if (!wait_posted(&sh->posted[k], (seq >> 1) & 1u, ctrl, status)) break;
-            const unsigned gid = sh->mailbox[k];
-            if (gid == ASPEN_TILE_NONE) break;
-            if (my_prof && tid == 0) { unsigned long long now = global_ns(); my_prof[PROF_SLOTS - 1] += now - t_mark; t_mark = now; }
-            const NasmDev &G = nasms[sh->tile_nasm[k]];
-            const TileDev T = sh->tile_desc[k];
-            const LayerDev &L = G.layers[T.layer];
-            run_tile<TENSOR_CORES, ATTENTION, SERVICE>(L, T, G, stage_mem, sh, ps, ctrl, status);
-            if (my_prof && tid == 0) {
+            const unsigned k = seq % tc::SLOTS;
+            if (!__all_sync(0xffffffffu, wait_posted(&sh->posted[k], (seq / tc::SLOTS) & 1u, ctrl, status))) break;
+            const tc::Slot &sl = sh->slots[k];
+            if (!sl.live) break;
+            if (my_prof && wt == 0) { unsigned long long now = global_ns(); my_prof[PROF_SLOTS - 1] += now - t_mark; t_mark = now; }
+            bool ok = true;
+            if (TENSOR_CORES && sl.layer.tc) ok = tc::epilogue_tile(sl, half, acc_uses, smem + tc::RING_BYTES, sh, ctrl, status);
+            else worker_tile<TENSOR_CORES>(sl, wt, smem + (TENSOR_CORES ? tc::RING_BYTES : 0u));
+            if (my_prof && wt == 0) {
                 unsigned long long now = global_ns();
-                my_prof[2 + T.layer % PROF_LAYERS] += now - t_mark; my_prof[2 + PROF_LAYERS + T.layer % PROF_LAYERS] += 1ull; t_mark = now;
+                const unsigned l = sl.tile.layer % PROF_LAYERS;
+                my_prof[2 + l] += now - t_mark; my_prof[2 + PROF_LAYERS + l] += 1ull; t_mark = now;
             }
-            tc::mbar_arrive(&sh->finished[k]);             // release (CTA scope): this thread's stores of the tile
+            __syncwarp();
+            if (lane == 0) tc::mbar_arrive(&sh->finished[k]);      // release (CTA scope): this warp's stores of the tile
+            if (!ok) break;
         }
+    } else if (TENSOR_CORES && lane == 0) {
+        if (warp == tc::WARP_A) single_thread_role<tc::WARP_A>(smem, sh, ctrl, status);
+        else if (warp == tc::WARP_B) single_thread_role<tc::WARP_B>(smem, sh, ctrl, status);
+        else single_thread_role<tc::WARP_MMA>(smem, sh, ctrl, status);
     }
-
+    __syncwarp();
     if (TENSOR_CORES) tc::tc_fence_before();
     __syncthreads();
-    if (TENSOR_CORES && warp == ctrl_warp + 1u) { tc::tc_fence_after(); tc::tmem_dealloc(sh->tmem_base, tc::TMEM_COLS); }
+    if (TENSOR_CORES && warp == tc::WARP_MMA) { tc::tc_fence_after(); tc::tmem_dealloc(sh->tmem_base, tc::TMEM_COLS); }
 }
 
 }  // namespace sched

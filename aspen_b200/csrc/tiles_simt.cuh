@@ -6,6 +6,7 @@
 // kernel.
 #pragma once
 #include "device_types.h"
+#include "gemm_ffma.cuh"
 #include "../../include/aspen_b200.h"
 
 // Barrier among the worker threads of a CTA only (the control warp does not take part).
@@ -83,7 +84,7 @@ __device__ __forceinline__ const float *input_pixel(const LayerDev &L, const Pix
 
 // ref src/tiled_kernels.c:613-638.  Pure streaming (12 bytes per element): four independent 16-byte
 // load pairs are in flight per thread before the first use.
-static __device__ __noinline__ void tile_residual(const LayerDev L, const TileDev T, unsigned tid, unsigned nthr) {
+static __device__ __noinline__ void tile_residual(const LayerDev &L, const TileDev &T, unsigned tid, unsigned nthr) {
     const unsigned h4 = T.tile_h >> 2, tail = T.tile_h & 3;
     const unsigned total = T.tile_w * h4;
     constexpr int U = 4;
@@ -125,7 +126,7 @@ static __device__ __noinline__ void tile_residual(const LayerDev L, const TileDe
 // issued before the first is used (a tap outside the image reads nothing and contributes the neutral element),
 // so the tile is bound by bandwidth instead of one load latency per tap.
 template <bool IS_MAX>
-static __device__ __noinline__ void tile_pool(const LayerDev L, const TileDev T, unsigned tid, unsigned nthr) {
+static __device__ __noinline__ void tile_pool(const LayerDev &L, const TileDev &T, unsigned tid, unsigned nthr) {
     const unsigned h4 = T.tile_h >> 2, per_col = h4 + (T.tile_h & 3);
     const float inv = 1.f / (float)(L.KH * L.KW);
     const float init = IS_MAX ? -INFINITY : 0.f;
@@ -205,7 +206,7 @@ __device__ __forceinline__ float warp_max(float v) {
 // A column of up to 1024 features is read ONCE: each lane keeps its up to eight 16-byte pieces in registers (all
 // loads issued before the first use), the warp reduces sum and sum of squares, and the normalised values are
 // written from the registers.  Longer or unaligned columns take the two-pass loop.
-static __device__ __noinline__ void tile_layernorm(const LayerDev L, const TileDev T, unsigned tid, unsigned nthr) {
+static __device__ __noinline__ void tile_layernorm(const LayerDev &L, const TileDev &T, unsigned tid, unsigned nthr) {
     const unsigned warp = tid >> 5, lane = tid & 31, nwarp = nthr >> 5;
     const unsigned M = T.tile_h;
     const float *gain = L.weight + T.pos_h;
@@ -275,7 +276,7 @@ static __device__ __noinline__ void tile_layernorm(const LayerDev L, const TileD
 }
 
 // ref src/tiled_kernels.c:640-673: max-subtracted softmax down each column.  One warp per column.
-static __device__ __noinline__ void tile_softmax(const LayerDev L, const TileDev T, unsigned tid, unsigned nthr) {
+static __device__ __noinline__ void tile_softmax(const LayerDev &L, const TileDev &T, unsigned tid, unsigned nthr) {
     const unsigned warp = tid >> 5, lane = tid & 31, nwarp = nthr >> 5;
     const unsigned M = T.tile_h;
     for (unsigned n = warp; n < T.tile_w; n += nwarp) {
@@ -292,7 +293,7 @@ static __device__ __noinline__ void tile_softmax(const LayerDev L, const TileDev
 }
 
 // ref src/tiled_kernels.c:675-709: box decode of one detection head.
-static __device__ __noinline__ void tile_yolo(const LayerDev L, const TileDev T, unsigned tid, unsigned nthr) {
+static __device__ __noinline__ void tile_yolo(const LayerDev &L, const TileDev &T, unsigned tid, unsigned nthr) {
     const unsigned C = L.p_out_c;
     const unsigned a_num = L.p_in_c / C, hw = L.IH * L.IW;
     for (unsigned i = tid; i < T.tile_w * C; i += nthr) {
@@ -315,7 +316,7 @@ static __device__ __noinline__ void tile_yolo(const LayerDev L, const TileDev T,
 }
 
 // ref src/tiled_kernels.c:711-741: nearest-neighbour upsample of PARENT_0 concatenated with PARENT_1.
-static __device__ __noinline__ void tile_append(const LayerDev L, const TileDev T, unsigned tid, unsigned nthr) {
+static __device__ __noinline__ void tile_append(const LayerDev &L, const TileDev &T, unsigned tid, unsigned nthr) {
     const unsigned c1 = L.p_in_c, c2 = L.p_out_c - L.p_in_c, C = c1 + c2;
     const unsigned w2 = L.OW, w1 = L.IW, s = L.p_stride;
     for (unsigned i = tid; i < T.tile_w * C; i += nthr) {
@@ -330,7 +331,7 @@ static __device__ __noinline__ void tile_append(const LayerDev L, const TileDev 
 }
 
 // ---- fp32 FFMA contraction tiles (validation mode) -----------------------------------------
-// out[col n][row m] = epilogue( sum_k  W(m, k) * X(n, k) ), fp32 multiply-add in k order.
+// out[col n][row m] = epilogue( sum_k  W(m, k) * X(n, k) ), fp32 multiply-add.
 //   conv     ref src/tiled_kernels.c:161-297   X(n,k): input pixel taps (kh, kw, ic), zero padding
 //   matmul   ref src/tiled_kernels.c:299-409   X(n,k): parent column n
 //   connected ref src/tiled_kernels.c:502-612  X(n,k): flattened sample n
@@ -376,7 +377,7 @@ __device__ __forceinline__ GemmView gemm_view(const LayerDev &L, const TileDev &
     return g;
 }
 
-// Layer-0 tile (service mode only): the uploaded input becomes the columns of the layer's activation matrix that the
+// Layer-0 tile: the uploaded input becomes the columns of the layer's activation matrix that the
 // tile covers -- what the host-launched unpack / rounding / embedding-gather / padded-copy kernels do for a run that
 // is launched per graph.  Sources are read through L2 (the host's DMA wrote them while this kernel was running).
 static __device__ void tile_input(const InputDev &I, const LayerDev &L, const TileDev &T, unsigned tid, unsigned nthr) {
@@ -453,85 +454,146 @@ static __device__ void tile_input(const InputDev &I, const LayerDev &L, const Ti
         }
 }
 
-static __device__ void tile_gemm_ffma(const LayerDev L, const TileDev T, unsigned tid, unsigned nthr) {
-    const GemmView g = gemm_view(L, T);
-    const unsigned mg = (T.tile_h + 3) >> 2;             // groups of 4 output rows
-    const bool vec = !g.w_transposed && (g.conv ? (L.IC & 3) == 0 : (g.K & 3) == 0) && L.a_vec4;
-    const bool is_k = L.type == K_ATTENTION_LAYER;
-    const float scale = is_k ? sqrtf((float)L.hd) : 1.f;
-    const unsigned q0 = is_k ? T.pos_w % L.seq : 0;
-    for (unsigned i = tid; i < mg * T.tile_w; i += nthr) {
-        const unsigned n = i % T.tile_w, m0 = (i / T.tile_w) * 4;
-        float acc[4] = {0.f, 0.f, 0.f, 0.f};
-        const float *w[4];
-        for (int r = 0; r < 4; r++) {
-            unsigned m = m0 + r < T.tile_h ? m0 + r : T.tile_h - 1;   // clamp: duplicates are discarded below
-            w[r] = g.w_transposed ? g.wbase + m : g.wbase + (size_t)m * g.wld;
-        }
-        if (g.conv) {
-            PixelWin pw = pixel_window(L, T.pos_w + n);
-            unsigned k = 0;
-            for (int kh = 0; kh < (int)L.KH; kh++)
-                for (int kw = 0; kw < (int)L.KW; kw++, k += L.IC) {
-                    const float *x = input_pixel(L, pw, kh, kw);
-                    if (!x) continue;
-                    if (vec) {
-                        for (unsigned c = 0; c < L.IC; c += 4) {
-                            float4 xv = ldcg4(x + c);
-                            for (int r = 0; r < 4; r++) {
-                                float4 wv = *reinterpret_cast<const float4 *>(w[r] + k + c);
-                                acc[r] = fmaf(wv.x, xv.x, acc[r]); acc[r] = fmaf(wv.y, xv.y, acc[r]);
-                                acc[r] = fmaf(wv.z, xv.z, acc[r]); acc[r] = fmaf(wv.w, xv.w, acc[r]);
-                            }
-                        }
-                    } else {
-                        for (unsigned c = 0; c < L.IC; c++) {
-                            float xv = ldcg1(x + c);
-                            for (int r = 0; r < 4; r++) acc[r] = fmaf(w[r][k + c], xv, acc[r]);
-                        }
-                    }
-                }
+// ---- contraction tiles in fp32 ------------------------------------------------------------------
+// Operand loaders of gemm_ffma.cuh over a layer's matrices.
+template <int NR>
+struct WeightRows {           // rows of W: weights, attention keys, or (transposed) attention values
+    const GemmView &g;
+    unsigned rows, k_end;     // rows of the tile, values of k that exist in memory
+    bool vec;
+    unsigned k0, at_row[NR];
+    bool ok[NR];
+    __device__ __forceinline__ WeightRows(const GemmView &v, unsigned r, unsigned ke, bool ve) : g(v), rows(r), k_end(ke), vec(ve), k0(0) {}
+    __device__ __forceinline__ void row(int i, unsigned r) { ok[i] = r < rows; at_row[i] = ok[i] ? r : 0u; }
+    __device__ __forceinline__ void at(unsigned k) { k0 = k; }
+    __device__ __forceinline__ void copy(unsigned dst, int i) const {
+        if (vec) {
+            const bool in = ok[i] && k0 < k_end;
+            fmablk::copy_async<16>(dst, g.wbase + (in ? (size_t)at_row[i] * g.wld + k0 : 0), in);
         } else {
-            const float *x = g.xbase + (size_t)n * g.xld;
-            if (vec) {
-                for (unsigned k = 0; k < g.K; k += 4) {
-                    float4 xv = ldcg4(x + k);
-                    for (int r = 0; r < 4; r++) {
-                        float4 wv = ldcg4(w[r] + k);
-                        acc[r] = fmaf(wv.x, xv.x, acc[r]); acc[r] = fmaf(wv.y, xv.y, acc[r]);
-                        acc[r] = fmaf(wv.z, xv.z, acc[r]); acc[r] = fmaf(wv.w, xv.w, acc[r]);
-                    }
-                }
-            } else {
-                for (unsigned k = 0; k < g.K; k++) {
-                    float xv = ldcg1(x + k);
-                    for (int r = 0; r < 4; r++) acc[r] = fmaf(ldcg1(g.w_transposed ? w[r] + (size_t)k * g.wld : w[r] + k), xv, acc[r]);
-                }
+            #pragma unroll
+            for (unsigned e = 0; e < 4; e++) {
+                const bool in = ok[i] && k0 + e < k_end;
+                const size_t off = g.w_transposed ? (size_t)(k0 + e) * g.wld + at_row[i] : (size_t)at_row[i] * g.wld + k0 + e;
+                fmablk::copy_async<4>(dst + e * 4u, g.wbase + (in ? off : 0), in);
             }
-        }
-        float *o = L.out + (size_t)(T.pos_w + n) * L.ldc + T.pos_h + m0;
-        for (int r = 0; r < 4; r++) {
-            if (m0 + r >= T.tile_h) break;
-            float v = acc[r];
-            if (is_k) {
-                if (L.masked && (T.pos_h + m0 + r) > (q0 + n)) v = -1e10f;
-                v = expf(v / scale);
-            } else if (L.type != V_ATTENTION_LAYER) {
-                if (L.bias) v += L.bias[T.pos_h + m0 + r];
-                v = activate(v, L.act);
-            }
-            o[r] = v;
         }
     }
-    if (is_k) {   // normalise every column by its sum (no max subtraction, as the reference)
-        worker_barrier(nthr);
+};
+template <int NR>
+struct ActivationRows {       // rows of X: columns of the parent matrix, or the taps of output pixels
+    const LayerDev &L;
+    const GemmView &g;
+    unsigned pos, cols;
+    bool vec;
+    unsigned k0, ic;
+    int kh, kw;
+    const float *p[NR];
+    PixelWin pw[NR];
+    bool ok[NR];
+    __device__ __forceinline__ ActivationRows(const LayerDev &l, const GemmView &v, unsigned po, unsigned c, bool ve)
+        : L(l), g(v), pos(po), cols(c), vec(ve), k0(0), ic(0), kh(0), kw(0) {}
+    __device__ __forceinline__ void row(int i, unsigned r) {
+        ok[i] = r < cols;
+        if (g.conv) pw[i] = pixel_window(L, pos + (ok[i] ? r : 0u));
+        else p[i] = g.xbase + (size_t)(ok[i] ? r : 0u) * g.xld;
+    }
+    __device__ __forceinline__ void at(unsigned k) {
+        k0 = k;
+        if (g.conv) { const unsigned tap = k / L.IC; ic = k - tap * L.IC; kh = (int)(tap / L.KW); kw = (int)(tap - (unsigned)kh * L.KW); }
+    }
+    __device__ __forceinline__ void copy(unsigned dst, int i) const {
+        if (vec) {
+            const float *src = nullptr;
+            if (ok[i] && k0 < g.K) {
+                if (g.conv) { src = input_pixel(L, pw[i], kh, kw); if (src) src += ic; }
+                else src = p[i] + k0;
+            }
+            fmablk::copy_async<16>(dst, src ? src : L.in0, src != nullptr);
+        } else {
+            unsigned c = ic;
+            int h = kh, w = kw;
+            #pragma unroll
+            for (unsigned e = 0; e < 4; e++) {
+                const float *src = nullptr;
+                if (ok[i] && k0 + e < g.K) {
+                    if (g.conv) { src = input_pixel(L, pw[i], h, w); if (src) src += c; }
+                    else src = p[i] + k0 + e;
+                }
+                fmablk::copy_async<4>(dst + e * 4u, src ? src : L.in0, src != nullptr);
+                if (g.conv && ++c == L.IC) { c = 0; if (++w == (int)L.KW) { w = 0; h++; } }
+            }
+        }
+    }
+};
+struct StoreTile {
+    const LayerDev &L;
+    const TileDev &T;
+    unsigned m0, n0, q0;
+    bool is_k;
+    float scale;
+    __device__ __forceinline__ void operator()(unsigned mi, unsigned ni, const float *v) const {
+        const unsigned m = m0 + mi, n = n0 + ni;
+        if (n >= T.tile_w || m >= T.tile_h) return;
+        float r[4];
+        #pragma unroll
+        for (unsigned j = 0; j < 4; j++) {
+            float x = v[j];
+            if (is_k) {
+                if (L.masked && T.pos_h + m + j > q0 + n) x = -1e10f;
+                x = expf(x / scale);
+            } else {
+                if (L.type != V_ATTENTION_LAYER) {
+                    if (L.bias && m + j < T.tile_h) x += L.bias[T.pos_h + m + j];
+                    x = activate(x, L.act);
+                }
+                x = store_round(x, L);
+            }
+            r[j] = x;
+        }
+        float *o = L.out + (size_t)(T.pos_w + n) * L.ldc + T.pos_h + m;
+        if (m + 4u <= T.tile_h && (reinterpret_cast<uintptr_t>(o) & 15u) == 0u) *reinterpret_cast<float4 *>(o) = make_float4(r[0], r[1], r[2], r[3]);
+        else
+            #pragma unroll
+            for (unsigned j = 0; j < 4; j++) if (m + j < T.tile_h) o[j] = r[j];
+    }
+};
+struct WorkerBarrier { __device__ __forceinline__ void operator()() const { worker_barrier(fmablk::THREADS); } };
+
+template <typename S>
+static __device__ __noinline__ void ffma_blocks(const LayerDev &L, const TileDev &T, unsigned tid, unsigned char *scratch) {
+    const GemmView g = gemm_view(L, T);
+    const bool is_k = L.type == K_ATTENTION_LAYER, weights = !is_k && L.type != V_ATTENTION_LAYER;
+    const bool vec_x = L.a_vec4 != 0, vec_w = weights || (is_k && L.a_vec4 != 0);      // weight rows are zero padded to Kpad
+    for (unsigned n0 = 0; n0 < T.tile_w; n0 += S::BN)
+        for (unsigned m0 = 0; m0 < T.tile_h; m0 += S::BM) {
+            GemmView b = g;
+            b.wbase += g.w_transposed ? (size_t)m0 : (size_t)m0 * g.wld;
+            if (!g.conv) b.xbase += (size_t)n0 * g.xld;
+            WeightRows<S::RW> lw(b, T.tile_h - m0, weights ? L.Kpad : g.K, vec_w);
+            ActivationRows<S::RX> lx(L, b, T.pos_w + n0, T.tile_w - n0, vec_x);
+            StoreTile out{L, T, m0, n0, is_k ? T.pos_w % L.seq : 0u, is_k, is_k ? sqrtf((float)L.hd) : 1.f};
+            fmablk::block<S>(scratch, tid, g.K, lw, lx, WorkerBarrier(), out);
+        }
+}
+
+// Tile in fp32 (ref src/tiled_kernels.c:21-490, 784-1038).  FULL: the fp32 mode, 96 KB of staging; the shape of the blocks
+// follows the tile (a shape larger than the tile would compute padding).  Otherwise the few layers of a tensor-core graph that
+// no TMA box can stage (IC % 32 != 0, head size % 32 != 0, ...).
+template <bool FULL>
+static __device__ void tile_gemm_ffma(const LayerDev &L, const TileDev &T, unsigned tid, unsigned nthr, unsigned char *scratch) {
+    if (!FULL) ffma_blocks<fmablk::Tight>(L, T, tid, scratch);
+    else if (T.tile_h > 64 && T.tile_w > 32) ffma_blocks<fmablk::Large>(L, T, tid, scratch);
+    else if (T.tile_h > 32 && T.tile_w > 32) ffma_blocks<fmablk::Medium>(L, T, tid, scratch);
+    else ffma_blocks<fmablk::Small>(L, T, tid, scratch);
+    if (L.type == K_ATTENTION_LAYER) {   // normalise every column by its sum (no max subtraction, as the reference)
         const unsigned warp = tid >> 5, lane = tid & 31, nwarp = nthr >> 5;
         for (unsigned n = warp; n < T.tile_w; n += nwarp) {
             float *o = L.out + (size_t)(T.pos_w + n) * L.ldc + T.pos_h;
             float s = 0.f;
             for (unsigned m = lane; m < T.tile_h; m += 32) s += ldcg1(o + m);
             s = warp_sum(s);
-            for (unsigned m = lane; m < T.tile_h; m += 32) o[m] = ldcg1(o + m) / s;
+            for (unsigned m = lane; m < T.tile_h; m += 32) o[m] = store_round(ldcg1(o + m) / s, L);
         }
     }
 }
