@@ -87,8 +87,9 @@ __device__ __forceinline__ bool mbar_test_wait(unsigned long long *bar, unsigned
                  : "=r"(ok) : "r"(smem_u32(bar)), "r"(parity) : "memory");
     return ok != 0;
 }
-// Bounded wait.  Returns false (and marks the run aborted) when the time budget runs out.  The common case is a handful of
-// try_waits (each suspends the thread for a while in hardware); clock, budget and abort flag are only looked at after many.
+// Bounded wait.  Returns false (and marks the run aborted) when the time budget runs out.  The one-thread roles are bound by the
+// length of their instruction stream, so the common case is four instructions; clock, budget and abort flag are only looked at
+// after some ten thousand try_waits (each suspends the thread for a while in hardware), out of the loop's way.
 __device__ __forceinline__ bool mbar_wait_slow(unsigned long long *bar, unsigned parity, CtrlDev *ctrl, StatusHost *status, unsigned where) {
     unsigned long long t0;
     asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t0));
@@ -111,9 +112,20 @@ __device__ __forceinline__ bool mbar_wait_slow(unsigned long long *bar, unsigned
     return false;
 }
 __device__ __forceinline__ bool mbar_wait(unsigned long long *bar, unsigned parity, CtrlDev *ctrl, StatusHost *status, unsigned where) {
-    #pragma unroll 1
-    for (unsigned spin = 0; spin < 4096u; spin++)
-        if (mbar_try_wait(bar, parity)) return true;
+    unsigned ok;
+    asm volatile("{\n\t.reg .pred p, q;\n\t.reg .u32 c;\n\t"
+                 "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+                 "@p bra DONE;\n\t"
+                 "mov.u32 c, 0;\n"
+                 "AGAIN:\n\t"
+                 "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+                 "@p bra DONE;\n\t"
+                 "add.u32 c, c, 1;\n\t"
+                 "setp.lt.u32 q, c, 10000;\n\t"
+                 "@q bra AGAIN;\n"
+                 "DONE:\n\t"
+                 "selp.u32 %0, 1, 0, p;\n\t}" : "=r"(ok) : "r"(smem_u32(bar)), "r"(parity) : "memory");
+    if (__builtin_expect(ok != 0u, 1)) return true;
     return mbar_wait_slow(bar, parity, ctrl, status, where);
 }
 
@@ -147,9 +159,18 @@ __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::
 __device__ __forceinline__ void tc_commit(unsigned long long *bar) {
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
 }
-__device__ __forceinline__ void tc_mma_tf32(unsigned d_tmem, unsigned long long adesc, unsigned long long bdesc, unsigned idesc, unsigned accumulate) {
-    asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\ttcgen05.mma.cta_group::1.kind::tf32 [%0], %1, %2, %3, p;\n\t}"
-                 ::"r"(d_tmem), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate) : "memory");
+// K-major, 128-byte swizzle, 8-row groups 1024 bytes apart; version 1 (sm_100) in bits 46-47.  Only the low word, which holds
+// the address, changes: leading byte offset (unused for swizzled K-major) in bits 16-29.
+constexpr unsigned UMMA_DESC_HIGH = (1024u >> 4) | 1u << 14 | 2u << 29;
+__device__ __forceinline__ unsigned umma_desc_low(unsigned smem_addr) { return (smem_addr >> 4) | 1u << 16; }
+// The four k = 8 steps of one stage.
+__device__ __forceinline__ void tc_mma_stage(unsigned d_tmem, unsigned alow, unsigned blow, unsigned idesc, unsigned accumulate) {
+    asm volatile("{\n\t.reg .pred p, t;\n\t.reg .b64 a, b;\n\t.reg .b32 al, bl;\n\tsetp.ne.b32 p, %4, 0;\n\tsetp.eq.b32 t, %4, %4;\n\t"
+                 "mov.b64 a, {%1, %5};\n\tmov.b64 b, {%2, %5};\n\ttcgen05.mma.cta_group::1.kind::tf32 [%0], a, b, %3, p;\n\t"
+                 "add.u32 al, %1, 2;\n\tadd.u32 bl, %2, 2;\n\tmov.b64 a, {al, %5};\n\tmov.b64 b, {bl, %5};\n\ttcgen05.mma.cta_group::1.kind::tf32 [%0], a, b, %3, t;\n\t"
+                 "add.u32 al, %1, 4;\n\tadd.u32 bl, %2, 4;\n\tmov.b64 a, {al, %5};\n\tmov.b64 b, {bl, %5};\n\ttcgen05.mma.cta_group::1.kind::tf32 [%0], a, b, %3, t;\n\t"
+                 "add.u32 al, %1, 6;\n\tadd.u32 bl, %2, 6;\n\tmov.b64 a, {al, %5};\n\tmov.b64 b, {bl, %5};\n\ttcgen05.mma.cta_group::1.kind::tf32 [%0], a, b, %3, t;\n\t}"
+                 ::"r"(d_tmem), "r"(alow), "r"(blow), "r"(idesc), "r"(accumulate), "r"(UMMA_DESC_HIGH) : "memory");
 }
 __device__ __forceinline__ void tmem_ld32(unsigned taddr, float *v) {
     unsigned *r = reinterpret_cast<unsigned *>(v);
@@ -176,16 +197,6 @@ __device__ __forceinline__ void tmem_st32(unsigned taddr, const float *v) {
     asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
 }
 
-// K-major, 128-byte swizzle, 8-row groups 1024 bytes apart; version 1 (sm_100) in bits 46-47.
-__device__ __forceinline__ unsigned long long umma_desc(unsigned smem_addr) {
-    unsigned long long d = 0;
-    d |= (unsigned long long)((smem_addr & 0x3ffffu) >> 4);
-    d |= (unsigned long long)1 << 16;                 // leading byte offset (unused for swizzled K-major)
-    d |= (unsigned long long)(1024 >> 4) << 32;       // stride byte offset
-    d |= (unsigned long long)1 << 46;
-    d |= (unsigned long long)2 << 61;                 // SWIZZLE_128B
-    return d;
-}
 // D fp32, A/B tf32, both K-major, M = 128, N = n.
 __device__ __forceinline__ unsigned umma_idesc(unsigned n) {
     return (1u << 4) | (2u << 7) | (2u << 10) | ((n >> 3) << 17) | ((128u >> 4) << 24);
@@ -349,9 +360,7 @@ __device__ __forceinline__ bool issue_mma(const Slot &sl, unsigned ring, Ring &r
                 if (!mbar_wait(&sh->full[r.s], r.parity(), ctrl, status, 3)) return false;
                 tc_fence_after();
                 const unsigned sA = ring + r.s * r.stage_bytes;
-                const unsigned long long adesc = umma_desc(sA), bdesc = umma_desc(sA + A_STAGE_BYTES);
-                #pragma unroll
-                for (unsigned k8 = 0; k8 < 4; k8++) tc_mma_tf32(d, adesc + 2ull * k8, bdesc + 2ull * k8, idesc, (kc | k8) != 0u);
+                tc_mma_stage(d, umma_desc_low(sA), umma_desc_low(sA + A_STAGE_BYTES), idesc, kc);
                 tc_commit(&sh->empty[r.s]);
                 r.step();
             }
