@@ -8,6 +8,8 @@
 // written to .nasm files) come out identical in milliseconds.
 #include "internal.h"
 
+#include <algorithm>
+#include <thread>
 #include <unordered_set>
 
 namespace {
@@ -55,6 +57,13 @@ void ParentFinder::run(ninst_t &ni, std::vector<unsigned int> &out, std::vector<
     const unsigned int w0 = ni.out_mat_pos[OUT_W], h0 = ni.out_mat_pos[OUT_H];
     const unsigned int tw = ni.tile_dims[OUT_W], th = ni.tile_dims[OUT_H];
     const unsigned int p0th = p0.ninst_tile_dims[OUT_H], p0tw = p0.ninst_tile_dims[OUT_W];
+    std::vector<unsigned int> cols, last_cols;
+    // Element-wise types: a column (row) inside the same parent tiles as the one before visits nothing new.
+    const unsigned int p1tw = p1 ? p1->ninst_tile_dims[OUT_W] : 0, p1th = p1 ? p1->ninst_tile_dims[OUT_H] : 0;
+    const bool same_shape = type == RESIDUAL_LAYER || type == SOFTMAX_LAYER || type == LAYERNORM_LAYER;
+    auto same_col = [&](unsigned int w) { return w != w0 && w % p0tw != 0 && (!p1 || w % p1tw != 0); };
+    auto same_row = [&](unsigned int h) { return h != h0 && h % p0th != 0 && (!p1 || h % p1th != 0); };
+    uint64_t last_q = ~0ull;
     std::unordered_set<uint64_t> done;   // signatures of element visits that cannot add anything new
     uint64_t last_sig = ~0ull;
 
@@ -68,18 +77,25 @@ void ParentFinder::run(ninst_t &ni, std::vector<unsigned int> &out, std::vector<
             tensor_pos_from_out_mat_pos(&ld, mp, tp);
             ip[BATCH] = tp[BATCH];
             if (ip[BATCH] >= batch) continue;
-            for (unsigned int c = 0; c < p[IN_C]; c += p0th - c % p0th) {   // first channel of each parent row block
-                ip[OUT_C] = c;
-                for (unsigned int kh = 0; kh < p[WEIGHT_H]; kh++) {
-                    ip[OUT_H] = tp[OUT_H] * p[STRIDE] + kh * p[DILATION] - p[PADDING];   // unsigned wrap == "negative"
-                    if (ip[OUT_H] >= p[IN_H]) continue;
-                    for (unsigned int kw = 0; kw < p[WEIGHT_W]; kw++) {
-                        ip[OUT_W] = tp[OUT_W] * p[STRIDE] + kw * p[DILATION] - p[PADDING];
-                        if (ip[OUT_W] >= p[IN_W]) continue;
-                        add(tile_from_tensor_pos(p0, ip));
-                    }
+            // the parent columns of the taps in visiting order, one entry per tile column; the channel blocks repeat them
+            cols.clear();
+            for (unsigned int kh = 0; kh < p[WEIGHT_H]; kh++) {
+                const unsigned int y = tp[OUT_H] * p[STRIDE] + kh * p[DILATION] - p[PADDING];   // unsigned wrap == "negative"
+                if (y >= p[IN_H]) continue;
+                for (unsigned int kw = 0; kw < p[WEIGHT_W]; kw++) {
+                    const unsigned int x = tp[OUT_W] * p[STRIDE] + kw * p[DILATION] - p[PADDING];
+                    if (x >= p[IN_W]) continue;
+                    ip[OUT_H] = y; ip[OUT_W] = x;
+                    unsigned int pos[2];
+                    out_mat_pos_from_tensor_pos(&p0, ip, pos);
+                    const unsigned int tc = pos[OUT_W] / p0tw;
+                    if (std::find(cols.begin(), cols.end(), tc) == cols.end()) cols.push_back(tc);
                 }
             }
+            if (cols == last_cols) continue;         // nothing new in this column
+            last_cols = cols;
+            for (unsigned int c = 0; c < p[IN_C]; c += p0th - c % p0th)   // first channel of each parent row block
+                for (unsigned int tc : cols) add(tile_of(p0, c, tc * p0tw));
         } else if (type == FC_LAYER) {
             // Column = one sample; reads every channel and pixel of it.
             const unsigned int b = w;
@@ -108,7 +124,17 @@ void ParentFinder::run(ninst_t &ni, std::vector<unsigned int> &out, std::vector<
         } else {
             // Element-wise dependent types: visit rows, skipping visits whose candidate list equals
             // that of an earlier visit (they can only produce duplicates).
+            if (same_shape && same_col(w)) continue;
+            if (type == K_ATTENTION_LAYER) {
+                const unsigned int per = seq * p[NUM_HEAD], b = w / per, head = (w % per) / seq;
+                const uint64_t q = ((uint64_t)(b * p[NUM_HEAD] + head) << 32) | ((b * seq + w % seq) / p0tw);
+                if (q == last_q) continue;           // same sample, head and query tile as the column before
+                last_q = q;
+            }
             for (unsigned int h = h0; h < h0 + th; h++) {
+                if (same_shape && same_row(h)) continue;
+                if (type == K_ATTENTION_LAYER && p1 && h != h0 && (w / (seq * p[NUM_HEAD]) * seq + h) % p1tw != 0) continue;
+                if (type == V_ATTENTION_LAYER && p1 && h != h0 && h % (p[NUM_HIDDEN] / p[NUM_HEAD]) != 0 && h % p1th != 0) continue;
                 mp[OUT_H] = h;
                 unsigned int tp[NUM_PARAM_ELEMENTS] = {}, ip[NUM_PARAM_ELEMENTS] = {};
                 tensor_pos_from_out_mat_pos(&ld, mp, tp);
@@ -209,26 +235,40 @@ void ParentFinder::run(ninst_t &ni, std::vector<unsigned int> &out, std::vector<
     list = &extra;
     if (type == RESIDUAL_LAYER && p1) {
         for (unsigned int w = w0; w < w0 + tw; w++)
-            for (unsigned int h = h0; h < h0 + th; h++) {
+            for (unsigned int h = h0; !same_col(w) && h < h0 + th; h++) {
+                if (same_row(h)) continue;
                 add(tile_of(p0, h, w));
                 add(tile_of(*p1, h, w));
             }
     } else if (type == SOFTMAX_LAYER) {
         for (unsigned int w = w0; w < w0 + tw; w++)
-            for (unsigned int h = h0; h < h0 + th; h++) add(tile_of(p0, h, w));
+            for (unsigned int h = h0; !same_col(w) && h < h0 + th; h++)
+                if (!same_row(h)) add(tile_of(p0, h, w));
     }
 }
 
 }  // namespace
 
+// Every tile's list stands by itself: the tiles are dealt to the host's cores in small runs.
 void graph_find_parents(nasm_t *nasm) {
-    ParentFinder pf(nasm);
-    for (auto &ni : nasm->ninst) {
-        ni.parent_ninst_idx.clear();
-        ni.extra_parent_idx.clear();
-        pf.run(ni, ni.parent_ninst_idx, ni.extra_parent_idx);
-        if (ni.parent_ninst_idx.size() > MAX_PARENT_NINST_NUM) ASPEN_ERR("ninst %u has more than %d parents\n", ni.ninst_idx, MAX_PARENT_NINST_NUM);
-    }
+    std::atomic<unsigned int> next{0};
+    const unsigned int n = nasm->num_ninst, run = 64;
+    auto work = [&] {
+        ParentFinder pf(nasm);
+        for (unsigned int at; (at = next.fetch_add(run)) < n;)
+            for (unsigned int i = at; i < std::min(n, at + run); i++) {
+                ninst_t &ni = nasm->ninst[i];
+                ni.parent_ninst_idx.clear();
+                ni.extra_parent_idx.clear();
+                pf.run(ni, ni.parent_ninst_idx, ni.extra_parent_idx);
+                if (ni.parent_ninst_idx.size() > MAX_PARENT_NINST_NUM) ASPEN_ERR("ninst %u has more than %d parents\n", ni.ninst_idx, MAX_PARENT_NINST_NUM);
+            }
+    };
+    const unsigned int cores = std::min(16u, std::max(1u, std::thread::hardware_concurrency()));
+    std::vector<std::thread> team;
+    for (unsigned int i = 1; i < cores && i * run < n; i++) team.emplace_back(work);
+    work();
+    for (std::thread &t : team) t.join();
 }
 
 // Children in ascending tile order, as the reference's forward scan yields (src/apu_nasm.c:544-576).
