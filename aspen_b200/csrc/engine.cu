@@ -4,10 +4,12 @@
 // sm_100 device every entry point fails with an error.
 #include "internal.h"
 #include "scheduler.cuh"
+#include "hostcopy.h"
 
 #include <cuda.h>
 #include <cuda_runtime.h>
 #include <algorithm>
+#include <memory>
 #include <mutex>
 #include <sched.h>
 #include <unordered_map>
@@ -199,6 +201,7 @@ struct Engine {
     unsigned long long idle_ns = 20000000ull;   // the kernel leaves after this long with no pass running
     cudaEvent_t svc_armed_ev = nullptr;
     unsigned svc_ahead = 32, run_ahead = 0;   // see CtrlDev::ahead: in service mode / in a launch per run
+    std::unique_ptr<HostCopy> copy;   // results into pageable memory
     unsigned long long *prof = nullptr;   // per-CTA time accounting, allocated when ASPEN_B200_PROFILE is set
 };
 
@@ -275,6 +278,7 @@ Engine *engine_create(int device, int precision, unsigned int /*num_dse_hint*/) 
     e->device = device;
     e->precision = precision;
     e->num_sms = prop.multiProcessorCount;
+    e->copy.reset(new HostCopy());
     unsigned long long v;
     e->n_ctas = (unsigned)e->num_sms;
     if (env_u64("ASPEN_B200_CTAS", &v) && v > 0 && v <= (unsigned long long)e->num_sms) e->n_ctas = (unsigned)v;
@@ -946,7 +950,7 @@ static int attach(Engine *e, nasm_t *nasm, const void *input_host, const int *id
             CUDA_TRY(cudaStreamSynchronize(e->stream));
         } else {
             CUDA_TRY(cudaMemcpyAsync(dst, input_host, n * sizeof(float), cudaMemcpyHostToDevice, e->io));
-            CUDA_TRY(cudaStreamSynchronize(e->io));
+            CUDA_TRY(cudaStreamSynchronize(e->io));      // the caller may reuse its buffer as soon as we return
         }
     }
     if (svc_done(dn)) dn->svc_armed++;
@@ -981,10 +985,10 @@ long engine_read_ldata(nasm_t *nasm, unsigned int idx, float *out) {
     if (!e->service && !svc_done(dn) && svc_serves(e, nasm)) svc_join(e, false);      // the graph is being computed
     // the copy engine packs strided matrices: a kernel could not start next to a resident one
     const size_t row = (size_t)ld.out_mat_dims[OUT_H] * sizeof(float);
-    const cudaError_t err = ld.out_mat_stride == ld.out_mat_dims[OUT_H]
-        ? cudaMemcpyAsync(out, src, n * sizeof(float), cudaMemcpyDeviceToHost, e->io)
+    const bool packed = ld.out_mat_stride == ld.out_mat_dims[OUT_H];
+    const cudaError_t err = packed ? e->copy->down(out, src, n * sizeof(float), e->io)
         : cudaMemcpy2DAsync(out, row, src, (size_t)ld.out_mat_stride * sizeof(float), row, ld.out_mat_dims[OUT_W], cudaMemcpyDeviceToHost, e->io);
-    if (err != cudaSuccess || cudaStreamSynchronize(e->io) != cudaSuccess) {
+    if (err != cudaSuccess || (!packed && cudaStreamSynchronize(e->io) != cudaSuccess)) {
         ASPEN_ERR("CUDA error reading layer %u: %s\n", idx, cudaGetErrorString(cudaGetLastError()));
         return -1;
     }
