@@ -208,6 +208,7 @@ struct Engine {
 struct DeviceNasm {
     Engine *e = nullptr;
     DeviceDnn *dd = nullptr;
+    std::unique_ptr<nasm_t> plan;   // the tiles the device executes; empty: the nasm's own
     float *arena = nullptr;
     size_t arena_bytes = 0;
     std::vector<size_t> ldata_off;
@@ -393,10 +394,27 @@ static void free_device_nasm(DeviceNasm *dn) {
     delete dn;
 }
 
-static int build_device_nasm(Engine *e, nasm_t *nasm) {
+// Layer `i` follows from layer `from` through per-token layers, at least one of which reads whole columns.
+static bool follows(const nasm_t *nasm, unsigned i, unsigned from, bool whole) {
+    if (i == (unsigned)-1 || i < from) return false;
+    if (i == from) return whole;
+    const LAYER_TYPE t = nasm->ldata[i].layer->type;
+    if (t != MATMUL_LAYER && t != LAYERNORM_LAYER && t != RESIDUAL_LAYER) return false;
+    whole = whole || t != RESIDUAL_LAYER;
+    return follows(nasm, nasm->ldata[i].parent_ldata_idx_arr[PARENT_0], from, whole) ||
+           (t == RESIDUAL_LAYER && follows(nasm, nasm->ldata[i].parent_ldata_idx_arr[PARENT_1], from, whole));
+}
+
+// The graph as the device executes it: layer geometry (strides, tiles) and lists.
+static const nasm_t *device_view(const nasm_t *nasm) { return nasm->dev->plan ? nasm->dev->plan.get() : nasm; }
+
+static int build_device_nasm(Engine *e, nasm_t *host_nasm) {
     DeviceNasm *dn = new DeviceNasm();
     dn->e = e;
-    nasm->dev = dn;
+    host_nasm->dev = dn;
+    const char *keep_tiles = getenv("ASPEN_B200_PLAN");      // 0: execute the nasm's own tiles
+    if (host_nasm->own_lists && !(keep_tiles && atoi(keep_tiles) == 0)) dn->plan.reset(plan_device_tiles(host_nasm, e->precision, e->n_ctas, e->service));
+    const nasm_t *nasm = device_view(host_nasm);
     if (upload_weights(nasm->dnn, e->device, e->precision, &dn->dd) != 0) return -1;
     // activation arena: one region per layer (no reuse: every layer output stays readable)
     dn->ldata_off.resize(nasm->num_ldata);
@@ -461,6 +479,7 @@ static int build_device_nasm(Engine *e, nasm_t *nasm) {
     const char *no_rows = getenv("ASPEN_B200_NO_ROW_BOXES");
     float *probs = nullptr;                                    // see K_ATTENTION below
     size_t probs_bytes = 0;
+    unsigned probs_reader = 0;
     std::vector<float *> moved(nasm->num_ldata, nullptr);      // layers that write elsewhere than into the arena
     for (unsigned i = 0; i < nasm->num_ldata; i++) {
         const aspen_layer_t &l = *nasm->ldata[i].layer;
@@ -544,14 +563,17 @@ static int build_device_nasm(Engine *e, nasm_t *nasm) {
         if (gemm_w && L.a_kind != tc::A_NONE && L.amap >= 0)
             L.wmap = add_map(L.weight, L.Kpad, layer_weight_rows(&l), (cuuint64_t)L.Kpad * sizeof(float), L.b_box);
         L.tc = L.a_kind != tc::A_NONE && L.amap >= 0 && L.wmap >= 0;
-        // Attention probabilities that only the attention_v layer reads need not stay: when hidden states may go, every such
-        // layer writes the same scratch matrix, which then lives in L2.  (A sample's scores of one layer are computed after all its
-        // attention outputs of the layer before: they follow from them through the projections.)
-        if (l.type == K_ATTENTION_LAYER && L.tc && !keep_hidden_states() && i != nasm->num_ldata - 1) {
-            unsigned readers = 0, v_readers = 0;
+        // ASPEN_B200_ATTN_FUSE=1 with hidden states given up: attention probabilities that only the attention_v layer reads do not
+        // stay; every such layer writes the same scratch matrix, which then lives in L2.  The layer's keys have to follow from
+        // the attention outputs of the layer before through per-token layers, one of which reads whole columns:
+        // all of a sample's probabilities have then been read before the next layer's are written.
+        const char *drop_probs = getenv("ASPEN_B200_ATTN_FUSE");
+        if (l.type == K_ATTENTION_LAYER && L.tc && drop_probs && atoi(drop_probs) != 0 && !keep_hidden_states() && i != nasm->num_ldata - 1 &&
+            (!probs || follows(nasm, p1, probs_reader, false))) {
+            unsigned readers = 0, v_readers = 0, reader = 0;
             for (unsigned j = 1; j < nasm->num_ldata; j++)
                 for (int k = PARENT_0; k <= PARENT_1; k++)
-                    if (nasm->ldata[j].parent_ldata_idx_arr[k] == i) { readers++; v_readers += k == PARENT_0 && nasm->ldata[j].layer->type == V_ATTENTION_LAYER; }
+                    if (nasm->ldata[j].parent_ldata_idx_arr[k] == i) { readers++; if (k == PARENT_0 && nasm->ldata[j].layer->type == V_ATTENTION_LAYER) { v_readers++; reader = j; } }
             const size_t bytes = nasm->ldata[i].out_mat_mem_size + 256;
             if (readers == 1 && v_readers == 1 && (!probs || bytes == probs_bytes)) {
                 if (!probs) {
@@ -561,6 +583,7 @@ static int build_device_nasm(Engine *e, nasm_t *nasm) {
                     probs_bytes = bytes;
                 }
                 L.out = probs;
+                probs_reader = reader;
                 moved[i] = probs;
             }
         }
@@ -581,7 +604,7 @@ static int build_device_nasm(Engine *e, nasm_t *nasm) {
     // (fused_other[producer] = that layer).  The residual layer's own tiles leave the device
     // graph.  ASPEN_B200_NO_FUSE=1 keeps the layers separate.
     std::vector<unsigned> fused_other(nasm->num_ldata, (unsigned)-1);
-    std::vector<unsigned char> written_by_parents(nasm->num_ldata, 0);
+    std::vector<unsigned> written_by(nasm->num_ldata, (unsigned)-1);      // residual layer -> the layer whose tiles write it
     const char *no_fuse = getenv("ASPEN_B200_NO_FUSE");
     if (e->precision == 0 && !(no_fuse && atoi(no_fuse) != 0)) {
         for (unsigned i = 1; i < nasm->num_ldata; i++) {
@@ -607,7 +630,7 @@ static int build_device_nasm(Engine *e, nasm_t *nasm) {
                 if (j != i && (nasm->ldata[j].parent_ldata_idx_arr[PARENT_0] == hi || nasm->ldata[j].parent_ldata_idx_arr[PARENT_1] == hi)) only_reader = false;
             L.res_elide = (!keep_hidden_states() && only_reader && hi != nasm->num_ldata - 1) ? 1u : 0u;
             fused_other[hi] = lo;
-            written_by_parents[i] = 1;
+            written_by[i] = hi;
         }
     }
     if (to_device(&dn->layers, layers) != 0) return -1;
@@ -617,70 +640,75 @@ static int build_device_nasm(Engine *e, nasm_t *nasm) {
         if (!maps.empty()) CUDA_TRY(cudaMemcpy(dn->wmaps, maps.data(), maps.size() * sizeof(CUtensorMap), cudaMemcpyHostToDevice));
     }
 
-    // Tiles, children (CSR).  A tile's count to reach is the length of its parent list plus
-    // the true-dependency supplement; the edges walked at completion are the host child lists (as the
-    // reference walks child_ninst_arr, src/dse.c:372-375) plus the supplement.  For a generated graph the
-    // two agree; a file whose lists disagree yields a tile that never becomes ready, which the
-    // scheduler reports as a stall.
-    const unsigned n = nasm->num_ninst;
+    // Tiles, children (CSR).
+    const unsigned n = nasm->num_ninst, n_input = nasm->ldata[0].num_ninst;
     std::vector<TileDev> tiles(n);
     std::vector<unsigned> need(n);
     std::vector<std::vector<unsigned>> kids(n);
-    const unsigned n_input = nasm->ldata[0].num_ninst;
+    bool fused = false;
+    for (unsigned i = 0; i < nasm->num_ldata; i++) fused = fused || written_by[i] != (unsigned)-1;
     for (unsigned t = 0; t < n; t++) {
         const ninst_t &ni = nasm->ninst[t];
         TileDev &T = tiles[t];
         T.layer = (unsigned)(ni.ldata - nasm->ldata.data());
         T.pos_h = ni.out_mat_pos[OUT_H]; T.pos_w = ni.out_mat_pos[OUT_W];
         T.tile_h = ni.tile_dims[OUT_H]; T.tile_w = ni.tile_dims[OUT_W];
-        need[t] = (unsigned)(ni.parent_ninst_idx.size() + ni.extra_parent_idx.size());
-        if (fused_other[T.layer] != (unsigned)-1) {
-            // the fused residual reads the other parent over this tile's own region: tiles of that layer's grid
-            // (rows fastest) that overlap it become parents too
-            const nasm_ldata_t &Q = nasm->ldata[fused_other[T.layer]];
-            const unsigned qh = Q.ninst_tile_dims[OUT_H], qw = Q.ninst_tile_dims[OUT_W];
-            const unsigned per_col = (Q.out_mat_dims[OUT_H] + qh - 1) / qh;
-            for (unsigned cw = T.pos_w / qw; cw <= (T.pos_w + T.tile_w - 1) / qw; cw++)
-                for (unsigned ch = T.pos_h / qh; ch <= (T.pos_h + T.tile_h - 1) / qh; ch++) {
-                    const unsigned par = Q.ninst_start + cw * per_col + ch;
-                    if (par >= Q.ninst_start + Q.num_ninst || par >= t) { ASPEN_ERR("fused residual: tile %u has no valid producer tile\n", t); return -1; }
-                    kids[par].push_back(t);
-                    need[t]++;
-                }
-        }
         for (unsigned par : ni.parent_ninst_idx)
             if (par >= n || par >= t) { ASPEN_ERR("tile %u lists parent %u that does not precede it\n", t, par); return -1; }
-        for (unsigned par : ni.extra_parent_idx) {
+        for (unsigned par : ni.extra_parent_idx)
             if (par >= n || par >= t) { ASPEN_ERR("tile %u lists parent %u that does not precede it\n", t, par); return -1; }
-            kids[par].push_back(t);
-        }
-        for (unsigned child : ni.child_ninst_idx) {
+        for (unsigned child : ni.child_ninst_idx)
             if (child >= n || child <= t) { ASPEN_ERR("tile %u lists child %u that does not follow it\n", t, child); return -1; }
-            kids[t].push_back(child);
-        }
-        if (t >= n_input && need[t] == 0) { ASPEN_ERR("tile %u of layer %u has no parents and can never run\n", t, T.layer); return -1; }
     }
-    // Tiles whose values their parents write (fused residual layers) are taken out of the device graph: each of their
-    // parent edges is replaced by edges to their children.
     unsigned n_bypassed = 0;
-    {
+    if (!fused) {
+        // A tile's count to reach is the length of its parent list plus the true-dependency supplement; the edges walked
+        // at completion are the host child lists (as the reference walks child_ninst_arr, src/dse.c:372-375) plus the
+        // supplement.  For a generated graph the two agree; a file whose lists disagree yields a tile that
+        // never becomes ready, which the scheduler reports as a stall.
+        for (unsigned t = 0; t < n; t++) {
+            const ninst_t &ni = nasm->ninst[t];
+            need[t] = (unsigned)(ni.parent_ninst_idx.size() + ni.extra_parent_idx.size());
+            kids[t].insert(kids[t].end(), ni.child_ninst_idx.begin(), ni.child_ninst_idx.end());
+            for (unsigned par : ni.extra_parent_idx) kids[par].push_back(t);
+        }
+    } else {
+        // Fused residual layers: their tiles leave the graph (the producer's tiles write their values), so whoever reads them
+        // waits for the producer's tiles instead; the producer's tiles also wait for the other operand over their own region.
         std::vector<std::vector<unsigned>> pars(n);
-        for (unsigned p = 0; p < n; p++)
-            for (unsigned c : kids[p]) pars[c].push_back(p);
-        for (unsigned t = n_input; t < n; t++) {
-            if (!written_by_parents[tiles[t].layer]) continue;
-            for (unsigned c : kids[t]) {                       // one edge t -> c becomes the edges p -> c
-                need[c] += (unsigned)pars[t].size() - 1u;
-                auto it = std::find(pars[c].begin(), pars[c].end(), t);
-                if (it != pars[c].end()) pars[c].erase(it);
-                for (unsigned p : pars[t]) { kids[p].push_back(c); pars[c].push_back(p); }
+        for (unsigned t = 0; t < n; t++) {
+            const ninst_t &ni = nasm->ninst[t];
+            const TileDev &T = tiles[t];
+            std::vector<unsigned> &list = pars[t];
+            const unsigned producer = written_by[T.layer];
+            auto reads = [&](unsigned par) {
+                if (producer != (unsigned)-1 && tiles[par].layer != producer) return;     // the producer waits for the rest
+                if (written_by[tiles[par].layer] != (unsigned)-1) list.insert(list.end(), pars[par].begin(), pars[par].end());
+                else list.push_back(par);
+            };
+            for (unsigned par : ni.parent_ninst_idx) reads(par);
+            for (unsigned par : ni.extra_parent_idx) reads(par);
+            if (fused_other[T.layer] != (unsigned)-1) {
+                // tiles of that layer's grid (rows fastest) that overlap this tile's region
+                const nasm_ldata_t &Q = nasm->ldata[fused_other[T.layer]];
+                const unsigned qh = Q.ninst_tile_dims[OUT_H], qw = Q.ninst_tile_dims[OUT_W];
+                const unsigned per_col = (Q.out_mat_dims[OUT_H] + qh - 1) / qh;
+                for (unsigned cw = T.pos_w / qw; cw <= (T.pos_w + T.tile_w - 1) / qw; cw++)
+                    for (unsigned ch = T.pos_h / qh; ch <= (T.pos_h + T.tile_h - 1) / qh; ch++) {
+                        const unsigned par = Q.ninst_start + cw * per_col + ch;
+                        if (par >= Q.ninst_start + Q.num_ninst || par >= t) { ASPEN_ERR("fused residual: tile %u has no valid producer tile\n", t); return -1; }
+                        reads(par);
+                    }
             }
-            for (unsigned p : pars[t]) kids[p].erase(std::remove(kids[p].begin(), kids[p].end(), t), kids[p].end());
-            kids[t].clear();
-            pars[t].clear();
-            n_bypassed++;
+            std::sort(list.begin(), list.end());
+            list.erase(std::unique(list.begin(), list.end()), list.end());
+            if (producer != (unsigned)-1) { n_bypassed++; continue; }
+            need[t] = (unsigned)list.size();
+            for (unsigned par : list) kids[par].push_back(t);
         }
     }
+    for (unsigned t = n_input; t < n; t++)
+        if (need[t] == 0 && written_by[tiles[t].layer] == (unsigned)-1) { ASPEN_ERR("tile %u of layer %u has no parents and can never run\n", t, tiles[t].layer); return -1; }
     std::vector<unsigned> children;   // pairs: (child tile, its layer << 16 | count it waits for)
     for (unsigned t = 0; t < n; t++) {
         tiles[t].child_off = (unsigned)(children.size() / 2);
@@ -919,7 +947,7 @@ static int attach(Engine *e, nasm_t *nasm, const void *input_host, const int *id
         if (e->service) { if (engine_wait_nasm(nasm) != 0) return -1; }
         else if (svc_serves(e, nasm) && svc_join(e, false) != 0) return -1;
     }
-    const nasm_ldata_t &l0 = nasm->ldata[0];
+    const nasm_ldata_t &l0 = device_view(nasm)->ldata[0];
     const size_t n = (size_t)l0.out_mat_dims[OUT_H] * l0.out_mat_dims[OUT_W];
     float *dst = dn->in_stage ? dn->in_stage : (float *)((char *)dn->arena + dn->ldata_off[0]);
     if (ids_host) {
@@ -979,7 +1007,7 @@ long engine_read_ldata(nasm_t *nasm, unsigned int idx, float *out) {
     if (!dn) return -1;
     Engine *e = dn->e;
     if (cudaSetDevice(e->device) != cudaSuccess) return -1;
-    const nasm_ldata_t &ld = nasm->ldata[idx];
+    const nasm_ldata_t &ld = device_view(nasm)->ldata[idx];
     const size_t n = (size_t)ld.out_mat_dims[OUT_H] * ld.out_mat_dims[OUT_W];
     const float *src = (const float *)((char *)dn->arena + dn->ldata_off[idx]);
     if (!e->service && !svc_done(dn) && svc_serves(e, nasm)) svc_join(e, false);      // the graph is being computed

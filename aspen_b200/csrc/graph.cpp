@@ -285,6 +285,7 @@ static nasm_t *create_full(aspen_dnn_t *dnn, unsigned int min_ninst, unsigned in
     if (!nasm) return nullptr;
     graph_find_parents(nasm);
     graph_set_children(nasm);
+    nasm->own_lists = true;
     return nasm;
 }
 
@@ -418,11 +419,20 @@ done:
         if (nasm) apu_destroy_nasm(nasm);
         return nullptr;
     }
-    // A file only carries the reference's lists; recompute the true-dependency supplement.
+    // A file only carries the reference's lists; recompute the true-dependency supplement, and see whether the file's lists are
+    // the ones the tiler gives.
     {
-        ParentFinder pf(nasm);
-        std::vector<unsigned int> scratch;
-        for (auto &ni : nasm->ninst) { scratch.clear(); ni.extra_parent_idx.clear(); pf.run(ni, scratch, ni.extra_parent_idx); }
+        std::vector<std::vector<unsigned int>> parents(nasm->num_ninst), children(nasm->num_ninst);
+        for (auto &ni : nasm->ninst) parents[ni.ninst_idx] = ni.parent_ninst_idx;
+        for (auto &ni : nasm->ninst) children[ni.ninst_idx].swap(ni.child_ninst_idx);
+        graph_find_parents(nasm);
+        graph_set_children(nasm);
+        nasm->own_lists = true;
+        for (auto &ni : nasm->ninst) {
+            nasm->own_lists = nasm->own_lists && ni.parent_ninst_idx == parents[ni.ninst_idx] && ni.child_ninst_idx == children[ni.ninst_idx];
+            ni.parent_ninst_idx.swap(parents[ni.ninst_idx]);
+            ni.child_ninst_idx.swap(children[ni.ninst_idx]);
+        }
     }
     nasm->has_graph = true;
     return nasm;

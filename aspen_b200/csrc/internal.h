@@ -99,6 +99,7 @@ struct nasm_t {
     uint64_t true_flops = 0;
     TileQuanta quanta;
     bool has_graph = false;
+    bool own_lists = false;        // parent / child lists are what the tiler gives (not changed by a file)
     // runtime side
     std::atomic<unsigned int> completed{0};
     DeviceNasm *dev = nullptr;     // device image (arena, descriptors, counters)
@@ -169,6 +170,7 @@ nasm_t *nasm_create_tiles(aspen_dnn_t *dnn, unsigned int flop_per_ninst, unsigne
 void graph_find_parents(nasm_t *nasm);
 void graph_set_children(nasm_t *nasm);
 // engine.cu (the only translation unit that touches CUDA)
+nasm_t *plan_device_tiles(const nasm_t *nasm, int precision, unsigned int sms, bool served);   // plan.cpp; nullptr: keep the nasm's tiles
 int engine_current_device();
 Engine *engine_create(int device, int precision, unsigned int num_dse_hint);
 void engine_destroy(Engine *e);

@@ -1,0 +1,181 @@
+// Device tile plan: the grid of tiles the GPU executes a graph with.
+//
+// A nasm's own tiles (tiler.cpp) follow the reference: their shapes are chosen for its CPU micro-kernels, they are graph node
+// ids, and .nasm files name them.  Tile VALUES do not depend on the shapes, so the device image of a graph is free to use its
+// own: with the reference's 64-row / 12-column quanta a 128-lane MMA would be mostly padding, and one quantum for a
+// whole network leaves SMs idle in the late layers or makes the early ones pay per tile.  Here every layer gets the
+// shape with the lowest estimated time on the SMs at hand.  The plan is a nasm of the same layers with that grid and
+// with the parents each tile reads (by region, so a graph of ten thousand tiles takes milliseconds).
+// Graphs whose lists a file has changed keep their own tiles and lists.
+#include "internal.h"
+
+#include <algorithm>
+#include <memory>
+
+namespace {
+
+struct Grid {
+    unsigned th = 1, tw = 1;       // tile rows, columns
+    unsigned seg = 1;              // tiles do not cross multiples of this many columns (a head's or sample's queries)
+    unsigned nh = 1, per_seg = 1;  // row tiles; column tiles of a segment
+    unsigned start = 0;
+};
+
+bool contraction(LAYER_TYPE t) { return t == CONV_LAYER || t == FC_LAYER || t == MATMUL_LAYER || t == K_ATTENTION_LAYER || t == V_ATTENTION_LAYER; }
+unsigned ceil_div(unsigned a, unsigned b) { return (a + b - 1) / b; }
+
+// Estimated microseconds of one tile of th x tw outputs with a k-deep contraction, `gap` of them between two tiles of an SM.
+// Tensor cores (measured, see tiles_tc.cuh): 0.29 us per 32-deep chunk of a 128 x <= 128 block, 0.38 of a 128 x 256 one; the
+// epilogue of a block takes 0.4 us per 32 rows and runs under the next block's main loop.
+double tile_us(bool tensor, unsigned th, unsigned tw, unsigned k, double gap) {
+    if (tensor) {
+        const unsigned chunks = ceil_div(k, 32), nb = ceil_div(tw, 128) * ceil_div(th, 256), rows = std::min(th, 256u);
+        const double loop = chunks * (rows > 128 ? 0.38 : 0.29), epi = 0.6 + 0.4 * ceil_div(rows, 32);
+        return gap + loop + epi + (nb - 1) * std::max(loop, epi);
+    }
+    // fp32 blocks (gemm_ffma.cuh): 128 FMAs a clock at the shape's share of the rate
+    const unsigned bm = th > 64 && tw > 32 ? 128 : th > 32 && tw > 32 ? 64 : 32, bn = bm == 32 ? 32 : 64;
+    return gap + (double)ceil_div(th, bm) * ceil_div(tw, bn) * bm * bn * k / (128.0 * 1900.0 * (bm == 32 ? 0.65 : 0.80));
+}
+
+Grid choose(const nasm_ldata_t &ld, const nasm_t *nasm, bool tensor, unsigned sms, bool served) {
+    const aspen_layer_t *l = ld.layer;
+    const unsigned *p = l->params;
+    const unsigned H = ld.out_mat_dims[OUT_H], W = ld.out_mat_dims[OUT_W];
+    Grid g;
+    g.seg = W;
+    if (contraction(l->type)) {
+        const bool ka = l->type == K_ATTENTION_LAYER, va = l->type == V_ATTENTION_LAYER;
+        if (ka || va) g.seg = nasm->tr_seq_len;
+        unsigned hs[8], nhs = 0;
+        if (ka) hs[nhs++] = H;                                      // the softmax reduces over all keys
+        else if (va) hs[nhs++] = p[NUM_HEAD] ? p[NUM_HIDDEN] / p[NUM_HEAD] : H;
+        else for (unsigned h : {512u, 256u, 128u, 64u, 32u}) if (h < 2 * H && (h <= 256 || tensor)) hs[nhs++] = h;
+        const unsigned k = ka ? p[NUM_HIDDEN] / std::max(1u, p[NUM_HEAD]) : va ? nasm->tr_seq_len : layer_contraction_k(l);
+        const unsigned quantum = tensor ? 128 : 32;
+        double best = 0;
+        for (unsigned i = 0; i < nhs; i++)
+            for (unsigned tw = quantum; tw < g.seg + quantum && tw <= 16 * quantum; tw += quantum) {
+                const unsigned tiles = ceil_div(H, hs[i]) * (W / g.seg) * ceil_div(g.seg, tw);
+                const double us = tile_us(tensor, std::min(hs[i], H), std::min(tw, g.seg), k, served ? 2.5 : 4.0);
+                const double share = (double)tiles / sms;
+                // Passes of other graphs fill the SMs a served layer leaves idle: its work counts, and, because the graphs in
+                // rotation are few, to a lesser degree the length of its longest tile.  A layer launched alone takes as many
+                // rounds as its busiest SM; the last, partly filled one overlaps in part with the next layer.
+                const double cost = served ? us * (share + 0.2) : us * (0.4 * std::max(1.0, share) + 0.6 * ceil_div(tiles, sms));
+                if (best == 0 || cost < best * 0.999) { best = cost; g.th = hs[i]; g.tw = tw; }
+            }
+    } else if (l->type == SOFTMAX_LAYER || l->type == YOLO_LAYER || l->type == APPEND_LAYER) {
+        g.th = ld.ninst_tile_dims[OUT_H]; g.tw = ld.ninst_tile_dims[OUT_W];
+    } else {
+        // memory-bound: whole columns, one tile per SM, more (up to four) where a tile then still writes 96 KB -- a tile costs
+        // some 4 us besides its transfers; few columns with many rows (a global pool) split the rows
+        g.th = H;
+        const unsigned want = (unsigned)std::min(4.0 * sms, std::max(1.0 * sms, (double)H * W * 4.0 / 98304.0));
+        g.tw = std::max(1u, ceil_div(W, want));
+        if (g.tw > 8) g.tw = (unsigned)round_up(g.tw, 8);
+        if (l->type == AVGPOOL_LAYER || l->type == MAXPOOL_LAYER)
+            while (g.th > 64 && g.th % 8 == 0 && ceil_div(H, g.th) * W < want / 2) g.th /= 2;
+    }
+    g.nh = ceil_div(H, g.th);
+    g.per_seg = ceil_div(g.seg, g.tw);
+    return g;
+}
+
+}  // namespace
+
+nasm_t *plan_device_tiles(const nasm_t *nasm, int precision, unsigned sms, bool served) {
+    std::unique_ptr<nasm_t> plan(new nasm_t());
+    plan->dnn = nasm->dnn;
+    plan->batch_size = nasm->batch_size;
+    plan->tr_seq_len = nasm->tr_seq_len;
+    plan->num_ldata = nasm->num_ldata;
+    plan->ldata = nasm->ldata;
+    std::vector<Grid> grid(plan->num_ldata);
+    unsigned total = 0;
+    for (unsigned i = 0; i < plan->num_ldata; i++) {
+        nasm_ldata_t &ld = plan->ldata[i];
+        ld.nasm = plan.get();
+        Grid &g = grid[i] = choose(nasm->ldata[i], nasm, precision == 0, sms, served);
+        const unsigned H = ld.out_mat_dims[OUT_H], W = ld.out_mat_dims[OUT_W];
+        if (H == 0 || W == 0 || W % g.seg != 0) return nullptr;
+        g.start = total;
+        ld.ninst_tile_dims[OUT_H] = g.th;
+        ld.ninst_tile_dims[OUT_W] = g.tw;
+        ld.out_mat_stride = (unsigned)round_up(H, 4);
+        ld.out_mat_mem_size = (size_t)ld.out_mat_stride * W * sizeof(float);
+        ld.ninst_start = total;
+        ld.num_ninst = g.nh * (W / g.seg) * g.per_seg;
+        total += ld.num_ninst;
+    }
+    plan->num_ninst = total;
+    plan->ninst.resize(total);
+    for (unsigned i = 0; i < plan->num_ldata; i++) {
+        nasm_ldata_t &ld = plan->ldata[i];
+        const aspen_layer_t *l = ld.layer;
+        const unsigned *p = l->params;
+        const Grid &g = grid[i];
+        const unsigned H = ld.out_mat_dims[OUT_H], seq = plan->tr_seq_len;
+        const unsigned i0 = ld.parent_ldata_idx_arr[PARENT_0], i1 = ld.parent_ldata_idx_arr[PARENT_1];
+        for (unsigned t = 0; t < ld.num_ninst; t++) {
+            ninst_t &ni = plan->ninst[g.start + t];
+            const unsigned ch = t % g.nh, cw = t / g.nh, seg = cw / g.per_seg, in_seg = (cw % g.per_seg) * g.tw;
+            const unsigned h0 = ch * g.th, h1 = std::min(H, h0 + g.th), w0 = seg * g.seg + in_seg, w1 = seg * g.seg + std::min(g.seg, in_seg + g.tw);
+            ni.ldata = &ld;
+            ni.ninst_idx = g.start + t;
+            ni.out_mat_pos[OUT_H] = h0; ni.out_mat_pos[OUT_W] = w0;
+            ni.tile_dims[OUT_H] = h1 - h0; ni.tile_dims[OUT_W] = w1 - w0;
+            // the tiles of parent layer `par` that overlap rows [r0, r1) x columns [c0, c1)
+            auto reads = [&](unsigned par, unsigned r0, unsigned r1, unsigned c0, unsigned c1) {
+                const Grid &q = grid[par];
+                const nasm_ldata_t &pl = plan->ldata[par];
+                r1 = std::min(r1, pl.out_mat_dims[OUT_H]); c1 = std::min(c1, pl.out_mat_dims[OUT_W]);
+                for (unsigned c = c0; c < c1;) {
+                    const unsigned s = c / q.seg, k = (c % q.seg) / q.tw, col = s * q.per_seg + k;
+                    for (unsigned r = r0 / q.th; r * q.th < r1; r++) ni.parent_ninst_idx.push_back(q.start + col * q.nh + r);
+                    c = s * q.seg + std::min(q.seg, (k + 1) * q.tw);
+                }
+            };
+            const unsigned all = 0xffffffffu;
+            if (l->type == INPUT_LAYER || i0 == (unsigned)-1) continue;
+            const bool like0 = plan->ldata[i0].out_mat_dims[OUT_W] == ld.out_mat_dims[OUT_W];
+            switch (l->type) {
+                case CONV_LAYER: case MAXPOOL_LAYER: case AVGPOOL_LAYER: {
+                    const unsigned OW = p[OUT_W], hw = p[OUT_H] * OW, IW = p[IN_W], IH = p[IN_H], s = p[STRIDE] ? p[STRIDE] : 1;
+                    const unsigned r0 = l->type == CONV_LAYER ? 0 : h0, r1 = l->type == CONV_LAYER ? all : h1;
+                    if (p[WEIGHT_H] == 1 && p[WEIGHT_W] == 1 && s == 1 && p[PADDING] == 0 && like0) { reads(i0, r0, r1, w0, w1); break; }
+                    // whole input rows; a tile that spans samples reads every row in between
+                    const unsigned b0 = w0 / hw, b1 = (w1 - 1) / hw, y0 = (w0 % hw) / OW * s, y1 = ((w1 - 1) % hw) / OW * s + p[WEIGHT_H] - 1;
+                    const unsigned first = y0 > p[PADDING] ? y0 - p[PADDING] : 0, last = std::min(IH - 1, y1 > p[PADDING] ? y1 - p[PADDING] : 0);
+                    reads(i0, r0, r1, (b0 * IH + std::min(first, IH - 1)) * IW, (b1 * IH + last + 1) * IW);
+                    break;
+                }
+                case FC_LAYER: { const unsigned px = p[IN_H] * p[IN_W]; reads(i0, 0, all, w0 * px, w1 * px); break; }
+                case MATMUL_LAYER: case LAYERNORM_LAYER: reads(i0, 0, all, w0, w1); break;
+                case RESIDUAL_LAYER:
+                    reads(i0, h0, h1, w0, w1);
+                    if (i1 != (unsigned)-1) reads(i1, h0, h1, w0, w1);
+                    break;
+                case K_ATTENTION_LAYER: {
+                    const unsigned heads = p[NUM_HEAD], hd = p[NUM_HIDDEN] / heads, b = w0 / (seq * heads), head = w0 / seq % heads, q0 = w0 % seq;
+                    reads(i0, head * hd, (head + 1) * hd, b * seq + q0, b * seq + q0 + (w1 - w0));
+                    if (i1 != (unsigned)-1) reads(i1, head * hd, (head + 1) * hd, b * seq + h0, b * seq + h1);
+                    break;
+                }
+                case V_ATTENTION_LAYER: {
+                    const unsigned heads = p[NUM_HEAD], hd = p[NUM_HIDDEN] / heads, b = w0 / seq, head = h0 / hd, c = (b * heads + head) * seq + w0 % seq;
+                    reads(i0, 0, all, c, c + (w1 - w0));
+                    if (i1 != (unsigned)-1) reads(i1, h0, h1, b * seq, (b + 1) * seq);
+                    break;
+                }
+                default:
+                    reads(i0, 0, all, 0, all);
+                    if (i1 != (unsigned)-1) reads(i1, 0, all, 0, all);
+                    break;
+            }
+            if (ni.parent_ninst_idx.empty()) return nullptr;
+        }
+    }
+    graph_set_children(plan.get());
+    return plan.release();
+}
