@@ -25,7 +25,11 @@ struct LayerDev {
     int wmap;                 // tensor map of the W-side operand (weights, PARENT_1 for attention keys, transposed values)
     int amap;                 // tensor map of the X-side operand (PARENT_0 activations)
     unsigned a_kind;          // X operand staging, see tiles_tc.cuh
-    unsigned b_box;           // rows of one box of the W-side map
+    unsigned a_multi;         // one X box covers all chunks of a stage (the map has a third dimension: the chunk)
+    unsigned b_rows;          // rows of the W-side box (one per stage): the tile's rows, at most 256
+    unsigned chunks;          // 32-deep chunks of the contraction
+    unsigned per_stage;       // chunks of one stage of the operand ring
+    unsigned stage_bytes, stages;
     unsigned a_vec4;          // fp32 tiles: operand rows can be fetched in 16-byte pieces (IC % 4 == 0 ...)
     unsigned round_out;       // store outputs rounded to TF32 (nearest): a tensor-core layer reads them
     unsigned PH;              // A_ROWS: rows per sample of the zero-padded copy of the input image
@@ -38,7 +42,7 @@ struct LayerDev {
     unsigned res_round;
     unsigned res_elide;       // the layer's own (pre-add) output has no other reader and is not written
     // A layer whose output is the value operand of an attention_v layer also writes it transposed: row = feature, column
-    // b * vt_seq + s (vt_seq = seq rounded up to 4: TMA coordinates are multiples of 16 bytes).  That copy is what the
+    // b * vt_seq + s (vt_seq = seq rounded up to 32, the columns in between are zero).  That copy is what the
     // attention tile's TMA reads as a K-major operand.  nullptr: no copy.  (attention_v itself: vt_seq of that copy.)
     float *vt_out;
     unsigned vt_ld, vt_seq;

@@ -374,7 +374,6 @@ static void fill_layer(const nasm_t *nasm, const DeviceNasm *dn, unsigned i, int
     L.p_out_c = p[OUT_C]; L.p_in_c = p[IN_C]; L.p_stride = p[STRIDE];
     L.wmap = -1;
     L.amap = -1;
-    L.b_box = 64;
     switch (l.type) {
         case CONV_LAYER: case FC_LAYER: L.a_vec4 = (L.IC % 4 == 0) && (L.ld0 % 4 == 0); break;
         case MATMUL_LAYER: L.a_vec4 = (L.K % 4 == 0) && (L.ld0 % 4 == 0); break;
@@ -430,17 +429,25 @@ static int build_device_nasm(Engine *e, nasm_t *host_nasm) {
     // layers + tensor maps (weights and, where the access pattern allows it, the parents' activations)
     std::vector<LayerDev> layers(nasm->num_ldata);
     std::vector<CUtensorMap> maps;
-    auto add_map = [&](const void *base, cuuint64_t inner, cuuint64_t outer, cuuint64_t stride_bytes, cuuint32_t box_rows) -> int {
+    // rows of `stride_bytes` with `inner` floats; boxes of 32 floats x box_rows (per = 0), or of `per` consecutive 32-float chunks
+    // x box_rows, the chunk being the third dimension (inner % 32 == 0)
+    auto add_map = [&](const void *base, cuuint64_t inner, cuuint64_t outer, cuuint64_t stride_bytes, cuuint32_t box_rows, cuuint32_t per) -> int {
         CUtensorMap m;
-        cuuint64_t dims[2] = {inner, outer};
-        cuuint64_t strides[1] = {stride_bytes};
-        cuuint32_t box[2] = {32, box_rows}, estr[2] = {1, 1};
-        CUresult r = get_encode_fn()(&m, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, const_cast<void *>(base), dims, strides, box, estr,
+        cuuint64_t dims[3] = {per ? 32 : inner, outer, inner / 32};
+        cuuint64_t strides[2] = {stride_bytes, 128};
+        cuuint32_t box[3] = {32, box_rows, per}, estr[3] = {1, 1, 1};
+        CUresult r = get_encode_fn()(&m, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, per ? 3 : 2, const_cast<void *>(base), dims, strides, box, estr,
                                      CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                                      CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
         if (r != CUDA_SUCCESS) { ASPEN_ERR("cuTensorMapEncodeTiled failed (%d)\n", (int)r); return -2; }
         maps.push_back(m);
         return (int)maps.size() - 1;
+    };
+    // The X operand by plain boxes: the chunks of a stage in one where the matrix allows it.
+    auto add_x_map = [&](LayerDev &L, const void *base, cuuint64_t inner, cuuint64_t outer, cuuint64_t stride_bytes) {
+        L.a_kind = tc::A_TMA;
+        L.a_multi = inner % 32 == 0;
+        L.amap = add_map(base, inner, outer, stride_bytes, 128, L.a_multi ? L.per_stage : 0);
     };
     // 3-D map of the padded input copy: (32 floats of a row, output pixel = `stride` input pixels apart, row)
     // Eight consecutive maps, the j-th with a box of 16 j pixels.  Returns the index of the first, or -2 when the driver
@@ -491,9 +498,18 @@ static int build_device_nasm(Engine *e, nasm_t *host_nasm) {
         const bool gemm_w = l.type == CONV_LAYER || l.type == FC_LAYER || l.type == MATMUL_LAYER;
         const unsigned p0 = nasm->ldata[i].parent_ldata_idx_arr[PARENT_0], p1 = nasm->ldata[i].parent_ldata_idx_arr[PARENT_1];
         const cuuint64_t W0 = p0 != (unsigned)-1 ? nasm->ldata[p0].out_mat_dims[OUT_W] : 0;
-        // rows of a W-side box: no larger than the tile's, so a tile loads nothing but its own rows (and the last box's padding)
+        // Operand ring: a W box holds the tile's rows; a stage holds as many chunks as keep the one-thread roles ahead of the MMAs
+        // (0.25 us of instructions per stage against 0.05 us of MMA per chunk of 32 rows, 0.1 of 64, 0.2 of 128, 0.4 of 256) while
+        // two or more stages fit.
         const unsigned th = nasm->ldata[i].ninst_tile_dims[OUT_H];
-        L.b_box = th >= 256 ? 256 : th >= 128 ? 128 : th >= 64 ? 64 : 32;
+        auto cut_ring = [&](unsigned k) {
+            L.b_rows = (unsigned)round_up(std::min(th, tc::BLOCK_ROWS), 16);
+            L.chunks = std::max(1u, (k + 31) / 32);
+            L.per_stage = std::min(L.chunks, L.b_rows <= 64 ? 4u : L.b_rows <= 128 ? 2u : 1u);
+            L.stage_bytes = L.per_stage * (tc::A_CHUNK_BYTES + L.b_rows * 128);
+            L.stages = std::min(tc::MAX_STAGES, tc::RING_BYTES / L.stage_bytes);
+        };
+        if (gemm_w || l.type == K_ATTENTION_LAYER || l.type == V_ATTENTION_LAYER) cut_ring(l.type == K_ATTENTION_LAYER ? L.hd : l.type == V_ATTENTION_LAYER ? L.seq : L.Kpad);
         // Row-box staging of an input convolution (see tiles_tc.cuh, A_ROWS): decided first, it changes the
         // weight layout the weight map is made from.
         bool rows_kind = false;
@@ -514,6 +530,7 @@ static int build_device_nasm(Engine *e, nasm_t *host_nasm) {
                 L.weight = dn->dd->weight_rows[i];
                 L.Kpad = L.KH * 32;
                 L.K = L.Kpad;
+                cut_ring(L.Kpad);
             } else {
                 cudaFree(dn->padded_in);
                 dn->padded_in = nullptr;
@@ -523,45 +540,41 @@ static int build_device_nasm(Engine *e, nasm_t *host_nasm) {
         if (rows_kind) {
             // X operand set above
         } else if (l.type == MATMUL_LAYER && aligned0) {
-            L.a_kind = tc::A_TMA;
-            L.amap = add_map(L.in0, L.H0, W0, (cuuint64_t)L.ld0 * sizeof(float), 128);
+            add_x_map(L, L.in0, L.H0, W0, (cuuint64_t)L.ld0 * sizeof(float));
         } else if (l.type == CONV_LAYER && aligned0 && L.KH == 1 && L.KW == 1 && L.stride == 1 && L.pad == 0) {
-            L.a_kind = tc::A_TMA;
-            L.amap = add_map(L.in0, L.H0, W0, (cuuint64_t)L.ld0 * sizeof(float), 128);
+            add_x_map(L, L.in0, L.H0, W0, (cuuint64_t)L.ld0 * sizeof(float));
         } else if (l.type == CONV_LAYER && aligned0 && L.IC % 32 == 0 && L.IC == L.H0 && L.KH * L.KW * L.IC == L.K && L.stride <= 8 && L.KH <= 64 && L.KW <= 64 &&
                    L.pad < L.KH && L.pad < L.KW) {
             L.amap = add_im2col_map(L);
             if (L.amap >= 0) L.a_kind = tc::A_IM2COL;
         } else if (l.type == FC_LAYER && L.ld0 == L.IC && L.K % 4 == 0) {
-            L.a_kind = tc::A_TMA;   // a sample's NHWC activations are one contiguous row of K values
-            L.amap = add_map(L.in0, L.K, nasm->batch_size, (cuuint64_t)L.IH * L.IW * L.ld0 * sizeof(float), 128);
+            // a sample's NHWC activations are one contiguous row of K values
+            add_x_map(L, L.in0, L.K, nasm->batch_size, (cuuint64_t)L.IH * L.IW * L.ld0 * sizeof(float));
         } else if (l.type == K_ATTENTION_LAYER) {
             // all keys of a query must fit the accumulators (512 columns); larger sequences run as fp32 tiles
-            if (L.hd % 32 == 0 && aligned0 && L.ld1 % 4 == 0 && L.seq <= tc::TMEM_COLS && th >= L.seq) {
-                L.a_kind = tc::A_TMA;
-                L.amap = add_map(L.in0, L.H0, W0, (cuuint64_t)L.ld0 * sizeof(float), 128);
-                L.wmap = add_map(L.in1, L.H1, nasm->ldata[p1].out_mat_dims[OUT_W], (cuuint64_t)L.ld1 * sizeof(float), L.b_box);
+            if (L.hd % 32 == 0 && L.H0 % 32 == 0 && L.H1 % 32 == 0 && aligned0 && L.ld1 % 4 == 0 && L.seq <= tc::TMEM_COLS && th >= L.seq) {
+                add_x_map(L, L.in0, L.H0, W0, (cuuint64_t)L.ld0 * sizeof(float));
+                L.wmap = add_map(L.in1, L.H1, nasm->ldata[p1].out_mat_dims[OUT_W], (cuuint64_t)L.ld1 * sizeof(float), L.b_rows, L.per_stage);
             }
         } else if (l.type == V_ATTENTION_LAYER && aligned0 && p1 != (unsigned)-1 && p1 < i && p1 != 0 && layers[p1].tc && !layers[p1].vt_out) {
             // The value operand W(m, k) = V[token k][feature m] is the transpose of how the value projection stores its
             // output; that projection, a tensor-core layer of this graph, writes a second, transposed copy into scratch memory.
-            const size_t seqp = round_up(L.seq, 4), ldt = round_up(seqp * nasm->batch_size, 32);
+            const size_t seqp = round_up(L.seq, 32), ldt = seqp * nasm->batch_size;
             float *vt = nullptr;
             CUDA_TRY(cudaMalloc(&vt, (size_t)L.H1 * ldt * sizeof(float) + 256));
             dn->scratch.push_back(vt);
             CUDA_TRY(cudaMemsetAsync(vt, 0, (size_t)L.H1 * ldt * sizeof(float) + 256, e->stream));
-            const int m = add_map(vt, ldt, L.H1, (cuuint64_t)ldt * sizeof(float), L.b_box);
+            const int m = add_map(vt, ldt, L.H1, (cuuint64_t)ldt * sizeof(float), L.b_rows, L.per_stage);
             if (m >= 0) {
                 layers[p1].vt_out = vt;
                 layers[p1].vt_ld = (unsigned)ldt;
                 layers[p1].vt_seq = L.vt_seq = (unsigned)seqp;
                 L.wmap = m;
-                L.a_kind = tc::A_TMA;
-                L.amap = add_map(L.in0, L.H0, W0, (cuuint64_t)L.ld0 * sizeof(float), 128);
+                add_x_map(L, L.in0, L.H0, W0, (cuuint64_t)L.ld0 * sizeof(float));
             }
         }
         if (gemm_w && L.a_kind != tc::A_NONE && L.amap >= 0)
-            L.wmap = add_map(L.weight, L.Kpad, layer_weight_rows(&l), (cuuint64_t)L.Kpad * sizeof(float), L.b_box);
+            L.wmap = add_map(L.weight, L.Kpad, layer_weight_rows(&l), (cuuint64_t)L.Kpad * sizeof(float), L.b_rows, L.per_stage);
         L.tc = L.a_kind != tc::A_NONE && L.amap >= 0 && L.wmap >= 0;
         // ASPEN_B200_ATTN_FUSE=1 with hidden states given up: attention probabilities that only the attention_v layer reads do not
         // stay; every such layer writes the same scratch matrix, which then lives in L2.  The layer's keys have to follow from

@@ -34,7 +34,7 @@ namespace tc {
 
 constexpr unsigned MAX_STAGES = 8;
 constexpr unsigned RING_BYTES = 192u * 1024u;
-constexpr unsigned A_STAGE_BYTES = 128 * 128;
+constexpr unsigned A_CHUNK_BYTES = 128 * 128;
 constexpr unsigned NW = 256;                       // worker threads
 constexpr unsigned WARP_A = 0, WARP_MMA = 1, WARP_SCHED = 2, WARP_B = 3, WARP_WORK = 4;   // workers: warps 4 .. 11 (warp % 4 = TMEM lane quarter)
 constexpr unsigned THREADS = 128 + NW;
@@ -213,33 +213,25 @@ __device__ __forceinline__ unsigned umma_idesc(unsigned n) {
 //   A_ROWS     convolution on the network input with <= 4 channels (the 7x7 stem): the input is kept as a zero-padded
 //              [sample][row][pixel][4] copy, the k axis is (kh, [kw][4] padded to 32), so one k-chunk of an output pixel
 //              is ONE contiguous 128-byte run of an input row, and 16 j consecutive output pixels of a row are a 3-D box
-// The W operand arrives in boxes of LayerDev::b_box rows: weights, attention keys (PARENT_1's matrix) or the transposed copy
-// of the attention values.  Layers that fit none of these run as fp32 FMA tiles (tile_gemm_ffma).
+// The W operand -- weights, attention keys (PARENT_1's matrix) or the transposed copy of the attention values -- arrives in one
+// box per stage; so does X where its map has the chunk as a third dimension (A_TMA over a multiple of 32).  Layers that
+// fit none of these run as fp32 FMA tiles (tile_gemm_ffma).
 enum { A_NONE = 0, A_TMA = 1, A_ROWS = 2, A_IM2COL = 3 };
 
-struct Geometry {             // of a posted contraction tile, the same in every role
-    unsigned k;               // contraction length, a multiple of 32
-    unsigned stage_bytes, stages;
-    int ax, ay, bx, by;       // box coordinates of (column 0 / row 0 of the tile, k = 0)
-};
+struct Origin { int ax, ay, bx, by; };      // box coordinates of column 0 / row 0 of a tile; x in chunks of 32
 
-__device__ __forceinline__ Geometry geometry(const LayerDev &L, const TileDev &T) {
-    Geometry g;
-    g.ax = 0; g.ay = (int)T.pos_w; g.bx = 0; g.by = (int)T.pos_h; g.k = L.Kpad;
+__device__ __forceinline__ Origin origin(const LayerDev &L, const TileDev &T) {
+    Origin g;
+    g.ax = 0; g.ay = (int)T.pos_w; g.bx = 0; g.by = (int)T.pos_h;
     if (L.type == K_ATTENTION_LAYER) {
         const unsigned per = L.seq * L.heads, b = T.pos_w / per, r = T.pos_w - b * per, head = r / L.seq, q0 = r - head * L.seq;
-        g.ax = g.bx = (int)(head * L.hd);
+        g.ax = g.bx = (int)(head * (L.hd >> 5));
         g.ay = (int)(b * L.seq + q0); g.by = (int)(b * L.seq + T.pos_h);
-        g.k = L.hd;
     } else if (L.type == V_ATTENTION_LAYER) {
         const unsigned b = T.pos_w / L.seq, head = T.pos_h / L.hd, q0 = T.pos_w - b * L.seq;
         g.ay = (int)((b * L.heads + head) * L.seq + q0);
-        g.bx = (int)(b * L.vt_seq);
-        g.k = (L.seq + 31u) & ~31u;
+        g.bx = (int)(b * (L.vt_seq >> 5));
     }
-    const unsigned rows = min(BLOCK_ROWS, T.tile_h), boxed = (rows + L.b_box - 1u) / L.b_box * L.b_box;
-    g.stage_bytes = A_STAGE_BYTES + ((boxed * 128u + 1023u) & ~1023u);
-    g.stages = min(MAX_STAGES, RING_BYTES / g.stage_bytes);
     return g;
 }
 
@@ -251,25 +243,25 @@ struct Ring {
 };
 
 // Producer side of a change of the ring's cut: every stage must have been read.
-__device__ __forceinline__ bool recut(Ring &r, const Geometry &g, Shared *sh, CtrlDev *ctrl, StatusHost *status) {
-    if (g.stage_bytes == r.stage_bytes) return true;
+__device__ __forceinline__ bool recut(Ring &r, const LayerDev &L, Shared *sh, CtrlDev *ctrl, StatusHost *status) {
+    if (L.stage_bytes == r.stage_bytes) return true;
     if (r.stage_bytes)
         for (unsigned i = 0; i < r.stages; i++)
             if (!mbar_wait(&sh->empty[i], ((r.uses >> i) & 1u) ^ 1u, ctrl, status, 8)) return false;
-    r.s = 0; r.stage_bytes = g.stage_bytes; r.stages = g.stages;
+    r.s = 0; r.stage_bytes = L.stage_bytes; r.stages = L.stages;
     return true;
 }
 
 // ---- X operand producer: one thread ----------------------------------------------------------------------------------
 __device__ __forceinline__ bool produce_a(const Slot &sl, unsigned ring, Ring &r, Shared *sh, CtrlDev *ctrl, StatusHost *status) {
     const LayerDev &L = sl.layer;
-    const Geometry g = geometry(L, sl.tile);
+    const Origin g = origin(L, sl.tile);
     const unsigned char *map = sl.maps + (size_t)L.amap * 128;
     // activations were written with ordinary (generic proxy) stores; TMA reads them through the async proxy
     asm volatile("fence.proxy.async.global;" ::: "memory");
-    if (!recut(r, g, sh, ctrl, status)) return false;
-    const unsigned kind = L.a_kind, tile_w = sl.tile.tile_w, tile_h = sl.tile.tile_h, pos_w = sl.tile.pos_w;
-    const unsigned OW = L.OW, OH = L.OH, KH = L.KH, KW = L.KW, IC = L.IC, PH = L.PH, stride = L.stride;
+    if (!recut(r, L, sh, ctrl, status)) return false;
+    const unsigned kind = L.a_kind, multi = L.a_multi, tile_w = sl.tile.tile_w, tile_h = sl.tile.tile_h, pos_w = sl.tile.pos_w;
+    const unsigned OW = L.OW, OH = L.OH, KW = L.KW, IC = L.IC, PH = L.PH, stride = L.stride, chunks = L.chunks, per = L.per_stage;
     const int pad = (int)L.pad;
     for (unsigned n0 = 0; n0 < tile_w; n0 += 128u) {
         unsigned px = 0, py = 0, pn = 0;             // first output pixel of the block
@@ -280,40 +272,43 @@ __device__ __forceinline__ bool produce_a(const Slot &sl, unsigned ring, Ring &r
             py = q / OW; px = q - py * OW;
         }
         for (unsigned mp = 0; mp < tile_h; mp += BLOCK_ROWS) {
-            if (kind == A_TMA) {
-                const int y = g.ay + (int)n0, x1 = g.ax + (int)g.k;
-                for (int x = g.ax; x < x1; x += 32) {
+            if (multi) {
+                const int y = g.ay + (int)n0;
+                for (unsigned ch = 0; ch < chunks; ch += per) {
                     if (!mbar_wait(&sh->empty[r.s], r.parity() ^ 1u, ctrl, status, 2)) return false;
-                    mbar_arrive_expect_tx(&sh->full[r.s], A_STAGE_BYTES);
-                    tma_load_2d(ring + r.s * r.stage_bytes, map, x, y, &sh->full[r.s]);
+                    mbar_arrive_expect_tx(&sh->full[r.s], per * A_CHUNK_BYTES);
+                    tma_load_3d(ring + r.s * r.stage_bytes, map, 0, y, g.ax + (int)ch, &sh->full[r.s]);
                     r.step();
                 }
-            } else if (kind == A_IM2COL) {
-                const int x0 = (int)(px * stride) - pad, y0 = (int)(py * stride) - pad;
-                for (unsigned kh = 0; kh < KH; kh++)
-                    for (unsigned kw = 0; kw < KW; kw++)
-                        for (unsigned c = 0; c < IC; c += 32u) {
-                            if (!mbar_wait(&sh->empty[r.s], r.parity() ^ 1u, ctrl, status, 2)) return false;
-                            mbar_arrive_expect_tx(&sh->full[r.s], A_STAGE_BYTES);
-                            tma_load_im2col(ring + r.s * r.stage_bytes, map, (int)c, x0, y0, (int)pn, kw, kh, &sh->full[r.s]);
-                            r.step();
+                continue;
+            }
+            unsigned kh = 0, kw = 0, c = 0;          // tap and first channel of the next chunk; c runs fastest
+            const int x0 = (int)(px * stride) - pad, y0 = (int)(py * stride) - pad;
+            for (unsigned ch = 0; ch < chunks; ch += per) {
+                const unsigned n = min(per, chunks - ch);
+                unsigned dst = ring + r.s * r.stage_bytes;
+                if (!mbar_wait(&sh->empty[r.s], r.parity() ^ 1u, ctrl, status, 2)) return false;
+                mbar_arrive_expect_tx(&sh->full[r.s], n * A_CHUNK_BYTES);
+                for (unsigned j = 0; j < n; j++, dst += A_CHUNK_BYTES) {
+                    if (kind == A_IM2COL) {
+                        tma_load_im2col(dst, map, (int)c, x0, y0, (int)pn, kw, kh, &sh->full[r.s]);
+                        c += 32u;
+                        if (c == IC) { c = 0; if (++kw == KW) { kw = 0; kh++; } }
+                    } else if (kind == A_TMA) {
+                        tma_load_2d(dst, map, (g.ax + (int)(ch + j)) * 32, g.ay + (int)n0, &sh->full[r.s]);
+                    } else {
+                        // the 128 pixels are cut where an output row ends; a run of 16 i pixels uses the layer's i-th consecutive map
+                        unsigned ow = px, oh = py, b = pn;
+                        for (unsigned done = 0; done < 128u;) {
+                            const unsigned len = min(128u - done, OW - ow);
+                            tma_load_3d(dst + done * 128u, map + (size_t)(len / 16u - 1u) * 128, 0, (int)ow, (int)(b * PH + oh * stride + ch + j), &sh->full[r.s]);
+                            done += len;
+                            ow += len;
+                            if (ow == OW) { ow = 0; if (++oh == OH) { oh = 0; b++; } }
                         }
-            } else {
-                // the 128 pixels are cut where an output row ends; a run of 16 j pixels uses the layer's j-th consecutive map
-                for (unsigned kh = 0; kh < KH; kh++) {
-                    if (!mbar_wait(&sh->empty[r.s], r.parity() ^ 1u, ctrl, status, 2)) return false;
-                    mbar_arrive_expect_tx(&sh->full[r.s], A_STAGE_BYTES);
-                    unsigned ow = px, oh = py, b = pn;
-                    for (unsigned done = 0; done < 128u;) {
-                        const unsigned len = min(128u - done, OW - ow);
-                        tma_load_3d(ring + r.s * r.stage_bytes + done * 128u, map + (size_t)(len / 16u - 1u) * 128, 0, (int)ow,
-                                    (int)(b * PH + oh * stride + kh), &sh->full[r.s]);
-                        done += len;
-                        ow += len;
-                        if (ow == OW) { ow = 0; if (++oh == OH) { oh = 0; b++; } }
                     }
-                    r.step();
                 }
+                r.step();
             }
         }
     }
@@ -323,44 +318,46 @@ __device__ __forceinline__ bool produce_a(const Slot &sl, unsigned ring, Ring &r
 // ---- W operand producer: one thread ----------------------------------------------------------------------------------
 __device__ __forceinline__ bool produce_b(const Slot &sl, unsigned ring, Ring &r, Shared *sh, CtrlDev *ctrl, StatusHost *status) {
     const LayerDev &L = sl.layer;
-    const Geometry g = geometry(L, sl.tile);
+    const Origin g = origin(L, sl.tile);
     const unsigned char *map = sl.maps + (size_t)L.wmap * 128;
     asm volatile("fence.proxy.async.global;" ::: "memory");
-    if (!recut(r, g, sh, ctrl, status)) return false;
-    const unsigned box = L.b_box, tile_w = sl.tile.tile_w, tile_h = sl.tile.tile_h;
+    if (!recut(r, L, sh, ctrl, status)) return false;
+    const unsigned tile_w = sl.tile.tile_w, tile_h = sl.tile.tile_h, chunks = L.chunks, per = L.per_stage, bytes = per * L.b_rows * 128u;
     for (unsigned n0 = 0; n0 < tile_w; n0 += 128u)
-        for (unsigned mp = 0; mp < tile_h; mp += BLOCK_ROWS) {
-            const unsigned boxes = (min(BLOCK_ROWS, tile_h - mp) + box - 1u) / box, bytes = boxes * box * 128u;
-            const int y = g.by + (int)mp, x1 = g.bx + (int)g.k;
-            for (int x = g.bx; x < x1; x += 32) {
+        for (unsigned mp = 0; mp < tile_h; mp += BLOCK_ROWS)
+            for (unsigned ch = 0; ch < chunks; ch += per) {
                 if (!mbar_wait(&sh->empty[r.s], r.parity() ^ 1u, ctrl, status, 9)) return false;
                 mbar_arrive_expect_tx(&sh->full[r.s], bytes);
-                const unsigned dst = ring + r.s * r.stage_bytes + A_STAGE_BYTES;
-                tma_load_2d(dst, map, x, y, &sh->full[r.s]);
-                for (unsigned j = 1; j < boxes; j++) tma_load_2d(dst + j * box * 128u, map, x, y + (int)(j * box), &sh->full[r.s]);
+                tma_load_3d(ring + r.s * r.stage_bytes + per * A_CHUNK_BYTES, map, 0, g.by + (int)mp, g.bx + (int)ch, &sh->full[r.s]);
                 r.step();
             }
-        }
     return true;
 }
 
 // ---- MMA issuer: one thread ------------------------------------------------------------------------------------------
 // `half`: accumulator half of the next block; `acc_uses`: parity of the uses of each half.
 __device__ __forceinline__ bool issue_mma(const Slot &sl, unsigned ring, Ring &r, unsigned &half, unsigned &acc_uses, Shared *sh, CtrlDev *ctrl, StatusHost *status) {
-    const Geometry g = geometry(sl.layer, sl.tile);
-    if (g.stage_bytes != r.stage_bytes) { r.s = 0; r.stage_bytes = g.stage_bytes; r.stages = g.stages; }
-    const unsigned tmem = sh->tmem_base, tile_w = sl.tile.tile_w, tile_h = sl.tile.tile_h;
+    const LayerDev &L = sl.layer;
+    if (L.stage_bytes != r.stage_bytes) { r.s = 0; r.stage_bytes = L.stage_bytes; r.stages = L.stages; }
+    const unsigned tmem = sh->tmem_base, tile_w = sl.tile.tile_w, tile_h = sl.tile.tile_h, chunks = L.chunks, per = L.per_stage;
+    const unsigned b_off = per * A_CHUNK_BYTES, b_step = (L.b_rows * 128u) >> 4;
     for (unsigned n0 = 0; n0 < tile_w; n0 += 128u)
         for (unsigned mp = 0; mp < tile_h; mp += BLOCK_ROWS) {
             const unsigned idesc = umma_idesc((min(BLOCK_ROWS, tile_h - mp) + 15u) & ~15u), d = tmem + half * BLOCK_ROWS;
             if (!mbar_wait(&sh->acc_empty[half], ((acc_uses >> half) & 1u) ^ 1u, ctrl, status, 6)) return false;
             acc_uses ^= 1u << half;
             tc_fence_after();
-            for (unsigned kc = 0; kc < g.k; kc += 32u) {
+            for (unsigned ch = 0; ch < chunks; ch += per) {
+                const unsigned n = min(per, chunks - ch), sA = ring + r.s * r.stage_bytes;
+                unsigned alow = umma_desc_low(sA), blow = umma_desc_low(sA + b_off);
                 if (!mbar_wait(&sh->full[r.s], r.parity(), ctrl, status, 3)) return false;
                 tc_fence_after();
-                const unsigned sA = ring + r.s * r.stage_bytes;
-                tc_mma_stage(d, umma_desc_low(sA), umma_desc_low(sA + A_STAGE_BYTES), idesc, kc);
+                tc_mma_stage(d, alow, blow, idesc, ch);
+                for (unsigned j = 1; j < n; j++) {
+                    alow += A_CHUNK_BYTES >> 4;
+                    blow += b_step;
+                    tc_mma_stage(d, alow, blow, idesc, 1u);
+                }
                 tc_commit(&sh->empty[r.s]);
                 r.step();
             }
