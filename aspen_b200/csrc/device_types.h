@@ -26,6 +26,7 @@ struct LayerDev {
     int amap;                 // tensor map of the X-side operand (PARENT_0 activations)
     unsigned a_kind;          // X operand staging, see tiles_tc.cuh
     unsigned a_multi;         // one X box covers all chunks of a stage (the map has a third dimension: the chunk)
+    unsigned a_rows;          // columns (MMA rows) of the X-side box: 128, or what a narrow layer has
     unsigned b_rows;          // rows of the W-side box (one per stage): the tile's rows, at most 256
     unsigned chunks;          // 32-deep chunks of the contraction
     unsigned per_stage;       // chunks of one stage of the operand ring

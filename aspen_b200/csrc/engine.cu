@@ -447,7 +447,7 @@ static int build_device_nasm(Engine *e, nasm_t *host_nasm) {
     auto add_x_map = [&](LayerDev &L, const void *base, cuuint64_t inner, cuuint64_t outer, cuuint64_t stride_bytes) {
         L.a_kind = tc::A_TMA;
         L.a_multi = inner % 32 == 0;
-        L.amap = add_map(base, inner, outer, stride_bytes, 128, L.a_multi ? L.per_stage : 0);
+        L.amap = add_map(base, inner, outer, stride_bytes, L.a_rows, L.a_multi ? L.per_stage : 0);
     };
     // 3-D map of the padded input copy: (32 floats of a row, output pixel = `stride` input pixels apart, row)
     // Eight consecutive maps, the j-th with a box of 16 j pixels.  Returns the index of the first, or -2 when the driver
@@ -467,7 +467,7 @@ static int build_device_nasm(Engine *e, nasm_t *host_nasm) {
         }
         return (int)first;
     };
-    // im2col map of a convolution's parent matrix: (channel, iw, ih, sample), boxes of 32 channels x 128 output pixels.  The
+    // im2col map of a convolution's parent matrix: (channel, iw, ih, sample), boxes of 32 channels x 128 (a_rows) output pixels.  The
     // corners bound the first tap of the first and last output pixel; the strides are the convolution's.
     auto add_im2col_map = [&](const LayerDev &L) -> int {
         CUtensorMap m;
@@ -476,7 +476,7 @@ static int build_device_nasm(Engine *e, nasm_t *host_nasm) {
         cuuint64_t strides[3] = {(cuuint64_t)L.ld0 * 4, (cuuint64_t)L.IW * L.ld0 * 4, (cuuint64_t)L.IH * L.IW * L.ld0 * 4};
         int lower[2] = {-pad, -pad}, upper[2] = {pad - (int)L.KW + 1, pad - (int)L.KH + 1};
         cuuint32_t estr[4] = {1, L.stride, L.stride, 1};
-        CUresult r = get_encode_im2col_fn()(&m, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, const_cast<float *>(L.in0), dims, strides, lower, upper, 32, 128, estr,
+        CUresult r = get_encode_im2col_fn()(&m, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, const_cast<float *>(L.in0), dims, strides, lower, upper, 32, L.a_rows, estr,
                                             CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                                             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
         if (r != CUDA_SUCCESS) return -2;
@@ -506,7 +506,8 @@ static int build_device_nasm(Engine *e, nasm_t *host_nasm) {
             L.b_rows = (unsigned)round_up(std::min(th, tc::BLOCK_ROWS), 16);
             L.chunks = std::max(1u, (k + 31) / 32);
             L.per_stage = std::min(L.chunks, L.b_rows <= 64 ? 4u : L.b_rows <= 128 ? 2u : 1u);
-            L.stage_bytes = L.per_stage * (tc::A_CHUNK_BYTES + L.b_rows * 128);
+            L.a_rows = std::min(128u, (unsigned)round_up(std::min(nasm->ldata[i].ninst_tile_dims[OUT_W], L.W), 8));
+            L.stage_bytes = L.per_stage * (L.a_rows + L.b_rows) * 128;
             L.stages = std::min(tc::MAX_STAGES, tc::RING_BYTES / L.stage_bytes);
         };
         if (gemm_w || l.type == K_ATTENTION_LAYER || l.type == V_ATTENTION_LAYER) cut_ring(l.type == K_ATTENTION_LAYER ? L.hd : l.type == V_ATTENTION_LAYER ? L.seq : L.Kpad);

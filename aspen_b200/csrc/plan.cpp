@@ -25,12 +25,13 @@ bool contraction(LAYER_TYPE t) { return t == CONV_LAYER || t == FC_LAYER || t ==
 unsigned ceil_div(unsigned a, unsigned b) { return (a + b - 1) / b; }
 
 // Estimated microseconds of one tile of th x tw outputs with a k-deep contraction, `gap` of them between two tiles of an SM.
-// Tensor cores (measured, see tiles_tc.cuh): 0.29 us per 32-deep chunk of a 128 x <= 128 block, 0.38 of a 128 x 256 one; the
-// epilogue of a block takes 0.4 us per 32 rows and runs under the next block's main loop.
+// Tensor cores (measured): a 32-deep chunk of a 128-column block takes 0.38 us with 256 rows (the MMAs' own rate), 0.28 with 128 and
+// 0.19 below (an MMA of 128 lanes takes as long with 32 rows as with 64); the epilogue of a block takes 0.4 us per 32 rows and
+// runs under the next block's main loop.
 double tile_us(bool tensor, unsigned th, unsigned tw, unsigned k, double gap) {
     if (tensor) {
         const unsigned chunks = ceil_div(k, 32), nb = ceil_div(tw, 128) * ceil_div(th, 256), rows = std::min(th, 256u);
-        const double loop = chunks * (rows > 128 ? 0.38 : 0.29), epi = 0.6 + 0.4 * ceil_div(rows, 32);
+        const double loop = chunks * (rows > 128 ? 0.38 : rows > 64 ? 0.28 : 0.19), epi = 0.6 + 0.4 * ceil_div(rows, 32);
         return gap + loop + epi + (nb - 1) * std::max(loop, epi);
     }
     // fp32 blocks (gemm_ffma.cuh): 128 FMAs a clock at the shape's share of the rate

@@ -21,7 +21,8 @@
 // stage take 0.14 us and of a 128 x 256 stage 0.28.  The loops below hold no division for the same reason.
 //
 // Staging.  Both operands are K-major, 32 fp32 (128 bytes) per row and k-chunk, in the 128-byte swizzled shared-memory
-// layout UMMA descriptors and TMA share.  The ring is cut into as many stages as the tile's row count allows (8 of 24 KB
+// layout UMMA descriptors and TMA share.  A narrow layer (few tokens, few pixels) stages only the columns it has; the MMA reads
+// 128 rows all the same, whatever lies there: those accumulator lanes have no reader.  The ring is cut into as many stages as the tile's row count allows (8 of 24 KB
 // for 64 rows, 6 of 32 KB for 128, 4 of 48 KB for 256); when the cut changes between two tiles both producers first
 // wait until the old stages have been read.
 //
@@ -34,7 +35,6 @@ namespace tc {
 
 constexpr unsigned MAX_STAGES = 8;
 constexpr unsigned RING_BYTES = 192u * 1024u;
-constexpr unsigned A_CHUNK_BYTES = 128 * 128;
 constexpr unsigned NW = 256;                       // worker threads
 constexpr unsigned WARP_A = 0, WARP_MMA = 1, WARP_SCHED = 2, WARP_B = 3, WARP_WORK = 4;   // workers: warps 4 .. 11 (warp % 4 = TMEM lane quarter)
 constexpr unsigned THREADS = 128 + NW;
@@ -261,7 +261,7 @@ __device__ __forceinline__ bool produce_a(const Slot &sl, unsigned ring, Ring &r
     asm volatile("fence.proxy.async.global;" ::: "memory");
     if (!recut(r, L, sh, ctrl, status)) return false;
     const unsigned kind = L.a_kind, multi = L.a_multi, tile_w = sl.tile.tile_w, tile_h = sl.tile.tile_h, pos_w = sl.tile.pos_w;
-    const unsigned OW = L.OW, OH = L.OH, KW = L.KW, IC = L.IC, PH = L.PH, stride = L.stride, chunks = L.chunks, per = L.per_stage;
+    const unsigned OW = L.OW, OH = L.OH, KW = L.KW, IC = L.IC, PH = L.PH, stride = L.stride, chunks = L.chunks, per = L.per_stage, chunk_bytes = L.a_rows * 128u;
     const int pad = (int)L.pad;
     for (unsigned n0 = 0; n0 < tile_w; n0 += 128u) {
         unsigned px = 0, py = 0, pn = 0;             // first output pixel of the block
@@ -276,7 +276,7 @@ __device__ __forceinline__ bool produce_a(const Slot &sl, unsigned ring, Ring &r
                 const int y = g.ay + (int)n0;
                 for (unsigned ch = 0; ch < chunks; ch += per) {
                     if (!mbar_wait(&sh->empty[r.s], r.parity() ^ 1u, ctrl, status, 2)) return false;
-                    mbar_arrive_expect_tx(&sh->full[r.s], per * A_CHUNK_BYTES);
+                    mbar_arrive_expect_tx(&sh->full[r.s], per * chunk_bytes);
                     tma_load_3d(ring + r.s * r.stage_bytes, map, 0, y, g.ax + (int)ch, &sh->full[r.s]);
                     r.step();
                 }
@@ -288,8 +288,8 @@ __device__ __forceinline__ bool produce_a(const Slot &sl, unsigned ring, Ring &r
                 const unsigned n = min(per, chunks - ch);
                 unsigned dst = ring + r.s * r.stage_bytes;
                 if (!mbar_wait(&sh->empty[r.s], r.parity() ^ 1u, ctrl, status, 2)) return false;
-                mbar_arrive_expect_tx(&sh->full[r.s], n * A_CHUNK_BYTES);
-                for (unsigned j = 0; j < n; j++, dst += A_CHUNK_BYTES) {
+                mbar_arrive_expect_tx(&sh->full[r.s], n * chunk_bytes);
+                for (unsigned j = 0; j < n; j++, dst += chunk_bytes) {
                     if (kind == A_IM2COL) {
                         tma_load_im2col(dst, map, (int)c, x0, y0, (int)pn, kw, kh, &sh->full[r.s]);
                         c += 32u;
@@ -322,13 +322,13 @@ __device__ __forceinline__ bool produce_b(const Slot &sl, unsigned ring, Ring &r
     const unsigned char *map = sl.maps + (size_t)L.wmap * 128;
     asm volatile("fence.proxy.async.global;" ::: "memory");
     if (!recut(r, L, sh, ctrl, status)) return false;
-    const unsigned tile_w = sl.tile.tile_w, tile_h = sl.tile.tile_h, chunks = L.chunks, per = L.per_stage, bytes = per * L.b_rows * 128u;
+    const unsigned tile_w = sl.tile.tile_w, tile_h = sl.tile.tile_h, chunks = L.chunks, per = L.per_stage, bytes = per * L.b_rows * 128u, b_off = per * L.a_rows * 128u;
     for (unsigned n0 = 0; n0 < tile_w; n0 += 128u)
         for (unsigned mp = 0; mp < tile_h; mp += BLOCK_ROWS)
             for (unsigned ch = 0; ch < chunks; ch += per) {
                 if (!mbar_wait(&sh->empty[r.s], r.parity() ^ 1u, ctrl, status, 9)) return false;
                 mbar_arrive_expect_tx(&sh->full[r.s], bytes);
-                tma_load_3d(ring + r.s * r.stage_bytes + per * A_CHUNK_BYTES, map, 0, g.by + (int)mp, g.bx + (int)ch, &sh->full[r.s]);
+                tma_load_3d(ring + r.s * r.stage_bytes + b_off, map, 0, g.by + (int)mp, g.bx + (int)ch, &sh->full[r.s]);
                 r.step();
             }
     return true;
@@ -340,7 +340,7 @@ __device__ __forceinline__ bool issue_mma(const Slot &sl, unsigned ring, Ring &r
     const LayerDev &L = sl.layer;
     if (L.stage_bytes != r.stage_bytes) { r.s = 0; r.stage_bytes = L.stage_bytes; r.stages = L.stages; }
     const unsigned tmem = sh->tmem_base, tile_w = sl.tile.tile_w, tile_h = sl.tile.tile_h, chunks = L.chunks, per = L.per_stage;
-    const unsigned b_off = per * A_CHUNK_BYTES, b_step = (L.b_rows * 128u) >> 4;
+    const unsigned b_off = per * L.a_rows * 128u, a_step = (L.a_rows * 128u) >> 4, b_step = (L.b_rows * 128u) >> 4;
     for (unsigned n0 = 0; n0 < tile_w; n0 += 128u)
         for (unsigned mp = 0; mp < tile_h; mp += BLOCK_ROWS) {
             const unsigned idesc = umma_idesc((min(BLOCK_ROWS, tile_h - mp) + 15u) & ~15u), d = tmem + half * BLOCK_ROWS;
@@ -354,7 +354,7 @@ __device__ __forceinline__ bool issue_mma(const Slot &sl, unsigned ring, Ring &r
                 tc_fence_after();
                 tc_mma_stage(d, alow, blow, idesc, ch);
                 for (unsigned j = 1; j < n; j++) {
-                    alow += A_CHUNK_BYTES >> 4;
+                    alow += a_step;
                     blow += b_step;
                     tc_mma_stage(d, alow, blow, idesc, 1u);
                 }
