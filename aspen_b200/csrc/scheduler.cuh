@@ -78,14 +78,22 @@ __device__ __forceinline__ unsigned ld_acquire_sys(const unsigned *p) {
     return v;
 }
 
+__device__ __forceinline__ void fence_gpu() { asm volatile("fence.acq_rel.gpu;" ::: "memory"); }
+__device__ __forceinline__ tc::GraphRef graph_ref(const NasmDev &G) {
+    return {G.layers, G.tiles, reinterpret_cast<const uint2 *>(G.children), G.dep, (const unsigned char *)G.wmaps, &G.input, G.svc, G.n_exec};
+}
+__device__ __forceinline__ tc::GraphRef graph_ref(const tc::Shared *sh, const NasmDev *nasms, unsigned g) {
+    return g < tc::CACHED_GRAPHS ? sh->graphs[g] : graph_ref(nasms[g]);
+}
+
 // Child update of a completed tile; called by the whole (converged) scheduler warp.  An edge is (child tile, layer << 16 |
 // count the child waits for); `e` holds this lane's first edge, fetched while the tile ran.
 // Returns a child this CTA should run next (only when want_keep), or 0.
-static __device__ __forceinline__ Entry complete_children(const NasmDev &G, unsigned g, uint2 e, unsigned child_off, unsigned child_cnt, CtrlDev *ctrl, Entry *queue, bool want_keep) {
+static __device__ __forceinline__ Entry complete_children(const tc::GraphRef &G, unsigned g, uint2 e, unsigned child_off, unsigned child_cnt, CtrlDev *ctrl, Entry *queue, unsigned cap, bool want_keep) {
     const unsigned lane = threadIdx.x & 31u;
-    const uint2 *edges = reinterpret_cast<const uint2 *>(G.children) + child_off;
+    const uint2 *edges = G.children + child_off;
     unsigned *dep = G.dep;
-    __threadfence();                                     // release: this tile's output
+    fence_gpu();                                         // release: this tile's output
     Entry next = 0;
     for (unsigned base = 0; base < child_cnt; base += 32u) {
         const unsigned idx = base + lane;
@@ -97,7 +105,7 @@ static __device__ __forceinline__ Entry complete_children(const NasmDev &G, unsi
         }
         unsigned mask = __ballot_sync(0xffffffffu, ready);
         if (mask == 0u) continue;
-        __threadfence();                                 // acquire the other parents' outputs (through the counters), then publish
+        fence_gpu();                                     // acquire the other parents' outputs (through the counters), then publish
         const Entry mine = make_entry(e.x, g, e.y >> 16);
         if (want_keep && next == 0) {
             const unsigned first = __ffs(mask) - 1u;
@@ -112,7 +120,7 @@ static __device__ __forceinline__ Entry complete_children(const NasmDev &G, unsi
             pos = __shfl_sync(0xffffffffu, pos, 0);
             if (ready) {
                 const unsigned rank = __popc(mask & ((1u << lane) - 1u));
-                if (pos + rank < ctrl->cap) st_release(&queue[pos + rank], mine);
+                if (pos + rank < cap) asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(&queue[pos + rank]), "l"(mine) : "memory");   // behind the fence
             }
         }
     }
@@ -258,9 +266,8 @@ __device__ __forceinline__ bool wait_posted(unsigned long long *bar, unsigned pa
 
 // Fills a slot with a ready tile and hands it to the roles (whole warp).  The tile's and the layer's descriptors are independent
 // loads; both and the graph's addresses are constant while the kernel runs.
-static __device__ __forceinline__ void post(tc::Slot &sl, unsigned long long &posted, const NasmDev *nasms, Entry entry) {
+static __device__ __forceinline__ void post(tc::Slot &sl, unsigned long long &posted, const tc::GraphRef &G, Entry entry) {
     const unsigned lane = threadIdx.x & 31u, g = (unsigned)(entry >> 48), layer = (unsigned)(entry >> 32) & 0xffffu, tile = (unsigned)entry - 1u;
-    const NasmDev &G = nasms[g];
     constexpr unsigned LW = sizeof(LayerDev) / 4, TW = sizeof(TileDev) / 4;
     static_assert(sizeof(LayerDev) % 4 == 0 && LW <= 96 && TW <= 32, "copied in words");
     const unsigned *lsrc = reinterpret_cast<const unsigned *>(G.layers + layer), *tsrc = reinterpret_cast<const unsigned *>(G.tiles + tile);
@@ -271,7 +278,7 @@ static __device__ __forceinline__ void post(tc::Slot &sl, unsigned long long &po
     #pragma unroll
     for (unsigned i = 0; i < 3; i++) if (i * 32u + lane < LW) reinterpret_cast<unsigned *>(&sl.layer)[i * 32u + lane] = lw[i];
     if (lane < TW) reinterpret_cast<unsigned *>(&sl.tile)[lane] = tw;
-    if (lane == 0) { sl.live = 1u; sl.nasm = g; sl.maps = (const unsigned char *)G.wmaps; sl.input = &G.input; }
+    if (lane == 0) { sl.live = 1u; sl.nasm = g; sl.maps = G.maps; sl.input = G.input; }
     __syncwarp();
     if (lane == 0) tc::mbar_arrive(&posted);
 }
@@ -291,14 +298,14 @@ static __device__ __noinline__ void scheduler_warp(const NasmDev *nasms, CtrlDev
     unsigned last_done = 0;
     unsigned long long t_progress = __shfl_sync(0xffffffffu, global_ns(), 0), t_mark = t_progress;
     const unsigned long long window = ctrl->stall_ns;
-    unsigned idle_spins = 30u, turn = 0, flags = 0, done = 0, ahead_turn = 0;   // the first idle turns already look for a pass to start
+    unsigned idle_spins = 30u, turn = 0, flags = 0, done = 0, ahead_turn = 0, q_tail = 0, q_head = 0;   // the first idle turns already look for a pass to start
     while (true) {
         bool progressed = false;
         // Control words (lanes 1 - 4) and the slot we wait on (lane 0) are read together: one L2 round trip a turn.  With a tile
-        // in work the control words are sampled every 8th turn.
+        // in work the control words are sampled every 64th turn: what the turn is then waiting for is the tile.
         unsigned word = 0;
         Entry slot = 0;
-        const bool sample = issued == retired || (turn++ & 7u) == 0u;
+        const bool sample = issued == retired || (turn++ & 63u) == 0u;
         if (sample && lane >= 1u && lane <= 4u) word = ld_relaxed(watch);
         if (ticket != ASPEN_TILE_NONE && lane == 0u) slot = ld_acquire(&queue[ticket]);
         if (sample) {
@@ -316,7 +323,7 @@ static __device__ __noinline__ void scheduler_warp(const NasmDev *nasms, CtrlDev
                 if (my_prof && lane == 0) t_mark = global_ns();
                 const tc::Slot &sl = sh->slots[k];
                 const unsigned g = sl.nasm;
-                const Entry child = complete_children(nasms[g], g, (retired & 1u) ? edge1 : edge0, sl.tile.child_off, sl.tile.child_cnt, ctrl, queue, kept == 0);
+                const Entry child = complete_children(graph_ref(sh, nasms, g), g, (retired & 1u) ? edge1 : edge0, sl.tile.child_off, sl.tile.child_cnt, ctrl, queue, cap, kept == 0);
                 if (child) kept = child;
                 if (my_prof && lane == 0) my_prof[1] += global_ns() - t_mark;
                 acct_nasm = g;
@@ -335,10 +342,11 @@ static __device__ __noinline__ void scheduler_warp(const NasmDev *nasms, CtrlDev
                 // the completion of the first runs beside the second.  A ticket held for a tile that is not there yet would
                 // keep that tile from an idle SM.
                 bool take = ticket == ASPEN_TILE_NONE && issued == retired;
-                if (ahead != 0u && !take && ticket == ASPEN_TILE_NONE && (ahead_turn++ & 7u) == 0u) {
-                    int backlog = 0;
-                    if (lane == 0) backlog = (int)(ld_relaxed(&ctrl->tail) - ld_relaxed(&ctrl->head));
-                    take = __shfl_sync(0xffffffffu, backlog, 0) >= (int)ahead;
+                if (ahead != 0u && !take && ticket == ASPEN_TILE_NONE) {
+                    // asked for in one turn, looked at some turns later: the turns in between do not wait for it
+                    if ((ahead_turn & 7u) == 0u && lane == 0) { q_tail = ld_relaxed(&ctrl->tail); q_head = ld_relaxed(&ctrl->head); }
+                    if ((ahead_turn & 7u) == 7u) take = __shfl_sync(0xffffffffu, (int)(q_tail - q_head), 0) >= (int)ahead;
+                    ahead_turn++;
                 }
                 if (take) {
                     unsigned t = lane == 0 ? atomicAdd(&ctrl->head, 1u) : 0u;
@@ -354,10 +362,11 @@ static __device__ __noinline__ void scheduler_warp(const NasmDev *nasms, CtrlDev
         // 3. post it: one tile in work, one behind it
         if (next) {
             const unsigned k = issued % tc::SLOTS;
-            post(sh->slots[k], sh->posted[k], nasms, next);
+            const tc::GraphRef G = graph_ref(sh, nasms, (unsigned)(next >> 48));
+            post(sh->slots[k], sh->posted[k], G, next);
             const tc::Slot &sl = sh->slots[k];
             uint2 e = make_uint2(0u, 1u);
-            if (lane < sl.tile.child_cnt) e = __ldg(reinterpret_cast<const uint2 *>(nasms[sl.nasm].children) + sl.tile.child_off + lane);
+            if (lane < sl.tile.child_cnt) e = __ldg(G.children + sl.tile.child_off + lane);
             if (issued & 1u) edge1 = e; else edge0 = e;
             issued++;
             progressed = true;
@@ -365,9 +374,10 @@ static __device__ __noinline__ void scheduler_warp(const NasmDev *nasms, CtrlDev
         // 4. completion accounting, behind everything that another tile may be waiting for
         if (acct) {
             unsigned t = 0;
-            if (lane == 0) { atomicAdd(&ctrl->done, 1u); t = atomicAdd(&nasms[acct_nasm].svc[SVC_COUNT], 1u) + 1u; }
+            const tc::GraphRef G = graph_ref(sh, nasms, acct_nasm);
+            if (lane == 0) { atomicAdd(&ctrl->done, 1u); t = atomicAdd(&G.svc[SVC_COUNT], 1u) + 1u; }
             t = __shfl_sync(0xffffffffu, t, 0);
-            if (t % nasms[acct_nasm].n_exec == 0u) end_of_pass(nasms, n_nasm, acct_nasm, t, ctrl, queue);
+            if (t % G.n_exec == 0u) end_of_pass(nasms, n_nasm, acct_nasm, t, ctrl, queue);
             acct = false;
         }
         // 5. end of launch / stall detection
@@ -463,6 +473,7 @@ scheduler_kernel(const NasmDev *nasms, CtrlDev *ctrl, Entry *queue, StatusHost *
         if (warp == tc::WARP_MMA) tc::tmem_alloc(&sh->tmem_base, tc::TMEM_COLS);
         tc::tc_fence_before();
     }
+    for (unsigned g = tid, n = min(tc::CACHED_GRAPHS, ctrl->n_nasm); g < n; g += threads<TENSOR_CORES>()) sh->graphs[g] = graph_ref(nasms[g]);
     __syncthreads();
     if (TENSOR_CORES) tc::tc_fence_after();
 

@@ -52,7 +52,22 @@ struct Slot {
     const InputDev *input;
 };
 
+// What the scheduler needs of a graph to hand out and retire its tiles; the first ones of a launch are kept in shared memory,
+// which takes an L2 round trip off both.
+struct GraphRef {
+    const LayerDev *layers;
+    const TileDev *tiles;
+    const uint2 *children;
+    unsigned *dep;
+    const unsigned char *maps;
+    const InputDev *input;
+    unsigned *svc;
+    unsigned n_exec;
+};
+constexpr unsigned CACHED_GRAPHS = 12;
+
 struct Shared {
+    GraphRef graphs[CACHED_GRAPHS];
     unsigned long long full[MAX_STAGES], empty[MAX_STAGES];    // stage filled (both producers) / read by the MMAs
     unsigned long long acc_full[2], acc_empty[2];              // accumulator half complete / read by the workers
     unsigned long long posted[SLOTS], finished[SLOTS];         // scheduler -> roles / roles -> scheduler
