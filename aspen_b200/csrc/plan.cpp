@@ -61,9 +61,10 @@ Grid choose(const nasm_ldata_t &ld, const nasm_t *nasm, bool tensor, unsigned sm
                 const double us = tile_us(tensor, std::min(hs[i], H), std::min(tw, g.seg), k, served ? 2.5 : 4.0);
                 const double share = (double)tiles / sms;
                 // Passes of other graphs fill the SMs a served layer leaves idle: its work counts, and, because the graphs in
-                // rotation are few, to a lesser degree the length of its longest tile.  A layer launched alone takes as many
+                // rotation are few, to a lesser degree the length of its longest tile
+                // (0.2 / 0.5 / 1.0 of it: 1.92 / 1.61 / 1.51 ms a request for ResNet-50 x 32 in bursts of twelve, 0.279 / 0.283 / 0.304 for x 4).  A layer launched alone takes as many
                 // rounds as its busiest SM; the last, partly filled one overlaps in part with the next layer.
-                const double cost = served ? us * (share + 0.2) : us * (0.4 * std::max(1.0, share) + 0.6 * ceil_div(tiles, sms));
+                const double cost = served ? us * (share + 0.5) : us * (0.4 * std::max(1.0, share) + 0.6 * ceil_div(tiles, sms));
                 if (best == 0 || cost < best * 0.999) { best = cost; g.th = hs[i]; g.tw = tw; }
             }
     } else if (l->type == SOFTMAX_LAYER || l->type == YOLO_LAYER || l->type == APPEND_LAYER) {

@@ -220,7 +220,14 @@ static __device__ __noinline__ void worker_tile(const tc::Slot &sl, unsigned wt,
     switch (L.type) {
         case CONV_LAYER: case FC_LAYER: case MATMUL_LAYER: case K_ATTENTION_LAYER: case V_ATTENTION_LAYER: tile_gemm_ffma<!TENSOR_CORES>(L, T, wt, tc::NW, scratch); break;
         case RESIDUAL_LAYER: tile_residual(L, T, wt, tc::NW); break;
-        case MAXPOOL_LAYER: tile_pool<true>(L, T, wt, tc::NW); break;
+        case MAXPOOL_LAYER:
+            // whole 16-byte pieces, and every window holds a pixel of the image
+            if (((T.tile_h | T.pos_h | L.ld0 | L.ldc) & 3u) == 0u && L.KH == L.KW && L.pad < L.KH && (L.OH - 1u) * L.stride < L.IH + L.pad &&
+                (L.OW - 1u) * L.stride < L.IW + L.pad && (L.KH == 2u || L.KH == 3u)) {
+                if (L.KH == 2u) tile_max_small<2, 2, 4>(L, T, wt, tc::NW);
+                else tile_max_small<3, 3, 2>(L, T, wt, tc::NW);
+            } else tile_pool<true>(L, T, wt, tc::NW);
+            break;
         case AVGPOOL_LAYER: tile_pool<false>(L, T, wt, tc::NW); break;
         case LAYERNORM_LAYER: tile_layernorm(L, T, wt, tc::NW); break;
         case SOFTMAX_LAYER: tile_softmax(L, T, wt, tc::NW); break;

@@ -125,6 +125,50 @@ static __device__ __noinline__ void tile_residual(const LayerDev &L, const TileD
 // items at a time; the window's taps are fetched nine at a time (a whole 3 x 3 window), all loads of both items
 // issued before the first is used (a tap outside the image reads nothing and contributes the neutral element),
 // so the tile is bound by bandwidth instead of one load latency per tap.
+// Max pooling with a small window, whole 16-byte pieces of channels: taps outside the image are moved to the nearest pixel inside,
+// which the window contains as well, so all KH x KW loads of U outputs are unconditional and in flight together.  With a
+// test per tap the loads went out a few at a time: 64 x 100352 outputs (3 x 3, stride 2) 158 -> 40 us per SM.
+template <int KH, int KW, int U>
+static __device__ __noinline__ void tile_max_small(const LayerDev &L, const TileDev &T, unsigned tid, unsigned nthr) {
+    const unsigned h4 = T.tile_h >> 2, total = T.tile_w * h4, pos_w = T.pos_w, pos_h = T.pos_h, hw = L.OH * L.OW, OW = L.OW;
+    const int IH = (int)L.IH, IW = (int)L.IW, stride = (int)L.stride, pad = (int)L.pad, act = L.act;
+    const size_t ld0 = L.ld0, ldc = L.ldc;
+    const float *in = L.in0;
+    float *out = L.out;
+    const bool round = L.round_out != 0;
+    for (unsigned i0 = tid; i0 < total; i0 += nthr * U) {
+        float4 v[U][KH * KW];
+        unsigned n[U], m[U];
+        #pragma unroll
+        for (int u = 0; u < U; u++) {
+            const unsigned i = min(i0 + u * nthr, total - 1u);       // past the end: the last piece again
+            n[u] = pos_w + i / h4;
+            m[u] = pos_h + 4u * (i % h4);
+            const unsigned b = n[u] / hw, r = n[u] - b * hw, oh = r / OW, ow = r - oh * OW;
+            const int y = (int)oh * stride - pad, x = (int)ow * stride - pad;
+            const float *img = in + (size_t)b * IH * IW * ld0 + m[u];
+            #pragma unroll
+            for (int kh = 0; kh < KH; kh++) {
+                const int ih = min(max(y + kh, 0), IH - 1);
+                #pragma unroll
+                for (int kw = 0; kw < KW; kw++) v[u][kh * KW + kw] = ldcg4(img + (size_t)(ih * IW + min(max(x + kw, 0), IW - 1)) * ld0);
+            }
+        }
+        #pragma unroll
+        for (int u = 0; u < U; u++) {
+            float4 a = v[u][0];
+            #pragma unroll
+            for (int k = 1; k < KH * KW; k++) {
+                const float4 x = v[u][k];
+                a.x = a.x >= x.x ? a.x : x.x; a.y = a.y >= x.y ? a.y : x.y; a.z = a.z >= x.z ? a.z : x.z; a.w = a.w >= x.w ? a.w : x.w;
+            }
+            if (act != NO_ACTIVATION && act != LINEAR) { a.x = activate(a.x, act); a.y = activate(a.y, act); a.z = activate(a.z, act); a.w = activate(a.w, act); }
+            if (round) { a.x = tf32_round(a.x); a.y = tf32_round(a.y); a.z = tf32_round(a.z); a.w = tf32_round(a.w); }
+            if (i0 + u * nthr < total) *reinterpret_cast<float4 *>(out + (size_t)n[u] * ldc + m[u]) = a;
+        }
+    }
+}
+
 template <bool IS_MAX>
 static __device__ __noinline__ void tile_pool(const LayerDev &L, const TileDev &T, unsigned tid, unsigned nthr) {
     const unsigned h4 = T.tile_h >> 2, per_col = h4 + (T.tile_h & 3);
@@ -212,11 +256,24 @@ static __device__ __noinline__ void tile_layernorm(const LayerDev &L, const Tile
     const float *gain = L.weight + T.pos_h;
     const float *shift = L.bias ? L.bias + T.pos_h : nullptr;
     const bool in_regs = M <= 1024u && (M & 3u) == 0u && ((L.ld0 | L.ldc | T.pos_h) & 3u) == 0u;
-    for (unsigned n = warp; n < T.tile_w; n += nwarp) {
-        const float *x = L.in0 + (size_t)(T.pos_w + n) * L.ld0 + T.pos_h;
-        float *y = L.out + (size_t)(T.pos_w + n) * L.ldc + T.pos_h;
-        if (in_regs) {
+    if (in_regs) {
+        // a column of a warp at a time, all its loads (and, once, the gains' and shifts') in flight before the first use; two columns
+        // at a time spill
+        const unsigned tile_w = T.tile_w, pos_w = T.pos_w, pos_h = T.pos_h;
+        const size_t ld0 = L.ld0, ldc = L.ldc;
+        const float *in = L.in0 + pos_h;
+        float *out = L.out + pos_h;
+        const bool round = L.round_out != 0;
+        float4 g[8], b[8];
+        #pragma unroll
+        for (unsigned q = 0; q < 8; q++) {
+            const unsigned m = lane * 4u + q * 128u;
+            g[q] = m < M ? __ldg(reinterpret_cast<const float4 *>(gain + m)) : make_float4(0.f, 0.f, 0.f, 0.f);
+            b[q] = m < M && shift ? __ldg(reinterpret_cast<const float4 *>(shift + m)) : make_float4(0.f, 0.f, 0.f, 0.f);
+        }
+        for (unsigned n = warp; n < tile_w; n += nwarp) {
             float4 v[8];
+            const float *x = in + (size_t)(pos_w + n) * ld0;
             #pragma unroll
             for (unsigned q = 0; q < 8; q++) {
                 const unsigned m = lane * 4u + q * 128u;
@@ -225,27 +282,31 @@ static __device__ __noinline__ void tile_layernorm(const LayerDev &L, const Tile
             float s = 0.f, ss = 0.f;
             #pragma unroll
             for (unsigned q = 0; q < 8; q++) {
-                s += v[q].x + v[q].y + v[q].z + v[q].w;
-                ss += v[q].x * v[q].x + v[q].y * v[q].y + v[q].z * v[q].z + v[q].w * v[q].w;
+                const float4 t = v[q];
+                s += t.x + t.y + t.z + t.w;
+                ss += t.x * t.x + t.y * t.y + t.z * t.z + t.w * t.w;
             }
             s = warp_sum(s);
             ss = warp_sum(ss);
-            const float mean = s / (float)M;
-            const float var = ss / (float)M - mean * mean;
-            const float inv = 1.f / sqrtf(var + 1e-6f);
+            const float mean = s / (float)M, var = ss / (float)M - mean * mean, inv = 1.f / sqrtf(var + 1e-6f);
+            float *y = out + (size_t)(pos_w + n) * ldc;
             #pragma unroll
             for (unsigned q = 0; q < 8; q++) {
                 const unsigned m = lane * 4u + q * 128u;
                 if (m < M) {
-                    const float4 g = *reinterpret_cast<const float4 *>(gain + m);
-                    float4 o = {(v[q].x - mean) * inv * g.x, (v[q].y - mean) * inv * g.y, (v[q].z - mean) * inv * g.z, (v[q].w - mean) * inv * g.w};
-                    if (shift) { const float4 b = *reinterpret_cast<const float4 *>(shift + m); o.x += b.x; o.y += b.y; o.z += b.z; o.w += b.w; }
-                    o.x = store_round(o.x, L); o.y = store_round(o.y, L); o.z = store_round(o.z, L); o.w = store_round(o.w, L);
+                    const float4 t = v[q];
+                    float4 o = {(t.x - mean) * inv * g[q].x, (t.y - mean) * inv * g[q].y, (t.z - mean) * inv * g[q].z, (t.w - mean) * inv * g[q].w};
+                    if (shift) { o.x += b[q].x; o.y += b[q].y; o.z += b[q].z; o.w += b[q].w; }
+                    if (round) { o.x = tf32_round(o.x); o.y = tf32_round(o.y); o.z = tf32_round(o.z); o.w = tf32_round(o.w); }
                     *reinterpret_cast<float4 *>(y + m) = o;
                 }
             }
-            continue;
         }
+        return;
+    }
+    for (unsigned n = warp; n < T.tile_w; n += nwarp) {
+        const float *x = L.in0 + (size_t)(T.pos_w + n) * L.ld0 + T.pos_h;
+        float *y = L.out + (size_t)(T.pos_w + n) * L.ldc + T.pos_h;
         float s = 0.f, ss = 0.f;
         const unsigned M4 = M & ~3u;
         for (unsigned m = lane * 4; m < M4; m += 128) {
@@ -400,6 +461,41 @@ static __device__ void tile_input(const InputDev &I, const LayerDev &L, const Ti
         return;
     }
     if (I.padded && I.stage && H <= 4u && T.pos_h == 0u) {
+        // an image of three channels, columns four floats apart: four pixels are three 16-byte loads, two such groups in flight
+        if (H == 3u && L.ldc == 4u && ((T.tile_w | T.pos_w) & 3u) == 0u) {
+            const unsigned hw = I.IH * I.IW, IW = I.IW, PH = I.PH, PW = I.PW, pad = I.pad, groups = T.tile_w >> 2, pos_w = T.pos_w;
+            const bool round = I.round != 0;
+            float4 *padded = reinterpret_cast<float4 *>(I.padded), *out = reinterpret_cast<float4 *>(L.out);
+            const float *stage = I.stage;
+            for (unsigned g0 = tid; g0 < groups; g0 += 2u * nthr) {
+                float f[2][12];
+                #pragma unroll
+                for (int u = 0; u < 2; u++) {
+                    const unsigned g = min(g0 + u * nthr, groups - 1u);
+                    #pragma unroll
+                    for (int q = 0; q < 3; q++) {
+                        const float4 t = ldcg4(stage + (size_t)(pos_w + 4u * g) * 3u + 4 * q);
+                        f[u][4 * q] = t.x; f[u][4 * q + 1] = t.y; f[u][4 * q + 2] = t.z; f[u][4 * q + 3] = t.w;
+                    }
+                }
+                #pragma unroll
+                for (int u = 0; u < 2; u++) {
+                    const unsigned g = g0 + u * nthr;
+                    if (g >= groups) break;
+                    const unsigned w = pos_w + 4u * g;
+                    unsigned b = w / hw, r = w - b * hw, ih = r / IW, iw = r - ih * IW;
+                    #pragma unroll
+                    for (int q = 0; q < 4; q++) {
+                        float4 v = make_float4(f[u][3 * q], f[u][3 * q + 1], f[u][3 * q + 2], 0.f);
+                        if (round) { v.x = tf32_round(v.x); v.y = tf32_round(v.y); v.z = tf32_round(v.z); }
+                        out[w + q] = v;
+                        padded[((size_t)b * PH + ih + pad) * PW + iw + pad] = v;
+                        if (++iw == IW) { iw = 0; if (++ih == I.IH) { ih = 0; b++; } }
+                    }
+                }
+            }
+            return;
+        }
         // an image: one thread per pixel reads its (up to four) channels once and writes both copies
         const unsigned hw = I.IH * I.IW;
         for (unsigned c = tid; c < T.tile_w; c += nthr) {
