@@ -5,6 +5,7 @@
 #include "internal.h"
 #include "scheduler.cuh"
 #include "hostcopy.h"
+#include "fp32.h"
 
 #include <cuda.h>
 #include <cuda_runtime.h>
@@ -294,8 +295,8 @@ Engine *engine_create(int device, int precision, unsigned int /*num_dse_hint*/) 
               cudaHostGetDevicePointer(&e->status_d, e->status_h, 0) == cudaSuccess;
     if (ok) {
         memset((void *)e->status_h, 0, sizeof(StatusHost));
-        const void *kernel = precision == 0 ? (const void *)sched::scheduler_kernel<true> : (const void *)sched::scheduler_kernel<false>;
-        ok = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)e->smem_bytes) == cudaSuccess;
+        ok = (precision == 0 ? cudaFuncSetAttribute(sched::scheduler_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)e->smem_bytes)
+                             : fp32_prepare(e->smem_bytes)) == cudaSuccess;
         ok = ok && cudaEventCreateWithFlags(&e->svc_armed_ev, cudaEventDisableTiming) == cudaSuccess;
         if (env_u64("ASPEN_B200_IDLE_MS", &v) && v > 0) e->idle_ns = v * 1000000ull;
         if (env_u64("ASPEN_B200_SVC_AHEAD", &v)) e->svc_ahead = (unsigned)v;
@@ -859,7 +860,7 @@ static int svc_launch(Engine *e, const std::vector<nasm_t *> &graphs, bool leave
     if (e->precision == 0)
         sched::scheduler_kernel<true><<<e->n_ctas, sched::threads<true>(), e->smem_bytes, e->stream>>>(e->nasms_d, e->ctrl, e->queue, e->status_d, e->prof);
     else
-        sched::scheduler_kernel<false><<<e->n_ctas, sched::threads<false>(), e->smem_bytes, e->stream>>>(e->nasms_d, e->ctrl, e->queue, e->status_d, e->prof);
+        fp32_launch(e->n_ctas, e->smem_bytes, e->stream, e->nasms_d, e->ctrl, e->queue, e->status_d, e->prof);
     e->launches++;
     CUDA_TRY(cudaGetLastError());
     e->svc_graphs = graphs;

@@ -34,9 +34,11 @@ double tile_us(bool tensor, unsigned th, unsigned tw, unsigned k, double gap) {
         const double loop = chunks * (rows > 128 ? 0.38 : rows > 64 ? 0.28 : 0.19), epi = 0.6 + 0.4 * ceil_div(rows, 32);
         return gap + loop + epi + (nb - 1) * std::max(loop, epi);
     }
-    // fp32 blocks (gemm_ffma.cuh): 128 FMAs a clock at the shape's share of the rate
-    const unsigned bm = th > 64 && tw > 32 ? 128 : th > 32 && tw > 32 ? 64 : 32, bn = bm == 32 ? 32 : 64;
-    return gap + (double)ceil_div(th, bm) * ceil_div(tw, bn) * bm * bn * k / (128.0 * 1900.0 * (bm == 32 ? 0.65 : 0.80));
+    // fp32 blocks (gemm_ffma.cuh), shapes as tile_gemm_ffma picks them: some 3 us for filling the pipeline, the reduction and the
+    // stores, then steps of 32, 64 or 128 of k
+    const int shape = th > 64 && tw > 32 ? 0 : th > 32 && tw > 32 ? 1 : 2;
+    const unsigned bm = shape == 0 ? 128 : shape == 1 ? 64 : 32, bn = shape == 2 ? 32 : 64, kt = 32u << shape;
+    return gap + (double)ceil_div(th, bm) * ceil_div(tw, bn) * (3.0 + ceil_div(k, kt) * (shape == 2 ? 1.3 : 2.0));
 }
 
 Grid choose(const nasm_ldata_t &ld, const nasm_t *nasm, bool tensor, unsigned sms, bool served) {

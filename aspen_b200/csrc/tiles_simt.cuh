@@ -551,74 +551,104 @@ static __device__ void tile_input(const InputDev &I, const LayerDev &L, const Ti
 }
 
 // ---- contraction tiles in fp32 ------------------------------------------------------------------
-// Operand loaders of gemm_ffma.cuh over a layer's matrices.
+// Operand loaders of gemm_ffma.cuh over a layer's matrices, one for each way an operand lies in memory: a loader that chose at run
+// time kept the addresses of every way in registers, and the blocks spilled.
 template <int NR>
-struct WeightRows {           // rows of W: weights, attention keys, or (transposed) attention values
+struct DenseRows {            // rows of k contiguous values, in 16-byte pieces: weights (zero padded to Kpad), keys, queries, tokens
+    const float *base;
+    unsigned rows, k_end, k0;
+    const float *p[NR];
+    __device__ __forceinline__ DenseRows(const float *b, unsigned r, unsigned ke) : base(b), rows(r), k_end(ke), k0(0) {}
+    __device__ __forceinline__ void row(int i, unsigned r, size_t ld) { p[i] = r < rows ? base + (size_t)r * ld : nullptr; }
+    __device__ __forceinline__ void at(unsigned k) { k0 = k; }
+    __device__ __forceinline__ void copy(unsigned dst, int i) const {
+        const bool in = p[i] != nullptr && k0 < k_end;
+        fmablk::copy_async<16>(dst, in ? p[i] + k0 : base, in);
+    }
+};
+template <int NR>
+struct WeightRows : DenseRows<NR> {
+    size_t ld;
+    __device__ __forceinline__ WeightRows(const GemmView &g, unsigned r, unsigned ke) : DenseRows<NR>(g.wbase, r, ke), ld(g.wld) {}
+    __device__ __forceinline__ void row(int i, unsigned r) { DenseRows<NR>::row(i, r, ld); }
+};
+template <int NR>
+struct TokenRows : DenseRows<NR> {
+    size_t ld;
+    __device__ __forceinline__ TokenRows(const LayerDev &, const GemmView &g, unsigned, unsigned cols) : DenseRows<NR>(g.xbase, cols, g.K), ld(g.xld) {}
+    __device__ __forceinline__ void row(int i, unsigned r) { DenseRows<NR>::row(i, r, ld); }
+};
+// n / d for n * d < 2^32: one multiplication (m = 0 stands for d = 1)
+__device__ __forceinline__ unsigned div_magic(unsigned d) { return d == 1u ? 0u : 0xffffffffu / d + 1u; }
+__device__ __forceinline__ unsigned fast_div(unsigned n, unsigned m) { return m ? __umulhi(n, m) : n; }
+template <int NR>
+struct PixelRows {            // taps of output pixels, channels in 16-byte pieces
+    const float *in0;
+    unsigned K, IC, KW, IH, IW, ld0, m_ic, m_kw, pos, cols, k0, ic;
+    int kh, kw;
+    const LayerDev &L;
+    const float *img[NR];     // the pixel's sample; nullptr: no such pixel
+    int y[NR], x[NR];
+    __device__ __forceinline__ PixelRows(const LayerDev &l, const GemmView &g, unsigned po, unsigned c)
+        : in0(l.in0), K(g.K), IC(l.IC), KW(l.KW), IH(l.IH), IW(l.IW), ld0(l.ld0), m_ic(div_magic(l.IC)), m_kw(div_magic(l.KW)), pos(po), cols(c), k0(0), ic(0),
+          kh(0), kw(0), L(l) {}
+    __device__ __forceinline__ void row(int i, unsigned r) {
+        const PixelWin w = pixel_window(L, pos + (r < cols ? r : 0u));
+        img[i] = r < cols ? in0 + (size_t)w.b * IH * IW * ld0 : nullptr;
+        y[i] = w.ih0; x[i] = w.iw0;
+    }
+    __device__ __forceinline__ void at(unsigned k) {
+        k0 = k;
+        const unsigned tap = fast_div(k, m_ic);
+        ic = k - tap * IC;
+        kh = (int)fast_div(tap, m_kw);
+        kw = (int)(tap - (unsigned)kh * KW);
+    }
+    __device__ __forceinline__ void copy(unsigned dst, int i) const {
+        const unsigned ih = (unsigned)(y[i] + kh), iw = (unsigned)(x[i] + kw);       // outside the image: negative or too large
+        const bool in = img[i] != nullptr && k0 < K && ih < IH && iw < IW;
+        fmablk::copy_async<16>(dst, in ? img[i] + (size_t)((ih * IW + iw) * ld0 + ic) : in0, in);
+    }
+};
+// The odd cases, value by value: transposed attention values, channel counts or heads that are no multiple of four.
+template <int NR>
+struct AnyWeightRows {
     const GemmView &g;
-    unsigned rows, k_end;     // rows of the tile, values of k that exist in memory
-    bool vec;
-    unsigned k0, at_row[NR];
+    unsigned rows, k_end, k0, at_row[NR];
     bool ok[NR];
-    __device__ __forceinline__ WeightRows(const GemmView &v, unsigned r, unsigned ke, bool ve) : g(v), rows(r), k_end(ke), vec(ve), k0(0) {}
+    __device__ __forceinline__ AnyWeightRows(const GemmView &v, unsigned r, unsigned ke) : g(v), rows(r), k_end(ke), k0(0) {}
     __device__ __forceinline__ void row(int i, unsigned r) { ok[i] = r < rows; at_row[i] = ok[i] ? r : 0u; }
     __device__ __forceinline__ void at(unsigned k) { k0 = k; }
     __device__ __forceinline__ void copy(unsigned dst, int i) const {
-        if (vec) {
-            const bool in = ok[i] && k0 < k_end;
-            fmablk::copy_async<16>(dst, g.wbase + (in ? (size_t)at_row[i] * g.wld + k0 : 0), in);
-        } else {
-            #pragma unroll
-            for (unsigned e = 0; e < 4; e++) {
-                const bool in = ok[i] && k0 + e < k_end;
-                const size_t off = g.w_transposed ? (size_t)(k0 + e) * g.wld + at_row[i] : (size_t)at_row[i] * g.wld + k0 + e;
-                fmablk::copy_async<4>(dst + e * 4u, g.wbase + (in ? off : 0), in);
-            }
+        #pragma unroll 1
+        for (unsigned e = 0; e < 4; e++) {
+            const bool in = ok[i] && k0 + e < k_end;
+            const size_t off = g.w_transposed ? (size_t)(k0 + e) * g.wld + at_row[i] : (size_t)at_row[i] * g.wld + k0 + e;
+            fmablk::copy_async<4>(dst + e * 4u, g.wbase + (in ? off : 0), in);
         }
     }
 };
 template <int NR>
-struct ActivationRows {       // rows of X: columns of the parent matrix, or the taps of output pixels
+struct AnyRows {
     const LayerDev &L;
     const GemmView &g;
-    unsigned pos, cols;
-    bool vec;
-    unsigned k0, ic;
-    int kh, kw;
-    const float *p[NR];
-    PixelWin pw[NR];
-    bool ok[NR];
-    __device__ __forceinline__ ActivationRows(const LayerDev &l, const GemmView &v, unsigned po, unsigned c, bool ve)
-        : L(l), g(v), pos(po), cols(c), vec(ve), k0(0), ic(0), kh(0), kw(0) {}
-    __device__ __forceinline__ void row(int i, unsigned r) {
-        ok[i] = r < cols;
-        if (g.conv) pw[i] = pixel_window(L, pos + (ok[i] ? r : 0u));
-        else p[i] = g.xbase + (size_t)(ok[i] ? r : 0u) * g.xld;
-    }
-    __device__ __forceinline__ void at(unsigned k) {
-        k0 = k;
-        if (g.conv) { const unsigned tap = k / L.IC; ic = k - tap * L.IC; kh = (int)(tap / L.KW); kw = (int)(tap - (unsigned)kh * L.KW); }
-    }
+    unsigned pos, cols, k0, at_row[NR];
+    __device__ __forceinline__ AnyRows(const LayerDev &l, const GemmView &v, unsigned po, unsigned c) : L(l), g(v), pos(po), cols(c), k0(0) {}
+    __device__ __forceinline__ void row(int i, unsigned r) { at_row[i] = r; }
+    __device__ __forceinline__ void at(unsigned k) { k0 = k; }
     __device__ __forceinline__ void copy(unsigned dst, int i) const {
-        if (vec) {
+        #pragma unroll 1
+        for (unsigned e = 0; e < 4; e++) {
+            const unsigned k = k0 + e;
             const float *src = nullptr;
-            if (ok[i] && k0 < g.K) {
-                if (g.conv) { src = input_pixel(L, pw[i], kh, kw); if (src) src += ic; }
-                else src = p[i] + k0;
+            if (at_row[i] < cols && k < g.K) {
+                if (g.conv) {
+                    const unsigned tap = k / L.IC;
+                    src = input_pixel(L, pixel_window(L, pos + at_row[i]), (int)(tap / L.KW), (int)(tap % L.KW));
+                    if (src) src += k - tap * L.IC;
+                } else src = g.xbase + (size_t)at_row[i] * g.xld + k;
             }
-            fmablk::copy_async<16>(dst, src ? src : L.in0, src != nullptr);
-        } else {
-            unsigned c = ic;
-            int h = kh, w = kw;
-            #pragma unroll
-            for (unsigned e = 0; e < 4; e++) {
-                const float *src = nullptr;
-                if (ok[i] && k0 + e < g.K) {
-                    if (g.conv) { src = input_pixel(L, pw[i], h, w); if (src) src += c; }
-                    else src = p[i] + k0 + e;
-                }
-                fmablk::copy_async<4>(dst + e * 4u, src ? src : L.in0, src != nullptr);
-                if (g.conv && ++c == L.IC) { c = 0; if (++w == (int)L.KW) { w = 0; h++; } }
-            }
+            fmablk::copy_async<4>(dst + e * 4u, src ? src : L.in0, src != nullptr);
         }
     }
 };
@@ -656,21 +686,26 @@ struct StoreTile {
 };
 struct WorkerBarrier { __device__ __forceinline__ void operator()() const { worker_barrier(fmablk::THREADS); } };
 
-template <typename S>
+template <typename S, template <int> class W, template <int> class X>
 static __device__ __noinline__ void ffma_blocks(const LayerDev &L, const TileDev &T, unsigned tid, unsigned char *scratch) {
     const GemmView g = gemm_view(L, T);
     const bool is_k = L.type == K_ATTENTION_LAYER, weights = !is_k && L.type != V_ATTENTION_LAYER;
-    const bool vec_x = L.a_vec4 != 0, vec_w = weights || (is_k && L.a_vec4 != 0);      // weight rows are zero padded to Kpad
+    const unsigned q0 = is_k ? T.pos_w % L.seq : 0u;
     for (unsigned n0 = 0; n0 < T.tile_w; n0 += S::BN)
         for (unsigned m0 = 0; m0 < T.tile_h; m0 += S::BM) {
             GemmView b = g;
             b.wbase += g.w_transposed ? (size_t)m0 : (size_t)m0 * g.wld;
             if (!g.conv) b.xbase += (size_t)n0 * g.xld;
-            WeightRows<S::RW> lw(b, T.tile_h - m0, weights ? L.Kpad : g.K, vec_w);
-            ActivationRows<S::RX> lx(L, b, T.pos_w + n0, T.tile_w - n0, vec_x);
-            StoreTile out{L, T, m0, n0, is_k ? T.pos_w % L.seq : 0u, is_k, is_k ? sqrtf((float)L.hd) : 1.f};
+            W<S::RW> lw(b, T.tile_h - m0, weights ? L.Kpad : g.K);
+            X<S::RX> lx(L, b, T.pos_w + n0, T.tile_w - n0);
+            StoreTile out{L, T, m0, n0, q0, is_k, is_k ? sqrtf((float)L.hd) : 1.f};
             fmablk::block<S>(scratch, tid, g.K, lw, lx, WorkerBarrier(), out);
         }
+}
+template <typename S>
+static __device__ __forceinline__ void ffma_shape(const LayerDev &L, const TileDev &T, unsigned tid, unsigned char *scratch) {
+    if (L.type == CONV_LAYER || L.type == FC_LAYER) ffma_blocks<S, WeightRows, PixelRows>(L, T, tid, scratch);
+    else ffma_blocks<S, WeightRows, TokenRows>(L, T, tid, scratch);
 }
 
 // Tile in fp32 (ref src/tiled_kernels.c:21-490, 784-1038).  FULL: the fp32 mode, 96 KB of staging; the shape of the blocks
@@ -678,10 +713,14 @@ static __device__ __noinline__ void ffma_blocks(const LayerDev &L, const TileDev
 // no TMA box can stage (IC % 32 != 0, head size % 32 != 0, ...).
 template <bool FULL>
 static __device__ void tile_gemm_ffma(const LayerDev &L, const TileDev &T, unsigned tid, unsigned nthr, unsigned char *scratch) {
-    if (!FULL) ffma_blocks<fmablk::Tight>(L, T, tid, scratch);
-    else if (T.tile_h > 64 && T.tile_w > 32) ffma_blocks<fmablk::Large>(L, T, tid, scratch);
-    else if (T.tile_h > 32 && T.tile_w > 32) ffma_blocks<fmablk::Medium>(L, T, tid, scratch);
-    else ffma_blocks<fmablk::Small>(L, T, tid, scratch);
+    const bool pieces = L.a_vec4 != 0 && L.type != V_ATTENTION_LAYER;
+    if (!FULL) {
+        if (pieces) ffma_shape<fmablk::Tight>(L, T, tid, scratch);
+        else ffma_blocks<fmablk::Tight, AnyWeightRows, AnyRows>(L, T, tid, scratch);
+    } else if (!pieces) ffma_blocks<fmablk::Small, AnyWeightRows, AnyRows>(L, T, tid, scratch);
+    else if (T.tile_h > 64 && T.tile_w > 32) ffma_shape<fmablk::Large>(L, T, tid, scratch);
+    else if (T.tile_h > 32 && T.tile_w > 32) ffma_shape<fmablk::Medium>(L, T, tid, scratch);
+    else ffma_shape<fmablk::Small>(L, T, tid, scratch);
     if (L.type == K_ATTENTION_LAYER) {   // normalise every column by its sum (no max subtraction, as the reference)
         const unsigned warp = tid >> 5, lane = tid & 31, nwarp = nthr >> 5;
         for (unsigned n = warp; n < T.tile_w; n += nwarp) {
