@@ -59,6 +59,15 @@ struct Rows {
     }
 };
 
+// The rare activations stay out of line: inlined 32 times their double-precision forms are many times the instruction cache.
+static __device__ __noinline__ float activate_rare(float x, int act) { return activate(x, act); }
+__device__ __forceinline__ float act_value(float x, int act) {
+    if (act == NO_ACTIVATION || act == LINEAR) return x;
+    if (act == RELU) return x > 0.f ? x : 0.f;
+    if (act == GELU) return 0.5f * x * (1.f + erff(x * 0.7071067811865475f));
+    return activate_rare(x, act);
+}
+
 struct Finish {
     const Args &a;
     unsigned m0, n0;
@@ -67,7 +76,7 @@ struct Finish {
         if (n >= a.n_cols || m >= a.m) return;
         float r[4];
         #pragma unroll
-        for (unsigned j = 0; j < 4; j++) r[j] = activate(v[j] + (a.bias && m + j < a.m ? __ldg(a.bias + m + j) : 0.f), a.act);
+        for (unsigned j = 0; j < 4; j++) r[j] = act_value(v[j] + (a.bias && m + j < a.m ? __ldg(a.bias + m + j) : 0.f), a.act);
         float *o = a.out + (size_t)n * a.m + m;
         if (a.vec_out && m + 4u <= a.m) *reinterpret_cast<float4 *>(o) = make_float4(r[0], r[1], r[2], r[3]);
         else
@@ -139,7 +148,7 @@ __global__ void __launch_bounds__(fmablk::THREADS) matmul_rows(const Args a) {
         for (int o = 16; o > 0; o >>= 1) acc[n] += __shfl_xor_sync(0xffffffffu, acc[n], o);
         if ((int)lane == n) mine = acc[n];
     }
-    if (lane < N && lane < a.n_cols) a.out[(size_t)lane * a.m + m] = activate(mine + (a.bias ? __ldg(a.bias + m) : 0.f), a.act);
+    if (lane < N && lane < a.n_cols) a.out[(size_t)lane * a.m + m] = act_value(mine + (a.bias ? __ldg(a.bias + m) : 0.f), a.act);
 }
 
 // Shape with the shortest longest SM: blocks are dealt whole, so an SM runs ceil(blocks / SMs) of them, each

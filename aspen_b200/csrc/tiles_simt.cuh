@@ -82,42 +82,50 @@ __device__ __forceinline__ const float *input_pixel(const LayerDev &L, const Pix
     return L.in0 + ((size_t)(w.b * (int)L.IH + ih) * L.IW + iw) * L.ld0;
 }
 
-// ref src/tiled_kernels.c:613-638.  Pure streaming (12 bytes per element): four independent 16-byte
-// load pairs are in flight per thread before the first use.
-static __device__ __noinline__ void tile_residual(const LayerDev &L, const TileDev &T, unsigned tid, unsigned nthr) {
-    const unsigned h4 = T.tile_h >> 2, tail = T.tile_h & 3;
-    const unsigned total = T.tile_w * h4;
-    constexpr int U = 4;
+// ref src/tiled_kernels.c:613-638.  Pure streaming (12 bytes per element): four independent 16-byte load pairs are in flight per
+// thread before the first use.  ReLU and no activation have loops of their own: with every activation inlined at each element the
+// loop outgrew the instruction cache (256 x 24 elements 9 - 17 us, now 4).
+enum { ACT_NONE = 0, ACT_RELU = 1, ACT_OTHER = 2 };
+template <int KIND>
+static __device__ __noinline__ void residual_loop(const LayerDev &L, const TileDev &T, unsigned tid, unsigned nthr) {
+    const unsigned h4 = T.tile_h >> 2, tail = T.tile_h & 3, tile_w = T.tile_w, pos_w = T.pos_w, pos_h = T.pos_h, total = tile_w * h4;
+    const size_t ld0 = L.ld0, ld1 = L.ld1, ldc = L.ldc;
+    const float *in0 = L.in0, *in1 = L.in1;
+    float *out = L.out;
+    const bool round = L.round_out != 0;
+    const int act = L.act;
+    auto one = [&](float x) {
+        if (KIND == ACT_RELU) x = x > 0.f ? x : 0.f;
+        if (KIND == ACT_OTHER) x = activate(x, act);
+        return round ? tf32_round(x) : x;
+    };
+    constexpr int U = KIND == ACT_OTHER ? 1 : 4;
     for (unsigned i0 = tid; i0 < total; i0 += nthr * U) {
         float4 a[U], b[U];
-        size_t off_o[U];
+        size_t off[U];
         #pragma unroll
         for (int u = 0; u < U; u++) {
-            const unsigned i = i0 + u * nthr;
-            if (i < total) {
-                const unsigned n = i / h4, j = i - n * h4;
-                const size_t col = T.pos_w + n;
-                const unsigned m = T.pos_h + 4 * j;
-                a[u] = ldcg4(L.in0 + col * L.ld0 + m);
-                b[u] = ldcg4(L.in1 + col * L.ld1 + m);
-                off_o[u] = col * L.ldc + m;
-            }
+            const unsigned i = min(i0 + u * nthr, total - 1u), n = i / h4, m = pos_h + 4u * (i - n * h4);
+            const size_t col = pos_w + n;
+            a[u] = ldcg4(in0 + col * ld0 + m);
+            b[u] = ldcg4(in1 + col * ld1 + m);
+            off[u] = col * ldc + m;
         }
         #pragma unroll
-        for (int u = 0; u < U; u++) {
-            if (i0 + u * nthr < total) {
-                float4 o = {finish(a[u].x + b[u].x, L), finish(a[u].y + b[u].y, L), finish(a[u].z + b[u].z, L), finish(a[u].w + b[u].w, L)};
-                *reinterpret_cast<float4 *>(L.out + off_o[u]) = o;
-            }
-        }
+        for (int u = 0; u < U; u++)
+            if (i0 + u * nthr < total)
+                *reinterpret_cast<float4 *>(out + off[u]) = make_float4(one(a[u].x + b[u].x), one(a[u].y + b[u].y), one(a[u].z + b[u].z), one(a[u].w + b[u].w));
     }
-    if (tail) {
-        for (unsigned i = tid; i < T.tile_w * tail; i += nthr) {
-            const unsigned n = i / tail, m = T.pos_h + 4 * h4 + (i - n * tail);
-            const size_t col = T.pos_w + n;
-            L.out[col * L.ldc + m] = finish(ldcg1(L.in0 + col * L.ld0 + m) + ldcg1(L.in1 + col * L.ld1 + m), L);
-        }
+    for (unsigned i = tid; i < tile_w * tail; i += nthr) {
+        const unsigned n = i / tail, m = pos_h + 4u * h4 + (i - n * tail);
+        const size_t col = pos_w + n;
+        out[col * ldc + m] = one(ldcg1(in0 + col * ld0 + m) + ldcg1(in1 + col * ld1 + m));
     }
+}
+static __device__ __forceinline__ void tile_residual(const LayerDev &L, const TileDev &T, unsigned tid, unsigned nthr) {
+    if (L.act == RELU) residual_loop<ACT_RELU>(L, T, tid, nthr);
+    else if (L.act == NO_ACTIVATION || L.act == LINEAR) residual_loop<ACT_NONE>(L, T, tid, nthr);
+    else residual_loop<ACT_OTHER>(L, T, tid, nthr);
 }
 
 // ref src/tiled_kernels.c:411-501.  Max ignores padded taps (all padded -> -inf); average divides by
@@ -652,36 +660,41 @@ struct AnyRows {
         }
     }
 };
+// Activations other than ReLU, and the softmax of the scores, are applied to the stored tile afterwards: inlined for each of a
+// thread's outputs their double-precision forms made the block's code many times the instruction cache.
+__device__ __forceinline__ bool late_activation(const LayerDev &L) {
+    return L.type != V_ATTENTION_LAYER && L.type != K_ATTENTION_LAYER && L.act != NO_ACTIVATION && L.act != LINEAR && L.act != RELU;
+}
+// Bias, ReLU, store of a block's outputs.  Everything it needs is copied here: a load through L, or of a bias that a store
+// might have changed, would wait for the store before it.
 struct StoreTile {
-    const LayerDev &L;
-    const TileDev &T;
-    unsigned m0, n0, q0;
-    bool is_k;
-    float scale;
+    const float *bias;
+    float *out;
+    size_t ldc;
+    unsigned tile_h, tile_w, pos_h, m0, n0;
+    int act;
+    bool round;
+    __device__ __forceinline__ StoreTile(const LayerDev &L, const TileDev &T, unsigned m, unsigned n)
+        : bias(L.type == V_ATTENTION_LAYER || L.type == K_ATTENTION_LAYER ? nullptr : L.bias), out(L.out + (size_t)T.pos_w * L.ldc + T.pos_h), ldc(L.ldc),
+          tile_h(T.tile_h), tile_w(T.tile_w), pos_h(T.pos_h), m0(m), n0(n), act(L.type == V_ATTENTION_LAYER ? (int)NO_ACTIVATION : L.act),
+          round(L.round_out != 0 && L.type != K_ATTENTION_LAYER && !late_activation(L)) {}
     __device__ __forceinline__ void operator()(unsigned mi, unsigned ni, const float *v) const {
         const unsigned m = m0 + mi, n = n0 + ni;
-        if (n >= T.tile_w || m >= T.tile_h) return;
+        if (n >= tile_w || m >= tile_h) return;
         float r[4];
         #pragma unroll
         for (unsigned j = 0; j < 4; j++) {
             float x = v[j];
-            if (is_k) {
-                if (L.masked && T.pos_h + m + j > q0 + n) x = -1e10f;
-                x = expf(x / scale);
-            } else {
-                if (L.type != V_ATTENTION_LAYER) {
-                    if (L.bias && m + j < T.tile_h) x += L.bias[T.pos_h + m + j];
-                    x = activate(x, L.act);
-                }
-                x = store_round(x, L);
-            }
+            if (bias && m + j < tile_h) x += __ldg(bias + pos_h + m + j);
+            if (act == RELU) x = x > 0.f ? x : 0.f;
+            if (round) x = tf32_round(x);
             r[j] = x;
         }
-        float *o = L.out + (size_t)(T.pos_w + n) * L.ldc + T.pos_h + m;
-        if (m + 4u <= T.tile_h && (reinterpret_cast<uintptr_t>(o) & 15u) == 0u) *reinterpret_cast<float4 *>(o) = make_float4(r[0], r[1], r[2], r[3]);
+        float *o = out + (size_t)n * ldc + m;
+        if (m + 4u <= tile_h && (reinterpret_cast<uintptr_t>(o) & 15u) == 0u) *reinterpret_cast<float4 *>(o) = make_float4(r[0], r[1], r[2], r[3]);
         else
             #pragma unroll
-            for (unsigned j = 0; j < 4; j++) if (m + j < T.tile_h) o[j] = r[j];
+            for (unsigned j = 0; j < 4; j++) if (m + j < tile_h) o[j] = r[j];
     }
 };
 struct WorkerBarrier { __device__ __forceinline__ void operator()() const { worker_barrier(fmablk::THREADS); } };
@@ -690,7 +703,6 @@ template <typename S, template <int> class W, template <int> class X>
 static __device__ __noinline__ void ffma_blocks(const LayerDev &L, const TileDev &T, unsigned tid, unsigned char *scratch) {
     const GemmView g = gemm_view(L, T);
     const bool is_k = L.type == K_ATTENTION_LAYER, weights = !is_k && L.type != V_ATTENTION_LAYER;
-    const unsigned q0 = is_k ? T.pos_w % L.seq : 0u;
     for (unsigned n0 = 0; n0 < T.tile_w; n0 += S::BN)
         for (unsigned m0 = 0; m0 < T.tile_h; m0 += S::BM) {
             GemmView b = g;
@@ -698,7 +710,7 @@ static __device__ __noinline__ void ffma_blocks(const LayerDev &L, const TileDev
             if (!g.conv) b.xbase += (size_t)n0 * g.xld;
             W<S::RW> lw(b, T.tile_h - m0, weights ? L.Kpad : g.K);
             X<S::RX> lx(L, b, T.pos_w + n0, T.tile_w - n0);
-            StoreTile out{L, T, m0, n0, q0, is_k, is_k ? sqrtf((float)L.hd) : 1.f};
+            StoreTile out(L, T, m0, n0);
             fmablk::block<S>(scratch, tid, g.K, lw, lx, WorkerBarrier(), out);
         }
 }
@@ -721,14 +733,27 @@ static __device__ void tile_gemm_ffma(const LayerDev &L, const TileDev &T, unsig
     else if (T.tile_h > 64 && T.tile_w > 32) ffma_shape<fmablk::Large>(L, T, tid, scratch);
     else if (T.tile_h > 32 && T.tile_w > 32) ffma_shape<fmablk::Medium>(L, T, tid, scratch);
     else ffma_shape<fmablk::Small>(L, T, tid, scratch);
-    if (L.type == K_ATTENTION_LAYER) {   // normalise every column by its sum (no max subtraction, as the reference)
-        const unsigned warp = tid >> 5, lane = tid & 31, nwarp = nthr >> 5;
-        for (unsigned n = warp; n < T.tile_w; n += nwarp) {
-            float *o = L.out + (size_t)(T.pos_w + n) * L.ldc + T.pos_h;
-            float s = 0.f;
-            for (unsigned m = lane; m < T.tile_h; m += 32) s += ldcg1(o + m);
+    const unsigned tile_h = T.tile_h, tile_w = T.tile_w;
+    float *tile = L.out + (size_t)T.pos_w * L.ldc + T.pos_h;
+    if (L.type == K_ATTENTION_LAYER) {
+        // mask, / sqrt(hd), exp, every column normalised by its sum (no max subtraction, as the reference)
+        const unsigned warp = tid >> 5, lane = tid & 31, nwarp = nthr >> 5, q0 = T.pos_w % L.seq;
+        const float scale = sqrtf((float)L.hd);
+        for (unsigned n = warp; n < tile_w; n += nwarp) {
+            float *o = tile + (size_t)n * L.ldc, s = 0.f;
+            for (unsigned m = lane; m < tile_h; m += 32) {
+                const float x = L.masked && T.pos_h + m > q0 + n ? -1e10f : ldcg1(o + m);
+                s += o[m] = expf(x / scale);
+            }
             s = warp_sum(s);
-            for (unsigned m = lane; m < T.tile_h; m += 32) o[m] = store_round(ldcg1(o + m) / s, L);
+            for (unsigned m = lane; m < tile_h; m += 32) o[m] = store_round(o[m] / s, L);
+        }
+    } else if (late_activation(L)) {
+        const int act = L.act;
+        const size_t ldc = L.ldc;
+        for (unsigned i = tid; i < tile_w * tile_h; i += nthr) {
+            float *o = tile + (size_t)(i / tile_h) * ldc + i % tile_h;
+            *o = store_round(activate(ldcg1(o), act), L);
         }
     }
 }
