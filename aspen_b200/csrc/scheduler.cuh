@@ -228,7 +228,11 @@ static __device__ __noinline__ void worker_tile(const tc::Slot &sl, unsigned wt,
                 else tile_max_small<3, 3, 2>(L, T, wt, tc::NW);
             } else tile_pool<true>(L, T, wt, tc::NW);
             break;
-        case AVGPOOL_LAYER: tile_pool<false>(L, T, wt, tc::NW); break;
+        case AVGPOOL_LAYER:
+            if (((T.tile_h | T.pos_h | L.ld0 | L.ldc) & 3u) == 0u && L.pad == 0u && (L.OH - 1u) * L.stride + L.KH <= L.IH && (L.OW - 1u) * L.stride + L.KW <= L.IW)
+                tile_avg_inside(L, T, wt, tc::NW);
+            else tile_pool<false>(L, T, wt, tc::NW);
+            break;
         case LAYERNORM_LAYER: tile_layernorm(L, T, wt, tc::NW); break;
         case SOFTMAX_LAYER: tile_softmax(L, T, wt, tc::NW); break;
         case YOLO_LAYER: tile_yolo(L, T, wt, tc::NW); break;

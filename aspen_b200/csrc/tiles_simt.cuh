@@ -177,6 +177,35 @@ static __device__ __noinline__ void tile_max_small(const LayerDev &L, const Tile
     }
 }
 
+// Average pooling whose windows lie inside the image (global pools): sixteen taps in flight, summed in order.  Tested tap by tap, a
+// 7 x 7 window took 20 us.
+static __device__ __noinline__ void tile_avg_inside(const LayerDev &L, const TileDev &T, unsigned tid, unsigned nthr) {
+    const unsigned h4 = T.tile_h >> 2, total = T.tile_w * h4, KW = L.KW, taps = L.KH * KW, IW = L.IW;
+    const size_t ld0 = L.ld0;
+    const float inv = 1.f / (float)taps;
+    for (unsigned i = tid; i < total; i += nthr) {
+        const unsigned n = T.pos_w + i / h4, m = T.pos_h + 4u * (i % h4);
+        const PixelWin w = pixel_window(L, n);
+        const float *img = L.in0 + ((size_t)(w.b * (int)L.IH + w.ih0) * IW + w.iw0) * ld0 + m;
+        float4 a = make_float4(0.f, 0.f, 0.f, 0.f);
+        unsigned kw = 0;
+        const float *p = img;
+        for (unsigned t0 = 0; t0 < taps; t0 += 16u) {
+            float4 v[16];
+            #pragma unroll
+            for (unsigned g = 0; g < 16; g++) {
+                v[g] = t0 + g < taps ? ldcg4(p) : make_float4(0.f, 0.f, 0.f, 0.f);
+                p += ld0;
+                if (++kw == KW) { kw = 0; p += (size_t)(IW - KW) * ld0; }
+            }
+            #pragma unroll
+            for (unsigned g = 0; g < 16; g++) { a.x += v[g].x; a.y += v[g].y; a.z += v[g].z; a.w += v[g].w; }
+        }
+        float *o = L.out + (size_t)n * L.ldc + m;
+        *reinterpret_cast<float4 *>(o) = make_float4(finish(a.x * inv, L), finish(a.y * inv, L), finish(a.z * inv, L), finish(a.w * inv, L));
+    }
+}
+
 template <bool IS_MAX>
 static __device__ __noinline__ void tile_pool(const LayerDev &L, const TileDev &T, unsigned tid, unsigned nthr) {
     const unsigned h4 = T.tile_h >> 2, per_col = h4 + (T.tile_h & 3);
