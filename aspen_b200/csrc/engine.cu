@@ -569,6 +569,7 @@ static int build_device_nasm(Engine *e, nasm_t *host_nasm) {
             const int m = add_map(vt, ldt, L.H1, (cuuint64_t)ldt * sizeof(float), L.b_rows, L.per_stage);
             if (m >= 0) {
                 layers[p1].vt_out = vt;
+                L.masked = nasm->ldata[p0].layer->type == K_ATTENTION_LAYER && layers[p0].tc && layers[p0].masked;   // its probabilities after the mask are zeros
                 layers[p1].vt_ld = (unsigned)ldt;
                 layers[p1].vt_seq = L.vt_seq = (unsigned)seqp;
                 L.wmap = m;

@@ -62,11 +62,12 @@ Grid choose(const nasm_ldata_t &ld, const nasm_t *nasm, bool tensor, unsigned sm
                 const unsigned tiles = ceil_div(H, hs[i]) * (W / g.seg) * ceil_div(g.seg, tw);
                 const double us = tile_us(tensor, std::min(hs[i], H), std::min(tw, g.seg), k, served ? 2.5 : 4.0);
                 const double share = (double)tiles / sms;
-                // Passes of other graphs fill the SMs a served layer leaves idle: its work counts, and, because the graphs in
-                // rotation are few, to a lesser degree the length of its longest tile
-                // (0.2 / 0.5 / 1.0 of it: 1.92 / 1.61 / 1.51 ms a request for ResNet-50 x 32 in bursts of twelve, 0.279 / 0.283 / 0.304 for x 4).  A layer launched alone takes as many
-                // rounds as its busiest SM; the last, partly filled one overlaps in part with the next layer.
-                const double cost = served ? us * (share + 0.5) : us * (0.4 * std::max(1.0, share) + 0.6 * ceil_div(tiles, sms));
+                // The layer's work, and the length of its longest tile: launched alone the last tiles of a layer run while the
+                // rest of the chip waits, served the passes of other graphs fill those SMs but the graphs in rotation are few.
+                // (Served, 0.2 / 0.5 / 1.0 tiles: 1.92 / 1.61 / 1.51 ms a request for ResNet-50 x 32 in bursts of twelve, 0.279 /
+                // 0.283 / 0.304 for x 4.  Launched, whole rounds of the SMs instead: GPT-2 8 x 512 2.93 ms, ResNet-50 x 32 1.64;
+                // 0.7 / 1.0 / 1.5 tiles: 2.59 / 2.64 / 3.06 and 1.57 / 1.54 / 1.55.)
+                const double cost = us * (share + (served ? 0.5 : 0.7));
                 if (best == 0 || cost < best * 0.999) { best = cost; g.th = hs[i]; g.tw = tw; }
             }
     } else if (l->type == SOFTMAX_LAYER || l->type == YOLO_LAYER || l->type == APPEND_LAYER) {

@@ -233,11 +233,17 @@ __device__ __forceinline__ unsigned umma_idesc(unsigned n) {
 // fit none of these run as fp32 FMA tiles (tile_gemm_ffma).
 enum { A_NONE = 0, A_TMA = 1, A_ROWS = 2, A_IM2COL = 3 };
 
-struct Origin { int ax, ay, bx, by; };      // box coordinates of column 0 / row 0 of a tile; x in chunks of 32
+// Box coordinates of column 0 / row 0 of a tile (x in chunks of 32), and, for attention values behind a causal mask, the keys its
+// first block of queries can see: the probabilities after them are zeros and are not multiplied.
+struct Origin {
+    int ax, ay, bx, by;
+    unsigned seen;
+    __device__ __forceinline__ unsigned chunks(const LayerDev &L, unsigned n0) const { return seen ? min(L.chunks, (seen + n0 + 31u) >> 5) : L.chunks; }
+};
 
 __device__ __forceinline__ Origin origin(const LayerDev &L, const TileDev &T) {
     Origin g;
-    g.ax = 0; g.ay = (int)T.pos_w; g.bx = 0; g.by = (int)T.pos_h;
+    g.ax = 0; g.ay = (int)T.pos_w; g.bx = 0; g.by = (int)T.pos_h; g.seen = 0;
     if (L.type == K_ATTENTION_LAYER) {
         const unsigned per = L.seq * L.heads, b = T.pos_w / per, r = T.pos_w - b * per, head = r / L.seq, q0 = r - head * L.seq;
         g.ax = g.bx = (int)(head * (L.hd >> 5));
@@ -246,6 +252,7 @@ __device__ __forceinline__ Origin origin(const LayerDev &L, const TileDev &T) {
         const unsigned b = T.pos_w / L.seq, head = T.pos_h / L.hd, q0 = T.pos_w - b * L.seq;
         g.ay = (int)((b * L.heads + head) * L.seq + q0);
         g.bx = (int)(b * (L.vt_seq >> 5));
+        if (L.masked) g.seen = q0 + 128u;
     }
     return g;
 }
@@ -276,9 +283,10 @@ __device__ __forceinline__ bool produce_a(const Slot &sl, unsigned ring, Ring &r
     asm volatile("fence.proxy.async.global;" ::: "memory");
     if (!recut(r, L, sh, ctrl, status)) return false;
     const unsigned kind = L.a_kind, multi = L.a_multi, tile_w = sl.tile.tile_w, tile_h = sl.tile.tile_h, pos_w = sl.tile.pos_w;
-    const unsigned OW = L.OW, OH = L.OH, KW = L.KW, IC = L.IC, PH = L.PH, stride = L.stride, chunks = L.chunks, per = L.per_stage, chunk_bytes = L.a_rows * 128u;
+    const unsigned OW = L.OW, OH = L.OH, KW = L.KW, IC = L.IC, PH = L.PH, stride = L.stride, per = L.per_stage, chunk_bytes = L.a_rows * 128u;
     const int pad = (int)L.pad;
     for (unsigned n0 = 0; n0 < tile_w; n0 += 128u) {
+        const unsigned chunks = g.chunks(L, n0);
         unsigned px = 0, py = 0, pn = 0;             // first output pixel of the block
         if (kind != A_TMA) {
             const unsigned n = pos_w + n0, hw = OH * OW;
@@ -337,10 +345,10 @@ __device__ __forceinline__ bool produce_b(const Slot &sl, unsigned ring, Ring &r
     const unsigned char *map = sl.maps + (size_t)L.wmap * 128;
     asm volatile("fence.proxy.async.global;" ::: "memory");
     if (!recut(r, L, sh, ctrl, status)) return false;
-    const unsigned tile_w = sl.tile.tile_w, tile_h = sl.tile.tile_h, chunks = L.chunks, per = L.per_stage, bytes = per * L.b_rows * 128u, b_off = per * L.a_rows * 128u;
+    const unsigned tile_w = sl.tile.tile_w, tile_h = sl.tile.tile_h, per = L.per_stage, bytes = per * L.b_rows * 128u, b_off = per * L.a_rows * 128u;
     for (unsigned n0 = 0; n0 < tile_w; n0 += 128u)
         for (unsigned mp = 0; mp < tile_h; mp += BLOCK_ROWS)
-            for (unsigned ch = 0; ch < chunks; ch += per) {
+            for (unsigned ch = 0, chunks = g.chunks(L, n0); ch < chunks; ch += per) {
                 if (!mbar_wait(&sh->empty[r.s], r.parity() ^ 1u, ctrl, status, 9)) return false;
                 mbar_arrive_expect_tx(&sh->full[r.s], bytes);
                 tma_load_3d(ring + r.s * r.stage_bytes + b_off, map, 0, g.by + (int)mp, g.bx + (int)ch, &sh->full[r.s]);
@@ -354,7 +362,8 @@ __device__ __forceinline__ bool produce_b(const Slot &sl, unsigned ring, Ring &r
 __device__ __forceinline__ bool issue_mma(const Slot &sl, unsigned ring, Ring &r, unsigned &half, unsigned &acc_uses, Shared *sh, CtrlDev *ctrl, StatusHost *status) {
     const LayerDev &L = sl.layer;
     if (L.stage_bytes != r.stage_bytes) { r.s = 0; r.stage_bytes = L.stage_bytes; r.stages = L.stages; }
-    const unsigned tmem = sh->tmem_base, tile_w = sl.tile.tile_w, tile_h = sl.tile.tile_h, chunks = L.chunks, per = L.per_stage;
+    const unsigned tmem = sh->tmem_base, tile_w = sl.tile.tile_w, tile_h = sl.tile.tile_h, per = L.per_stage;
+    const Origin g = origin(L, sl.tile);
     const unsigned b_off = per * L.a_rows * 128u, a_step = (L.a_rows * 128u) >> 4, b_step = (L.b_rows * 128u) >> 4;
     for (unsigned n0 = 0; n0 < tile_w; n0 += 128u)
         for (unsigned mp = 0; mp < tile_h; mp += BLOCK_ROWS) {
@@ -362,7 +371,7 @@ __device__ __forceinline__ bool issue_mma(const Slot &sl, unsigned ring, Ring &r
             if (!mbar_wait(&sh->acc_empty[half], ((acc_uses >> half) & 1u) ^ 1u, ctrl, status, 6)) return false;
             acc_uses ^= 1u << half;
             tc_fence_after();
-            for (unsigned ch = 0; ch < chunks; ch += per) {
+            for (unsigned ch = 0, chunks = g.chunks(L, n0); ch < chunks; ch += per) {
                 const unsigned n = min(per, chunks - ch), sA = ring + r.s * r.stage_bytes;
                 unsigned alow = umma_desc_low(sA), blow = umma_desc_low(sA + b_off);
                 if (!mbar_wait(&sh->full[r.s], r.parity(), ctrl, status, 3)) return false;
@@ -620,7 +629,7 @@ static __device__ __noinline__ bool softmax_block(const Slot &sl, unsigned n0, u
     const size_t ldc = L.ldc;
     const unsigned lane = threadIdx.x & 31u, warp = (threadIdx.x >> 5) - WARP_WORK, lane0 = (warp & 3u) * 32u, first = warp >> 2;
     const unsigned cols_left = tile_w - n0, n_valid = cols_left > lane0 ? min(32u, cols_left - lane0) : 0u;
-    const unsigned pieces = (tile_h + 31u) >> 5, two = tile_h > BLOCK_ROWS ? 1u : 0u;
+    const unsigned two = tile_h > BLOCK_ROWS ? 1u : 0u;
     float *stage = reinterpret_cast<float *>(epi + warp * 4096u), *other = reinterpret_cast<float *>(epi + (warp ^ 4u) * 4096u);
     float *out = L.out + (size_t)(pos_w + n0 + lane0) * ldc + pos_h;
     const unsigned acc = sh->tmem_base + (lane0 << 16);
@@ -631,7 +640,8 @@ static __device__ __noinline__ bool softmax_block(const Slot &sl, unsigned n0, u
     ok = __all_sync(0xffffffffu, ok);
     tc_fence_after();
     const bool live = ok && n_valid;
-    // rows past the last query of the warp are masked for all its columns: nothing to compute there
+    // Keys past the last query of the warp are masked for all its columns: nothing to compute, and nothing to store -- the matrix
+    // is zero from the start, and nothing else ever writes there.
     const unsigned last = q - lane + 32u, seen = masked ? min(tile_h, last - min(last, pos_h)) : tile_h, seen_pieces = (seen + 31u) >> 5;
     float v[32], sum = 0.f;
     Piece p;
@@ -654,17 +664,12 @@ static __device__ __noinline__ bool softmax_block(const Slot &sl, unsigned n0, u
     worker_sync();
     const float inv_sum = 1.f / sum;
     if (live)
-        for (unsigned c = first; c < pieces; c += 2u) {
-            if (c < seen_pieces) {
-                tmem_ld32(acc + (half ^ (c >> 3)) * BLOCK_ROWS + (c & 7u) * 32u, v);
-                #pragma unroll
-                for (unsigned j = 0; j < 32; j++) v[j] *= inv_sum;
-                transpose(stage, v, p);
-                if (rnd) round_piece(p);
-            } else {
-                #pragma unroll
-                for (unsigned i = 0; i < 8; i++) p.x[i] = make_float4(0.f, 0.f, 0.f, 0.f);
-            }
+        for (unsigned c = first; c < seen_pieces; c += 2u) {
+            tmem_ld32(acc + (half ^ (c >> 3)) * BLOCK_ROWS + (c & 7u) * 32u, v);
+            #pragma unroll
+            for (unsigned j = 0; j < 32; j++) v[j] *= inv_sum;
+            transpose(stage, v, p);
+            if (rnd) round_piece(p);
             store_piece(p, out + c * 32u, ldc, n_valid, min(32u, tile_h - c * 32u));
         }
     tc_fence_before();
