@@ -196,6 +196,7 @@ struct Engine {
     unsigned long long pipe_ns = 1000000000ull;
     unsigned long long launches = 0;
     bool service = false;             // service mode: one kernel serves pass after pass of its graphs until dse_group_stop (see scheduler.cuh)
+    bool uploading = false;           // inputs were copied on the compute stream since a launch or a read
     bool svc_live = false;            // a kernel was launched and has not yet been seen to end
     std::vector<nasm_t *> svc_graphs; // the graphs that kernel serves
     std::vector<nasm_t *> svc_pool;   // every graph of the group's rpool that has a device image: what the next launch serves
@@ -866,6 +867,7 @@ static int svc_launch(Engine *e, const std::vector<nasm_t *> &graphs, bool leave
     CUDA_TRY(cudaGetLastError());
     e->svc_graphs = graphs;
     e->svc_live = true;
+    e->uploading = false;
     return 0;
 }
 
@@ -947,6 +949,20 @@ static int upload_embedding(DeviceDnn *dd, const aspen_dnn_t *dnn) {
     return 0;
 }
 
+// Host to device, complete (or staged by the driver) on return: the caller may reuse its buffer.  With no kernel of the group in
+// flight a pageable source is copied in stream order ahead of the next launch, without waiting for the DMA; otherwise on
+// the transfer stream, beside a running kernel.
+static cudaError_t upload(Engine *e, void *dst, const void *src, size_t bytes) {
+    cudaPointerAttributes attr;
+    const bool pageable = cudaPointerGetAttributes(&attr, src) == cudaSuccess && attr.type == cudaMemoryTypeUnregistered;
+    if (pageable && !e->service && !e->svc_live) {
+        e->uploading = true;
+        return cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, e->stream);
+    }
+    const cudaError_t err = cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, e->io);
+    return err != cudaSuccess ? err : cudaStreamSynchronize(e->io);
+}
+
 // rpool_add_nasm*: uploads (input_host, or ids_host, or neither: zeros; keep_input: what the graph holds) and asks for a pass.
 static int attach(Engine *e, nasm_t *nasm, const void *input_host, const int *ids_host, bool keep_input) {
     CUDA_TRY(cudaSetDevice(e->device));
@@ -983,8 +999,7 @@ static int attach(Engine *e, nasm_t *nasm, const void *input_host, const int *id
             if (!dn->ids_stage) CUDA_TRY(cudaMalloc(&dn->ids_stage, (size_t)l0.out_mat_dims[OUT_W] * sizeof(int)));
             dn->svc_ids = true;
         }
-        CUDA_TRY(cudaMemcpyAsync(dn->ids_stage, ids_host, (size_t)l0.out_mat_dims[OUT_W] * sizeof(int), cudaMemcpyHostToDevice, e->io));
-        CUDA_TRY(cudaStreamSynchronize(e->io));       // the caller may reuse its buffer as soon as we return
+        CUDA_TRY(upload(e, dn->ids_stage, ids_host, (size_t)l0.out_mat_dims[OUT_W] * sizeof(int)));
     } else if (!keep_input) {
         if (dn->svc_ids) { if (svc_halt(e) != 0) return -1; dn->svc_ids = false; }
         if (!input_host) {
@@ -993,8 +1008,7 @@ static int attach(Engine *e, nasm_t *nasm, const void *input_host, const int *id
             CUDA_TRY(cudaMemsetAsync(dst, 0, n * sizeof(float), e->stream));
             CUDA_TRY(cudaStreamSynchronize(e->stream));
         } else {
-            CUDA_TRY(cudaMemcpyAsync(dst, input_host, n * sizeof(float), cudaMemcpyHostToDevice, e->io));
-            CUDA_TRY(cudaStreamSynchronize(e->io));      // the caller may reuse its buffer as soon as we return
+            CUDA_TRY(upload(e, dst, input_host, n * sizeof(float)));
         }
     }
     if (svc_done(dn)) dn->svc_armed++;
@@ -1027,6 +1041,7 @@ long engine_read_ldata(nasm_t *nasm, unsigned int idx, float *out) {
     const size_t n = (size_t)ld.out_mat_dims[OUT_H] * ld.out_mat_dims[OUT_W];
     const float *src = (const float *)((char *)dn->arena + dn->ldata_off[idx]);
     if (!e->service && !svc_done(dn) && svc_serves(e, nasm)) svc_join(e, false);      // the graph is being computed
+    if (e->uploading && !e->svc_live) { cudaStreamSynchronize(e->stream); e->uploading = false; }
     // the copy engine packs strided matrices: a kernel could not start next to a resident one
     const size_t row = (size_t)ld.out_mat_dims[OUT_H] * sizeof(float);
     const bool packed = ld.out_mat_stride == ld.out_mat_dims[OUT_H];

@@ -22,6 +22,7 @@ class HostCopy {
 public:
     static constexpr size_t PIECE = 512u << 10, SLOTS = 16;
     static constexpr size_t MIN_BYTES = 1u << 20;      // below, waking the threads costs more than they save
+    static constexpr size_t SMALL = 256u << 10;        // up to here one pinned buffer and a memcpy (the driver's staging takes 10 us more)
 
     HostCopy() {}
     HostCopy(const HostCopy &) = delete;
@@ -34,6 +35,7 @@ public:
         for (std::thread &t : team_) t.join();
         for (cudaEvent_t e : ev_) if (e) cudaEventDestroy(e);
         if (ring_) cudaFreeHost(ring_);
+        if (small_) cudaFreeHost(small_);
     }
     // Returns once the copy is complete.
     cudaError_t down(void *host, const void *dev, size_t bytes, cudaStream_t st);
@@ -70,7 +72,7 @@ private:
         }
     }
 
-    void *ring_ = nullptr;
+    void *ring_ = nullptr, *small_ = nullptr;
     cudaEvent_t ev_[SLOTS] = {};
     std::vector<std::thread> team_;
     std::mutex m_;
@@ -88,6 +90,12 @@ private:
 inline cudaError_t HostCopy::down(void *host, const void *dev, size_t bytes, cudaStream_t st) {
     cudaPointerAttributes attr;
     const bool pinned = cudaPointerGetAttributes(&attr, host) == cudaSuccess && attr.type != cudaMemoryTypeUnregistered;
+    if (bytes <= SMALL && !pinned && (small_ || cudaHostAlloc(&small_, SMALL, cudaHostAllocDefault) == cudaSuccess)) {
+        cudaError_t e = cudaMemcpyAsync(small_, dev, bytes, cudaMemcpyDeviceToHost, st);
+        if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+        if (e == cudaSuccess) memcpy(host, small_, bytes);
+        return e;
+    }
     if (bytes < MIN_BYTES || pinned || !start()) {
         const cudaError_t e = cudaMemcpyAsync(host, dev, bytes, cudaMemcpyDeviceToHost, st);
         return e != cudaSuccess ? e : cudaStreamSynchronize(st);

@@ -481,19 +481,35 @@ __device__ __forceinline__ GemmView gemm_view(const LayerDev &L, const TileDev &
 static __device__ void tile_input(const InputDev &I, const LayerDev &L, const TileDev &T, unsigned tid, unsigned nthr) {
     const unsigned H = L.H;
     if (I.ids) {
-        const unsigned m4 = T.tile_h >> 2;
-        for (unsigned i = tid; i < T.tile_w * m4; i += nthr) {
-            const unsigned c = i / m4, j = T.pos_h + (i - c * m4) * 4u;
-            const size_t t = T.pos_w + c;
-            int id = __ldcg(I.ids + t);
-            id = id < 0 ? 0 : (id >= (int)I.emb_vocab ? (int)I.emb_vocab - 1 : id);
-            float4 v = __ldg(reinterpret_cast<const float4 *>(I.emb_tok + (size_t)id * H + j));
-            if (I.emb_pos) {
-                const float4 p = __ldg(reinterpret_cast<const float4 *>(I.emb_pos + (size_t)(t % I.emb_seq) * H + j));
-                v.x += p.x; v.y += p.y; v.z += p.z; v.w += p.w;
+        // four pieces of rows in flight: each needs its id first
+        const unsigned m4 = T.tile_h >> 2, total = T.tile_w * m4, pos_w = T.pos_w, pos_h = T.pos_h;
+        const bool round = I.round != 0;
+        const size_t ldc = L.ldc;
+        float *out = L.out;
+        for (unsigned i0 = tid; i0 < total; i0 += 4u * nthr) {
+            unsigned t[4], j[4];
+            int id[4];
+            float4 v[4], p[4];
+            #pragma unroll
+            for (int u = 0; u < 4; u++) {
+                const unsigned i = min(i0 + u * nthr, total - 1u), c = i / m4;
+                t[u] = pos_w + c;
+                j[u] = pos_h + (i - c * m4) * 4u;
+                id[u] = __ldcg(I.ids + t[u]);
             }
-            if (I.round) { v.x = tf32_round(v.x); v.y = tf32_round(v.y); v.z = tf32_round(v.z); v.w = tf32_round(v.w); }
-            *reinterpret_cast<float4 *>(L.out + t * L.ldc + j) = v;
+            #pragma unroll
+            for (int u = 0; u < 4; u++) {
+                id[u] = id[u] < 0 ? 0 : (id[u] >= (int)I.emb_vocab ? (int)I.emb_vocab - 1 : id[u]);
+                v[u] = __ldg(reinterpret_cast<const float4 *>(I.emb_tok + (size_t)id[u] * H + j[u]));
+                if (I.emb_pos) p[u] = __ldg(reinterpret_cast<const float4 *>(I.emb_pos + (size_t)(t[u] % I.emb_seq) * H + j[u]));
+                else p[u] = make_float4(0.f, 0.f, 0.f, 0.f);
+            }
+            #pragma unroll
+            for (int u = 0; u < 4; u++) {
+                if (I.emb_pos) { v[u].x += p[u].x; v[u].y += p[u].y; v[u].z += p[u].z; v[u].w += p[u].w; }
+                if (round) { v[u].x = tf32_round(v[u].x); v[u].y = tf32_round(v[u].y); v[u].z = tf32_round(v[u].z); v[u].w = tf32_round(v[u].w); }
+                if (i0 + u * nthr < total) *reinterpret_cast<float4 *>(out + (size_t)t[u] * ldc + j[u]) = v[u];
+            }
         }
         return;
     }

@@ -1,0 +1,53 @@
+"""Sizes where the kernels' splits change: blocks of the allocation-free matmul, the operand ring's cuts and the tile plan's edges,
+attention over one and two accumulator halves, results that leave through the pinned ring."""
+import numpy as np
+import pytest
+
+import harness
+from aspen_b200 import api, cfgs, weights
+from oracle import port
+from test_zz_no_alloc import oracle_matmul
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("n,k,m", [(1, 1, 1), (2, 130, 33), (4, 128, 9), (8, 257, 64), (9, 31, 32), (33, 1021, 31), (65, 64, 129), (190, 66, 700), (700, 40, 641)])
+@pytest.mark.parametrize("act", [0, 4, 8])
+def test_noalloc_blocks_at_their_edges(n, k, m, act):
+    import torch
+    rng = np.random.default_rng(n * 1000 + k)
+    x = rng.standard_normal((n, k), dtype=np.float32)
+    w = (rng.standard_normal((m, k), dtype=np.float32) / np.sqrt(k)).astype(np.float32)
+    b = rng.standard_normal((m,), dtype=np.float32)
+    xd, wd, bd = (torch.from_numpy(a).cuda() for a in (x, w, b))
+    od = torch.full((n, m), float("nan"), device="cuda")
+    torch.cuda.synchronize()
+    rc = api.lib().aspen_b200_matmul_noalloc(xd.data_ptr(), wd.data_ptr(), bd.data_ptr(), od.data_ptr(), n, k, m, act, None)
+    assert rc == 0, api.last_error()
+    want = oracle_matmul(x, w, b, act)
+    bad, ea, er = harness.compare(od.cpu().numpy(), want, 1e-4, 1e-5 * float(np.abs(want).max()))
+    assert bad == 0, f"{bad} mismatches, max abs {ea:.3e}, max rel {er:.3e}"
+
+
+@pytest.mark.parametrize("name,batch,seq,precision", [("tiny_attn", 1, 1, 0), ("tiny_attn", 3, 33, 0), ("tiny_attn", 1, 129, 0), ("tiny_attn_causal", 2, 255, 0),
+                                                      ("tiny_attn_causal", 1, 257, 0), ("tiny_attn_causal", 1, 300, 1), ("tiny_transformer", 64, 128, 0),
+                                                      ("tiny_cnn", 1, 0, 0), ("tiny_cnn", 33, 0, 0), ("tiny_cnn", 9, 0, 1), ("custom", 1, 0, 0), ("custom", 130, 0, 0),
+                                                      ("custom", 3, 0, 1)])
+def test_every_layer_at_the_edges_of_the_plan(name, batch, seq, precision, workdir):
+    cfg, wf = harness.prepare(name, workdir)
+    dev = harness.Device(cfg, wf, batch, seq, 20, precision, 1)
+    x = harness.make_input(name, dev.input_shape())
+    for _ in range(2):                                        # a second pass over the same memory
+        assert dev.run(x) == 0, api.last_error()
+    kw, scheme, (wseed, _) = harness.NETS[name]
+    text, wl = cfgs.BUILDERS[harness._BUILDER.get(name, name)](**kw)
+    outs = port.run(text, weights.make_weights(wl, wseed, scheme), x, batch, seq)
+    for i in range(1, dev.nasm.num_ldata):
+        got, want = dev.nasm.ldata(i), outs[i]
+        scale = float(np.abs(want).max())
+        if precision == 1:
+            bad, ea, er = harness.compare(got, want, 1e-4, 1e-5 * scale)
+            assert bad == 0, f"layer {i}: {bad} mismatches, max abs {ea:.3e}, max rel {er:.3e}"
+        else:
+            assert float(np.abs(got.astype(np.float64) - want).max()) <= 1e-2 * scale, f"layer {i}"
+    dev.close()
