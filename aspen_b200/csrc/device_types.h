@@ -22,6 +22,8 @@ struct LayerDev {
     unsigned p_out_c, p_in_c, p_stride;                  // yolo / append raw cfg parameters
     const float *anchors;
     unsigned tc;              // the layer's tiles run on the tensor cores
+    unsigned gemv;            // at most 8 columns, each one contiguous run of K values: dot products (tile_gemv)
+    unsigned x_ld;            // ... distance between those columns
     int wmap;                 // tensor map of the W-side operand (weights, PARENT_1 for attention keys, transposed values)
     int amap;                 // tensor map of the X-side operand (PARENT_0 activations)
     unsigned a_kind;          // X operand staging, see tiles_tc.cuh

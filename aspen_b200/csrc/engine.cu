@@ -383,6 +383,10 @@ static void fill_layer(const nasm_t *nasm, const DeviceNasm *dn, unsigned i, int
         case V_ATTENTION_LAYER: L.a_vec4 = (L.seq % 4 == 0) && (L.ld0 % 4 == 0); break;
         default: L.a_vec4 = 0; break;
     }
+    if (gemv_layer(ld) && L.a_vec4 && (l.type != FC_LAYER || L.ld0 == L.IC || L.KH * L.KW == 1)) {
+        L.gemv = 1;
+        L.x_ld = l.type == FC_LAYER ? L.KH * L.KW * L.ld0 : L.ld0;
+    }
 }
 
 static void free_device_nasm(DeviceNasm *dn) {
@@ -496,7 +500,7 @@ static int build_device_nasm(Engine *e, nasm_t *host_nasm) {
         fill_layer(nasm, dn, i, e->precision, L);
         if (nasm->ldata[i].parent_ldata_idx_arr[PARENT_0] != (unsigned)-1 && moved[nasm->ldata[i].parent_ldata_idx_arr[PARENT_0]])
             L.in0 = moved[nasm->ldata[i].parent_ldata_idx_arr[PARENT_0]];
-        if (e->precision != 0) continue;
+        if (e->precision != 0 || L.gemv) continue;
         const bool gemm_w = l.type == CONV_LAYER || l.type == FC_LAYER || l.type == MATMUL_LAYER;
         const unsigned p0 = nasm->ldata[i].parent_ldata_idx_arr[PARENT_0], p1 = nasm->ldata[i].parent_ldata_idx_arr[PARENT_1];
         const cuuint64_t W0 = p0 != (unsigned)-1 ? nasm->ldata[p0].out_mat_dims[OUT_W] : 0;

@@ -170,6 +170,7 @@ nasm_t *nasm_create_tiles(aspen_dnn_t *dnn, unsigned int flop_per_ninst, unsigne
 void graph_find_parents(nasm_t *nasm);
 void graph_set_children(nasm_t *nasm);
 // engine.cu (the only translation unit that touches CUDA)
+bool gemv_layer(const nasm_ldata_t &ld);          // plan.cpp: so few columns that a tile is dot products with whole weight rows
 nasm_t *plan_device_tiles(const nasm_t *nasm, int precision, unsigned int sms, bool served);   // plan.cpp; nullptr: keep the nasm's tiles
 int engine_current_device();
 Engine *engine_create(int device, int precision, unsigned int num_dse_hint);

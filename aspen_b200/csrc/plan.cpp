@@ -47,7 +47,11 @@ Grid choose(const nasm_ldata_t &ld, const nasm_t *nasm, bool tensor, unsigned sm
     const unsigned H = ld.out_mat_dims[OUT_H], W = ld.out_mat_dims[OUT_W];
     Grid g;
     g.seg = W;
-    if (contraction(l->type)) {
+    if (gemv_layer(ld)) {
+        // dot products, a warp a row: two tiles per SM, none smaller than its eight warps' rows, so that every SM fetches weights
+        g.th = (unsigned)round_up(std::min(64u, std::max(8u, ceil_div(H, 2 * sms))), 8);
+        g.tw = W;
+    } else if (contraction(l->type)) {
         const bool ka = l->type == K_ATTENTION_LAYER, va = l->type == V_ATTENTION_LAYER;
         if (ka || va) g.seg = nasm->tr_seq_len;
         unsigned hs[8], nhs = 0;
@@ -88,6 +92,15 @@ Grid choose(const nasm_ldata_t &ld, const nasm_t *nasm, bool tensor, unsigned sm
 }
 
 }  // namespace
+
+// Up to 8 columns a weight is worth at most 8 multiplications a load; beyond, the sums of one row no longer fit the registers beside
+// the loads in flight, and a 32-column MMA tile or fp32 block takes over.
+bool gemv_layer(const nasm_ldata_t &ld) {
+    const unsigned *p = ld.layer->params;
+    const LAYER_TYPE t = ld.layer->type;
+    return ld.out_mat_dims[OUT_W] <= 8 && (t == MATMUL_LAYER || t == FC_LAYER ||
+                                           (t == CONV_LAYER && p[WEIGHT_H] == 1 && p[WEIGHT_W] == 1 && p[STRIDE] <= 1 && p[PADDING] == 0));
+}
 
 nasm_t *plan_device_tiles(const nasm_t *nasm, int precision, unsigned sms, bool served) {
     std::unique_ptr<nasm_t> plan(new nasm_t());
