@@ -649,7 +649,7 @@ def report(args, world, workload, batch, net, ms, max_ms, block_max, e2e_max, se
         "roofline": {"bound": "tensor", "achieved": achieved_tf, "peak": peak_tf, "unit": "TFLOP/s", "frac": achieved_tf / peak_tf,
                      "traffic": TRAFFIC_BYTES_PER_STEP[workload] * args.steps if workload in TRAFFIC_BYTES_PER_STEP else None,
                      "traffic_per_step": TRAFFIC_BYTES_PER_STEP.get(workload), "peak_source": peak_src,
-                     "note": "kernel = persistent scheduler_kernel<true, false, true> (whole tile graphs, all layer types; one launch per timed block); "
+                     "note": "kernel = persistent scheduler_kernel<true> (whole tile graphs, all layer types; one launch per timed block); "
                              "operands are TF32: see peak_tf32"},
     }
     if world == 1 and not args.no_extras:

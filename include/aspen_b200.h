@@ -217,7 +217,7 @@ double aspen_b200_group_time_runs(dse_group_t *dse_group, unsigned int warmup, u
  * that must allocate or free device memory (a graph's first use, its destruction) stop the kernel first and the next
  * run or wait starts it again.  Left idle for 20 ms (ASPEN_B200_IDLE_MS) the kernel leaves by itself.
  * Off by default: each dse_group_run then launches the scheduler for the graphs armed at that moment.
- * Returns 0, or -1 on error.  Graphs that use the fused attention tile are not served in this mode. */
+ * Returns 0, or -1 on error. */
 int aspen_b200_dse_group_set_service(dse_group_t *dse_group, int on);
 
 /* Timed execution in service mode: `passes` passes dealt round robin to the graphs of the group's rpool (inputs as
