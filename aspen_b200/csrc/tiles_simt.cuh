@@ -7,6 +7,7 @@
 #pragma once
 #include "device_types.h"
 #include "gemm_ffma.cuh"
+#include "index_div.h"
 #include "../../include/aspen_b200.h"
 
 // Barrier among the worker threads of a CTA only (the control warp does not take part).
@@ -631,9 +632,6 @@ struct TokenRows : DenseRows<NR> {
     __device__ __forceinline__ TokenRows(const LayerDev &, const GemmView &g, unsigned, unsigned cols) : DenseRows<NR>(g.xbase, cols, g.K), ld(g.xld) {}
     __device__ __forceinline__ void row(int i, unsigned r) { DenseRows<NR>::row(i, r, ld); }
 };
-// n / d for n * d < 2^32: one multiplication (m = 0 stands for d = 1)
-__device__ __forceinline__ unsigned div_magic(unsigned d) { return d == 1u ? 0u : 0xffffffffu / d + 1u; }
-__device__ __forceinline__ unsigned fast_div(unsigned n, unsigned m) { return m ? __umulhi(n, m) : n; }
 template <int NR>
 struct PixelRows {            // taps of output pixels, channels in 16-byte pieces
     const float *in0;
@@ -652,9 +650,9 @@ struct PixelRows {            // taps of output pixels, channels in 16-byte piec
     }
     __device__ __forceinline__ void at(unsigned k) {
         k0 = k;
-        const unsigned tap = fast_div(k, m_ic);
+        const unsigned tap = div_by(k, IC, m_ic);
         ic = k - tap * IC;
-        kh = (int)fast_div(tap, m_kw);
+        kh = (int)div_by(tap, KW, m_kw);
         kw = (int)(tap - (unsigned)kh * KW);
     }
     __device__ __forceinline__ void copy(unsigned dst, int i) const {

@@ -52,3 +52,25 @@ def test_every_layer_at_the_edges_of_the_plan(name, batch, seq, precision, workd
         else:
             assert float(np.abs(got.astype(np.float64) - want).max()) <= 1e-2 * scale, f"layer {i}"
     dev.close()
+
+
+@pytest.mark.parametrize("channels", [200704, 300000])
+def test_connected_layer_over_more_channels_than_a_product_of_indices_can_hold(channels, workdir):
+    """fp32 blocks find the channel of a k by a multiplication; k times the channel count passes 2^32 here.  The last pieces of k
+    carry most of the sum, so one that is taken as lying outside the image shows."""
+    n, m = 9, 16
+    rng = np.random.default_rng(channels)
+    x = rng.standard_normal((n, channels), dtype=np.float32)
+    x[:, -64:] *= 100.0
+    w = (rng.standard_normal((m, channels), dtype=np.float32) / np.sqrt(channels)).astype(np.float32)
+    b = rng.standard_normal((m,), dtype=np.float32)
+    cfg, wf = f"{workdir}/wide_{channels}.cfg", f"{workdir}/wide_{channels}.bin"
+    with open(cfg, "w") as f:
+        f.write(f"[net]\nheight=1\nwidth=1\nchannels={channels}\n\n[connected]\noutput={m}\nactivation=linear\n")
+    weights.write_aspen_data(wf, [(w.reshape(m, channels, 1, 1), b)])
+    dev = harness.Device(cfg, wf, n, 0, 4, precision=1, profile=1)
+    assert dev.run(x) == 0, api.last_error()
+    want = x.astype(np.float64) @ w.astype(np.float64).T + b
+    bad, ea, er = harness.compare(dev.nasm.ldata(1), want, 1e-4, 1e-5 * float(np.abs(want).max()))
+    dev.close()
+    assert bad == 0, f"{bad} mismatches, max abs {ea:.3e}, max rel {er:.3e}"

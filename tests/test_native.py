@@ -1,0 +1,25 @@
+"""Host code of the library that no entry point reaches by itself, compiled into small C++ programs: index arithmetic of the kernels
+over its whole range, and calls of the CUDA runtime or of the C library that fail (fakes of those calls; no GPU is involved)."""
+import os
+import subprocess
+
+
+
+HERE = os.path.dirname(os.path.abspath(__file__))
+LIBDIR = os.path.join(os.path.dirname(HERE), "aspen_b200")
+CUDA_INCLUDE = os.path.join(os.environ.get("CUDA_HOME", "/usr/local/cuda"), "include")
+
+
+def build(name, workdir, *flags):
+    exe = os.path.join(workdir, name)
+    subprocess.run(["g++", "-std=c++17", "-O1", "-Wall", os.path.join(HERE, "native", name + ".cpp"), "-o", exe, *flags], check=True)
+    return exe
+
+
+def passes(exe, *args, timeout=60):
+    r = subprocess.run([exe, *args], capture_output=True, text=True, timeout=timeout)
+    assert r.returncode == 0, r.stdout + r.stderr
+
+
+def test_division_by_multiplication_is_exact(workdir):
+    passes(build("index_div", workdir))
