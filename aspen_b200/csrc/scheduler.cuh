@@ -331,6 +331,7 @@ static __device__ __noinline__ void scheduler_warp(const NasmDev *nasms, CtrlDev
             unsigned ok = lane == 0 ? (unsigned)tc::mbar_test_wait(&sh->finished[k], (retired / tc::SLOTS) & 1u) : 0u;
             ok = __shfl_sync(0xffffffffu, ok, 0);
             if (ok) {
+                __syncwarp();                    // a shuffle orders no memory: what lane 0 has observed holds for the lanes that release it
                 if (my_prof && lane == 0) t_mark = global_ns();
                 const tc::Slot &sl = sh->slots[k];
                 const unsigned g = sl.nasm;
