@@ -14,6 +14,7 @@
 #include <atomic>
 #include <condition_variable>
 #include <cstring>
+#include <exception>
 #include <mutex>
 #include <thread>
 #include <vector>
@@ -41,14 +42,26 @@ public:
     cudaError_t down(void *host, const void *dev, size_t bytes, cudaStream_t st);
 
 private:
+    // The ring counts as there once everything that goes with it is; otherwise what was made is given back, the copy goes through
+    // the driver, and the next large one tries again.
     bool start() {
         if (ring_) return true;
-        if (cudaHostAlloc(&ring_, PIECE * SLOTS, cudaHostAllocDefault) != cudaSuccess) { ring_ = nullptr; cudaGetLastError(); return false; }
-        for (cudaEvent_t &e : ev_)
-            if (cudaEventCreateWithFlags(&e, cudaEventDisableTiming) != cudaSuccess) return false;
-        const unsigned n = std::min(8u, std::max(2u, std::thread::hardware_concurrency() / 2u));
-        for (unsigned i = 0; i < n; i++) team_.emplace_back([this] { loop(); });
-        return true;
+        void *ring = nullptr;
+        size_t made = 0;
+        bool ok = cudaHostAlloc(&ring, PIECE * SLOTS, cudaHostAllocDefault) == cudaSuccess;
+        while (ok && made < SLOTS && (ok = cudaEventCreateWithFlags(&ev_[made], cudaEventDisableTiming) == cudaSuccess)) made++;
+        if (ok) {
+            const unsigned n = std::min(8u, std::max(2u, std::thread::hardware_concurrency() / 2u));
+            try {
+                for (unsigned i = 0; i < n; i++) team_.emplace_back([this] { loop(); });
+            } catch (const std::exception &) {     // no more threads: those that there are do the work
+            }
+            if (!team_.empty()) { ring_ = ring; return true; }
+        }
+        for (size_t i = 0; i < made; i++) { cudaEventDestroy(ev_[i]); ev_[i] = nullptr; }
+        if (ring) cudaFreeHost(ring);
+        cudaGetLastError();
+        return false;
     }
     void loop() {
         for (unsigned seen = 0;;) {

@@ -3,6 +3,8 @@ over its whole range, and calls of the CUDA runtime or of the C library that fai
 import os
 import subprocess
 
+import pytest
+
 
 
 HERE = os.path.dirname(os.path.abspath(__file__))
@@ -16,10 +18,20 @@ def build(name, workdir, *flags):
     return exe
 
 
-def passes(exe, *args, timeout=60):
+def passes(exe, *args, timeout=20):
     r = subprocess.run([exe, *args], capture_output=True, text=True, timeout=timeout)
     assert r.returncode == 0, r.stdout + r.stderr
 
 
 def test_division_by_multiplication_is_exact(workdir):
     passes(build("index_div", workdir))
+
+
+@pytest.fixture(scope="module")
+def host_copy(tmp_path_factory):
+    return build("host_copy", str(tmp_path_factory.mktemp("native")), "-I", CUDA_INCLUDE, "-rdynamic", "-lpthread", "-ldl")
+
+
+@pytest.mark.parametrize("fault", [(), ("event", "1"), ("event", "16"), ("ring",), ("thread", "1"), ("thread", "2")], ids=" ".join)
+def test_results_arrive_whatever_part_of_the_copy_team_cannot_be_made(host_copy, fault):
+    passes(host_copy, *fault)
