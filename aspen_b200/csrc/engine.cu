@@ -303,6 +303,7 @@ Engine *engine_create(int device, int precision, unsigned int /*num_dse_hint*/) 
         if (env_u64("ASPEN_B200_SVC_AHEAD", &v)) e->svc_ahead = (unsigned)v;
         if (env_u64("ASPEN_B200_SERVICE", &v)) e->service = v != 0;      // for programs that cannot call aspen_b200_dse_group_set_service
         if (env_u64("ASPEN_B200_RUN_AHEAD", &v)) e->run_ahead = (unsigned)v;
+        e->copy->prepare(0);
     }
     if (ok && getenv("ASPEN_B200_PROFILE")) {
         size_t bytes = (size_t)e->n_ctas * sched::PROF_SLOTS * sizeof(unsigned long long);
@@ -749,6 +750,8 @@ static int build_device_nasm(Engine *e, nasm_t *host_nasm) {
     const nasm_ldata_t &l0 = nasm->ldata[0];
     if (l0.out_mat_stride != l0.out_mat_dims[OUT_H])
         CUDA_TRY(cudaMalloc(&dn->in_stage, std::max<size_t>((size_t)l0.out_mat_dims[OUT_H] * l0.out_mat_dims[OUT_W], 1) * sizeof(float)));
+    const nasm_ldata_t &last = nasm->ldata[nasm->num_ldata - 1];      // the result, which may be read beside a resident kernel
+    e->copy->prepare((size_t)last.out_mat_dims[OUT_H] * last.out_mat_dims[OUT_W] * sizeof(float));
     NasmDev &H = dn->host;
     memset(&H, 0, sizeof H);
     H.layers = dn->layers; H.tiles = dn->tiles; H.children = dn->children; H.dep = dn->dep; H.wmaps = dn->wmaps;
@@ -1049,6 +1052,9 @@ long engine_read_ldata(nasm_t *nasm, unsigned int idx, float *out) {
     // the copy engine packs strided matrices: a kernel could not start next to a resident one
     const size_t row = (size_t)ld.out_mat_dims[OUT_H] * sizeof(float);
     const bool packed = ld.out_mat_stride == ld.out_mat_dims[OUT_H];
+    // memory for large results is pinned when one is first read with no resident kernel; beside one, dse_get_nasm_result finds what
+    // its graph's image asked for when it was built
+    if (!(e->service && e->svc_live)) e->copy->prepare(n * sizeof(float));
     const cudaError_t err = packed ? e->copy->down(out, src, n * sizeof(float), e->io)
         : cudaMemcpy2DAsync(out, row, src, (size_t)ld.out_mat_stride * sizeof(float), row, ld.out_mat_dims[OUT_W], cudaMemcpyDeviceToHost, e->io);
     if (err != cudaSuccess || (!packed && cudaStreamSynchronize(e->io) != cudaSuccess)) {

@@ -5,8 +5,9 @@
 // a few threads copy (and fault) the pieces that the DMA engine has moved into a pinned ring.
 // B200 host, 16 cores: 12.6 MB into a fresh buffer 1.97 -> 0.57 ms, 6.3 MB 0.91 -> 0.31.  Uploads stay with the driver: it
 // reads resident pages at 13 - 20 GB/s, and the same team filling the ring was no faster.
-// The threads and the ring (8 MB) belong to one engine, are made on its first large result and end with it; an engine's
-// calls come from one host thread.
+// The threads, the ring (8 MB) and the small buffer belong to one engine and end with it; an engine's calls come from one host
+// thread.  Pinned memory is allocated by `prepare`, which the engine calls only while no kernel of it is resident: a copy beside
+// a resident kernel uses what there is, and the driver's staging otherwise.
 #pragma once
 #include <cuda_runtime.h>
 
@@ -37,6 +38,11 @@ public:
         for (cudaEvent_t e : ev_) if (e) cudaEventDestroy(e);
         if (ring_) cudaFreeHost(ring_);
         if (small_) cudaFreeHost(small_);
+    }
+    // Makes what copies of up to `bytes` use.  Nothing is lost if it fails: those copies then go through the driver.
+    void prepare(size_t bytes) {
+        if (!small_ && cudaHostAlloc(&small_, SMALL, cudaHostAllocDefault) != cudaSuccess) { small_ = nullptr; cudaGetLastError(); }
+        if (bytes >= MIN_BYTES) start();
     }
     // Returns once the copy is complete.
     cudaError_t down(void *host, const void *dev, size_t bytes, cudaStream_t st);
@@ -103,13 +109,13 @@ private:
 inline cudaError_t HostCopy::down(void *host, const void *dev, size_t bytes, cudaStream_t st) {
     cudaPointerAttributes attr;
     const bool pinned = cudaPointerGetAttributes(&attr, host) == cudaSuccess && attr.type != cudaMemoryTypeUnregistered;
-    if (bytes <= SMALL && !pinned && (small_ || cudaHostAlloc(&small_, SMALL, cudaHostAllocDefault) == cudaSuccess)) {
+    if (bytes <= SMALL && !pinned && small_) {
         cudaError_t e = cudaMemcpyAsync(small_, dev, bytes, cudaMemcpyDeviceToHost, st);
         if (e == cudaSuccess) e = cudaStreamSynchronize(st);
         if (e == cudaSuccess) memcpy(host, small_, bytes);
         return e;
     }
-    if (bytes < MIN_BYTES || pinned || !start()) {
+    if (bytes < MIN_BYTES || pinned || !ring_) {
         const cudaError_t e = cudaMemcpyAsync(host, dev, bytes, cudaMemcpyDeviceToHost, st);
         return e != cudaSuccess ? e : cudaStreamSynchronize(st);
     }

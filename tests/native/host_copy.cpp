@@ -2,6 +2,7 @@
 //   host_copy event N      the N-th cudaEventCreateWithFlags fails
 //   host_copy ring         cudaHostAlloc fails
 //   host_copy thread N     pthread_create fails from the N-th call on
+//   host_copy resident     nothing was prepared: no copy may allocate
 // Every copy has to end, with the right bytes, and what a failed start has made has to be given back.
 #include "../../aspen_b200/csrc/hostcopy.h"
 
@@ -12,13 +13,14 @@
 #include <cstdlib>
 #include <string>
 
-static int g_event_fails = -1, g_thread_fails = -1, g_events = 0, g_threads = 0, g_live_events = 0, g_live_blocks = 0;
+static int g_event_fails = -1, g_thread_fails = -1, g_events = 0, g_threads = 0, g_live_events = 0, g_live_blocks = 0, g_allocs = 0;
 static bool g_ring_fails = false;
 
 extern "C" {
 cudaError_t cudaHostAlloc(void **p, size_t n, unsigned) {
     if (g_ring_fails && n > HostCopy::SMALL) return cudaErrorMemoryAllocation;
     g_live_blocks++;
+    g_allocs++;
     return (*p = malloc(n)) ? cudaSuccess : cudaErrorMemoryAllocation;
 }
 cudaError_t cudaFreeHost(void *p) { g_live_blocks--; free(p); return cudaSuccess; }
@@ -54,8 +56,11 @@ int main(int argc, char **argv) {
         HostCopy copy;
         for (size_t bytes : {(size_t)1000, HostCopy::SMALL + 4, HostCopy::MIN_BYTES, 40 * HostCopy::PIECE + 12, 3 * HostCopy::PIECE}) {
             std::vector<char> src(bytes), dst(bytes);
+            if (what != "resident") copy.prepare(bytes);
+            const int allocs = g_allocs;
             for (size_t i = 0; i < bytes; i++) src[i] = (char)(i * 2654435761u >> 13);
             if (copy.down(dst.data(), src.data(), bytes, nullptr) != cudaSuccess || src != dst) { printf("copy of %zu bytes is wrong\n", bytes); bad = 1; }
+            if (g_allocs != allocs) { printf("copy of %zu bytes allocates pinned memory\n", bytes); bad = 1; }
         }
     }
     if (g_live_events || g_live_blocks) { printf("%d events and %d blocks are left\n", g_live_events, g_live_blocks); bad = 1; }

@@ -32,6 +32,6 @@ def host_copy(tmp_path_factory):
     return build("host_copy", str(tmp_path_factory.mktemp("native")), "-I", CUDA_INCLUDE, "-rdynamic", "-lpthread", "-ldl")
 
 
-@pytest.mark.parametrize("fault", [(), ("event", "1"), ("event", "16"), ("ring",), ("thread", "1"), ("thread", "2")], ids=" ".join)
+@pytest.mark.parametrize("fault", [(), ("event", "1"), ("event", "16"), ("ring",), ("thread", "1"), ("thread", "2"), ("resident",)], ids=" ".join)
 def test_results_arrive_whatever_part_of_the_copy_team_cannot_be_made(host_copy, fault):
     passes(host_copy, *fault)
