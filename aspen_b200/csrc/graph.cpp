@@ -9,6 +9,7 @@
 #include "internal.h"
 
 #include <algorithm>
+#include <exception>
 #include <thread>
 #include <unordered_set>
 
@@ -266,7 +267,10 @@ void graph_find_parents(nasm_t *nasm) {
     };
     const unsigned int cores = std::min(16u, std::max(1u, std::thread::hardware_concurrency()));
     std::vector<std::thread> team;
-    for (unsigned int i = 1; i < cores && i * run < n; i++) team.emplace_back(work);
+    try {
+        for (unsigned int i = 1; i < cores && i * run < n; i++) team.emplace_back(work);
+    } catch (const std::exception &) {     // no more threads: this one and those that there are do the work
+    }
     work();
     for (std::thread &t : team) t.join();
 }

@@ -5,6 +5,9 @@ import subprocess
 
 import pytest
 
+import harness
+from aspen_b200 import api
+
 
 
 HERE = os.path.dirname(os.path.abspath(__file__))
@@ -35,3 +38,14 @@ def host_copy(tmp_path_factory):
 @pytest.mark.parametrize("fault", [(), ("event", "1"), ("event", "16"), ("ring",), ("thread", "1"), ("thread", "2"), ("resident",)], ids=" ".join)
 def test_results_arrive_whatever_part_of_the_copy_team_cannot_be_made(host_copy, fault):
     passes(host_copy, *fault)
+
+
+def test_a_graph_is_the_same_with_any_number_of_threads(workdir):
+    api.lib()
+    exe = build("few_threads", workdir, "-rdynamic", f"-L{LIBDIR}", "-laspen_b200", f"-Wl,-rpath,{LIBDIR}", "-lpthread", "-ldl")
+    cfg, _ = harness.prepare("custom", workdir)
+    files = [os.path.join(workdir, f"threads_{n}.nasm") for n in (1, 3, 1000)]
+    for n, f in zip((1, 3, 1000), files):
+        passes(exe, str(n), cfg, "16", f)
+    graphs = [open(f, "rb").read() for f in files]
+    assert graphs[0] == graphs[1] == graphs[2] and len(graphs[0]) > 100000
