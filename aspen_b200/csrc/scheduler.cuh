@@ -41,6 +41,7 @@
 // parent's data through the counter's RMW chain) before it publishes or keeps the child.
 #pragma once
 #include "tiles_tc.cuh"
+#include "worker_loop.h"
 
 namespace sched {
 
@@ -462,6 +463,56 @@ static __device__ __forceinline__ void single_thread_role(unsigned char *smem, t
     }
 }
 
+// What a worker warp does at each step of worker_loop.
+template <bool TENSOR_CORES>
+struct WorkerWarp {
+    unsigned char *smem;
+    tc::Shared *sh;
+    CtrlDev *ctrl;
+    StatusHost *status;
+    unsigned long long *prof;
+    unsigned wt;                                 // worker thread 0 .. tc::NW - 1
+    unsigned half = 0, acc_uses = 0;
+    unsigned long long t_mark = 0;
+
+    __device__ __forceinline__ const tc::Slot &slot(unsigned seq) const { return sh->slots[seq % tc::SLOTS]; }
+    __device__ __forceinline__ bool tensor(const tc::Slot &sl) const { return TENSOR_CORES && sl.layer.tc; }
+    __device__ __forceinline__ bool posted(unsigned seq) {
+        if (prof && seq == 0) t_mark = global_ns();
+        return __all_sync(0xffffffffu, wait_posted(&sh->posted[seq % tc::SLOTS], (seq / tc::SLOTS) & 1u, ctrl, status));
+    }
+    __device__ __forceinline__ bool live(unsigned seq) const { return slot(seq).live != 0u; }
+    // the softmax of attention scores, and fp32 blocks
+    __device__ __forceinline__ bool meets(unsigned seq) const {
+        const LayerDev &L = slot(seq).layer;
+        return L.type == K_ATTENTION_LAYER || (!tensor(slot(seq)) && !L.gemv && (L.type == CONV_LAYER || L.type == FC_LAYER || L.type == MATMUL_LAYER || L.type == V_ATTENTION_LAYER));
+    }
+    __device__ __forceinline__ bool agree(bool yes) const {
+        unsigned all;
+        __syncwarp();
+        asm volatile("{\n\t.reg .pred p, q;\n\tsetp.ne.u32 p, %1, 0;\n\tbar.red.and.pred q, 1, %2, p;\n\tselp.u32 %0, 1, 0, q;\n\t}"
+                     : "=r"(all) : "r"(yes ? 1u : 0u), "r"(tc::NW) : "memory");
+        return all != 0u;
+    }
+    __device__ __forceinline__ bool run(unsigned seq) {
+        const tc::Slot &sl = slot(seq);
+        if (prof && wt == 0) { unsigned long long now = global_ns(); prof[PROF_SLOTS - 1] += now - t_mark; t_mark = now; }
+        bool ok = true;
+        if (tensor(sl)) ok = tc::epilogue_tile(sl, half, acc_uses, smem + tc::RING_BYTES, sh, ctrl, status);
+        else worker_tile<TENSOR_CORES>(sl, wt, smem + (TENSOR_CORES ? tc::RING_BYTES : 0u));
+        if (prof && wt == 0) {
+            unsigned long long now = global_ns();
+            const unsigned l = sl.tile.layer % PROF_LAYERS;
+            prof[2 + l] += now - t_mark; prof[2 + PROF_LAYERS + l] += 1ull; t_mark = now;
+        }
+        return ok;
+    }
+    __device__ __forceinline__ void finished(unsigned seq) const {
+        __syncwarp();
+        if ((wt & 31u) == 0u) tc::mbar_arrive(&sh->finished[seq % tc::SLOTS]);      // release (CTA scope): this warp's stores of the tile
+    }
+};
+
 // Registers move from the first warpgroup to the two of workers: 128 x 104 + 256 x 200 = 384 x 168, what the launch holds.
 constexpr int ROLE_REGISTERS = 104, WORKER_REGISTERS = 200;
 static_assert(128 * ROLE_REGISTERS + 256 * WORKER_REGISTERS <= 384 * 168, "register split");
@@ -503,27 +554,8 @@ scheduler_kernel(const NasmDev *nasms, CtrlDev *ctrl, Entry *queue, StatusHost *
     if (warp == sched_warp) {
         scheduler_warp(nasms, ctrl, queue, status, sh, my_prof);
     } else if (warp >= first_worker) {
-        const unsigned wt = tid - first_worker * 32u;
-        unsigned half = 0, acc_uses = 0;
-        unsigned long long t_mark = my_prof ? global_ns() : 0ull;
-        for (unsigned seq = 0;; seq++) {
-            const unsigned k = seq % tc::SLOTS;
-            if (!__all_sync(0xffffffffu, wait_posted(&sh->posted[k], (seq / tc::SLOTS) & 1u, ctrl, status))) break;
-            const tc::Slot &sl = sh->slots[k];
-            if (!sl.live) break;
-            if (my_prof && wt == 0) { unsigned long long now = global_ns(); my_prof[PROF_SLOTS - 1] += now - t_mark; t_mark = now; }
-            bool ok = true;
-            if (TENSOR_CORES && sl.layer.tc) ok = tc::epilogue_tile(sl, half, acc_uses, smem + tc::RING_BYTES, sh, ctrl, status);
-            else worker_tile<TENSOR_CORES>(sl, wt, smem + (TENSOR_CORES ? tc::RING_BYTES : 0u));
-            if (my_prof && wt == 0) {
-                unsigned long long now = global_ns();
-                const unsigned l = sl.tile.layer % PROF_LAYERS;
-                my_prof[2 + l] += now - t_mark; my_prof[2 + PROF_LAYERS + l] += 1ull; t_mark = now;
-            }
-            __syncwarp();
-            if (lane == 0) tc::mbar_arrive(&sh->finished[k]);      // release (CTA scope): this warp's stores of the tile
-            if (!ok) break;
-        }
+        WorkerWarp<TENSOR_CORES> w{smem, sh, ctrl, status, my_prof, tid - first_worker * 32u};
+        worker_loop(w);
     } else if (TENSOR_CORES && lane == 0) {
         if (warp == tc::WARP_A) single_thread_role<tc::WARP_A>(smem, sh, ctrl, status);
         else if (warp == tc::WARP_B) single_thread_role<tc::WARP_B>(smem, sh, ctrl, status);

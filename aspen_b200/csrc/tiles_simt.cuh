@@ -824,8 +824,8 @@ static __device__ void tile_gemm_ffma(const LayerDev &L, const TileDev &T, unsig
     if (L.gemv) { tile_gemv(L, T, tid, nthr); return; }
     const bool pieces = L.a_vec4 != 0 && L.type != V_ATTENTION_LAYER;
     if (!FULL) {
-        // The staging is the epilogue's transposing buffers, one per warp: a warp may still be storing the tensor-core tile before.
-        worker_barrier(nthr);
+        // The staging is the epilogue's transposing buffers, one per warp: a warp may still be storing the tensor-core tile before when
+        // another comes here, and the warps have met since (worker_loop).
         if (pieces) ffma_shape<fmablk::Tight>(L, T, tid, scratch);
         else ffma_blocks<fmablk::Tight, AnyWeightRows, AnyRows>(L, T, tid, scratch);
     } else if (!pieces) ffma_blocks<fmablk::Small, AnyWeightRows, AnyRows>(L, T, tid, scratch);

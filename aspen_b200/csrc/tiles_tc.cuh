@@ -27,7 +27,7 @@
 // wait until the old stages have been read.
 //
 // Every wait is bounded: when a time budget runs out the thread records an error and raises the abort flag, every role
-// leaves its loop, producers let their copies land, and the CTA frees its TMEM and exits.
+// leaves its loop, producers let their copies land, and the CTA frees its TMEM and exits.  (The workers' barriers: worker_loop.h.)
 #pragma once
 #include "tiles_simt.cuh"
 
@@ -621,7 +621,8 @@ __device__ __forceinline__ void worker_sync() { asm volatile("bar.sync 1, %0;" :
 // src/tiled_kernels.c:859-876).  All keys of 128 queries are in TMEM at once: one block, or two (both accumulator halves) for
 // more than 256 keys.  The two warps of a query quarter take alternate pieces and add their sums; the exponentials go back
 // to TMEM, so each is computed once.  `parity`: acc_full parity of each half.
-static __device__ __noinline__ bool softmax_block(const Slot &sl, unsigned n0, unsigned half, unsigned parity, unsigned char *epi, Shared *sh, CtrlDev *ctrl,
+// `ok` false: the warp has given up before; it only meets the others at the barriers.
+static __device__ __noinline__ bool softmax_block(const Slot &sl, unsigned n0, unsigned half, unsigned parity, bool ok, unsigned char *epi, Shared *sh, CtrlDev *ctrl,
                                                   StatusHost *status) {
     const LayerDev &L = sl.layer;
     const unsigned tile_w = sl.tile.tile_w, tile_h = sl.tile.tile_h, pos_w = sl.tile.pos_w, pos_h = sl.tile.pos_h;
@@ -635,7 +636,7 @@ static __device__ __noinline__ bool softmax_block(const Slot &sl, unsigned n0, u
     const unsigned acc = sh->tmem_base + (lane0 << 16);
     const float scale = 1.4426950408889634f / sqrtf((float)L.hd);
     const unsigned q = pos_w % L.seq + n0 + lane0 + lane;
-    bool ok = mbar_wait(&sh->acc_full[half], (parity >> half) & 1u, ctrl, status, 4);
+    ok = ok && mbar_wait(&sh->acc_full[half], (parity >> half) & 1u, ctrl, status, 4);
     if (two) ok = ok && mbar_wait(&sh->acc_full[half ^ 1u], (parity >> (half ^ 1u)) & 1u, ctrl, status, 4);
     ok = __all_sync(0xffffffffu, ok);
     tc_fence_after();
@@ -686,9 +687,10 @@ __device__ __forceinline__ bool epilogue_tile(const Slot &sl, unsigned &half, un
     const unsigned tile_w = sl.tile.tile_w, tile_h = sl.tile.tile_h;
     float *stage = reinterpret_cast<float *>(epi + ((threadIdx.x >> 5) - WARP_WORK) * 4096u);
     const bool softmax = sl.layer.type == K_ATTENTION_LAYER, res = sl.layer.res_out != nullptr;
+    bool ok = true;
     for (unsigned n0 = 0; n0 < tile_w; n0 += 128u) {
         if (softmax) {
-            if (!softmax_block(sl, n0, half, acc_uses, epi, sh, ctrl, status)) return false;
+            ok = softmax_block(sl, n0, half, acc_uses, ok, epi, sh, ctrl, status);
             if (tile_h > BLOCK_ROWS) acc_uses ^= 3u;
             else { acc_uses ^= 1u << half; half ^= 1u; }
             continue;
@@ -701,7 +703,7 @@ __device__ __forceinline__ bool epilogue_tile(const Slot &sl, unsigned &half, un
             half ^= 1u;
         }
     }
-    return true;
+    return ok;
 }
 
 }  // namespace tc

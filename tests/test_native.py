@@ -49,3 +49,8 @@ def test_a_graph_is_the_same_with_any_number_of_threads(workdir):
         passes(exe, str(n), cfg, "16", f)
     graphs = [open(f, "rb").read() for f in files]
     assert graphs[0] == graphs[1] == graphs[2] and len(graphs[0]) > 100000
+
+
+@pytest.mark.parametrize("seed", ["1", "2", "3"])
+def test_every_worker_warp_leaves_whichever_waits_give_up(seed, workdir):
+    passes(build("worker_loop", workdir, "-lpthread"), seed)
