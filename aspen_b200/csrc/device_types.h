@@ -3,6 +3,8 @@
 #pragma once
 #include <cstdint>
 
+#include "index_div.h"
+
 // Layer types / activations use the ABI enum values of include/aspen_b200.h.
 
 struct LayerDev {
@@ -33,6 +35,7 @@ struct LayerDev {
     unsigned chunks;          // 32-deep chunks of the contraction
     unsigned per_stage;       // chunks of one stage of the operand ring
     unsigned stage_bytes, stages;
+    Divisor by_ic, by_kw;     // division by IC, KW
     unsigned a_vec4;          // fp32 tiles: operand rows can be fetched in 16-byte pieces (IC % 4 == 0 ...)
     unsigned round_out;       // store outputs rounded to TF32 (nearest): a tensor-core layer reads them
     unsigned PH;              // A_ROWS: rows per sample of the zero-padded copy of the input image

@@ -373,6 +373,7 @@ static void fill_layer(const nasm_t *nasm, const DeviceNasm *dn, unsigned i, int
     L.KH = p[WEIGHT_H]; L.KW = p[WEIGHT_W]; L.stride = p[STRIDE] ? p[STRIDE] : 1; L.pad = p[PADDING];
     if (l.type == FC_LAYER) { L.KH = p[IN_H]; L.KW = p[IN_W]; L.OH = 1; L.OW = 1; L.stride = 1; L.pad = 0; }
     if (dn->dd->ic_pad[i] && L.ld0 >= dn->dd->ic_pad[i]) { L.IC = dn->dd->ic_pad[i]; L.K = L.KH * L.KW * L.IC; }
+    L.by_ic = make_divisor(L.IC); L.by_kw = make_divisor(L.KW);
     L.seq = nasm->tr_seq_len; L.heads = p[NUM_HEAD]; L.hd = p[NUM_HEAD] ? p[NUM_HIDDEN] / p[NUM_HEAD] : 0; L.masked = p[MASKED];
     L.p_out_c = p[OUT_C]; L.p_in_c = p[IN_C]; L.p_stride = p[STRIDE];
     L.wmap = -1;

@@ -1,4 +1,4 @@
-// Division by a number that is fixed for a whole tile, as one multiplication.
+// Division of an index by a number that is fixed for a layer, as a multiplication and a shift.
 #pragma once
 
 #ifdef __CUDACC__
@@ -7,16 +7,26 @@
 #define INDEX_DIV_FN inline
 #endif
 
-// ceil(2^32 / d); 0 stands for d = 1
-INDEX_DIV_FN unsigned div_magic(unsigned d) { return d == 1u ? 0u : 0xffffffffu / d + 1u; }
+struct Divisor {
+    unsigned magic, shift;      // magic 0: the divisor is 1
+};
 
-// n / d, m = div_magic(d), for every n with n + d < 2^32.  The product's high word is the quotient or, where n times m's rounding
-// passes 2^32 (n * d >= 2^32 at the earliest: a connected layer over more than 65536 channels reaches that), one more.
-INDEX_DIV_FN unsigned div_by(unsigned n, unsigned d, unsigned m) {
-#ifdef __CUDA_ARCH__
-    const unsigned q = m ? __umulhi(n, m) : n;
-#else
-    const unsigned q = m ? (unsigned)(((unsigned long long)n * m) >> 32) : n;
-#endif
-    return q * d > n ? q - 1u : q;
+// With 2^shift < d <= 2^(shift + 1) and magic = ceil(2^(32 + shift) / d), which fits 32 bits, n * magic / 2^(32 + shift) exceeds
+// n / d by less than n / 2^(32 + shift): the quotient is exact while n * d < 2^(32 + shift), that is for every n < 2^31.
+inline Divisor make_divisor(unsigned d) {
+    Divisor v = {0u, 0u};
+    if (d <= 1u) return v;
+    while ((d - 1u) >> (v.shift + 1u)) v.shift++;
+    v.magic = (unsigned)(((1ull << (32u + v.shift)) + d - 1u) / d);
+    return v;
 }
+
+// n / d for d >= 2 (and n < 2^31)
+INDEX_DIV_FN unsigned div_by_2_up(unsigned n, Divisor v) {
+#ifdef __CUDA_ARCH__
+    return __umulhi(n, v.magic) >> v.shift;
+#else
+    return (unsigned)(((unsigned long long)n * v.magic) >> 32) >> v.shift;
+#endif
+}
+INDEX_DIV_FN unsigned div_by(unsigned n, Divisor v) { return v.magic ? div_by_2_up(n, v) : n; }

@@ -7,7 +7,6 @@
 #pragma once
 #include "device_types.h"
 #include "gemm_ffma.cuh"
-#include "index_div.h"
 #include "../../include/aspen_b200.h"
 
 // Barrier among the worker threads of a CTA only (the control warp does not take part).
@@ -635,14 +634,15 @@ struct TokenRows : DenseRows<NR> {
 template <int NR>
 struct PixelRows {            // taps of output pixels, channels in 16-byte pieces
     const float *in0;
-    unsigned K, IC, KW, IH, IW, ld0, m_ic, m_kw, pos, cols, k0, ic;
+    unsigned K, IC, KW, IH, IW, ld0, pos, cols, k0, ic;
+    Divisor by_ic, by_kw;
     int kh, kw;
     const LayerDev &L;
     const float *img[NR];     // the pixel's sample; nullptr: no such pixel
     int y[NR], x[NR];
     __device__ __forceinline__ PixelRows(const LayerDev &l, const GemmView &g, unsigned po, unsigned c)
-        : in0(l.in0), K(g.K), IC(l.IC), KW(l.KW), IH(l.IH), IW(l.IW), ld0(l.ld0), m_ic(div_magic(l.IC)), m_kw(div_magic(l.KW)), pos(po), cols(c), k0(0), ic(0),
-          kh(0), kw(0), L(l) {}
+        : in0(l.in0), K(g.K), IC(l.IC), KW(l.KW), IH(l.IH), IW(l.IW), ld0(l.ld0), pos(po), cols(c), k0(0), ic(0),
+          by_ic(l.by_ic), by_kw(l.by_kw), kh(0), kw(0), L(l) {}
     __device__ __forceinline__ void row(int i, unsigned r) {
         const PixelWin w = pixel_window(L, pos + (r < cols ? r : 0u));
         img[i] = r < cols ? in0 + (size_t)w.b * IH * IW * ld0 : nullptr;
@@ -650,9 +650,9 @@ struct PixelRows {            // taps of output pixels, channels in 16-byte piec
     }
     __device__ __forceinline__ void at(unsigned k) {
         k0 = k;
-        const unsigned tap = div_by(k, IC, m_ic);
+        const unsigned tap = div_by_2_up(k, by_ic);            // whole pieces: at least four channels
         ic = k - tap * IC;
-        kh = (int)div_by(tap, KW, m_kw);
+        kh = (int)div_by(tap, by_kw);
         kw = (int)(tap - (unsigned)kh * KW);
     }
     __device__ __forceinline__ void copy(unsigned dst, int i) const {
