@@ -491,39 +491,44 @@ __device__ __forceinline__ void round_piece(Piece &p) {
     for (unsigned i = 0; i < 8; i++) { p.x[i].x = tf32_round(p.x[i].x); p.x[i].y = tf32_round(p.x[i].y); p.x[i].z = tf32_round(p.x[i].z); p.x[i].w = tf32_round(p.x[i].w); }
 }
 
-// Activations of the tensor-core epilogue: single precision and free of calls (a call would put the epilogue's registers on the
-// stack); the fp32 tiles keep `activate`, which follows the reference's double-precision forms.
-__device__ __forceinline__ float act_fast(float x, int act) {
+// Activations of the tensor-core epilogue.  ReLU, leaky ReLU and the two GELUs are branch-free single precision on the registers.
+__device__ __forceinline__ float act_inline(float x, int act) {
     switch (act) {
         case RELU: return fmaxf(x, 0.f);
         case GELU: return gelu_erf_fast(x);
         case GELU_ACCURATE: return gelu_tanh_fast(x);
-        case LEAKY_RELU: return x > 0.f ? x : 0.1f * x;
-        case ELU: return x > 0.f ? x : 0.1f * (__expf(x) - 1.f);
-        case SELU: return x > 0.f ? 1.0507f * x : 1.0507f * 1.67326f * (__expf(x) - 1.f);
-        case SIGMOID: return __fdividef(1.f, 1.f + __expf(-fmaxf(x, -80.f)));
-        case TANH: return 1.f - __fdividef(2.f, 1.f + __expf(2.f * fminf(fmaxf(x, -15.f), 15.f)));
-        default: return x;   // NO_ACTIVATION, LINEAR
+        default: return x > 0.f ? x : fmaf(x, 0.1f, x * (float)(0.1 - (double)0.1f));   // LEAKY_RELU: 0.1 in two parts, rounded once
     }
 }
 template <int ACT>
 __device__ __forceinline__ void act_piece(Piece &p) {
     #pragma unroll
     for (unsigned i = 0; i < 8; i++) {
-        p.x[i].x = act_fast(p.x[i].x, ACT); p.x[i].y = act_fast(p.x[i].y, ACT); p.x[i].z = act_fast(p.x[i].z, ACT); p.x[i].w = act_fast(p.x[i].w, ACT);
+        p.x[i].x = act_inline(p.x[i].x, ACT); p.x[i].y = act_inline(p.x[i].y, ACT); p.x[i].z = act_inline(p.x[i].z, ACT); p.x[i].w = act_inline(p.x[i].w, ACT);
     }
 }
-__device__ __forceinline__ void activate_piece(Piece &p, int act) {
+// The others are the reference's double-precision forms (`activate`): in single precision exp(x) - 1 cancels.  Their code once, in a
+// loop over the lane's 32 values in its warp's buffer: inlined for each value it would be many times the instruction cache.
+static __device__ __noinline__ void act_buffer(float *mine, int act) {
+    #pragma unroll 1
+    for (unsigned e = 0; e < 32; e++) mine[e * 32u] = activate(mine[e * 32u], act);
+}
+__device__ __forceinline__ void activate_piece(Piece &p, int act, float *stage) {
     switch (act) {
+        case NO_ACTIVATION: case LINEAR: break;
         case RELU: act_piece<RELU>(p); break;
         case GELU: act_piece<GELU>(p); break;
         case GELU_ACCURATE: act_piece<GELU_ACCURATE>(p); break;
         case LEAKY_RELU: act_piece<LEAKY_RELU>(p); break;
-        case ELU: act_piece<ELU>(p); break;
-        case SELU: act_piece<SELU>(p); break;
-        case SIGMOID: act_piece<SIGMOID>(p); break;
-        case TANH: act_piece<TANH>(p); break;
-        default: break;
+        default: {
+            float *mine = stage + (threadIdx.x & 31u);
+            #pragma unroll
+            for (unsigned i = 0; i < 8; i++) { mine[i * 128u] = p.x[i].x; mine[i * 128u + 32u] = p.x[i].y; mine[i * 128u + 64u] = p.x[i].z; mine[i * 128u + 96u] = p.x[i].w; }
+            act_buffer(mine, act);
+            #pragma unroll
+            for (unsigned i = 0; i < 8; i++) p.x[i] = make_float4(mine[i * 128u], mine[i * 128u + 32u], mine[i * 128u + 64u], mine[i * 128u + 96u]);
+            __syncwarp();      // the buffer's next use is another lane's
+        }
     }
 }
 
@@ -580,7 +585,7 @@ static __device__ __noinline__ bool epilogue_block(const Slot &sl, unsigned n0, 
             #pragma unroll
             for (unsigned i = 0; i < 8; i++) { p.x[i].x += b.x; p.x[i].y += b.y; p.x[i].z += b.z; p.x[i].w += b.w; }
             if (bias && c + 2u < pieces) b = load_bias(bias + m0 + m + 64u + quad, (int)(rows - (c + 2u) * 32u) - (int)quad);
-            activate_piece(p, act);
+            activate_piece(p, act, stage);
             if (rnd) round_piece(p);
             if (own) store_piece(p, out + m, ldc, n_valid, valid);
             if (!RES && vt) {
@@ -602,7 +607,7 @@ static __device__ __noinline__ bool epilogue_block(const Slot &sl, unsigned n0, 
                     r.x[i] = r2.x[i];
                 }
                 if (c + 4u < pieces) load_piece(r2, rin + (c + 4u) * 32u, ld_res, n_valid, min(32u, rows - (c + 4u) * 32u));
-                activate_piece(p, act2);
+                activate_piece(p, act2, stage);
                 if (rnd2) round_piece(p);
                 store_piece(p, out2 + m, ld_out2, n_valid, valid);
             }

@@ -74,3 +74,34 @@ def test_connected_layer_over_more_channels_than_a_product_of_indices_can_hold(c
     bad, ea, er = harness.compare(dev.nasm.ldata(1), want, 1e-4, 1e-5 * float(np.abs(want).max()))
     dev.close()
     assert bad == 0, f"{bad} mismatches, max abs {ea:.3e}, max rel {er:.3e}"
+
+
+_ACT64 = {"logistic": lambda x: 1.0 / (1.0 + np.exp(-x)), "tanh": np.tanh, "leaky": lambda x: np.where(x > 0, x, 0.1 * x),
+          "elu": lambda x: np.where(x > 0, x, 0.1 * (np.exp(x) - 1.0)), "selu": lambda x: np.where(x > 0, 1.0507 * x, 1.0507 * 1.67326 * (np.exp(x) - 1.0))}
+
+
+@pytest.mark.parametrize("act", sorted(_ACT64))
+def test_activations_of_the_tensor_core_epilogue_are_rounded_once(act, workdir):
+    """Matmul and fused residual add, outputs from 1e-7 to 10: the activation of what the same network gives with `linear`, in 64 bits,
+    to the last place of fp32 (the reference's double-precision forms, src/naive_kernels.c:11-57)."""
+    d, n = 96, 70
+    rng = np.random.default_rng(31)
+    x = (rng.standard_normal((n, d)) * 10.0 ** rng.uniform(-7, 1, (n, 1))).astype(np.float32)
+    ws = [((rng.standard_normal((d, d)) / np.sqrt(d)).astype(np.float32), np.zeros(d, np.float32)) for _ in range(2)]
+    wf = f"{workdir}/act_{act}.bin"
+    weights.write_aspen_data(wf, ws)
+    outs = []
+    for a in ("linear", act):
+        cfg = f"{workdir}/act_{act}_{a}.cfg"
+        with open(cfg, "w") as f:
+            f.write(f"[net]\nM={d}\nheight=1\nfilters={d}\n\n[matmul]\nM={d}\nactivation={a}\n\n[matmul]\nM={d}\nparent=-2\n\n"
+                    f"[shortcut]\nfrom=-3\nM={d}\nactivation={a}\n\n")
+        dev = harness.Device(cfg, wf, 1, n, 4, 0, 1)
+        assert dev.run(x) == 0, api.last_error()
+        outs.append([dev.nasm.ldata(i).copy() for i in (1, 3)])
+        dev.close()
+    for layer, lin, got in zip((1, 3), *outs):
+        want = _ACT64[act](lin.astype(np.float64))
+        assert float(np.abs(want).max()) > 0
+        off = np.abs(got.astype(np.float64) - want) / np.spacing(np.abs(want).astype(np.float32))
+        assert float(off.max()) <= 1.0, f"layer {layer}: {off.max():.1f} units in the last place at {lin.ravel()[off.argmax()]:.3e}"
