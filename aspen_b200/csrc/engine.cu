@@ -585,7 +585,9 @@ static int build_device_nasm(Engine *e, nasm_t *host_nasm) {
         }
         if (gemm_w && L.a_kind != tc::A_NONE && L.amap >= 0)
             L.wmap = add_map(L.weight, L.Kpad, layer_weight_rows(&l), (cuuint64_t)L.Kpad * sizeof(float), L.b_rows, L.per_stage);
-        L.tc = L.a_kind != tc::A_NONE && L.amap >= 0 && L.wmap >= 0;
+        // the epilogue stores 16-byte pieces: a tile has to start on one (a head of ten features does not)
+        const bool aligned_out = L.ldc % 4 == 0 && (th % 4 == 0 || th >= L.H);
+        L.tc = L.a_kind != tc::A_NONE && L.amap >= 0 && L.wmap >= 0 && aligned_out;
         // ASPEN_B200_ATTN_FUSE=1 with hidden states given up: attention probabilities that only the attention_v layer reads do not
         // stay; every such layer writes the same scratch matrix, which then lives in L2.  The layer's keys have to follow from
         // the attention outputs of the layer before through per-token layers, one of which reads whole columns:
@@ -642,6 +644,7 @@ static int build_device_nasm(Engine *e, nasm_t *host_nasm) {
                 Q.out_mat_dims[OUT_H] != R.out_mat_dims[OUT_H] || Q.out_mat_dims[OUT_W] != R.out_mat_dims[OUT_W])
                 continue;
             LayerDev &L = layers[hi];
+            if ((layers[lo].ldc | layers[i].ldc) % 4 != 0) continue;
             L.res_in = layers[lo].out; L.res_ld_in = layers[lo].ldc;
             L.res_out = layers[i].out; L.res_ld_out = layers[i].ldc;
             L.res_act = layers[i].act; L.res_round = layers[i].round_out;

@@ -88,7 +88,8 @@ __device__ __forceinline__ const float *input_pixel(const LayerDev &L, const Pix
 enum { ACT_NONE = 0, ACT_RELU = 1, ACT_OTHER = 2 };
 template <int KIND>
 static __device__ __noinline__ void residual_loop(const LayerDev &L, const TileDev &T, unsigned tid, unsigned nthr) {
-    const unsigned h4 = T.tile_h >> 2, tail = T.tile_h & 3, tile_w = T.tile_w, pos_w = T.pos_w, pos_h = T.pos_h, total = tile_w * h4;
+    const unsigned h4 = ((T.pos_h | L.ld0 | L.ld1 | L.ldc) & 3u) ? 0u : T.tile_h >> 2, tail = T.tile_h - 4u * h4;      // whole aligned pieces, and the rest
+    const unsigned tile_w = T.tile_w, pos_w = T.pos_w, pos_h = T.pos_h, total = tile_w * h4;
     const size_t ld0 = L.ld0, ld1 = L.ld1, ldc = L.ldc;
     const float *in0 = L.in0, *in1 = L.in1;
     float *out = L.out;
@@ -208,7 +209,7 @@ static __device__ __noinline__ void tile_avg_inside(const LayerDev &L, const Til
 
 template <bool IS_MAX>
 static __device__ __noinline__ void tile_pool(const LayerDev &L, const TileDev &T, unsigned tid, unsigned nthr) {
-    const unsigned h4 = T.tile_h >> 2, per_col = h4 + (T.tile_h & 3);
+    const unsigned h4 = ((T.pos_h | L.ld0 | L.ldc) & 3u) ? 0u : T.tile_h >> 2, per_col = T.tile_h - 3u * h4;   // whole aligned pieces, and the rest
     const float inv = 1.f / (float)(L.KH * L.KW);
     const float init = IS_MAX ? -INFINITY : 0.f;
     const unsigned taps = L.KH * L.KW, total = T.tile_w * per_col;
@@ -292,7 +293,7 @@ static __device__ __noinline__ void tile_layernorm(const LayerDev &L, const Tile
     const unsigned M = T.tile_h;
     const float *gain = L.weight + T.pos_h;
     const float *shift = L.bias ? L.bias + T.pos_h : nullptr;
-    const bool in_regs = M <= 1024u && (M & 3u) == 0u && ((L.ld0 | L.ldc | T.pos_h) & 3u) == 0u;
+    const bool aligned = ((L.ld0 | L.ldc | T.pos_h) & 3u) == 0u, in_regs = aligned && M <= 1024u && (M & 3u) == 0u;
     if (in_regs) {
         // a column of a warp at a time, all its loads (and, once, the gains' and shifts') in flight before the first use; two columns
         // at a time spill
@@ -345,7 +346,7 @@ static __device__ __noinline__ void tile_layernorm(const LayerDev &L, const Tile
         const float *x = L.in0 + (size_t)(T.pos_w + n) * L.ld0 + T.pos_h;
         float *y = L.out + (size_t)(T.pos_w + n) * L.ldc + T.pos_h;
         float s = 0.f, ss = 0.f;
-        const unsigned M4 = M & ~3u;
+        const unsigned M4 = aligned ? M & ~3u : 0u;
         for (unsigned m = lane * 4; m < M4; m += 128) {
             float4 v = ldcg4(x + m);
             s += v.x + v.y + v.z + v.w;

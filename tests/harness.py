@@ -16,6 +16,9 @@ NETS = {
     # head size 32: the smallest the fused attention tile takes (the 4-head variants above have head size 16)
     "tiny_attn": ({"heads": 2}, "n002", (21, 20)),
     "tiny_attn_causal": ({"heads": 2, "masked": True, "pre_ln": True}, "n002", (23, 22)),
+    # heads of 10 and 12 features: tiles of one head's rows do not start on 16-byte boundaries, or only every other one does
+    "tiny_heads10": ({"d": 40, "heads": 4}, "n002", (25, 24)),
+    "tiny_heads12": ({"d": 48, "heads": 4, "masked": True, "pre_ln": True}, "n002", (27, 26)),
     "custom": ({}, "he", (5, 6)),
     "tiny_yolo": ({}, "he", (17, 16)),
     "tiny_acts": ({}, "he", (19, 18)),
@@ -26,7 +29,8 @@ NETS = {
     # GPT-2 with the tail the reference's cfg leaves out: final layernorm and the 50257-row output head
     "gpt2_lm": ({"with_lm_head": True}, "n002", (4, 4)),
 }
-_BUILDER = {"tiny_gpt": "tiny_transformer", "gpt2_lm": "gpt2_124M", "tiny_attn": "tiny_transformer", "tiny_attn_causal": "tiny_transformer"}
+_BUILDER = {"tiny_gpt": "tiny_transformer", "gpt2_lm": "gpt2_124M", "tiny_attn": "tiny_transformer", "tiny_attn_causal": "tiny_transformer",
+            "tiny_heads10": "tiny_transformer", "tiny_heads12": "tiny_transformer"}
 
 
 def prepare(name: str, workdir: str):

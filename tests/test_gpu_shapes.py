@@ -35,8 +35,24 @@ def test_noalloc_blocks_at_their_edges(n, k, m, act):
                                                       ("custom", 3, 0, 1), ("custom", 2, 0, 0), ("custom", 5, 0, 0), ("custom", 8, 0, 0), ("custom", 9, 0, 0),
                                                       ("custom", 8, 0, 1), ("tiny_attn", 1, 7, 1), ("tiny_transformer", 1, 5, 0), ("tiny_cnn", 4, 0, 0)])
 def test_every_layer_at_the_edges_of_the_plan(name, batch, seq, precision, workdir):
+    every_layer_matches(name, batch, seq, precision, 1, workdir)
+
+
+@pytest.mark.parametrize("name,batch,seq", [("tiny_heads10", 2, 40), ("tiny_heads12", 3, 24), ("tiny_heads10", 1, 9), ("tiny_cnn", 2, 0), ("tiny_acts", 3, 0)])
+@pytest.mark.parametrize("precision", [0, 1])
+@pytest.mark.parametrize("plan,quanta", [("1", None), ("0", None), ("0", (10, 12)), ("0", (6, 40))])
+def test_tiles_that_start_anywhere(name, batch, seq, precision, plan, quanta, workdir, monkeypatch):
+    """Heads of ten or twelve features, and graphs executed with their own tiles (ASPEN_B200_PLAN=0) of odd heights: rows and strides that
+    are no multiple of four, in every kind of tile."""
+    monkeypatch.setenv("ASPEN_B200_PLAN", plan)
+    if quanta:
+        api.lib().aspen_b200_set_tile_quanta(*quanta, 100000)
+    every_layer_matches(name, batch, seq, precision, 2 if quanta else 0, workdir)
+
+
+def every_layer_matches(name, batch, seq, precision, profile, workdir):
     cfg, wf = harness.prepare(name, workdir)
-    dev = harness.Device(cfg, wf, batch, seq, 20, precision, 1)
+    dev = harness.Device(cfg, wf, batch, seq, 20, precision, profile)
     x = harness.make_input(name, dev.input_shape())
     for _ in range(2):                                        # a second pass over the same memory
         assert dev.run(x) == 0, api.last_error()
