@@ -68,7 +68,7 @@ def test_tiler_and_graph_match_reference_fixture(path, workdir):
     dnn.close()
 
 
-@pytest.mark.skipif(not os.path.isdir(REFDIR), reason="reference tree not mounted")
+@pytest.mark.skipif(not os.path.isdir(os.path.join(REFDIR, "files")), reason="reference tree not mounted")
 @pytest.mark.parametrize("net,fname", [("resnet50", "resnet50_B2.nasm"), ("resnet50", "resnet50_B4.nasm")])
 def test_shipped_nasm_files_load(net, fname, workdir):
     cfg = os.path.join(workdir, net + "_s.cfg")
@@ -83,7 +83,7 @@ def test_shipped_nasm_files_load(net, fname, workdir):
     dnn.close()
 
 
-@pytest.mark.skipif(not os.path.isdir(REFDIR), reason="reference tree not mounted")
+@pytest.mark.skipif(not os.path.isdir(os.path.join(REFDIR, "files")), reason="reference tree not mounted")
 @pytest.mark.parametrize("net", ["resnet50", "vgg16", "bert_base", "gpt2_124M", "custom"])
 def test_generated_cfg_equals_reference_cfg(net, workdir):
     """The cfg builders stand in for the reference's files/*.cfg on machines without the reference."""
