@@ -7,11 +7,14 @@
 
 // Layer types / activations use the ABI enum values of include/aspen_b200.h.
 
+// How the X operand (activations) of a contraction layer reaches shared memory on the tensor-core path; see tiles_tc.cuh.
+enum { A_NONE = 0, A_TMA = 1, A_IM2COL = 2 };
+
 struct LayerDev {
     int type;                 // LAYER_TYPE
     int act;                  // LAYER_ACT
     float *out;               // own activation matrix: column-major, H rows contiguous, W columns
-    unsigned ldc, H, W;       // column stride (floats), logical rows, columns
+    unsigned ldc, H, W;       // column stride (floats; of every layer a multiple of 4), logical rows, columns
     const float *in0;         // PARENT_0 activations
     unsigned ld0, H0;
     const float *in1;         // PARENT_1 activations
@@ -28,7 +31,7 @@ struct LayerDev {
     unsigned x_ld;            // ... distance between those columns
     int wmap;                 // tensor map of the W-side operand (weights, PARENT_1 for attention keys, transposed values)
     int amap;                 // tensor map of the X-side operand (PARENT_0 activations)
-    unsigned a_kind;          // X operand staging, see tiles_tc.cuh
+    unsigned a_kind;          // A_*
     unsigned a_multi;         // one X box covers all chunks of a stage (the map has a third dimension: the chunk)
     unsigned a_rows;          // columns (MMA rows) of the X-side box: 128, or what a narrow layer has
     unsigned b_rows;          // rows of the W-side box (one per stage): the tile's rows, at most 256
@@ -38,7 +41,8 @@ struct LayerDev {
     Divisor by_ic, by_kw;     // division by IC, KW
     unsigned a_vec4;          // fp32 tiles: operand rows can be fetched in 16-byte pieces (IC % 4 == 0 ...)
     unsigned round_out;       // store outputs rounded to TF32 (nearest): a tensor-core layer reads them
-    unsigned PH;              // A_ROWS: rows per sample of the zero-padded copy of the input image
+    // A_IM2COL: channels of a tap (rounded up to whole chunks), taps of a row, input pixels between two output pixels, padding
+    unsigned tap_c, tap_kw, tap_sx, tap_sy, tap_pad;
     // A residual layer fused into this (convolution / matmul) layer's epilogue: besides its own output the tile
     // also writes res_out = act(own + res_in) for the same region.  res_out == nullptr: nothing fused.
     const float *res_in;
@@ -69,7 +73,7 @@ struct InputDev {
     const int *ids;           // token ids as uploaded (one per column), nullptr otherwise
     const float *emb_tok, *emb_pos;
     unsigned emb_vocab, emb_seq;
-    float *padded;            // zero-padded [sample][PH][PW][4] copy of the image (A_ROWS), nullptr otherwise
+    float *padded;            // zero-padded [sample][PH][PW][4] copy of the image for a convolution on it, nullptr otherwise
     unsigned IC, IH, IW, PH, PW, pad;
     unsigned round;           // values are rounded to TF32 (nearest)
 };

@@ -70,8 +70,8 @@ struct DeviceDnn {
     std::vector<float *> bias;
     std::vector<float *> anchors;
     std::vector<unsigned> kpad;
-    std::vector<float *> weight_rows;   // tensor-core path, input convolutions with <= 4 channels: k = (kh, [kw][4] padded to 32)
-    std::vector<unsigned> ic_pad;     // conv on the network input with IC % 4 != 0: channels padded to this many (0: not padded)
+    std::vector<float *> weight_boxes;  // A_IM2COL layers whose taps are not whole 32-value chunks: every tap zero padded (OperandForm::k)
+    std::vector<unsigned> ic_pad;     // conv on the network input, connected layer, with IC % 4 != 0: channels padded to this many (0: not padded)
     bool have[2] = {false, false};
     float *emb_token = nullptr, *emb_position = nullptr;   // embedding tables, uploaded on first use
 };
@@ -98,7 +98,7 @@ static int upload_weights(aspen_dnn_t *dnn, int device, int precision, DeviceDnn
         dd->anchors.assign(dnn->num_layers, nullptr);
         dd->kpad.assign(dnn->num_layers, 0);
         dd->ic_pad.assign(dnn->num_layers, 0);
-        dd->weight_rows.assign(dnn->num_layers, nullptr);
+        dd->weight_boxes.assign(dnn->num_layers, nullptr);
         dnn->dev[device] = dd;
     }
     *out = dd;
@@ -109,11 +109,11 @@ static int upload_weights(aspen_dnn_t *dnn, int device, int precision, DeviceDnn
         if (w) {
             unsigned rows = layer_weight_rows(&l);
             unsigned k = l.type == LAYERNORM_LAYER ? 1 : layer_contraction_k(&l);
-            // A convolution straight on the network input with an odd channel count (the 3-channel
-            // stem): the input matrix keeps its pad rows zero, so the device copy pads every tap to a
-            // multiple of 4 channels with zero weights and the tile reads 16-byte pieces.
+            // A convolution straight on the network input with an odd channel count (the 3-channel stem), and a connected layer
+            // over padded columns: the parent's pad rows stay zero, so the device copy pads every tap to a multiple of 4 channels
+            // with zero weights and the tile reads 16-byte pieces, or the whole sample as one row.
             unsigned ic = l.params[IN_C], icp = ic;
-            if (l.type == CONV_LAYER && l.parent_layers[PARENT_0] && l.parent_layers[PARENT_0]->type == INPUT_LAYER && ic % 4 != 0) {
+            if (ic % 4 != 0 && (l.type == FC_LAYER || (l.type == CONV_LAYER && l.parent_layers[PARENT_0] && l.parent_layers[PARENT_0]->type == INPUT_LAYER))) {
                 icp = (unsigned)round_up(ic, 4);
                 dd->ic_pad[i] = icp;
             }
@@ -130,18 +130,16 @@ static int upload_weights(aspen_dnn_t *dnn, int device, int precision, DeviceDnn
                 }
             CUDA_TRY(cudaMalloc(&dd->weight[precision][i], padded.size() * sizeof(float) + 256));
             CUDA_TRY(cudaMemcpy(dd->weight[precision][i], padded.data(), padded.size() * sizeof(float), cudaMemcpyHostToDevice));
-            if (precision == 0 && l.type == CONV_LAYER && l.parent_layers[PARENT_0] && l.parent_layers[PARENT_0]->type == INPUT_LAYER && ic <= 4 &&
-                l.params[WEIGHT_W] <= 8 && !dd->weight_rows[i]) {
-                // second copy for the row-box staging: one 32-float chunk per filter row, (kw, channel) inside it
-                const unsigned KH = l.params[WEIGHT_H], KW = l.params[WEIGHT_W];
-                std::vector<float> rowsw((size_t)rows * KH * 32, 0.f);
+            const OperandForm form = operand_form(&l);
+            if (precision == 0 && form.kind == A_IM2COL && (form.image || (ic % 32 != 0 && form.kh * form.kw > 1)) && !dd->weight_boxes[i]) {
+                const unsigned window = k / ic, in_row = form.image ? l.params[WEIGHT_W] : 1, cp = (unsigned)round_up(form.c, 32);
+                std::vector<float> boxes((size_t)rows * form.k(), 0.f);
                 for (unsigned r = 0; r < rows; r++)
-                    for (unsigned kh = 0; kh < KH; kh++)
-                        for (unsigned kw = 0; kw < KW; kw++)
-                            for (unsigned c = 0; c < ic; c++)
-                                rowsw[((size_t)r * KH + kh) * 32 + kw * 4 + c] = round_to_tf32(src[(size_t)r * k + (kh * KW + kw) * ic + c]);
-                CUDA_TRY(cudaMalloc(&dd->weight_rows[i], rowsw.size() * sizeof(float) + 256));
-                CUDA_TRY(cudaMemcpy(dd->weight_rows[i], rowsw.data(), rowsw.size() * sizeof(float), cudaMemcpyHostToDevice));
+                    for (unsigned t = 0; t < window; t++)
+                        for (unsigned c = 0; c < ic; c++)
+                            boxes[(size_t)r * form.k() + t / in_row * cp + t % in_row * 4 + c] = round_to_tf32(src[(size_t)r * k + t * ic + c]);
+                CUDA_TRY(cudaMalloc(&dd->weight_boxes[i], boxes.size() * sizeof(float) + 256));
+                CUDA_TRY(cudaMemcpy(dd->weight_boxes[i], boxes.data(), boxes.size() * sizeof(float), cudaMemcpyHostToDevice));
             }
         }
         if (b && !dd->bias[i]) {
@@ -166,7 +164,7 @@ void engine_release_dnn(aspen_dnn_t *dnn) {
         for (int p = 0; p < 2; p++)
             for (float *ptr : dd->weight[p]) cudaFree(ptr);
         for (float *ptr : dd->bias) cudaFree(ptr);
-        for (float *ptr : dd->weight_rows) cudaFree(ptr);
+        for (float *ptr : dd->weight_boxes) cudaFree(ptr);
         for (float *ptr : dd->anchors) cudaFree(ptr);
         cudaFree(dd->emb_token);
         cudaFree(dd->emb_position);
@@ -210,7 +208,7 @@ struct Engine {
 struct DeviceNasm {
     Engine *e = nullptr;
     DeviceDnn *dd = nullptr;
-    std::unique_ptr<nasm_t> plan;   // the tiles the device executes; empty: the nasm's own
+    std::unique_ptr<nasm_t> plan;   // the tiles the device executes
     float *arena = nullptr;
     size_t arena_bytes = 0;
     std::vector<size_t> ldata_off;
@@ -228,7 +226,7 @@ struct DeviceNasm {
     float *in_stage = nullptr;          // packed input as uploaded (strided layer 0), spread by the layer-0 tiles
     int *ids_stage = nullptr;           // token ids as uploaded
     std::vector<float *> scratch;       // transposed copies of attention value matrices (LayerDev::vt_out), shared probabilities
-    // A_ROWS: zero-padded [sample][PH][PW][4] copy of the input image (borders stay zero), written by the layer-0 tiles
+    // zero-padded [sample][PH][PW][4] copy of the input image (borders stay zero), written by the layer-0 tiles (OperandForm::image)
     float *padded_in = nullptr;
     unsigned pin_ph = 0, pin_pw = 0, pin_pad = 0, pin_ic = 0, pin_ih = 0, pin_iw = 0;
 };
@@ -372,7 +370,7 @@ static void fill_layer(const nasm_t *nasm, const DeviceNasm *dn, unsigned i, int
     L.IC = p[IN_C]; L.IH = p[IN_H]; L.IW = p[IN_W]; L.OH = p[OUT_H]; L.OW = p[OUT_W];
     L.KH = p[WEIGHT_H]; L.KW = p[WEIGHT_W]; L.stride = p[STRIDE] ? p[STRIDE] : 1; L.pad = p[PADDING];
     if (l.type == FC_LAYER) { L.KH = p[IN_H]; L.KW = p[IN_W]; L.OH = 1; L.OW = 1; L.stride = 1; L.pad = 0; }
-    if (dn->dd->ic_pad[i] && L.ld0 >= dn->dd->ic_pad[i]) { L.IC = dn->dd->ic_pad[i]; L.K = L.KH * L.KW * L.IC; }
+    if (dn->dd->ic_pad[i]) { L.IC = dn->dd->ic_pad[i]; L.K = L.KH * L.KW * L.IC; }
     L.by_ic = make_divisor(L.IC); L.by_kw = make_divisor(L.KW);
     L.seq = nasm->tr_seq_len; L.heads = p[NUM_HEAD]; L.hd = p[NUM_HEAD] ? p[NUM_HIDDEN] / p[NUM_HEAD] : 0; L.masked = p[MASKED];
     L.p_out_c = p[OUT_C]; L.p_in_c = p[IN_C]; L.p_stride = p[STRIDE];
@@ -413,7 +411,7 @@ static bool follows(const nasm_t *nasm, unsigned i, unsigned from, bool whole) {
 }
 
 // The graph as the device executes it: layer geometry (strides, tiles) and lists.
-static const nasm_t *device_view(const nasm_t *nasm) { return nasm->dev->plan ? nasm->dev->plan.get() : nasm; }
+static const nasm_t *device_view(const nasm_t *nasm) { return nasm->dev->plan.get(); }
 
 static int build_device_nasm(Engine *e, nasm_t *host_nasm) {
     DeviceNasm *dn = new DeviceNasm();
@@ -421,7 +419,8 @@ static int build_device_nasm(Engine *e, nasm_t *host_nasm) {
     host_nasm->dev = dn;
     const char *keep_tiles = getenv("ASPEN_B200_PLAN");      // 0: execute the nasm's own tiles
     if (host_nasm->own_lists && !(keep_tiles && atoi(keep_tiles) == 0)) dn->plan.reset(plan_device_tiles(host_nasm, e->precision, e->n_ctas, e->service));
-    const nasm_t *nasm = device_view(host_nasm);
+    if (!dn->plan) dn->plan.reset(own_device_tiles(host_nasm));
+    const nasm_t *nasm = dn->plan.get();
     if (upload_weights(nasm->dnn, e->device, e->precision, &dn->dd) != 0) return -1;
     // activation arena: one region per layer (no reuse: every layer output stays readable)
     dn->ldata_off.resize(nasm->num_ldata);
@@ -453,45 +452,25 @@ static int build_device_nasm(Engine *e, nasm_t *host_nasm) {
     };
     // The X operand by plain boxes: the chunks of a stage in one where the matrix allows it.
     auto add_x_map = [&](LayerDev &L, const void *base, cuuint64_t inner, cuuint64_t outer, cuuint64_t stride_bytes) {
-        L.a_kind = tc::A_TMA;
+        L.a_kind = A_TMA;
         L.a_multi = inner % 32 == 0;
         L.amap = add_map(base, inner, outer, stride_bytes, L.a_rows, L.a_multi ? L.per_stage : 0);
     };
-    // 3-D map of the padded input copy: (32 floats of a row, output pixel = `stride` input pixels apart, row)
-    // Eight consecutive maps, the j-th with a box of 16 j pixels.  Returns the index of the first, or -2 when the driver
-    // does not take such (overlapping) maps: the layer then keeps the gather.
-    auto add_rows_map = [&](const void *base, unsigned OW, unsigned stride, unsigned PW, cuuint64_t rows_total) -> int {
-        const size_t first = maps.size();
-        for (unsigned j = 1; j <= 8; j++) {
-            CUtensorMap m;
-            cuuint64_t dims[3] = {32, OW, rows_total};
-            cuuint64_t strides[2] = {(cuuint64_t)stride * 16, (cuuint64_t)PW * 16};
-            cuuint32_t box[3] = {32, std::min(16 * j, OW), 1}, estr[3] = {1, 1, 1};
-            CUresult r = get_encode_fn()(&m, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3, const_cast<void *>(base), dims, strides, box, estr,
-                                         CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                                         CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-            if (r != CUDA_SUCCESS) { maps.resize(first); return -2; }
-            maps.push_back(m);
-        }
-        return (int)first;
-    };
-    // im2col map of a convolution's parent matrix: (channel, iw, ih, sample), boxes of 32 channels x 128 (a_rows) output pixels.  The
-    // corners bound the first tap of the first and last output pixel; the strides are the convolution's.
-    auto add_im2col_map = [&](const LayerDev &L) -> int {
+    // im2col map: (channel, column, row, sample) with those extents and distances in floats, boxes of 32 channels x a_rows output pixels.
+    // The corners bound the first tap of the first and last output pixel; sx, sy: input pixels between two output pixels.
+    auto add_im2col_map = [&](const float *base, const unsigned (&extent)[4], const size_t (&ld)[3], int lower, int upper_x, int upper_y, unsigned sx, unsigned sy,
+                              unsigned a_rows) -> int {
         CUtensorMap m;
-        const int pad = (int)L.pad;
-        cuuint64_t dims[4] = {L.IC, L.IW, L.IH, nasm->batch_size};
-        cuuint64_t strides[3] = {(cuuint64_t)L.ld0 * 4, (cuuint64_t)L.IW * L.ld0 * 4, (cuuint64_t)L.IH * L.IW * L.ld0 * 4};
-        int lower[2] = {-pad, -pad}, upper[2] = {pad - (int)L.KW + 1, pad - (int)L.KH + 1};
-        cuuint32_t estr[4] = {1, L.stride, L.stride, 1};
-        CUresult r = get_encode_im2col_fn()(&m, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, const_cast<float *>(L.in0), dims, strides, lower, upper, 32, L.a_rows, estr,
+        cuuint64_t dims[4] = {extent[0], extent[1], extent[2], extent[3]}, strides[3] = {ld[0] * 4, ld[1] * 4, ld[2] * 4};
+        int low[2] = {lower, lower}, up[2] = {upper_x, upper_y};
+        cuuint32_t estr[4] = {1, sx, sy, 1};
+        CUresult r = get_encode_im2col_fn()(&m, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, const_cast<float *>(base), dims, strides, low, up, 32, a_rows, estr,
                                             CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                                             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-        if (r != CUDA_SUCCESS) return -2;
+        if (r != CUDA_SUCCESS) { ASPEN_ERR("cuTensorMapEncodeIm2col failed (%d)\n", (int)r); return -2; }
         maps.push_back(m);
         return (int)maps.size() - 1;
     };
-    const char *no_rows = getenv("ASPEN_B200_NO_ROW_BOXES");
     float *probs = nullptr;                                    // see K_ATTENTION below
     size_t probs_bytes = 0;
     unsigned probs_reader = 0;
@@ -519,53 +498,44 @@ static int build_device_nasm(Engine *e, nasm_t *host_nasm) {
             L.stages = std::min(tc::MAX_STAGES, tc::RING_BYTES / L.stage_bytes);
         };
         if (gemm_w || l.type == K_ATTENTION_LAYER || l.type == V_ATTENTION_LAYER) cut_ring(l.type == K_ATTENTION_LAYER ? L.hd : l.type == V_ATTENTION_LAYER ? L.seq : L.Kpad);
-        // Row-box staging of an input convolution (see tiles_tc.cuh, A_ROWS): decided first, it changes the
-        // weight layout the weight map is made from.
-        bool rows_kind = false;
-        if (l.type == CONV_LAYER && p0 == 0 && dn->dd->weight_rows[i] && !dn->padded_in && !(no_rows && atoi(no_rows) != 0) &&
-            L.OW % 16 == 0 && nasm->ldata[i].out_mat_dims[OUT_W] % 128 == 0 && nasm->ldata[i].ninst_tile_dims[OUT_W] % 128 == 0) {
-            const unsigned s_ = L.stride, pad = L.pad;
-            const unsigned PW = std::max(L.IW + 2 * pad, s_ * (L.OW - 1) + 8), PH = std::max(L.IH + 2 * pad, s_ * (L.OH - 1) + L.KH);
-            const size_t bytes = (size_t)nasm->batch_size * PH * PW * 4 * sizeof(float);
-            CUDA_TRY(cudaMalloc(&dn->padded_in, bytes + 256));
-            CUDA_TRY(cudaMemsetAsync(dn->padded_in, 0, bytes + 256, e->stream));
-            const int m = add_rows_map(dn->padded_in, L.OW, s_, PW, (cuuint64_t)nasm->batch_size * PH);
-            if (m >= 0) {
-                dn->pin_ph = PH; dn->pin_pw = PW; dn->pin_pad = pad; dn->pin_ic = l.params[IN_C]; dn->pin_ih = L.IH; dn->pin_iw = L.IW;
-                rows_kind = true;
-                L.a_kind = tc::A_ROWS;
-                L.amap = m;
-                L.PH = PH;
-                L.weight = dn->dd->weight_rows[i];
-                L.Kpad = L.KH * 32;
-                L.K = L.Kpad;
-                cut_ring(L.Kpad);
+        const OperandForm form = operand_form(&l);
+        const float *dense = L.weight;
+        const unsigned dense_kpad = L.Kpad;
+        if (form.kind == A_IM2COL && L.H0 == l.params[IN_C]) {
+            if (dn->dd->weight_boxes[i]) { L.weight = dn->dd->weight_boxes[i]; L.Kpad = form.k(); }
+            cut_ring(L.Kpad);
+            L.a_kind = A_IM2COL;
+            L.tap_c = (unsigned)round_up(form.c, 32);
+            L.tap_kw = form.kw;
+            L.tap_sy = L.stride;
+            if (form.image) {
+                // the padded copy as a tensor whose columns are output columns: a row of the window is 4 * KW consecutive values
+                const unsigned s_ = L.stride, PW = std::max(L.IW + 2 * L.pad, s_ * (L.OW - 1) + L.KW), PH = std::max(L.IH + 2 * L.pad, s_ * (L.OH - 1) + L.KH);
+                const size_t bytes = (size_t)nasm->batch_size * PH * PW * 4 * sizeof(float);
+                CUDA_TRY(cudaMalloc(&dn->padded_in, bytes + 256));
+                CUDA_TRY(cudaMemsetAsync(dn->padded_in, 0, bytes + 256, e->stream));
+                dn->pin_ph = PH; dn->pin_pw = PW; dn->pin_pad = L.pad; dn->pin_ic = l.params[IN_C]; dn->pin_ih = L.IH; dn->pin_iw = L.IW;
+                L.tap_sx = 1; L.tap_pad = 0;
+                L.amap = add_im2col_map(dn->padded_in, {form.c, L.OW, s_ * (L.OH - 1) + L.KH, nasm->batch_size}, {(size_t)s_ * 4, (size_t)PW * 4, (size_t)PH * PW * 4},
+                                        0, 0, 1 - (int)L.KH, 1, s_, L.a_rows);
             } else {
-                cudaFree(dn->padded_in);
-                dn->padded_in = nullptr;
+                L.tap_sx = L.stride; L.tap_pad = L.pad;
+                L.amap = add_im2col_map(L.in0, {form.c, L.IW, L.IH, nasm->batch_size}, {L.ld0, (size_t)L.IW * L.ld0, (size_t)L.IH * L.IW * L.ld0}, -(int)L.pad,
+                                        (int)L.pad - (int)L.KW + 1, (int)L.pad - (int)L.KH + 1, L.stride, L.stride, L.a_rows);
             }
-        }
-        const bool aligned0 = L.ld0 % 4 == 0;
-        if (rows_kind) {
-            // X operand set above
-        } else if (l.type == MATMUL_LAYER && aligned0) {
+            if (L.amap < 0) return -1;
+        } else if (form.kind == A_TMA && (l.type == MATMUL_LAYER || l.type == CONV_LAYER)) {
             add_x_map(L, L.in0, L.H0, W0, (cuuint64_t)L.ld0 * sizeof(float));
-        } else if (l.type == CONV_LAYER && aligned0 && L.KH == 1 && L.KW == 1 && L.stride == 1 && L.pad == 0) {
-            add_x_map(L, L.in0, L.H0, W0, (cuuint64_t)L.ld0 * sizeof(float));
-        } else if (l.type == CONV_LAYER && aligned0 && L.IC % 32 == 0 && L.IC == L.H0 && L.KH * L.KW * L.IC == L.K && L.stride <= 8 && L.KH <= 64 && L.KW <= 64 &&
-                   L.pad < L.KH && L.pad < L.KW) {
-            L.amap = add_im2col_map(L);
-            if (L.amap >= 0) L.a_kind = tc::A_IM2COL;
-        } else if (l.type == FC_LAYER && L.ld0 == L.IC && L.K % 4 == 0) {
-            // a sample's NHWC activations are one contiguous row of K values
+        } else if (l.type == FC_LAYER && (L.ld0 == L.IC || L.KH * L.KW == 1)) {
+            // a sample's NHWC activations are one contiguous row of K values (own tiles may leave more rows between its columns)
             add_x_map(L, L.in0, L.K, nasm->batch_size, (cuuint64_t)L.IH * L.IW * L.ld0 * sizeof(float));
         } else if (l.type == K_ATTENTION_LAYER) {
             // all keys of a query must fit the accumulators (512 columns); larger sequences run as fp32 tiles
-            if (L.hd % 32 == 0 && L.H0 % 32 == 0 && L.H1 % 32 == 0 && aligned0 && L.ld1 % 4 == 0 && L.seq <= tc::TMEM_COLS && th >= L.seq) {
+            if (L.hd % 32 == 0 && L.H0 % 32 == 0 && L.H1 % 32 == 0 && L.seq <= tc::TMEM_COLS && th >= L.seq) {
                 add_x_map(L, L.in0, L.H0, W0, (cuuint64_t)L.ld0 * sizeof(float));
                 L.wmap = add_map(L.in1, L.H1, nasm->ldata[p1].out_mat_dims[OUT_W], (cuuint64_t)L.ld1 * sizeof(float), L.b_rows, L.per_stage);
             }
-        } else if (l.type == V_ATTENTION_LAYER && aligned0 && p1 != (unsigned)-1 && p1 < i && p1 != 0 && layers[p1].tc && !layers[p1].vt_out) {
+        } else if (l.type == V_ATTENTION_LAYER && p1 != (unsigned)-1 && p1 < i && p1 != 0 && layers[p1].tc && !layers[p1].vt_out) {
             // The value operand W(m, k) = V[token k][feature m] is the transpose of how the value projection stores its
             // output; that projection, a tensor-core layer of this graph, writes a second, transposed copy into scratch memory.
             const size_t seqp = round_up(L.seq, 32), ldt = seqp * nasm->batch_size;
@@ -583,11 +553,12 @@ static int build_device_nasm(Engine *e, nasm_t *host_nasm) {
                 add_x_map(L, L.in0, L.H0, W0, (cuuint64_t)L.ld0 * sizeof(float));
             }
         }
-        if (gemm_w && L.a_kind != tc::A_NONE && L.amap >= 0)
+        if (gemm_w && L.a_kind != A_NONE && L.amap >= 0)
             L.wmap = add_map(L.weight, L.Kpad, layer_weight_rows(&l), (cuuint64_t)L.Kpad * sizeof(float), L.b_rows, L.per_stage);
         // the epilogue stores 16-byte pieces: a tile has to start on one (a head of ten features does not)
-        const bool aligned_out = L.ldc % 4 == 0 && (th % 4 == 0 || th >= L.H);
-        L.tc = L.a_kind != tc::A_NONE && L.amap >= 0 && L.wmap >= 0 && aligned_out;
+        const bool aligned_out = th % 4 == 0 || th >= L.H;
+        L.tc = L.a_kind != A_NONE && L.amap >= 0 && L.wmap >= 0 && aligned_out;
+        if (!L.tc) { L.weight = dense; L.Kpad = dense_kpad; }       // fp32 blocks walk the taps as they are
         // ASPEN_B200_ATTN_FUSE=1 with hidden states given up: attention probabilities that only the attention_v layer reads do not
         // stay; every such layer writes the same scratch matrix, which then lives in L2.  The layer's keys have to follow from
         // the attention outputs of the layer before through per-token layers, one of which reads whole columns:
@@ -644,7 +615,6 @@ static int build_device_nasm(Engine *e, nasm_t *host_nasm) {
                 Q.out_mat_dims[OUT_H] != R.out_mat_dims[OUT_H] || Q.out_mat_dims[OUT_W] != R.out_mat_dims[OUT_W])
                 continue;
             LayerDev &L = layers[hi];
-            if ((layers[lo].ldc | layers[i].ldc) % 4 != 0) continue;
             L.res_in = layers[lo].out; L.res_ld_in = layers[lo].ldc;
             L.res_out = layers[i].out; L.res_ld_out = layers[i].ldc;
             L.res_act = layers[i].act; L.res_round = layers[i].round_out;

@@ -171,7 +171,16 @@ void graph_find_parents(nasm_t *nasm);
 void graph_set_children(nasm_t *nasm);
 // engine.cu (the only translation unit that touches CUDA)
 bool gemv_layer(const nasm_ldata_t &ld);          // plan.cpp: so few columns that a tile is dot products with whole weight rows
+// How TMA boxes find the operands of a contraction layer, from its shape alone (plan.cpp).  A_NONE: they do not, its tiles run in fp32.
+struct OperandForm {
+    unsigned kind = 0;             // A_* (device_types.h)
+    bool image = false;            // convolution on an image of at most 4 channels: a row of the window is one tap of 4 * width "channels"
+    unsigned c = 0, kh = 1, kw = 1;
+    unsigned k() const { return kh * kw * (unsigned)round_up(c, 32); }      // A_IM2COL: k of the weights, every tap in whole chunks
+};
+OperandForm operand_form(const aspen_layer_t *l);
 nasm_t *plan_device_tiles(const nasm_t *nasm, int precision, unsigned int sms, bool served);   // plan.cpp; nullptr: keep the nasm's tiles
+nasm_t *own_device_tiles(const nasm_t *nasm);      // plan.cpp: the nasm's tiles, columns a multiple of 16 bytes apart
 int engine_current_device();
 Engine *engine_create(int device, int precision, unsigned int num_dse_hint);
 void engine_destroy(Engine *e);

@@ -8,6 +8,7 @@
 // with the parents each tile reads (by region, so a graph of ten thousand tiles takes milliseconds).
 // Graphs whose lists a file has changed keep their own tiles and lists.
 #include "internal.h"
+#include "device_types.h"
 
 #include <algorithm>
 #include <memory>
@@ -100,6 +101,50 @@ bool gemv_layer(const nasm_ldata_t &ld) {
     const LAYER_TYPE t = ld.layer->type;
     return ld.out_mat_dims[OUT_W] <= 8 && (t == MATMUL_LAYER || t == FC_LAYER ||
                                            (t == CONV_LAYER && p[WEIGHT_H] == 1 && p[WEIGHT_W] == 1 && p[STRIDE] <= 1 && p[PADDING] == 0));
+}
+
+OperandForm operand_form(const aspen_layer_t *l) {
+    const unsigned *p = l->params;
+    OperandForm f;
+    f.c = p[IN_C];
+    switch (l->type) {
+        case MATMUL_LAYER: case FC_LAYER: case K_ATTENTION_LAYER: case V_ATTENTION_LAYER: f.kind = A_TMA; break;
+        case CONV_LAYER: {
+            const unsigned stride = p[STRIDE] ? p[STRIDE] : 1;
+            if (p[WEIGHT_H] == 1 && p[WEIGHT_W] == 1 && stride == 1 && p[PADDING] == 0) { f.kind = A_TMA; break; }
+            // limits of an im2col tensor map; a window that lies in the padding alone is left out
+            if (stride > 8 || p[WEIGHT_H] > 64 || p[WEIGHT_W] > 64 || p[PADDING] >= p[WEIGHT_H] || p[PADDING] >= p[WEIGHT_W]) break;
+            f.kind = A_IM2COL;
+            f.kh = p[WEIGHT_H]; f.kw = p[WEIGHT_W];
+            // one convolution of a network reads the image that way (there is one padded copy): the first
+            const aspen_layer_t *first = l->dnn->layers.data(), *in = l->parent_layers[PARENT_0];
+            f.image = in && in->type == INPUT_LAYER && p[IN_C] <= 4;
+            for (; first < l; first++)
+                if (first->type == CONV_LAYER && first->parent_layers[PARENT_0] == in && operand_form(first).image) f.image = false;
+            if (f.image) { f.c = 4 * f.kw; f.kw = 1; }
+            break;
+        }
+        default: break;
+    }
+    return f;
+}
+
+nasm_t *own_device_tiles(const nasm_t *nasm) {
+    nasm_t *own = new nasm_t();
+    own->dnn = nasm->dnn;
+    own->batch_size = nasm->batch_size;
+    own->tr_seq_len = nasm->tr_seq_len;
+    own->num_ldata = nasm->num_ldata;
+    own->num_ninst = nasm->num_ninst;
+    own->ldata = nasm->ldata;
+    own->ninst = nasm->ninst;
+    for (nasm_ldata_t &ld : own->ldata) {
+        ld.nasm = own;
+        ld.out_mat_stride = (unsigned)round_up(ld.out_mat_stride, 4);
+        ld.out_mat_mem_size = std::max(ld.out_mat_mem_size, (size_t)ld.out_mat_stride * ld.out_mat_dims[OUT_W] * sizeof(float));
+    }
+    for (ninst_t &ni : own->ninst) ni.ldata = own->ldata.data() + (ni.ldata - nasm->ldata.data());
+    return own;
 }
 
 nasm_t *plan_device_tiles(const nasm_t *nasm, int precision, unsigned sms, bool served) {

@@ -220,18 +220,17 @@ __device__ __forceinline__ unsigned umma_idesc(unsigned n) {
 
 
 // How the X operand of a layer reaches shared memory (chosen on the host, LayerDev::a_kind):
-//   A_TMA      one 32 x 128 box per k-chunk straight from the parent's [columns][rows] matrix: matmul, 1x1 stride-1
-//              convolution, attention, connected layers over an unpadded parent
-//   A_IM2COL   any convolution with IC % 32 == 0: TMA im2col boxes.  The parent is a (channel, iw, ih, sample) tensor; one
-//              chunk is 32 channels of one tap for 128 consecutive output pixels, wherever they cross the end of an image row
-//              or of a sample; taps outside the image arrive as zeros.  No im2col matrix exists.
-//   A_ROWS     convolution on the network input with <= 4 channels (the 7x7 stem): the input is kept as a zero-padded
-//              [sample][row][pixel][4] copy, the k axis is (kh, [kw][4] padded to 32), so one k-chunk of an output pixel
-//              is ONE contiguous 128-byte run of an input row, and 16 j consecutive output pixels of a row are a 3-D box
+//   A_TMA      boxes straight from the parent's [columns][rows] matrix: matmul, 1x1 stride-1 convolution, attention, connected
+//              layers over an unpadded parent.  One box per k-chunk, or per stage where the map has the chunk as a third dimension
+//   A_IM2COL   any other convolution: TMA im2col boxes.  The parent is a (channel, iw, ih, sample) tensor; one chunk is 32
+//              channels of one tap for 128 consecutive output pixels, wherever they cross the end of an image row or of a
+//              sample; taps outside the image and channels past the last arrive as zeros (the weights hold every tap in whole
+//              chunks).  No im2col matrix exists.  A connected layer over padded columns is a window as large as its image.
+//              A convolution on an image of at most 4 channels (the 7x7 stem) reads a zero-padded [sample][row][pixel][4] copy of
+//              it: a row of the window is 4 * KW consecutive floats there, the tensor's columns are the output's (a stride apart,
+//              overlapping), and KH rows of 28 floats take 7 chunks where 49 taps of 3 channels would take 49.
 // The W operand -- weights, attention keys (PARENT_1's matrix) or the transposed copy of the attention values -- arrives in one
-// box per stage; so does X where its map has the chunk as a third dimension (A_TMA over a multiple of 32).  Layers that
-// fit none of these run as fp32 FMA tiles (tile_gemm_ffma).
-enum { A_NONE = 0, A_TMA = 1, A_ROWS = 2, A_IM2COL = 3 };
+// box per stage.  Layers that fit none of these run as fp32 FMA tiles (tile_gemm_ffma).
 
 // Box coordinates of column 0 / row 0 of a tile (x in chunks of 32), and, for attention values behind a causal mask, the keys its
 // first block of queries can see: the probabilities after them are zeros and are not multiplied.
@@ -282,13 +281,14 @@ __device__ __forceinline__ bool produce_a(const Slot &sl, unsigned ring, Ring &r
     // activations were written with ordinary (generic proxy) stores; TMA reads them through the async proxy
     asm volatile("fence.proxy.async.global;" ::: "memory");
     if (!recut(r, L, sh, ctrl, status)) return false;
-    const unsigned kind = L.a_kind, multi = L.a_multi, tile_w = sl.tile.tile_w, tile_h = sl.tile.tile_h, pos_w = sl.tile.pos_w;
-    const unsigned OW = L.OW, OH = L.OH, KW = L.KW, IC = L.IC, PH = L.PH, stride = L.stride, per = L.per_stage, chunk_bytes = L.a_rows * 128u;
-    const int pad = (int)L.pad;
+    const bool im2col = L.a_kind == A_IM2COL;
+    const unsigned multi = L.a_multi, tile_w = sl.tile.tile_w, tile_h = sl.tile.tile_h, pos_w = sl.tile.pos_w;
+    const unsigned OW = L.OW, OH = L.OH, KW = L.tap_kw, C = L.tap_c, sx = L.tap_sx, sy = L.tap_sy, per = L.per_stage, chunk_bytes = L.a_rows * 128u;
+    const int pad = (int)L.tap_pad;
     for (unsigned n0 = 0; n0 < tile_w; n0 += 128u) {
         const unsigned chunks = g.chunks(L, n0);
         unsigned px = 0, py = 0, pn = 0;             // first output pixel of the block
-        if (kind != A_TMA) {
+        if (im2col) {
             const unsigned n = pos_w + n0, hw = OH * OW;
             pn = n / hw;
             const unsigned q = n - pn * hw;
@@ -306,30 +306,18 @@ __device__ __forceinline__ bool produce_a(const Slot &sl, unsigned ring, Ring &r
                 continue;
             }
             unsigned kh = 0, kw = 0, c = 0;          // tap and first channel of the next chunk; c runs fastest
-            const int x0 = (int)(px * stride) - pad, y0 = (int)(py * stride) - pad;
+            const int x0 = (int)(px * sx) - pad, y0 = (int)(py * sy) - pad;
             for (unsigned ch = 0; ch < chunks; ch += per) {
                 const unsigned n = min(per, chunks - ch);
                 unsigned dst = ring + r.s * r.stage_bytes;
                 if (!mbar_wait(&sh->empty[r.s], r.parity() ^ 1u, ctrl, status, 2)) return false;
                 mbar_arrive_expect_tx(&sh->full[r.s], n * chunk_bytes);
                 for (unsigned j = 0; j < n; j++, dst += chunk_bytes) {
-                    if (kind == A_IM2COL) {
+                    if (im2col) {
                         tma_load_im2col(dst, map, (int)c, x0, y0, (int)pn, kw, kh, &sh->full[r.s]);
                         c += 32u;
-                        if (c == IC) { c = 0; if (++kw == KW) { kw = 0; kh++; } }
-                    } else if (kind == A_TMA) {
-                        tma_load_2d(dst, map, (g.ax + (int)(ch + j)) * 32, g.ay + (int)n0, &sh->full[r.s]);
-                    } else {
-                        // the 128 pixels are cut where an output row ends; a run of 16 i pixels uses the layer's i-th consecutive map
-                        unsigned ow = px, oh = py, b = pn;
-                        for (unsigned done = 0; done < 128u;) {
-                            const unsigned len = min(128u - done, OW - ow);
-                            tma_load_3d(dst + done * 128u, map + (size_t)(len / 16u - 1u) * 128, 0, (int)ow, (int)(b * PH + oh * stride + ch + j), &sh->full[r.s]);
-                            done += len;
-                            ow += len;
-                            if (ow == OW) { ow = 0; if (++oh == OH) { oh = 0; b++; } }
-                        }
-                    }
+                        if (c == C) { c = 0; if (++kw == KW) { kw = 0; kh++; } }
+                    } else tma_load_2d(dst, map, (g.ax + (int)(ch + j)) * 32, g.ay + (int)n0, &sh->full[r.s]);
                 }
                 r.step();
             }

@@ -96,22 +96,21 @@ def test_every_layer_matches_oracle(name, batch, seq, mn, precision, profile, wo
     dev.close()
 
 
-@pytest.mark.skipif(not ref.available(), reason="needs the reference build")
-@pytest.mark.parametrize("env", [{"ASPEN_B200_NO_ROW_BOXES": "1"}, {"ASPEN_B200_IM2COL": "0"}, {"ASPEN_B200_IM2COL": "2"},
-                                 {"ASPEN_B200_NO_FUSE": "1", "ASPEN_B200_IM2COL": "2"}])
-def test_every_operand_staging_matches_oracle(env, workdir, monkeypatch):
-    """ResNet-50 with each way of staging the convolution operands forced: stem by gather instead of row boxes,
-    strided layers by gather instead of strided boxes, every 3x3 layer by strided boxes instead of shifted
-    box + fix-up.  All must meet the same per-layer bound against the reference."""
+@pytest.mark.parametrize("env", [{"ASPEN_B200_NO_FUSE": "1"}, {"ASPEN_B200_PLAN": "0"}, {"ASPEN_B200_PLAN": "0", "ASPEN_B200_NO_FUSE": "1"}], ids=" ".join)
+@pytest.mark.parametrize("name,batch,profile", [("tiny_cnn", 3, 1), ("tiny_acts", 3, 1), ("resnet50", 3, 1), ("resnet50", 2, 0)])
+def test_every_way_of_executing_a_network_matches_oracle(env, name, batch, profile, workdir, monkeypatch):
+    """Residual layers on their own instead of in their producer's epilogue, and the graph's own tiles instead of the device plan's
+    (operand stagings: tests/test_gpu_shapes.py)."""
+    if name == "resnet50" and not ref.available():
+        pytest.skip("plain-C oracle is too slow for this size; needs the reference build")
     for k, v in env.items():
         monkeypatch.setenv(k, v)
-    cfg, wf = harness.prepare("resnet50", workdir)
-    dev = harness.Device(cfg, wf, 3, 0, 100, 0, 1)
-    x = harness.make_input("resnet50", dev.input_shape())
+    cfg, wf = harness.prepare(name, workdir)
+    dev = harness.Device(cfg, wf, batch, 0, 100 if name == "resnet50" else 8, 0, profile)
+    x = harness.make_input(name, dev.input_shape())
     assert dev.run(x) == 0, api.last_error()
-    outs = oracle_layers("resnet50", cfg, wf, 3, 0, 100, x)
-    worst = check_layers(dev, outs, 0, "resnet50")
-    assert worst < TF32_NORM
+    outs = oracle_layers(name, cfg, wf, batch, 0, 100 if name == "resnet50" else 8, x)
+    check_layers(dev, outs, 0, name)
     dev.close()
 
 

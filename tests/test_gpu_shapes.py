@@ -59,6 +59,11 @@ def every_layer_matches(name, batch, seq, precision, profile, workdir):
     kw, scheme, (wseed, _) = harness.NETS[name]
     text, wl = cfgs.BUILDERS[harness._BUILDER.get(name, name)](**kw)
     outs = port.run(text, weights.make_weights(wl, wseed, scheme), x, batch, seq)
+    layers_match(dev, outs, precision)
+    dev.close()
+
+
+def layers_match(dev, outs, precision):
     for i in range(1, dev.nasm.num_ldata):
         got, want = dev.nasm.ldata(i), outs[i]
         scale = float(np.abs(want).max())
@@ -67,6 +72,39 @@ def every_layer_matches(name, batch, seq, precision, profile, workdir):
             assert bad == 0, f"layer {i}: {bad} mismatches, max abs {ea:.3e}, max rel {er:.3e}"
         else:
             assert float(np.abs(got.astype(np.float64) - want).max()) <= 1e-2 * scale, f"layer {i}"
+
+
+def _conv_net(side, channels, layers, out):
+    """cfg and weighted layers: convolutions (channels, size, stride, pad) one after the other and a connected layer over the last."""
+    text, wl = f"[net]\nheight={side}\nwidth={side}\nchannels={channels}\n\n", []
+    for c, size, stride, pad in layers:
+        text += f"[convolutional]\nfilters={c}\nsize={size}\nstride={stride}\npad={pad}\nactivation=relu\n\n"
+        wl.append(("conv", (c, channels, size, size), channels * size * size))
+        side, channels = (side + 2 * pad - size) // stride + 1, c
+    wl.append(("fc", (out, channels, side, side), channels * side * side))
+    return text + f"[connected]\noutput={out}\nactivation=linear\n", wl
+
+
+@pytest.mark.parametrize("batch,side,channels,layers", [
+    (3, 30, 3, [(48, 7, 2, 3), (24, 3, 1, 1), (33, 3, 2, 1), (64, 1, 2, 0), (10, 1, 1, 0)]),       # rows of 15 pixels; channels no multiple of 32, or of 4
+    (12, 37, 1, [(20, 11, 4, 2), (96, 3, 1, 0), (12, 5, 1, 2)]),                                   # one channel, a window of two chunks a row
+    (9, 18, 4, [(40, 3, 1, 1), (6, 3, 3, 2), (70, 2, 1, 1)]),
+    (11, 9, 3, []),                                                                                # connected straight to the image
+    (2, 17, 9, [(5, 3, 1, 1), (36, 4, 2, 1)]),                                                     # an input of more than four channels
+    (2, 21, 3, [(36, 3, 1, 4), (40, 3, 9, 1)])])                                                   # windows that lie in the padding, a stride past TMA's: fp32 blocks
+@pytest.mark.parametrize("precision", [0, 1])
+def test_convolutions_of_any_channel_count_and_width(batch, side, channels, layers, precision, workdir):
+    text, wl = _conv_net(side, channels, layers, 13)
+    cfg, wf = f"{workdir}/conv_{side}.cfg", f"{workdir}/conv_{side}.bin"
+    with open(cfg, "w") as f:
+        f.write(text)
+    ws = weights.make_weights(wl, 41, "he")
+    weights.write_aspen_data(wf, ws)
+    dev = harness.Device(cfg, wf, batch, 0, 20, precision, 1)
+    x = np.random.default_rng(side).standard_normal(dev.input_shape(), dtype=np.float32)
+    for _ in range(2):
+        assert dev.run(x) == 0, api.last_error()
+    layers_match(dev, port.run(text, ws, x, batch, 0), precision)
     dev.close()
 
 

@@ -54,3 +54,19 @@ def test_a_graph_is_the_same_with_any_number_of_threads(workdir):
 @pytest.mark.parametrize("seed", ["1", "2", "3"])
 def test_every_worker_warp_leaves_whichever_waits_give_up(seed, workdir):
     passes(build("worker_loop", workdir, "-lpthread"), seed)
+
+
+def test_layers_of_any_channel_count_have_a_form_for_the_tensor_cores(workdir):
+    """300 x 300 image, 48- and 24-channel convolutions: every contraction reaches the tensor cores, the taps of the weights in whole
+    chunks of 32; a second convolution on the image goes tap by tap, and what an im2col map cannot hold does not go at all."""
+    api.lib()
+    exe = build("operand_forms", workdir, f"-L{LIBDIR}", "-laspen_b200", f"-Wl,-rpath,{LIBDIR}")
+    cfg = os.path.join(workdir, "forms.cfg")
+    conv = "[convolutional]\nfilters={}\nsize={}\nstride={}\npad={}\n{}\n"
+    with open(cfg, "w") as f:
+        f.write("[net]\nheight=300\nwidth=300\nchannels=3\n\n" + conv.format(48, 7, 2, 3, "") + conv.format(24, 3, 1, 1, "") + conv.format(64, 1, 1, 0, "") +
+                conv.format(8, 1, 2, 0, "") + conv.format(8, 3, 1, 1, "parent=-5\n") + conv.format(8, 3, 1, 3, "") + conv.format(8, 3, 9, 1, "") +
+                "[connected]\noutput=10\n\n")
+    r = subprocess.run([exe, cfg], capture_output=True, text=True, check=True).stdout.split("\n")
+    forms = [tuple(int(v) for v in line.split()[1:]) for line in r[1:9]]
+    assert forms == [(2, 1, 7 * 32), (2, 0, 9 * 64), (1, 0, 0), (2, 0, 64), (2, 0, 9 * 32), (0, 0, 0), (0, 0, 0), (1, 0, 0)]
