@@ -8,7 +8,7 @@
 // Layer types / activations use the ABI enum values of include/aspen_b200.h.
 
 // How the X operand (activations) of a contraction layer reaches shared memory on the tensor-core path; see tiles_tc.cuh.
-enum { A_NONE = 0, A_TMA = 1, A_IM2COL = 2 };
+enum { A_NONE = 0, A_TMA = 1, A_IM2COL = 2, A_HEAD = 3 };
 
 struct LayerDev {
     int type;                 // LAYER_TYPE

@@ -130,7 +130,7 @@ static int upload_weights(aspen_dnn_t *dnn, int device, int precision, DeviceDnn
                 }
             CUDA_TRY(cudaMalloc(&dd->weight[precision][i], padded.size() * sizeof(float) + 256));
             CUDA_TRY(cudaMemcpy(dd->weight[precision][i], padded.data(), padded.size() * sizeof(float), cudaMemcpyHostToDevice));
-            const OperandForm form = operand_form(&l);
+            const OperandForm form = operand_form(&l, 0);
             if (precision == 0 && form.kind == A_IM2COL && (form.image || (ic % 32 != 0 && form.kh * form.kw > 1)) && !dd->weight_boxes[i]) {
                 const unsigned window = k / ic, in_row = form.image ? l.params[WEIGHT_W] : 1, cp = (unsigned)round_up(form.c, 32);
                 std::vector<float> boxes((size_t)rows * form.k(), 0.f);
@@ -450,6 +450,19 @@ static int build_device_nasm(Engine *e, nasm_t *host_nasm) {
         maps.push_back(m);
         return (int)maps.size() - 1;
     };
+    // (feature of a head, head, column): boxes of 32 features of one head x box_rows columns; what a box holds past the head's last
+    // feature arrives as zeros
+    auto add_head_map = [&](const void *base, const LayerDev &L, cuuint64_t columns, unsigned ld, cuuint32_t box_rows) -> int {
+        CUtensorMap m;
+        cuuint64_t dims[3] = {L.hd, L.heads, columns}, strides[2] = {(cuuint64_t)L.hd * 4, (cuuint64_t)ld * 4};
+        cuuint32_t box[3] = {32, 1, box_rows}, estr[3] = {1, 1, 1};
+        CUresult r = get_encode_fn()(&m, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3, const_cast<void *>(base), dims, strides, box, estr,
+                                     CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                                     CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+        if (r != CUDA_SUCCESS) { ASPEN_ERR("cuTensorMapEncodeTiled failed (%d)\n", (int)r); return -2; }
+        maps.push_back(m);
+        return (int)maps.size() - 1;
+    };
     // The X operand by plain boxes: the chunks of a stage in one where the matrix allows it.
     auto add_x_map = [&](LayerDev &L, const void *base, cuuint64_t inner, cuuint64_t outer, cuuint64_t stride_bytes) {
         L.a_kind = A_TMA;
@@ -498,7 +511,7 @@ static int build_device_nasm(Engine *e, nasm_t *host_nasm) {
             L.stages = std::min(tc::MAX_STAGES, tc::RING_BYTES / L.stage_bytes);
         };
         if (gemm_w || l.type == K_ATTENTION_LAYER || l.type == V_ATTENTION_LAYER) cut_ring(l.type == K_ATTENTION_LAYER ? L.hd : l.type == V_ATTENTION_LAYER ? L.seq : L.Kpad);
-        const OperandForm form = operand_form(&l);
+        const OperandForm form = operand_form(&l, L.seq);
         const float *dense = L.weight;
         const unsigned dense_kpad = L.Kpad;
         if (form.kind == A_IM2COL && L.H0 == l.params[IN_C]) {
@@ -530,10 +543,16 @@ static int build_device_nasm(Engine *e, nasm_t *host_nasm) {
             // a sample's NHWC activations are one contiguous row of K values (own tiles may leave more rows between its columns)
             add_x_map(L, L.in0, L.K, nasm->batch_size, (cuuint64_t)L.IH * L.IW * L.ld0 * sizeof(float));
         } else if (l.type == K_ATTENTION_LAYER) {
-            // all keys of a query must fit the accumulators (512 columns); larger sequences run as fp32 tiles
-            if (L.hd % 32 == 0 && L.H0 % 32 == 0 && L.H1 % 32 == 0 && L.seq <= tc::TMEM_COLS && th >= L.seq) {
+            const cuuint64_t W1 = nasm->ldata[p1].out_mat_dims[OUT_W];
+            if (th < L.seq || L.H0 != L.heads * L.hd || L.H1 != L.H0) {
+                // tiles of a part of the keys: the softmax needs them all
+            } else if (form.kind == A_TMA) {
                 add_x_map(L, L.in0, L.H0, W0, (cuuint64_t)L.ld0 * sizeof(float));
-                L.wmap = add_map(L.in1, L.H1, nasm->ldata[p1].out_mat_dims[OUT_W], (cuuint64_t)L.ld1 * sizeof(float), L.b_rows, L.per_stage);
+                L.wmap = add_map(L.in1, L.H1, W1, (cuuint64_t)L.ld1 * sizeof(float), L.b_rows, L.per_stage);
+            } else if (form.kind == A_HEAD) {
+                L.a_kind = A_HEAD;
+                L.amap = add_head_map(L.in0, L, W0, L.ld0, L.a_rows);
+                L.wmap = add_head_map(L.in1, L, W1, L.ld1, L.b_rows);
             }
         } else if (l.type == V_ATTENTION_LAYER && p1 != (unsigned)-1 && p1 < i && p1 != 0 && layers[p1].tc && !layers[p1].vt_out) {
             // The value operand W(m, k) = V[token k][feature m] is the transpose of how the value projection stores its

@@ -178,7 +178,7 @@ struct OperandForm {
     unsigned c = 0, kh = 1, kw = 1;
     unsigned k() const { return kh * kw * (unsigned)round_up(c, 32); }      // A_IM2COL: k of the weights, every tap in whole chunks
 };
-OperandForm operand_form(const aspen_layer_t *l);
+OperandForm operand_form(const aspen_layer_t *l, unsigned seq);
 nasm_t *plan_device_tiles(const nasm_t *nasm, int precision, unsigned int sms, bool served);   // plan.cpp; nullptr: keep the nasm's tiles
 nasm_t *own_device_tiles(const nasm_t *nasm);      // plan.cpp: the nasm's tiles, columns a multiple of 16 bytes apart
 int engine_current_device();

@@ -103,12 +103,19 @@ bool gemv_layer(const nasm_ldata_t &ld) {
                                            (t == CONV_LAYER && p[WEIGHT_H] == 1 && p[WEIGHT_W] == 1 && p[STRIDE] <= 1 && p[PADDING] == 0));
 }
 
-OperandForm operand_form(const aspen_layer_t *l) {
+OperandForm operand_form(const aspen_layer_t *l, unsigned seq) {
     const unsigned *p = l->params;
     OperandForm f;
     f.c = p[IN_C];
     switch (l->type) {
-        case MATMUL_LAYER: case FC_LAYER: case K_ATTENTION_LAYER: case V_ATTENTION_LAYER: f.kind = A_TMA; break;
+        case MATMUL_LAYER: case FC_LAYER: case V_ATTENTION_LAYER: f.kind = A_TMA; break;
+        case K_ATTENTION_LAYER: {
+            // all keys of a query have to fit the accumulators, and a head has to start on a 16-byte boundary
+            const unsigned hd = p[NUM_HEAD] ? p[NUM_HIDDEN] / p[NUM_HEAD] : 0;
+            if (hd == 0 || hd % 4 != 0 || seq > 512) break;
+            f.kind = hd % 32 == 0 ? A_TMA : A_HEAD;
+            break;
+        }
         case CONV_LAYER: {
             const unsigned stride = p[STRIDE] ? p[STRIDE] : 1;
             if (p[WEIGHT_H] == 1 && p[WEIGHT_W] == 1 && stride == 1 && p[PADDING] == 0) { f.kind = A_TMA; break; }
@@ -120,7 +127,7 @@ OperandForm operand_form(const aspen_layer_t *l) {
             const aspen_layer_t *first = l->dnn->layers.data(), *in = l->parent_layers[PARENT_0];
             f.image = in && in->type == INPUT_LAYER && p[IN_C] <= 4;
             for (; first < l; first++)
-                if (first->type == CONV_LAYER && first->parent_layers[PARENT_0] == in && operand_form(first).image) f.image = false;
+                if (first->type == CONV_LAYER && first->parent_layers[PARENT_0] == in && operand_form(first, seq).image) f.image = false;
             if (f.image) { f.c = 4 * f.kw; f.kw = 1; }
             break;
         }

@@ -229,6 +229,8 @@ __device__ __forceinline__ unsigned umma_idesc(unsigned n) {
 //              A convolution on an image of at most 4 channels (the 7x7 stem) reads a zero-padded [sample][row][pixel][4] copy of
 //              it: a row of the window is 4 * KW consecutive floats there, the tensor's columns are the output's (a stride apart,
 //              overlapping), and KH rows of 28 floats take 7 chunks where 49 taps of 3 channels would take 49.
+//   A_HEAD     attention scores with heads that are no multiple of 32 features: the parent is a (feature, head, column) tensor for
+//              queries and keys alike, one box per k-chunk, zeros past the head's last feature
 // The W operand -- weights, attention keys (PARENT_1's matrix) or the transposed copy of the attention values -- arrives in one
 // box per stage.  Layers that fit none of these run as fp32 FMA tiles (tile_gemm_ffma).
 
@@ -245,7 +247,7 @@ __device__ __forceinline__ Origin origin(const LayerDev &L, const TileDev &T) {
     g.ax = 0; g.ay = (int)T.pos_w; g.bx = 0; g.by = (int)T.pos_h; g.seen = 0;
     if (L.type == K_ATTENTION_LAYER) {
         const unsigned per = L.seq * L.heads, b = T.pos_w / per, r = T.pos_w - b * per, head = r / L.seq, q0 = r - head * L.seq;
-        g.ax = g.bx = (int)(head * (L.hd >> 5));
+        g.ax = g.bx = (int)(L.a_kind == A_HEAD ? head : head * (L.hd >> 5));
         g.ay = (int)(b * L.seq + q0); g.by = (int)(b * L.seq + T.pos_h);
     } else if (L.type == V_ATTENTION_LAYER) {
         const unsigned b = T.pos_w / L.seq, head = T.pos_h / L.hd, q0 = T.pos_w - b * L.seq;
@@ -281,7 +283,7 @@ __device__ __forceinline__ bool produce_a(const Slot &sl, unsigned ring, Ring &r
     // activations were written with ordinary (generic proxy) stores; TMA reads them through the async proxy
     asm volatile("fence.proxy.async.global;" ::: "memory");
     if (!recut(r, L, sh, ctrl, status)) return false;
-    const bool im2col = L.a_kind == A_IM2COL;
+    const bool im2col = L.a_kind == A_IM2COL, heads = L.a_kind == A_HEAD;
     const unsigned multi = L.a_multi, tile_w = sl.tile.tile_w, tile_h = sl.tile.tile_h, pos_w = sl.tile.pos_w;
     const unsigned OW = L.OW, OH = L.OH, KW = L.tap_kw, C = L.tap_c, sx = L.tap_sx, sy = L.tap_sy, per = L.per_stage, chunk_bytes = L.a_rows * 128u;
     const int pad = (int)L.tap_pad;
@@ -317,7 +319,8 @@ __device__ __forceinline__ bool produce_a(const Slot &sl, unsigned ring, Ring &r
                         tma_load_im2col(dst, map, (int)c, x0, y0, (int)pn, kw, kh, &sh->full[r.s]);
                         c += 32u;
                         if (c == C) { c = 0; if (++kw == KW) { kw = 0; kh++; } }
-                    } else tma_load_2d(dst, map, (g.ax + (int)(ch + j)) * 32, g.ay + (int)n0, &sh->full[r.s]);
+                    } else if (heads) tma_load_3d(dst, map, (int)(ch + j) * 32, g.ax, g.ay + (int)n0, &sh->full[r.s]);
+                    else tma_load_2d(dst, map, (g.ax + (int)(ch + j)) * 32, g.ay + (int)n0, &sh->full[r.s]);
                 }
                 r.step();
             }
@@ -334,6 +337,19 @@ __device__ __forceinline__ bool produce_b(const Slot &sl, unsigned ring, Ring &r
     asm volatile("fence.proxy.async.global;" ::: "memory");
     if (!recut(r, L, sh, ctrl, status)) return false;
     const unsigned tile_w = sl.tile.tile_w, tile_h = sl.tile.tile_h, per = L.per_stage, bytes = per * L.b_rows * 128u, b_off = per * L.a_rows * 128u;
+    if (L.a_kind == A_HEAD) {
+        for (unsigned n0 = 0; n0 < tile_w; n0 += 128u)
+            for (unsigned mp = 0; mp < tile_h; mp += BLOCK_ROWS)
+                for (unsigned ch = 0, chunks = L.chunks; ch < chunks; ch += per) {
+                    const unsigned n = min(per, chunks - ch), box = L.b_rows * 128u;
+                    if (!mbar_wait(&sh->empty[r.s], r.parity() ^ 1u, ctrl, status, 9)) return false;
+                    mbar_arrive_expect_tx(&sh->full[r.s], n * box);
+                    for (unsigned j = 0; j < n; j++)
+                        tma_load_3d(ring + r.s * r.stage_bytes + b_off + j * box, map, (int)(ch + j) * 32, g.bx, g.by + (int)mp, &sh->full[r.s]);
+                    r.step();
+                }
+        return true;
+    }
     for (unsigned n0 = 0; n0 < tile_w; n0 += 128u)
         for (unsigned mp = 0; mp < tile_h; mp += BLOCK_ROWS)
             for (unsigned ch = 0, chunks = g.chunks(L, n0); ch < chunks; ch += per) {

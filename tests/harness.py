@@ -19,6 +19,7 @@ NETS = {
     # heads of 10 and 12 features: tiles of one head's rows do not start on 16-byte boundaries, or only every other one does
     "tiny_heads10": ({"d": 40, "heads": 4}, "n002", (25, 24)),
     "tiny_heads12": ({"d": 48, "heads": 4, "masked": True, "pre_ln": True}, "n002", (27, 26)),
+    "tiny_heads80": ({"d": 160, "heads": 2}, "n002", (29, 28)),     # heads of two and a half 32-feature chunks
     "custom": ({}, "he", (5, 6)),
     "tiny_yolo": ({}, "he", (17, 16)),
     "tiny_acts": ({}, "he", (19, 18)),
@@ -30,7 +31,7 @@ NETS = {
     "gpt2_lm": ({"with_lm_head": True}, "n002", (4, 4)),
 }
 _BUILDER = {"tiny_gpt": "tiny_transformer", "gpt2_lm": "gpt2_124M", "tiny_attn": "tiny_transformer", "tiny_attn_causal": "tiny_transformer",
-            "tiny_heads10": "tiny_transformer", "tiny_heads12": "tiny_transformer"}
+            "tiny_heads10": "tiny_transformer", "tiny_heads12": "tiny_transformer", "tiny_heads80": "tiny_transformer"}
 
 
 def prepare(name: str, workdir: str):

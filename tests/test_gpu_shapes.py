@@ -33,7 +33,9 @@ def test_noalloc_blocks_at_their_edges(n, k, m, act):
                                                       ("tiny_attn_causal", 1, 257, 0), ("tiny_attn_causal", 1, 300, 1), ("tiny_transformer", 64, 128, 0),
                                                       ("tiny_cnn", 1, 0, 0), ("tiny_cnn", 33, 0, 0), ("tiny_cnn", 9, 0, 1), ("custom", 1, 0, 0), ("custom", 130, 0, 0),
                                                       ("custom", 3, 0, 1), ("custom", 2, 0, 0), ("custom", 5, 0, 0), ("custom", 8, 0, 0), ("custom", 9, 0, 0),
-                                                      ("custom", 8, 0, 1), ("tiny_attn", 1, 7, 1), ("tiny_transformer", 1, 5, 0), ("tiny_cnn", 4, 0, 0)])
+                                                      ("custom", 8, 0, 1), ("tiny_attn", 1, 7, 1),
+                                                      ("tiny_heads80", 2, 40, 0), ("tiny_heads80", 1, 300, 0), ("tiny_heads80", 1, 40, 1), ("tiny_heads12", 3, 130, 0),
+                                                      ("tiny_gpt", 1, 512, 0), ("tiny_attn", 1, 520, 0), ("tiny_attn_causal", 1, 520, 1), ("tiny_transformer", 1, 5, 0), ("tiny_cnn", 4, 0, 0)])
 def test_every_layer_at_the_edges_of_the_plan(name, batch, seq, precision, workdir):
     every_layer_matches(name, batch, seq, precision, 1, workdir)
 

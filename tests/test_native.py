@@ -6,7 +6,7 @@ import subprocess
 import pytest
 
 import harness
-from aspen_b200 import api
+from aspen_b200 import api, cfgs
 
 
 
@@ -56,17 +56,28 @@ def test_every_worker_warp_leaves_whichever_waits_give_up(seed, workdir):
     passes(build("worker_loop", workdir, "-lpthread"), seed)
 
 
-def test_layers_of_any_channel_count_have_a_form_for_the_tensor_cores(workdir):
-    """300 x 300 image, 48- and 24-channel convolutions: every contraction reaches the tensor cores, the taps of the weights in whole
-    chunks of 32; a second convolution on the image goes tap by tap, and what an im2col map cannot hold does not go at all."""
+def operand_forms(workdir, text, seq=0):
     api.lib()
     exe = build("operand_forms", workdir, f"-L{LIBDIR}", "-laspen_b200", f"-Wl,-rpath,{LIBDIR}")
     cfg = os.path.join(workdir, "forms.cfg")
-    conv = "[convolutional]\nfilters={}\nsize={}\nstride={}\npad={}\n{}\n"
     with open(cfg, "w") as f:
-        f.write("[net]\nheight=300\nwidth=300\nchannels=3\n\n" + conv.format(48, 7, 2, 3, "") + conv.format(24, 3, 1, 1, "") + conv.format(64, 1, 1, 0, "") +
-                conv.format(8, 1, 2, 0, "") + conv.format(8, 3, 1, 1, "parent=-5\n") + conv.format(8, 3, 1, 3, "") + conv.format(8, 3, 9, 1, "") +
-                "[connected]\noutput=10\n\n")
-    r = subprocess.run([exe, cfg], capture_output=True, text=True, check=True).stdout.split("\n")
-    forms = [tuple(int(v) for v in line.split()[1:]) for line in r[1:9]]
+        f.write(text)
+    r = subprocess.run([exe, cfg, str(seq)], capture_output=True, text=True, check=True).stdout
+    return [tuple(int(v) for v in line.split()[1:]) for line in r.split("\n")[1:-1]]
+
+
+def test_layers_of_any_channel_count_have_a_form_for_the_tensor_cores(workdir):
+    """300 x 300 image, 48- and 24-channel convolutions: every contraction reaches the tensor cores, the taps of the weights in whole
+    chunks of 32; a second convolution on the image goes tap by tap, and what an im2col map cannot hold does not go at all."""
+    conv = "[convolutional]\nfilters={}\nsize={}\nstride={}\npad={}\n{}\n"
+    forms = operand_forms(workdir, "[net]\nheight=300\nwidth=300\nchannels=3\n\n" + conv.format(48, 7, 2, 3, "") + conv.format(24, 3, 1, 1, "") +
+                          conv.format(64, 1, 1, 0, "") + conv.format(8, 1, 2, 0, "") + conv.format(8, 3, 1, 1, "parent=-5\n") + conv.format(8, 3, 1, 3, "") +
+                          conv.format(8, 3, 9, 1, "") + "[connected]\noutput=10\n\n")
     assert forms == [(2, 1, 7 * 32), (2, 0, 9 * 64), (1, 0, 0), (2, 0, 64), (2, 0, 9 * 32), (0, 0, 0), (0, 0, 0), (1, 0, 0)]
+
+
+@pytest.mark.parametrize("heads,d,seq,form", [(2, 64, 100, 1), (2, 160, 100, 3), (4, 48, 512, 3), (4, 40, 100, 0), (2, 64, 513, 0)])
+def test_attention_heads_of_a_multiple_of_four_have_a_form_for_the_tensor_cores(heads, d, seq, form, workdir):
+    text, _ = cfgs.transformer(1, d, heads, d, pre_ln=False, masked=False, act="gelu")
+    forms = operand_forms(workdir, text, seq)
+    assert [f[0] for f in forms[:6]] == [1, 1, 1, form, 1, 1]
