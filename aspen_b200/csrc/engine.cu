@@ -502,6 +502,8 @@ static int build_device_nasm(Engine *e, nasm_t *host_nasm) {
         // (0.25 us of instructions per stage against 0.05 us of MMA per chunk of 32 rows, 0.1 of 64, 0.2 of 128, 0.4 of 256) while
         // two or more stages fit.
         const unsigned th = nasm->ldata[i].ninst_tile_dims[OUT_H];
+        // the epilogue stores 16-byte pieces: a tile has to start on one (a head of ten features does not)
+        const bool aligned_out = th % 4 == 0 || th >= L.H;
         auto cut_ring = [&](unsigned k) {
             L.b_rows = (unsigned)round_up(std::min(th, tc::BLOCK_ROWS), 16);
             L.chunks = std::max(1u, (k + 31) / 32);
@@ -554,28 +556,26 @@ static int build_device_nasm(Engine *e, nasm_t *host_nasm) {
                 L.amap = add_head_map(L.in0, L, W0, L.ld0, L.a_rows);
                 L.wmap = add_head_map(L.in1, L, W1, L.ld1, L.b_rows);
             }
-        } else if (l.type == V_ATTENTION_LAYER && p1 != (unsigned)-1 && p1 < i && p1 != 0 && layers[p1].tc && !layers[p1].vt_out) {
-            // The value operand W(m, k) = V[token k][feature m] is the transpose of how the value projection stores its
-            // output; that projection, a tensor-core layer of this graph, writes a second, transposed copy into scratch memory.
+        } else if (l.type == V_ATTENTION_LAYER && aligned_out && p1 != (unsigned)-1 && p1 < i && nasm->ldata[p1].layer->type != K_ATTENTION_LAYER) {
+            // The value operand W(m, k) = V[token k][feature m] is the transpose of how the values' layer stores its output; that
+            // layer writes a second, transposed copy into scratch memory: in the epilogue of a tensor-core projection, else by a loop
+            // over the stored tile.  Several attention_v layers over the same values share it.
             const size_t seqp = round_up(L.seq, 32), ldt = seqp * nasm->batch_size;
-            float *vt = nullptr;
-            CUDA_TRY(cudaMalloc(&vt, (size_t)L.H1 * ldt * sizeof(float) + 256));
-            dn->scratch.push_back(vt);
-            CUDA_TRY(cudaMemsetAsync(vt, 0, (size_t)L.H1 * ldt * sizeof(float) + 256, e->stream));
-            const int m = add_map(vt, ldt, L.H1, (cuuint64_t)ldt * sizeof(float), L.b_rows, L.per_stage);
-            if (m >= 0) {
-                layers[p1].vt_out = vt;
-                L.masked = nasm->ldata[p0].layer->type == K_ATTENTION_LAYER && layers[p0].tc && layers[p0].masked;   // its probabilities after the mask are zeros
-                layers[p1].vt_ld = (unsigned)ldt;
-                layers[p1].vt_seq = L.vt_seq = (unsigned)seqp;
-                L.wmap = m;
-                add_x_map(L, L.in0, L.H0, W0, (cuuint64_t)L.ld0 * sizeof(float));
+            LayerDev &V = layers[p1];
+            if (!V.vt_out) {
+                CUDA_TRY(cudaMalloc(&V.vt_out, (size_t)L.H1 * ldt * sizeof(float) + 256));
+                dn->scratch.push_back(V.vt_out);
+                CUDA_TRY(cudaMemsetAsync(V.vt_out, 0, (size_t)L.H1 * ldt * sizeof(float) + 256, e->stream));
+                V.vt_ld = (unsigned)ldt;
+                V.vt_seq = (unsigned)seqp;
             }
+            L.wmap = add_map(V.vt_out, ldt, L.H1, (cuuint64_t)ldt * sizeof(float), L.b_rows, L.per_stage);
+            L.masked = nasm->ldata[p0].layer->type == K_ATTENTION_LAYER && layers[p0].tc && layers[p0].masked;   // its probabilities after the mask are zeros
+            L.vt_seq = (unsigned)seqp;
+            add_x_map(L, L.in0, L.H0, W0, (cuuint64_t)L.ld0 * sizeof(float));
         }
         if (gemm_w && L.a_kind != A_NONE && L.amap >= 0)
             L.wmap = add_map(L.weight, L.Kpad, layer_weight_rows(&l), (cuuint64_t)L.Kpad * sizeof(float), L.b_rows, L.per_stage);
-        // the epilogue stores 16-byte pieces: a tile has to start on one (a head of ten features does not)
-        const bool aligned_out = th % 4 == 0 || th >= L.H;
         L.tc = L.a_kind != A_NONE && L.amap >= 0 && L.wmap >= 0 && aligned_out;
         if (!L.tc) { L.weight = dense; L.Kpad = dense_kpad; }       // fp32 blocks walk the taps as they are
         // ASPEN_B200_ATTN_FUSE=1 with hidden states given up: attention probabilities that only the attention_v layer reads do not
@@ -628,7 +628,7 @@ static int build_device_nasm(Engine *e, nasm_t *host_nasm) {
             if (a == (unsigned)-1 || b == (unsigned)-1 || a == b) continue;
             const unsigned hi = std::max(a, b), lo = std::min(a, b);
             const LAYER_TYPE t = nasm->ldata[hi].layer->type;
-            if ((t != CONV_LAYER && t != MATMUL_LAYER) || !layers[hi].tc || layers[hi].res_out || layers[hi].vt_out) continue;
+            if ((t != CONV_LAYER && t != MATMUL_LAYER) || !layers[hi].tc || layers[hi].res_out || layers[hi].vt_out || layers[i].vt_out) continue;
             const nasm_ldata_t &R = nasm->ldata[i], &P = nasm->ldata[hi], &Q = nasm->ldata[lo];
             if (P.out_mat_dims[OUT_H] != R.out_mat_dims[OUT_H] || P.out_mat_dims[OUT_W] != R.out_mat_dims[OUT_W] ||
                 Q.out_mat_dims[OUT_H] != R.out_mat_dims[OUT_H] || Q.out_mat_dims[OUT_W] != R.out_mat_dims[OUT_W])

@@ -241,6 +241,7 @@ static __device__ __noinline__ void worker_tile(const tc::Slot &sl, unsigned wt,
         case INPUT_LAYER: tile_input(*sl.input, L, T, wt, tc::NW); break;
         default: break;
     }
+    if (TENSOR_CORES && L.vt_out) tile_transposed_copy(L, T, wt, tc::NW);
 }
 
 // ---- the persistent kernel -------------------------------------------------------------------
@@ -482,10 +483,12 @@ struct WorkerWarp {
         return __all_sync(0xffffffffu, wait_posted(&sh->posted[seq % tc::SLOTS], (seq / tc::SLOTS) & 1u, ctrl, status));
     }
     __device__ __forceinline__ bool live(unsigned seq) const { return slot(seq).live != 0u; }
-    // the softmax of attention scores, and fp32 blocks
+    // the softmax of attention scores, fp32 blocks, and a stored tile that is read back for its transposed copy
     __device__ __forceinline__ bool meets(unsigned seq) const {
         const LayerDev &L = slot(seq).layer;
-        return L.type == K_ATTENTION_LAYER || (!tensor(slot(seq)) && !L.gemv && (L.type == CONV_LAYER || L.type == FC_LAYER || L.type == MATMUL_LAYER || L.type == V_ATTENTION_LAYER));
+        if (L.type == K_ATTENTION_LAYER) return true;
+        if (tensor(slot(seq))) return false;
+        return L.vt_out != nullptr || (!L.gemv && (L.type == CONV_LAYER || L.type == FC_LAYER || L.type == MATMUL_LAYER || L.type == V_ATTENTION_LAYER));
     }
     __device__ __forceinline__ bool agree(bool yes) const {
         unsigned all;

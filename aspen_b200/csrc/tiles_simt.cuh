@@ -476,6 +476,21 @@ __device__ __forceinline__ GemmView gemm_view(const LayerDev &L, const TileDev &
     return g;
 }
 
+// The stored tile once more, transposed, for an attention_v layer that reads its values (LayerDev::vt_out).  The values of a projection
+// on the tensor cores are written by its epilogue; this is for layers of any other kind.  Consecutive threads write consecutive
+// tokens of a feature.
+static __device__ __noinline__ void tile_transposed_copy(const LayerDev &L, const TileDev &T, unsigned tid, unsigned nthr) {
+    const unsigned tile_w = T.tile_w, total = tile_w * T.tile_h, pos_w = T.pos_w, pos_h = T.pos_h, seq = L.seq, vt_seq = L.vt_seq;
+    const size_t ldc = L.ldc, vt_ld = L.vt_ld;
+    const float *in = L.out;
+    float *out = L.vt_out;
+    worker_barrier(nthr);
+    for (unsigned i = tid; i < total; i += nthr) {
+        const unsigned m = pos_h + i / tile_w, col = pos_w + i % tile_w, b = col / seq;
+        out[(size_t)m * vt_ld + (size_t)b * vt_seq + (col - b * seq)] = ldcg1(in + (size_t)col * ldc + m);
+    }
+}
+
 // Layer-0 tile: the uploaded input becomes the columns of the layer's activation matrix that the
 // tile covers -- what the host-launched unpack / rounding / embedding-gather / padded-copy kernels do for a run that
 // is launched per graph.  Sources are read through L2 (the host's DMA wrote them while this kernel was running).

@@ -110,6 +110,29 @@ def test_convolutions_of_any_channel_count_and_width(batch, side, channels, laye
     dev.close()
 
 
+@pytest.mark.parametrize("batch,seq", [(1, 7), (2, 45), (1, 130)])
+@pytest.mark.parametrize("precision", [0, 1])
+def test_attention_over_values_of_any_layer(batch, seq, precision, workdir):
+    """Values without a projection of their own: a layernorm's output (twice), the network's input, a residual add, and a residual add
+    that would otherwise be computed by its producer."""
+    d, h = 64, 2
+    k, v = f"n_head={h}\nn_embd={d}\n", f"[attention_v]\nM={d}\nn_head={h}\nn_embd={d}\n"
+    text = (f"[net]\nM={d}\nheight=1\nfilters={d}\n\n[layernorm]\nM={d}\n\n[matmul]\nM={d}\n{k}\n[matmul]\nM={d}\nparent=-2\n{k}\n"
+            f"[attention_k]\nparent=-1\nfrom=-2\nM=1\nK={d // h}\n{k}\n{v}parent=-1\nfrom=-4\n\n{v}parent=-2\nfrom=-5\n\n{v}parent=-3\nfrom=-7\n\n"
+            f"[shortcut]\nfrom=-3\nM={d}\n\n{v}parent=-5\nfrom=-1\n\n[matmul]\nM={d}\n\n[shortcut]\nfrom=-2\nM={d}\n\n{v}parent=-8\nfrom=-1\n\n")
+    cfg, wf = f"{workdir}/values.cfg", f"{workdir}/values.bin"
+    with open(cfg, "w") as f:
+        f.write(text)
+    ws = weights.make_weights([("layernorm", (d,), d)] + [("matmul", (d, d), d)] * 3, 43, "he")
+    weights.write_aspen_data(wf, ws)
+    dev = harness.Device(cfg, wf, batch, seq, 20, precision, 1)
+    x = np.random.default_rng(seq).standard_normal(dev.input_shape(), dtype=np.float32)
+    for _ in range(2):
+        assert dev.run(x) == 0, api.last_error()
+    layers_match(dev, port.run(text, ws, x, batch, seq), precision)
+    dev.close()
+
+
 @pytest.mark.parametrize("channels", [200704, 300000])
 def test_connected_layer_over_more_channels_than_a_product_of_indices_can_hold(channels, workdir):
     """fp32 blocks find the channel of a k by a multiplication; k times the channel count passes 2^32 here.  The last pieces of k
