@@ -556,7 +556,7 @@ static int build_device_nasm(Engine *e, nasm_t *host_nasm) {
                 L.amap = add_head_map(L.in0, L, W0, L.ld0, L.a_rows);
                 L.wmap = add_head_map(L.in1, L, W1, L.ld1, L.b_rows);
             }
-        } else if (l.type == V_ATTENTION_LAYER && aligned_out && p1 != (unsigned)-1 && p1 < i && nasm->ldata[p1].layer->type != K_ATTENTION_LAYER) {
+        } else if (l.type == V_ATTENTION_LAYER && form.kind == A_TMA && aligned_out && p1 != (unsigned)-1 && p1 < i && nasm->ldata[p1].layer->type != K_ATTENTION_LAYER) {
             // The value operand W(m, k) = V[token k][feature m] is the transpose of how the values' layer stores its output; that
             // layer writes a second, transposed copy into scratch memory: in the epilogue of a tensor-core projection, else by a loop
             // over the stored tile.  Several attention_v layers over the same values share it.

@@ -25,15 +25,27 @@ struct Grid {
 bool contraction(LAYER_TYPE t) { return t == CONV_LAYER || t == FC_LAYER || t == MATMUL_LAYER || t == K_ATTENTION_LAYER || t == V_ATTENTION_LAYER; }
 unsigned ceil_div(unsigned a, unsigned b) { return (a + b - 1) / b; }
 
+// What runs the tiles of a contraction layer.
+enum Path { TENSOR, BESIDE_RING, FP32 };      // tensor cores / fp32 blocks in a tensor-core graph (no operand form) / fp32 mode
+
+Path path_of(const aspen_layer_t *l, int precision, unsigned seq) { return precision != 0 ? FP32 : operand_form(l, seq).kind != A_NONE ? TENSOR : BESIDE_RING; }
+
 // Estimated microseconds of one tile of th x tw outputs with a k-deep contraction, `gap` of them between two tiles of an SM.
 // Tensor cores (measured): a 32-deep chunk of a 128-column block takes 0.38 us with 256 rows (the MMAs' own rate), 0.28 with 128 and
 // 0.19 below (an MMA of 128 lanes takes as long with 32 rows as with 64); the epilogue of a block takes 0.4 us per 32 rows and
 // runs under the next block's main loop.
-double tile_us(bool tensor, unsigned th, unsigned tw, unsigned k, double gap) {
-    if (tensor) {
+// Beside the ring (measured): 64 x 32 blocks, 0.8 us and 1.0 per 32 of k (3 x 3 layers of 48 and 24 channels), 1.6 where operands
+// come value by value (attention with heads of 10); the softmax of scores 1.4 us per 1024.
+double tile_us(Path path, const aspen_layer_t *l, unsigned th, unsigned tw, unsigned k, double gap) {
+    if (path == TENSOR) {
         const unsigned chunks = ceil_div(k, 32), nb = ceil_div(tw, 128) * ceil_div(th, 256), rows = std::min(th, 256u);
         const double loop = chunks * (rows > 128 ? 0.38 : rows > 64 ? 0.28 : 0.19), epi = 0.6 + 0.4 * ceil_div(rows, 32);
         return gap + loop + epi + (nb - 1) * std::max(loop, epi);
+    }
+    if (path == BESIDE_RING) {
+        const bool pieces = l->type == CONV_LAYER ? l->params[IN_C] % 4 == 0 : l->type == K_ATTENTION_LAYER && k % 4 == 0;
+        const double softmax = l->type == K_ATTENTION_LAYER ? 1.4 * th * tw / 1024 : 0;
+        return gap + ceil_div(th, 64) * ceil_div(tw, 32) * (0.8 + ceil_div(k, 32) * (pieces ? 1.0 : 1.6)) + softmax;
     }
     // fp32 blocks (gemm_ffma.cuh), shapes as tile_gemm_ffma picks them: some 3 us for filling the pipeline, the reduction and the
     // stores, then steps of 32, 64 or 128 of k
@@ -42,7 +54,7 @@ double tile_us(bool tensor, unsigned th, unsigned tw, unsigned k, double gap) {
     return gap + (double)ceil_div(th, bm) * ceil_div(tw, bn) * (3.0 + ceil_div(k, kt) * (shape == 2 ? 1.3 : 2.0));
 }
 
-Grid choose(const nasm_ldata_t &ld, const nasm_t *nasm, bool tensor, unsigned sms, bool served) {
+Grid choose(const nasm_ldata_t &ld, const nasm_t *nasm, int precision, unsigned sms, bool served) {
     const aspen_layer_t *l = ld.layer;
     const unsigned *p = l->params;
     const unsigned H = ld.out_mat_dims[OUT_H], W = ld.out_mat_dims[OUT_W];
@@ -53,19 +65,20 @@ Grid choose(const nasm_ldata_t &ld, const nasm_t *nasm, bool tensor, unsigned sm
         g.th = (unsigned)round_up(std::min(64u, std::max(8u, ceil_div(H, 2 * sms))), 8);
         g.tw = W;
     } else if (contraction(l->type)) {
+        const Path path = path_of(l, precision, nasm->tr_seq_len);
         const bool ka = l->type == K_ATTENTION_LAYER, va = l->type == V_ATTENTION_LAYER;
         if (ka || va) g.seg = nasm->tr_seq_len;
         unsigned hs[8], nhs = 0;
         if (ka) hs[nhs++] = H;                                      // the softmax reduces over all keys
         else if (va) hs[nhs++] = p[NUM_HEAD] ? p[NUM_HIDDEN] / p[NUM_HEAD] : H;
-        else for (unsigned h : {512u, 256u, 128u, 64u, 32u}) if (h < 2 * H && (h <= 256 || tensor)) hs[nhs++] = h;
+        else for (unsigned h : {512u, 256u, 128u, 64u, 32u}) if (h < 2 * H && (h <= 256 || path == TENSOR)) hs[nhs++] = h;
         const unsigned k = ka ? p[NUM_HIDDEN] / std::max(1u, p[NUM_HEAD]) : va ? nasm->tr_seq_len : layer_contraction_k(l);
-        const unsigned quantum = tensor ? 128 : 32;
+        const unsigned quantum = path == TENSOR ? 128 : 32;
         double best = 0;
         for (unsigned i = 0; i < nhs; i++)
             for (unsigned tw = quantum; tw < g.seg + quantum && tw <= 16 * quantum; tw += quantum) {
                 const unsigned tiles = ceil_div(H, hs[i]) * (W / g.seg) * ceil_div(g.seg, tw);
-                const double us = tile_us(tensor, std::min(hs[i], H), std::min(tw, g.seg), k, served ? 2.5 : 4.0);
+                const double us = tile_us(path, l, std::min(hs[i], H), std::min(tw, g.seg), k, served ? 2.5 : 4.0);
                 const double share = (double)tiles / sms;
                 // The layer's work, and the length of its longest tile: launched alone the last tiles of a layer run while the
                 // rest of the chip waits, served the passes of other graphs fill those SMs but the graphs in rotation are few.
@@ -108,7 +121,10 @@ OperandForm operand_form(const aspen_layer_t *l, unsigned seq) {
     OperandForm f;
     f.c = p[IN_C];
     switch (l->type) {
-        case MATMUL_LAYER: case FC_LAYER: case V_ATTENTION_LAYER: f.kind = A_TMA; break;
+        case MATMUL_LAYER: case FC_LAYER: f.kind = A_TMA; break;
+        case V_ATTENTION_LAYER:            // a tile is a head's rows and has to start on a 16-byte boundary
+            if (p[NUM_HEAD] && p[NUM_HIDDEN] / p[NUM_HEAD] % 4 == 0) f.kind = A_TMA;
+            break;
         case K_ATTENTION_LAYER: {
             // all keys of a query have to fit the accumulators, and a head has to start on a 16-byte boundary
             const unsigned hd = p[NUM_HEAD] ? p[NUM_HIDDEN] / p[NUM_HEAD] : 0;
@@ -166,7 +182,7 @@ nasm_t *plan_device_tiles(const nasm_t *nasm, int precision, unsigned sms, bool 
     for (unsigned i = 0; i < plan->num_ldata; i++) {
         nasm_ldata_t &ld = plan->ldata[i];
         ld.nasm = plan.get();
-        Grid &g = grid[i] = choose(nasm->ldata[i], nasm, precision == 0, sms, served);
+        Grid &g = grid[i] = choose(nasm->ldata[i], nasm, precision, sms, served);
         const unsigned H = ld.out_mat_dims[OUT_H], W = ld.out_mat_dims[OUT_W];
         if (H == 0 || W == 0 || W % g.seg != 0) return nullptr;
         g.start = total;

@@ -76,8 +76,24 @@ def test_layers_of_any_channel_count_have_a_form_for_the_tensor_cores(workdir):
     assert forms == [(2, 1, 7 * 32), (2, 0, 9 * 64), (1, 0, 0), (2, 0, 64), (2, 0, 9 * 32), (0, 0, 0), (0, 0, 0), (1, 0, 0)]
 
 
-@pytest.mark.parametrize("heads,d,seq,form", [(2, 64, 100, 1), (2, 160, 100, 3), (4, 48, 512, 3), (4, 40, 100, 0), (2, 64, 513, 0)])
+@pytest.mark.parametrize("heads,d,seq,form", [(2, 64, 100, 1), (2, 160, 100, 3), (4, 48, 512, 3), (4, 40, 100, 0), (2, 64, 513, 0)])   # 0: not
 def test_attention_heads_of_a_multiple_of_four_have_a_form_for_the_tensor_cores(heads, d, seq, form, workdir):
     text, _ = cfgs.transformer(1, d, heads, d, pre_ln=False, masked=False, act="gelu")
     forms = operand_forms(workdir, text, seq)
-    assert [f[0] for f in forms[:6]] == [1, 1, 1, form, 1, 1]
+    assert [f[0] for f in forms[:6]] == [1, 1, 1, form, 1 if d // heads % 4 == 0 else 0, 1]
+
+
+@pytest.mark.parametrize("batch,seq,d,heads", [(2, 600, 256, 4), (8, 128, 120, 12)])
+def test_the_plan_spreads_layers_that_do_not_run_on_the_tensor_cores(batch, seq, d, heads, workdir):
+    """Scores of 600 keys, or of heads of 10: fp32 blocks one after the other on an SM, so no SM may be left with the work of several
+    (costed as tensor-core tiles they were 40 and 96 tiles for 148 SMs)."""
+    api.lib()
+    text, _ = cfgs.transformer(1, d, heads, d, pre_ln=False, masked=False, act="gelu")
+    exe = build("plan_tiles", workdir, f"-L{LIBDIR}", "-laspen_b200", f"-Wl,-rpath,{LIBDIR}")
+    cfg = os.path.join(workdir, "plan.cfg")
+    with open(cfg, "w") as f:
+        f.write(text)
+    r = subprocess.run([exe, cfg, str(batch), str(seq), "148"], capture_output=True, text=True, check=True).stdout
+    layers = [(line.split()[0], [int(v) for v in line.split()[1:]]) for line in r.split("\n")[:-1]]
+    th, tw, tiles = next(v for t, v in layers if "K_ATTENTION" in t)
+    assert tiles >= 148 and th == seq
