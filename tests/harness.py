@@ -13,7 +13,7 @@ NETS = {
     "tiny_cnn": ({}, "he", (11, 10)),
     "tiny_transformer": ({}, "n002", (13, 12)),
     "tiny_gpt": ({"masked": True, "pre_ln": True}, "n002", (15, 14)),
-    # head size 32: the smallest the fused attention tile takes (the 4-head variants above have head size 16)
+    # head size 32, one whole chunk of k (the 4-head variants above have head size 16)
     "tiny_attn": ({"heads": 2}, "n002", (21, 20)),
     "tiny_attn_causal": ({"heads": 2, "masked": True, "pre_ln": True}, "n002", (23, 22)),
     # heads of 10 and 12 features: tiles of one head's rows do not start on 16-byte boundaries, or only every other one does
