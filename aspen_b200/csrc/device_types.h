@@ -21,7 +21,7 @@ struct LayerDev {
     unsigned ld1, H1;
     const float *weight;      // [rows][Kpad] fp32, K contiguous, zero padded; layernorm: gain[rows]
     const float *bias;        // [rows]
-    unsigned K, Kpad, rows;
+    unsigned K, Kpad;
     unsigned IC, IH, IW, OH, OW, KH, KW, stride, pad;     // conv / pool geometry
     unsigned seq, heads, hd, masked;                     // attention
     unsigned p_out_c, p_in_c, p_stride;                  // yolo / append raw cfg parameters
@@ -63,7 +63,6 @@ struct TileDev {
     unsigned pos_h, pos_w;    // position in the layer's output matrix
     unsigned tile_h, tile_w;  // clipped extents
     unsigned child_off, child_cnt;
-    unsigned need;            // number of parent tiles (true dependencies)
 };
 
 // The layer-0 tiles run on the device and turn what the host uploaded into the layer's activation matrix, so a
@@ -93,7 +92,7 @@ struct NasmDev {
     unsigned *dep;                   // [n_tiles] parents completed since the launch
     volatile unsigned *completed;    // mapped host word: number of the last complete pass
     const void *wmaps;               // CUtensorMap[]
-    unsigned n_tiles, n_layers;
+    unsigned n_tiles;
     unsigned *svc;                   // SVC_* words in device memory
     unsigned n_exec;                 // tiles that complete in one pass (every tile but the ones whose parents write their values)
     unsigned n_input;                // layer-0 tiles (local ids 0 .. n_input-1): the seeds of a pass
@@ -113,7 +112,6 @@ struct CtrlDev {
     unsigned long long pipe_ns;    // time budget of in-kernel pipeline waits
     unsigned svc_stop;       // host request: leave once no pass is running or asked for
     unsigned svc_close;      // set by the device: everybody leaves (no error)
-    unsigned busy;           // graphs with a pass in progress
     unsigned ahead;          // a busy CTA lines up a second tile when at least this many ready tiles wait unclaimed (0: never)
     unsigned long long idle_ns;    // leave after this long without a pass in progress
 };

@@ -364,7 +364,6 @@ static void fill_layer(const nasm_t *nasm, const DeviceNasm *dn, unsigned i, int
     L.weight = dn->dd->weight[precision][i];
     L.bias = dn->dd->bias[i];
     L.anchors = dn->dd->anchors[i];
-    L.rows = layer_weight_rows(&l);
     L.K = layer_contraction_k(&l);
     L.Kpad = dn->dd->kpad[i];
     L.IC = p[IN_C]; L.IH = p[IN_H]; L.IW = p[IN_W]; L.OH = p[OUT_H]; L.OW = p[OUT_W];
@@ -749,7 +748,7 @@ static int build_device_nasm(Engine *e, nasm_t *host_nasm) {
     memset(&H, 0, sizeof H);
     H.layers = dn->layers; H.tiles = dn->tiles; H.children = dn->children; H.dep = dn->dep; H.wmaps = dn->wmaps;
     H.completed = dn->svc_done_d; H.svc = dn->svc_d;
-    H.n_tiles = n; H.n_layers = nasm->num_ldata; H.n_exec = n - n_bypassed; H.n_input = n_input;
+    H.n_tiles = n; H.n_exec = n - n_bypassed; H.n_input = n_input;
     return 0;
 }
 
@@ -1126,8 +1125,6 @@ double engine_time_passes(Engine *e, const std::vector<nasm_t *> &nasms, unsigne
     svc_pool_add(e, nasms);
     return timed(e, e->svc_pool, warmup, passes, launches, true);
 }
-
-void engine_flush() {}
 
 // Sums the per-CTA time accounting (ASPEN_B200_PROFILE=1) into out[PROF_SLOTS] and clears it.
 int engine_read_profile(Engine *e, unsigned long long *out, unsigned *n_ctas) {

@@ -140,8 +140,9 @@ unsigned int layer_weight_rows(const aspen_layer_t *l);
 // tiler.cpp
 extern TileQuanta g_quanta;
 
-// Output pixels per block of a convolution staged by strided TMA boxes, chosen so that a block is whole output
-// rows of one sample (or whole samples when a sample has at most 128 pixels): the block is then a single box.
+// Columns per tile quantum of a convolution when tiles are whole MMA blocks (column quantum 128): whole output rows of one sample, or
+// whole samples when a sample has at most 128 pixels.  The device executes a grid of its own and needs no such shape; graphs made
+// with these quanta, and the .nasm files written of them, name these tiles.
 inline unsigned conv_block_width(unsigned OW, unsigned OH) {
     if (OW == 0 || OH == 0 || OW > 128) return 128;
     if (OW * OH <= 128) return (128 / (OW * OH)) * OW * OH;
@@ -150,8 +151,7 @@ inline unsigned conv_block_width(unsigned OW, unsigned OH) {
         if (OH % d == 0) k = d;
     return k * OW;
 }
-// The convolutions that get that staging when tiles are whole MMA blocks (column quantum 128): IC a multiple of
-// 32 and neither a 1x1 stride-1 layer (plain 2-D boxes) nor a stride-1 "same" layer (shifted box + fix-up).
+// The convolutions that it applies to: IC a multiple of 32 and neither a 1x1 stride-1 layer nor a stride-1 "same" layer.
 inline bool conv_uses_row_blocks(const aspen_layer_t *l) {
     if (l->type != CONV_LAYER) return false;
     const unsigned *p = l->params;
@@ -198,5 +198,4 @@ int engine_status(Engine *e);
 long engine_read_ldata(nasm_t *nasm, unsigned int ldata_idx, float *out_packed);
 double engine_time_runs(Engine *e, const std::vector<nasm_t *> &nasms, unsigned int warmup, unsigned int iters, unsigned long long *launches);
 void engine_release_dnn(aspen_dnn_t *dnn);
-void engine_flush();
 int engine_read_profile(Engine *e, unsigned long long *out, unsigned *n_ctas);

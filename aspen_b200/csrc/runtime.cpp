@@ -228,7 +228,8 @@ extern "C" int aspen_b200_group_profile(dse_group_t *g, unsigned long long *out6
     return g ? engine_read_profile(g->engine, out64, n_ctas) : -1;
 }
 
-extern "C" void aspen_flush_dynamic_memory(void) { engine_flush(); }
+// The reference returns cached host blocks here; this library caches none.
+extern "C" void aspen_flush_dynamic_memory(void) {}
 
 extern "C" int aspen_b200_set_device(int device);   // engine.cu
 

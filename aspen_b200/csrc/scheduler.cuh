@@ -149,7 +149,6 @@ static __device__ unsigned svc_scan(const NasmDev *nasms, unsigned n_nasm, CtrlD
                     const unsigned started = ld_relaxed(&G.svc[SVC_STARTED]);
                     if (ld_acquire_sys(&G.svc[SVC_TARGET]) != started) {
                         asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(&G.svc[SVC_STARTED]), "r"(started + 1u) : "memory");
-                        atomicAdd(&ctrl->busy, 1u);
                         go = 4u;
                     } else asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(&G.svc[SVC_IDLE]), "r"(1u) : "memory");
                 } else go = 1u;
@@ -175,7 +174,6 @@ static __device__ void end_of_pass(const NasmDev *nasms, unsigned n_nasm, unsign
         __threadfence_system();
         *G.completed = ld_relaxed(&G.svc[SVC_BASE]) + t / G.n_exec;          // mapped host word: number of the pass that is complete
         __threadfence_system();
-        atomicSub(&ctrl->busy, 1u);
         asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(&G.svc[SVC_IDLE]), "r"(1u) : "memory");
     }
     __syncwarp();
@@ -209,7 +207,7 @@ static __global__ void arm_kernel(const NasmDev *nasms, CtrlDev *ctrl, Entry *qu
     if (t0 == 0 && a.g0 == 0) {
         ctrl->head = 0u; ctrl->tail = 0u; ctrl->done = 0u; ctrl->total = a.total; ctrl->cap = a.cap; ctrl->n_nasm = a.n_nasm;
         ctrl->abort = 0u; ctrl->stop = 0u; ctrl->stall_ns = a.stall_ns; ctrl->pipe_ns = a.pipe_ns;
-        ctrl->svc_stop = a.svc_stop; ctrl->svc_close = 0u; ctrl->busy = 0u; ctrl->idle_ns = a.idle_ns; ctrl->ahead = a.ahead;
+        ctrl->svc_stop = a.svc_stop; ctrl->svc_close = 0u; ctrl->idle_ns = a.idle_ns; ctrl->ahead = a.ahead;
     }
 }
 

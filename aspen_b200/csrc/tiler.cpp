@@ -70,15 +70,14 @@ static bool out_mat_info(nasm_ldata_t *ld) {
     }
 }
 
-// First guess: grow a (h_min x w_min) tile until it holds flop_per_ninst of work, rows first.
-// Column quantum of a layer: the global one, except for convolutions staged by strided TMA boxes when tiles are
-// whole MMA blocks -- their tiles are made of blocks of whole output rows (conv_block_width).
+// Column quantum of a layer: the global one, but for some convolutions when tiles are whole MMA blocks (conv_block_width).
 static unsigned int layer_w_quantum(const nasm_ldata_t *ld) {
     const TileQuanta &q = ld->nasm->quanta;
     if (q.w_min == 128 && conv_uses_row_blocks(ld->layer)) return conv_block_width(ld->layer->params[OUT_W], ld->layer->params[OUT_H]);
     return q.w_min;
 }
 
+// First guess: grow a (h_min x w_min) tile until it holds flop_per_ninst of work, rows first.
 static void initial_tile_dims(nasm_ldata_t *ld) {
     const TileQuanta &q = ld->nasm->quanta;
     const unsigned int w_min = layer_w_quantum(ld);
