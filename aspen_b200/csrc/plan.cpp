@@ -6,7 +6,8 @@
 // whole network leaves SMs idle in the late layers or makes the early ones pay per tile.  Here every layer gets the
 // shape with the lowest estimated time on the SMs at hand.  The plan is a nasm of the same layers with that grid and
 // with the parents each tile reads (by region, so a graph of ten thousand tiles takes milliseconds).
-// Graphs whose lists a file has changed keep their own tiles and lists.
+// Graphs whose lists a file has changed keep their own tiles and lists.  A plan is made for launched or for served passes, whichever
+// mode the group is in when the graph's image is built; it stays when the mode changes later (the values are the same).
 #include "internal.h"
 #include "device_types.h"
 
@@ -31,9 +32,9 @@ enum Path { TENSOR, BESIDE_RING, FP32 };      // tensor cores / fp32 blocks in a
 Path path_of(const aspen_layer_t *l, int precision, unsigned seq) { return precision != 0 ? FP32 : operand_form(l, seq).kind != A_NONE ? TENSOR : BESIDE_RING; }
 
 // Estimated microseconds of one tile of th x tw outputs with a k-deep contraction, `gap` of them between two tiles of an SM.
-// Tensor cores (measured): a 32-deep chunk of a 128-column block takes 0.38 us with 256 rows (the MMAs' own rate), 0.28 with 128 and
-// 0.19 below (an MMA of 128 lanes takes as long with 32 rows as with 64); the epilogue of a block takes 0.4 us per 32 rows and
-// runs under the next block's main loop.
+// Tensor cores: what a 32-deep chunk of a 128-column block takes inside a network, where part of the operands comes from HBM -- 0.38 us
+// with 256 rows, 0.28 with 128 and 0.19 below (0.30 - 0.37, 0.22 and 0.16 with everything in L2: tiles_tc.cuh); the epilogue of a
+// block takes 0.4 us per 32 rows and runs under the next block's main loop.
 // Beside the ring (measured): 64 x 32 blocks, 0.8 us and 1.0 per 32 of k (3 x 3 layers of 48 and 24 channels), 1.6 where operands
 // come value by value (attention with heads of 10); the softmax of scores 1.4 us per 1024.
 double tile_us(Path path, const aspen_layer_t *l, unsigned th, unsigned tw, unsigned k, double gap) {
@@ -82,9 +83,11 @@ Grid choose(const nasm_ldata_t &ld, const nasm_t *nasm, int precision, unsigned 
                 const double share = (double)tiles / sms;
                 // The layer's work, and the length of its longest tile: launched alone the last tiles of a layer run while the
                 // rest of the chip waits, served the passes of other graphs fill those SMs but the graphs in rotation are few.
-                // (Served, 0.2 / 0.5 / 1.0 tiles: 1.92 / 1.61 / 1.51 ms a request for ResNet-50 x 32 in bursts of twelve, 0.279 /
-                // 0.283 / 0.304 for x 4.  Launched, whole rounds of the SMs instead: GPT-2 8 x 512 2.93 ms, ResNet-50 x 32 1.64;
-                // 0.7 / 1.0 / 1.5 tiles: 2.59 / 2.64 / 3.06 and 1.57 / 1.54 / 1.55.)
+                // (Launched, whole rounds of the SMs instead: GPT-2 8 x 512 2.93 ms, ResNet-50 x 32 1.64; 0.7 / 1.0 / 1.5 tiles:
+                // 2.59 / 2.64 / 3.06 and 1.57 / 1.54 / 1.55.)  Served, the best weight falls with the work that the other graphs
+                // offer each SM, which a plan of one graph does not know: three graphs of ResNet-50 x 32 in bursts of twelve take
+                // 1.92 / 1.61 / 1.51 ms a request with 0.2 / 0.5 / 1.0 tiles, eight of x 4 take 0.279 / 0.283 / 0.304.  0.5 lies
+                // between the two.
                 const double cost = us * (share + (served ? 0.5 : 0.7));
                 if (best == 0 || cost < best * 0.999) { best = cost; g.th = hs[i]; g.tw = tw; }
             }

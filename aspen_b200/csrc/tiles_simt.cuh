@@ -129,11 +129,6 @@ static __device__ __forceinline__ void tile_residual(const LayerDev &L, const Ti
     else residual_loop<ACT_OTHER>(L, T, tid, nthr);
 }
 
-// ref src/tiled_kernels.c:411-501.  Max ignores padded taps (all padded -> -inf); average divides by
-// the full window size, padding counted.  A thread owns four channels of an output pixel and works on two such
-// items at a time; the window's taps are fetched nine at a time (a whole 3 x 3 window), all loads of both items
-// issued before the first is used (a tap outside the image reads nothing and contributes the neutral element),
-// so the tile is bound by bandwidth instead of one load latency per tap.
 // Max pooling with a small window, whole 16-byte pieces of channels: taps outside the image are moved to the nearest pixel inside,
 // which the window contains as well, so all KH x KW loads of U outputs are unconditional and in flight together.  With a
 // test per tap the loads went out a few at a time: 64 x 100352 outputs (3 x 3, stride 2) 158 -> 40 us per SM.
@@ -207,6 +202,11 @@ static __device__ __noinline__ void tile_avg_inside(const LayerDev &L, const Til
     }
 }
 
+// Pooling of any window (ref src/tiled_kernels.c:411-501).  Max ignores padded taps (all padded -> -inf); average divides by
+// the full window size, padding counted.  A thread owns four channels of an output pixel and works on two such
+// items at a time; the window's taps are fetched nine at a time (a whole 3 x 3 window), all loads of both items
+// issued before the first is used (a tap outside the image reads nothing and contributes the neutral element),
+// so the tile is bound by bandwidth instead of one load latency per tap.
 template <bool IS_MAX>
 static __device__ __noinline__ void tile_pool(const LayerDev &L, const TileDev &T, unsigned tid, unsigned nthr) {
     const unsigned h4 = ((T.pos_h | L.ld0 | L.ldc) & 3u) ? 0u : T.tile_h >> 2, per_col = T.tile_h - 3u * h4;   // whole aligned pieces, and the rest
@@ -491,9 +491,9 @@ static __device__ __noinline__ void tile_transposed_copy(const LayerDev &L, cons
     }
 }
 
-// Layer-0 tile: the uploaded input becomes the columns of the layer's activation matrix that the
-// tile covers -- what the host-launched unpack / rounding / embedding-gather / padded-copy kernels do for a run that
-// is launched per graph.  Sources are read through L2 (the host's DMA wrote them while this kernel was running).
+// Layer-0 tile: the uploaded input becomes the columns of the layer's activation matrix that the tile covers: scatter into the column
+// stride, rounding, embedding rows of token ids, and the zero-padded copy of a small image.  Sources are read through L2: the
+// host's DMA may have written them while this kernel was running.
 static __device__ void tile_input(const InputDev &I, const LayerDev &L, const TileDev &T, unsigned tid, unsigned nthr) {
     const unsigned H = L.H;
     if (I.ids) {
@@ -833,8 +833,9 @@ static __device__ __forceinline__ void tile_gemv(const LayerDev &L, const TileDe
 }
 
 // Tile in fp32 (ref src/tiled_kernels.c:21-490, 784-1038).  FULL: the fp32 mode, 96 KB of staging; the shape of the blocks
-// follows the tile (a shape larger than the tile would compute padding).  Otherwise the few layers of a tensor-core graph that
-// no TMA box can stage (IC % 32 != 0, head size % 32 != 0, ...).
+// follows the tile (a shape larger than the tile would compute padding).  Otherwise the few layers of a tensor-core graph without an
+// operand form: scores of heads that are no multiple of four features or of more than 512 keys, values of such heads, convolutions
+// past an im2col map's limits.
 template <bool FULL>
 static __device__ void tile_gemm_ffma(const LayerDev &L, const TileDev &T, unsigned tid, unsigned nthr, unsigned char *scratch) {
     if (L.gemv) { tile_gemv(L, T, tid, nthr); return; }

@@ -5,26 +5,30 @@
 // features, m contiguous in memory).  The MMA is issued as D[128 x N] with
 //     MMA-M (128 TMEM lanes)  <- 128 consecutive tile columns n   (operand "X": activations)
 //     MMA-N (<=256 TMEM cols) <- tile rows m                      (operand "W": weights / keys / V)
-// so each epilogue thread owns one output column n and writes runs of contiguous m, and the
-// K-attention softmax (a reduction over m) stays inside one thread.
+// so an accumulator lane is one output column n.  The epilogue transposes 32 x 32 pieces through shared memory, after which
+// consecutive lanes store consecutive m; the K-attention softmax (a reduction over m) sums a lane's own column, half of the
+// pieces in each of the two warps of a query quarter.
 //
 // Roles.  A tile is a sequence of 128 x (<= 256) blocks, and four kinds of warps walk the same sequence, each at its own pace
 // and across tile boundaries; nothing but mbarriers connects them:
-//     warp A, warp B   one thread each: TMA boxes of the X / W operand into a ring of stages (32 fp32 of k per stage)
-//     warp MMA         one thread: four tcgen05.mma (k = 8 each) per stage, accumulators alternate between two halves of TMEM
+//     warp A, warp B   one thread each: TMA boxes of the X / W operand into a ring of stages (32 fp32 of k a chunk, up to four chunks
+//                      a stage)
+//     warp MMA         one thread: four tcgen05.mma (k = 8 each) per chunk, accumulators alternate between two halves of TMEM
 //     8 worker warps   epilogue: TMEM -> registers -> bias, activation, residual add, softmax -> memory; they also run the
 //                      memory-bound tiles
 // so the operands of the next block (or of the next tile, once the scheduler has posted one) stream in and are multiplied
 // while the previous block is written out.
-// Two threads feed the ring because one is not fast enough: a probe that only waits and issues measured 0.24 us per stage
-// for one thread with two boxes (0.32 with five), whatever their size up to 48 KB, while the four MMAs of a 128 x 128
-// stage take 0.14 us and of a 128 x 256 stage 0.28.  The loops below hold no division for the same reason.
+// What bounds the k loop.  A one-thread role takes 0.17 us for a wait and a box whatever it holds (a probe that only waits and
+// issues; 0.24 with two boxes, 0.043 a chunk with four chunks in a box), so two threads feed the ring and narrow tiles take several
+// chunks a stage.  A chunk of a 128-column block then takes 0.16 us with 32 or 64 rows, 0.22 with 128 and 0.30 - 0.37 with 256 (all
+// SMs at work, operands in L2; 256 rows is the rate of the measured dense TF32 peak).  The loops below hold no division for the
+// same reason.
 //
 // Staging.  Both operands are K-major, 32 fp32 (128 bytes) per row and k-chunk, in the 128-byte swizzled shared-memory
 // layout UMMA descriptors and TMA share.  A narrow layer (few tokens, few pixels) stages only the columns it has; the MMA reads
-// 128 rows all the same, whatever lies there: those accumulator lanes have no reader.  The ring is cut into as many stages as the tile's row count allows (8 of 24 KB
-// for 64 rows, 6 of 32 KB for 128, 4 of 48 KB for 256); when the cut changes between two tiles both producers first
-// wait until the old stages have been read.
+// 128 rows all the same, whatever lies there: those accumulator lanes have no reader.  The ring is cut into stages of four
+// chunks for tiles of up to 64 rows (2 stages of 96 KB), two up to 128 (3 of 64 KB), one above (4 of 48 KB); when the cut
+// changes between two tiles both producers first wait until the old stages have been read.
 //
 // Every wait is bounded: when a time budget runs out the thread records an error and raises the abort flag, every role
 // leaves its loop, producers let their copies land, and the CTA frees its TMEM and exits.  (The workers' barriers: worker_loop.h.)
@@ -452,7 +456,7 @@ __device__ __forceinline__ void store_piece(const Piece &p, float *out /*(n = 0,
 }
 // The other operand of a fused residual add.  A warp asks for it two of its pieces ahead (the first ones before the
 // accumulator is waited for), so it lands under the main loop or under the previous pieces' stores: one piece ahead measured
-// 142 us for a 256 x 768 tile with k = 64 (every piece waits for HBM), two ahead 74.
+// 142 us for a 256 x 768 tile with k = 64 (every piece waits for HBM), two ahead 74, and 51 once rare activations had left the loop.
 __device__ __forceinline__ void load_piece(Piece &p, const float *in, size_t ld, unsigned n_valid, unsigned m_valid) {
     const unsigned lane = threadIdx.x & 31u, m = (lane & 7u) * 4u, n0 = lane >> 3;
     const float *src = in + (size_t)n0 * ld + m;
