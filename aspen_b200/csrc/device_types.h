@@ -27,6 +27,7 @@ struct LayerDev {
     unsigned p_out_c, p_in_c, p_stride;                  // yolo / append raw cfg parameters
     const float *anchors;
     unsigned tc;              // the layer's tiles run on the tensor cores
+    unsigned meets;           // its tiles have barriers of the worker warps: the softmax of scores, fp32 blocks, a stored tile read back (vt_out)
     unsigned gemv;            // at most 8 columns, each one contiguous run of K values: dot products (tile_gemv)
     unsigned x_ld;            // ... distance between those columns
     int wmap;                 // tensor map of the W-side operand (weights, PARENT_1 for attention keys, transposed values)
@@ -58,7 +59,7 @@ struct LayerDev {
     unsigned vt_ld, vt_seq;
 };
 
-struct TileDev {
+struct alignas(32) TileDev {        // a whole sector, one load for the scheduler
     unsigned layer;
     unsigned pos_h, pos_w;    // position in the layer's output matrix
     unsigned tile_h, tile_w;  // clipped extents

@@ -613,6 +613,10 @@ static int build_device_nasm(Engine *e, nasm_t *host_nasm) {
         }
     }
     dn->round_input = layers[0].round_out != 0;
+    for (LayerDev &L : layers) {
+        const bool contraction = L.type == CONV_LAYER || L.type == FC_LAYER || L.type == MATMUL_LAYER || L.type == K_ATTENTION_LAYER || L.type == V_ATTENTION_LAYER;
+        L.meets = L.tc ? L.type == K_ATTENTION_LAYER : L.vt_out != nullptr || (contraction && !L.gemv);
+    }
     // Residual fusion (tensor-core path): a residual layer whose later parent is a convolution or a matmul
     // is computed in that parent's epilogue, which then needs the earlier parent's tiles of the same region
     // (fused_other[producer] = that layer).  The residual layer's own tiles leave the device

@@ -481,13 +481,7 @@ struct WorkerWarp {
         return __all_sync(0xffffffffu, wait_posted(&sh->posted[seq % tc::SLOTS], (seq / tc::SLOTS) & 1u, ctrl, status));
     }
     __device__ __forceinline__ bool live(unsigned seq) const { return slot(seq).live != 0u; }
-    // the softmax of attention scores, fp32 blocks, and a stored tile that is read back for its transposed copy
-    __device__ __forceinline__ bool meets(unsigned seq) const {
-        const LayerDev &L = slot(seq).layer;
-        if (L.type == K_ATTENTION_LAYER) return true;
-        if (tensor(slot(seq))) return false;
-        return L.vt_out != nullptr || (!L.gemv && (L.type == CONV_LAYER || L.type == FC_LAYER || L.type == MATMUL_LAYER || L.type == V_ATTENTION_LAYER));
-    }
+    __device__ __forceinline__ bool meets(unsigned seq) const { return slot(seq).layer.meets != 0u; }
     __device__ __forceinline__ bool agree(bool yes) const {
         unsigned all;
         __syncwarp();

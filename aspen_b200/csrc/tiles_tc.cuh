@@ -287,22 +287,37 @@ __device__ __forceinline__ bool produce_a(const Slot &sl, unsigned ring, Ring &r
     // activations were written with ordinary (generic proxy) stores; TMA reads them through the async proxy
     asm volatile("fence.proxy.async.global;" ::: "memory");
     if (!recut(r, L, sh, ctrl, status)) return false;
-    const bool im2col = L.a_kind == A_IM2COL, heads = L.a_kind == A_HEAD;
-    const unsigned multi = L.a_multi, tile_w = sl.tile.tile_w, tile_h = sl.tile.tile_h, pos_w = sl.tile.pos_w;
-    const unsigned OW = L.OW, OH = L.OH, KW = L.tap_kw, C = L.tap_c, sx = L.tap_sx, sy = L.tap_sy, per = L.per_stage, chunk_bytes = L.a_rows * 128u;
-    const int pad = (int)L.tap_pad;
+    const unsigned kind = L.a_kind, tile_w = sl.tile.tile_w, tile_h = sl.tile.tile_h, per = L.per_stage, chunk_bytes = L.a_rows * 128u;
+    if (kind == A_IM2COL) {
+        const unsigned pos_w = sl.tile.pos_w, OW = L.OW, hw = L.OH * OW, KW = L.tap_kw, C = L.tap_c, sx = L.tap_sx, sy = L.tap_sy, chunks = L.chunks;
+        const int pad = (int)L.tap_pad;
+        for (unsigned n0 = 0; n0 < tile_w; n0 += 128u) {
+            const unsigned n = pos_w + n0, pn = n / hw, q = n - pn * hw, py = q / OW, px = q - py * OW;      // first output pixel of the block
+            const int x0 = (int)(px * sx) - pad, y0 = (int)(py * sy) - pad;
+            for (unsigned mp = 0; mp < tile_h; mp += BLOCK_ROWS) {
+                unsigned kh = 0, kw = 0, c = 0;      // tap and first channel of the next chunk; c runs fastest
+                for (unsigned ch = 0; ch < chunks; ch += per) {
+                    const unsigned count = min(per, chunks - ch);
+                    unsigned dst = ring + r.s * r.stage_bytes;
+                    if (!mbar_wait(&sh->empty[r.s], r.parity() ^ 1u, ctrl, status, 2)) return false;
+                    mbar_arrive_expect_tx(&sh->full[r.s], count * chunk_bytes);
+                    for (unsigned j = 0; j < count; j++, dst += chunk_bytes) {
+                        tma_load_im2col(dst, map, (int)c, x0, y0, (int)pn, kw, kh, &sh->full[r.s]);
+                        c += 32u;
+                        if (c == C) { c = 0; if (++kw == KW) { kw = 0; kh++; } }
+                    }
+                    r.step();
+                }
+            }
+        }
+        return true;
+    }
+    const bool multi = L.a_multi != 0;
     for (unsigned n0 = 0; n0 < tile_w; n0 += 128u) {
         const unsigned chunks = g.chunks(L, n0);
-        unsigned px = 0, py = 0, pn = 0;             // first output pixel of the block
-        if (im2col) {
-            const unsigned n = pos_w + n0, hw = OH * OW;
-            pn = n / hw;
-            const unsigned q = n - pn * hw;
-            py = q / OW; px = q - py * OW;
-        }
+        const int y = g.ay + (int)n0;
         for (unsigned mp = 0; mp < tile_h; mp += BLOCK_ROWS) {
             if (multi) {
-                const int y = g.ay + (int)n0;
                 for (unsigned ch = 0; ch < chunks; ch += per) {
                     if (!mbar_wait(&sh->empty[r.s], r.parity() ^ 1u, ctrl, status, 2)) return false;
                     mbar_arrive_expect_tx(&sh->full[r.s], per * chunk_bytes);
@@ -311,20 +326,14 @@ __device__ __forceinline__ bool produce_a(const Slot &sl, unsigned ring, Ring &r
                 }
                 continue;
             }
-            unsigned kh = 0, kw = 0, c = 0;          // tap and first channel of the next chunk; c runs fastest
-            const int x0 = (int)(px * sx) - pad, y0 = (int)(py * sy) - pad;
             for (unsigned ch = 0; ch < chunks; ch += per) {
-                const unsigned n = min(per, chunks - ch);
+                const unsigned count = min(per, chunks - ch);
                 unsigned dst = ring + r.s * r.stage_bytes;
                 if (!mbar_wait(&sh->empty[r.s], r.parity() ^ 1u, ctrl, status, 2)) return false;
-                mbar_arrive_expect_tx(&sh->full[r.s], n * chunk_bytes);
-                for (unsigned j = 0; j < n; j++, dst += chunk_bytes) {
-                    if (im2col) {
-                        tma_load_im2col(dst, map, (int)c, x0, y0, (int)pn, kw, kh, &sh->full[r.s]);
-                        c += 32u;
-                        if (c == C) { c = 0; if (++kw == KW) { kw = 0; kh++; } }
-                    } else if (heads) tma_load_3d(dst, map, (int)(ch + j) * 32, g.ax, g.ay + (int)n0, &sh->full[r.s]);
-                    else tma_load_2d(dst, map, (g.ax + (int)(ch + j)) * 32, g.ay + (int)n0, &sh->full[r.s]);
+                mbar_arrive_expect_tx(&sh->full[r.s], count * chunk_bytes);
+                for (unsigned j = 0; j < count; j++, dst += chunk_bytes) {
+                    if (kind == A_HEAD) tma_load_3d(dst, map, (int)(ch + j) * 32, g.ax, y, &sh->full[r.s]);
+                    else tma_load_2d(dst, map, (g.ax + (int)(ch + j)) * 32, y, &sh->full[r.s]);
                 }
                 r.step();
             }
