@@ -371,7 +371,7 @@ static void fill_layer(const nasm_t *nasm, const DeviceNasm *dn, unsigned i, int
     if (l.type == FC_LAYER) { L.KH = p[IN_H]; L.KW = p[IN_W]; L.OH = 1; L.OW = 1; L.stride = 1; L.pad = 0; }
     if (dn->dd->ic_pad[i]) { L.IC = dn->dd->ic_pad[i]; L.K = L.KH * L.KW * L.IC; }
     L.by_ic = make_divisor(L.IC); L.by_kw = make_divisor(L.KW);
-    L.seq = nasm->tr_seq_len; L.heads = p[NUM_HEAD]; L.hd = p[NUM_HEAD] ? p[NUM_HIDDEN] / p[NUM_HEAD] : 0; L.masked = p[MASKED];
+    L.seq = nasm->tr_seq_len; L.heads = p[NUM_HEAD]; L.hd = p[NUM_HEAD] ? p[NUM_HIDDEN] / p[NUM_HEAD] : 0; L.masked = p[MASKED] != 0;
     L.p_out_c = p[OUT_C]; L.p_in_c = p[IN_C]; L.p_stride = p[STRIDE];
     L.wmap = -1;
     L.amap = -1;
@@ -506,7 +506,7 @@ static int build_device_nasm(Engine *e, nasm_t *host_nasm) {
         auto cut_ring = [&](unsigned k) {
             L.b_rows = (unsigned)round_up(std::min(th, tc::BLOCK_ROWS), 16);
             L.chunks = std::max(1u, (k + 31) / 32);
-            L.per_stage = std::min(L.chunks, L.b_rows <= 64 ? 4u : L.b_rows <= 128 ? 2u : 1u);
+            L.per_stage = (unsigned char)std::min(L.chunks, L.b_rows <= 64 ? 4u : L.b_rows <= 128 ? 2u : 1u);
             L.a_rows = std::min(128u, (unsigned)round_up(std::min(nasm->ldata[i].ninst_tile_dims[OUT_W], L.W), 8));
             L.stage_bytes = L.per_stage * (L.a_rows + L.b_rows) * 128;
             L.stages = std::min(tc::MAX_STAGES, tc::RING_BYTES / L.stage_bytes);

@@ -280,14 +280,13 @@ __device__ __forceinline__ bool wait_posted(unsigned long long *bar, unsigned pa
 static __device__ __forceinline__ void post(tc::Slot &sl, unsigned long long &posted, const tc::GraphRef &G, Entry entry) {
     const unsigned lane = threadIdx.x & 31u, g = (unsigned)(entry >> 48), layer = (unsigned)(entry >> 32) & 0xffffu, tile = (unsigned)entry - 1u;
     constexpr unsigned LW = sizeof(LayerDev) / 4, TW = sizeof(TileDev) / 4;
-    static_assert(sizeof(LayerDev) % 4 == 0 && LW <= 96 && TW <= 32, "copied in words");
+    static_assert(LW == 64 && TW <= 32, "copied in words");
     const unsigned *lsrc = reinterpret_cast<const unsigned *>(G.layers + layer), *tsrc = reinterpret_cast<const unsigned *>(G.tiles + tile);
-    unsigned lw[3] = {}, tw = 0;
-    #pragma unroll
-    for (unsigned i = 0; i < 3; i++) if (i * 32u + lane < LW) lw[i] = __ldg(lsrc + i * 32u + lane);
+    const unsigned l0 = __ldg(lsrc + lane), l1 = __ldg(lsrc + 32u + lane);
+    unsigned tw = 0;
     if (lane < TW) tw = __ldg(tsrc + lane);
-    #pragma unroll
-    for (unsigned i = 0; i < 3; i++) if (i * 32u + lane < LW) reinterpret_cast<unsigned *>(&sl.layer)[i * 32u + lane] = lw[i];
+    reinterpret_cast<unsigned *>(&sl.layer)[lane] = l0;
+    reinterpret_cast<unsigned *>(&sl.layer)[32u + lane] = l1;
     if (lane < TW) reinterpret_cast<unsigned *>(&sl.tile)[lane] = tw;
     if (lane == 0) { sl.live = 1u; sl.nasm = g; sl.maps = G.maps; sl.input = G.input; }
     __syncwarp();
