@@ -461,23 +461,27 @@ static __device__ __forceinline__ void single_thread_role(unsigned char *smem, t
     }
 }
 
-// What a worker warp does at each step of worker_loop.
+// What a worker warp does at each step of worker_loop.  It keeps next to nothing across a tile -- the tiles are calls, and what does not
+// fit the registers that they leave would come back by an L2 round trip.
 template <bool TENSOR_CORES>
 struct WorkerWarp {
-    unsigned char *smem;
-    tc::Shared *sh;
     CtrlDev *ctrl;
     StatusHost *status;
-    unsigned long long *prof;
-    unsigned wt;                                 // worker thread 0 .. tc::NW - 1
+    unsigned long long *prof;                    // of all CTAs, or nullptr
     unsigned half = 0, acc_uses = 0;
-    unsigned long long t_mark = 0;
 
-    __device__ __forceinline__ const tc::Slot &slot(unsigned seq) const { return sh->slots[seq % tc::SLOTS]; }
-    __device__ __forceinline__ bool tensor(const tc::Slot &sl) const { return TENSOR_CORES && sl.layer.tc; }
+    __device__ __forceinline__ static unsigned char *smem() { extern __shared__ __align__(1024) unsigned char work[]; return work; }
+    __device__ __forceinline__ static tc::Shared *sh() { return reinterpret_cast<tc::Shared *>(smem() + work_bytes<TENSOR_CORES>()); }
+    __device__ __forceinline__ static unsigned wt() { return threadIdx.x - (TENSOR_CORES ? tc::WARP_WORK : 1u) * 32u; }     // worker thread 0 .. tc::NW - 1
+    __device__ __forceinline__ static tc::Slot &slot(unsigned seq) { return sh()->slots[seq % tc::SLOTS]; }
+    // time since the last call, for the accounting of the CTA (one thread)
+    __device__ __forceinline__ static unsigned long long lap() {
+        const unsigned long long now = global_ns(), t = now - sh()->prof_mark;
+        sh()->prof_mark = now;
+        return t;
+    }
     __device__ __forceinline__ bool posted(unsigned seq) {
-        if (prof && seq == 0) t_mark = global_ns();
-        return __all_sync(0xffffffffu, wait_posted(&sh->posted[seq % tc::SLOTS], (seq / tc::SLOTS) & 1u, ctrl, status));
+        return __all_sync(0xffffffffu, wait_posted(&sh()->posted[seq % tc::SLOTS], (seq / tc::SLOTS) & 1u, ctrl, status));
     }
     __device__ __forceinline__ bool live(unsigned seq) const { return slot(seq).live != 0u; }
     __device__ __forceinline__ bool meets(unsigned seq) const { return slot(seq).layer.meets != 0u; }
@@ -489,21 +493,19 @@ struct WorkerWarp {
         return all != 0u;
     }
     __device__ __forceinline__ bool run(unsigned seq) {
-        const tc::Slot &sl = slot(seq);
-        if (prof && wt == 0) { unsigned long long now = global_ns(); prof[PROF_SLOTS - 1] += now - t_mark; t_mark = now; }
+        if (prof && wt() == 0) prof[(size_t)blockIdx.x * PROF_SLOTS + PROF_SLOTS - 1] += lap();
         bool ok = true;
-        if (tensor(sl)) ok = tc::epilogue_tile(sl, half, acc_uses, smem + tc::RING_BYTES, sh, ctrl, status);
-        else worker_tile<TENSOR_CORES>(sl, wt, smem + (TENSOR_CORES ? tc::RING_BYTES : 0u));
-        if (prof && wt == 0) {
-            unsigned long long now = global_ns();
-            const unsigned l = sl.tile.layer % PROF_LAYERS;
-            prof[2 + l] += now - t_mark; prof[2 + PROF_LAYERS + l] += 1ull; t_mark = now;
+        if (TENSOR_CORES && slot(seq).layer.tc) ok = tc::epilogue_tile(slot(seq), half, acc_uses, smem() + tc::RING_BYTES, sh(), ctrl, status);
+        else worker_tile<TENSOR_CORES>(slot(seq), wt(), smem() + (TENSOR_CORES ? tc::RING_BYTES : 0u));
+        if (prof && wt() == 0) {
+            unsigned long long *mine = prof + (size_t)blockIdx.x * PROF_SLOTS + 2 + slot(seq).tile.layer % PROF_LAYERS;
+            mine[0] += lap(); mine[PROF_LAYERS] += 1ull;
         }
         return ok;
     }
     __device__ __forceinline__ void finished(unsigned seq) const {
         __syncwarp();
-        if ((wt & 31u) == 0u) tc::mbar_arrive(&sh->finished[seq % tc::SLOTS]);      // release (CTA scope): this warp's stores of the tile
+        if ((threadIdx.x & 31u) == 0u) tc::mbar_arrive(&sh()->finished[seq % tc::SLOTS]);      // release (CTA scope): this warp's stores of the tile
     }
 };
 
@@ -520,6 +522,7 @@ scheduler_kernel(const NasmDev *nasms, CtrlDev *ctrl, Entry *queue, StatusHost *
     constexpr unsigned sched_warp = TENSOR_CORES ? tc::WARP_SCHED : 0u, first_worker = TENSOR_CORES ? tc::WARP_WORK : 1u;
 
     if (tid == 0) {
+        sh->prof_mark = global_ns();
         for (unsigned s = 0; s < tc::MAX_STAGES; s++) { tc::mbar_init(&sh->full[s], 2u); tc::mbar_init(&sh->empty[s], 1u); }
         for (unsigned h = 0; h < 2; h++) { tc::mbar_init(&sh->acc_full[h], 1u); tc::mbar_init(&sh->acc_empty[h], tc::NW / 32u); }
         for (unsigned k = 0; k < tc::SLOTS; k++) { tc::mbar_init(&sh->posted[k], 1u); tc::mbar_init(&sh->finished[k], tc::NW / 32u + (TENSOR_CORES ? 3u : 0u)); }
@@ -537,8 +540,6 @@ scheduler_kernel(const NasmDev *nasms, CtrlDev *ctrl, Entry *queue, StatusHost *
     // Optional time accounting per CTA: [0] scheduler idle polls, [1] completion + child update (ns),
     // [2 + layer] ns the workers spent on tiles of that layer (index modulo PROF_LAYERS),
     // [2 + PROF_LAYERS + layer] tile counts, [PROF_SLOTS - 1] ns the workers waited for a tile.
-    unsigned long long *my_prof = prof ? prof + (size_t)blockIdx.x * PROF_SLOTS : nullptr;
-
     // The first four warps need few registers, the workers many: a spill costs an L2 round trip here, because the ring leaves
     // almost no L1 (with 168 registers for everybody the epilogue of a 256 x 128 block took 12 us instead of 6).
     if (TENSOR_CORES) {
@@ -546,9 +547,9 @@ scheduler_kernel(const NasmDev *nasms, CtrlDev *ctrl, Entry *queue, StatusHost *
         else asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(ROLE_REGISTERS));
     }
     if (warp == sched_warp) {
-        scheduler_warp(nasms, ctrl, queue, status, sh, my_prof);
+        scheduler_warp(nasms, ctrl, queue, status, sh, prof ? prof + (size_t)blockIdx.x * PROF_SLOTS : nullptr);
     } else if (warp >= first_worker) {
-        WorkerWarp<TENSOR_CORES> w{smem, sh, ctrl, status, my_prof, tid - first_worker * 32u};
+        WorkerWarp<TENSOR_CORES> w{ctrl, status, prof};
         worker_loop(w);
     } else if (TENSOR_CORES && lane == 0) {
         if (warp == tc::WARP_A) single_thread_role<tc::WARP_A>(smem, sh, ctrl, status);

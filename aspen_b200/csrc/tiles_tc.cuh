@@ -75,6 +75,7 @@ struct Shared {
     unsigned long long full[MAX_STAGES], empty[MAX_STAGES];    // stage filled (both producers) / read by the MMAs
     unsigned long long acc_full[2], acc_empty[2];              // accumulator half complete / read by the workers
     unsigned long long posted[SLOTS], finished[SLOTS];         // scheduler -> roles / roles -> scheduler
+    unsigned long long prof_mark;                              // time accounting: when the workers' last step ended
     unsigned tmem_base;
     Slot slots[SLOTS];
 };
