@@ -13,8 +13,8 @@
 //     The line lies at 8: with 16 columns the 32 x 32 blocks below are faster (19.9 against 23.6 us at k = 768, m = 3072).
 //   * larger: the fp32 FMA blocks of gemm_ffma.cuh, shape by `pick_shape`.
 // B200, wall time of a call, launch and wait included (before: the tile queue of the scheduler kernel, set up by a kernel of
-// its own, scalar FMAs from global memory):  1 x 768 x 768 97 -> 14 us, 333 x 770 x 1000 2447 -> 42 us,
-// 4096 x 768 x 3072 4650 -> 470 us (columns x k x rows).
+// its own, scalar FMAs from global memory):  1 x 768 x 768 95 -> 17 us, 333 x 770 x 1000 2430 -> 44 us,
+// 4096 x 768 x 3072 4640 -> 467 us (columns x k x rows).
 #include "internal.h"
 #include "tiles_simt.cuh"
 #include "gemm_ffma.cuh"

@@ -84,7 +84,7 @@ __device__ __forceinline__ const float *input_pixel(const LayerDev &L, const Pix
 
 // ref src/tiled_kernels.c:613-638.  Pure streaming (12 bytes per element): four independent 16-byte load pairs are in flight per
 // thread before the first use.  ReLU and no activation have loops of their own: with every activation inlined at each element the
-// loop outgrew the instruction cache (256 x 24 elements 9 - 17 us, now 4).
+// loop outgrew the instruction cache (256 x 24 elements 9 - 17 us, now 2.0 - 2.6).
 enum { ACT_NONE = 0, ACT_RELU = 1, ACT_OTHER = 2 };
 template <int KIND>
 static __device__ __noinline__ void residual_loop(const LayerDev &L, const TileDev &T, unsigned tid, unsigned nthr) {
@@ -131,7 +131,7 @@ static __device__ __forceinline__ void tile_residual(const LayerDev &L, const Ti
 
 // Max pooling with a small window, whole 16-byte pieces of channels: taps outside the image are moved to the nearest pixel inside,
 // which the window contains as well, so all KH x KW loads of U outputs are unconditional and in flight together.  With a
-// test per tap the loads went out a few at a time: 64 x 100352 outputs (3 x 3, stride 2) 158 -> 40 us per SM.
+// test per tap the loads went out a few at a time: 64 x 100352 outputs (3 x 3, stride 2), launched alone, 158 -> 40 us per SM.
 template <int KH, int KW, int U>
 static __device__ __noinline__ void tile_max_small(const LayerDev &L, const TileDev &T, unsigned tid, unsigned nthr) {
     const unsigned h4 = T.tile_h >> 2, total = T.tile_w * h4, pos_w = T.pos_w, pos_h = T.pos_h, hw = L.OH * L.OW, OW = L.OW;

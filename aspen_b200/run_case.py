@@ -8,7 +8,7 @@ through rpool / dse and prints the device time per run.  Used for profiler captu
 persistent scheduler kernel on small cases.
 
 `--layer-table` (sets ASPEN_B200_PROFILE=1 before the library loads) prints, per layer shape class,
-the tiles per run, the executors' microseconds per tile and what that is per SM: TFLOP/s for the
+the device's tiles per run ("graph tile" is the host graph's), the workers' microseconds per tile and what that is per SM: TFLOP/s for the
 contraction tiles (2 M N K per tile), GB/s of algorithmic bytes for the memory-bound tiles
 (residual 12 B per element, layernorm 8 B, pooling 4 B x (inputs read once + outputs), softmax 8 B),
 each with its fraction of one SM's share of the roof given by --tensor-peak / --hbm-peak.
@@ -51,7 +51,7 @@ def layer_table(api, nasm, dnn, prof, runs, n_sms, tensor_peak_tf, hbm_peak_gbs)
         else:
             c["bytes"] += 8.0 * elems
     tf_sm, gb_sm = tensor_peak_tf / n_sms, hbm_peak_gbs / n_sms
-    out = ["| layer type | out rows x cols | K | tile | layers | tiles/run | us/tile | per SM | of one SM's roof |", "|---|---|---|---|---|---|---|---|---|"]
+    out = ["| layer type | out rows x cols | K | graph tile | layers | tiles/run | us/tile | per SM | of one SM's roof |", "|---|---|---|---|---|---|---|---|---|"]
     for (tname, H, W, k, th, tw), c in classes.items():
         us = c["ns"] / max(c["tiles"], 1) / 1e3
         if tname in GEMM_TYPES:

@@ -41,15 +41,13 @@ WORKLOADS = {
     "bert_base": ("bert_base", 32, 128, "n002", 3, 3),
     "vgg16": ("vgg16", 16, 0, "he", 2, 2),
 }
-# DRAM bytes per pass, from the ncu capture of the service-mode kernel summarised in profiles/ (265 MB per batch-4 pass, scaled by 8:
+# DRAM bytes per pass, from the ncu capture of the service-mode kernel summarised in profiles/ (237 MB per batch-4 pass, scaled by 8:
 # activation traffic grows with the batch).  A timed launch serves `steps` passes.
-TRAFFIC_BYTES_PER_STEP = {"resnet50": 2.12e9}
+TRAFFIC_BYTES_PER_STEP = {"resnet50": 1.90e9}
 # Tiling of the nasm per workload: (row quantum, column quantum, min_ninst_per_ldata).  Tensor-core shaped
-# quanta; the values a graph computes do not depend on them.  Each is the best of a measured sweep
-# (quanta 64-256, min_ninst 100-592).
+# quanta; the values a graph computes do not depend on them.
 TILING = {"resnet50": (128, 128, 100), "bert_base": (256, 128, 148), "vgg16": (128, 128, 180)}
-# The tile counts above are the best of a sweep in service mode (consecutive passes overlap, so fewer, larger tiles win); a graph
-# that is launched by itself is latency bound in its narrow layers and wants more tiles per layer (180 / 296).
+# These shape the host graph (ids, files; `host_graph_tiles`).  The device executes a grid of its own, chosen per layer.
 
 
 def log(*a):
@@ -554,7 +552,7 @@ def extra_legs(args, rank, world, wd, net, workload):
         b.group.set_service(False)
         tf = b.flops * steps / (float(np.median(bms)) * 1e-3) / 1e12
         extras["bert_base"] = {"metric": "sequences_per_sec", "config": {"workload": "bert_base_s128_bs32_per_gpu", "tile_quanta": list(b.tiling[:2]),
-                                                                          "min_ninst_per_ldata": b.tiling[2], "tiles": b.nasms[0].num_ninst},
+                                                                          "min_ninst_per_ldata": b.tiling[2], "host_graph_tiles": b.nasms[0].num_ninst},
                                "value": job_value(b.batch, steps, world, bmax), "unit": "seq/s", "ms_per_step": bmax / steps,
                                "e2e": {"value": job_value(b.batch, steps, world, be2e), "unit": "seq/s", "h2d_bytes_per_step": b.h2d_bytes,
                                        "input": "token ids (int32), embedded on the device",
@@ -587,7 +585,7 @@ def extra_legs(args, rank, world, wd, net, workload):
             want = net.out.reshape(gb, -1)
             ok = bool(whole.shape == want.shape and np.abs(whole - want).max() <= 2e-3 * np.abs(want).max()
                       and (whole.argmax(1) == want.argmax(1)).all())
-        extras["strong"] = {"config": {"workload": f"{workload}_global_bs{gb}", "per_gpu_batch": hi - lo, "tiles_per_gpu": s.nasms[0].num_ninst,
+        extras["strong"] = {"config": {"workload": f"{workload}_global_bs{gb}", "per_gpu_batch": hi - lo, "host_graph_tiles_per_gpu": s.nasms[0].num_ninst,
                                        "execution": f"service mode, {rotation} shards in rotation per GPU"},
                             "value": gb * steps / (smax * 1e-3), "unit": "inf/s", "ms_per_step": smax / steps, "scaling": "strong",
                             "e2e_value": gb * steps / (se2e * 1e-3), "gathered_equals_single_gpu_batch": ok}
@@ -631,7 +629,7 @@ def report(args, world, workload, batch, net, ms, max_ms, block_max, e2e_max, se
         "ms_per_step": max_ms / args.steps, "higher_is_better": True, "scaling": "weak", "vs_baseline": None, "dtype": "tf32",
         "data": "synthetic",
         "config": {"workload": f"{workload}_bs{batch}_per_gpu", "seq_len": seq or None, "tile_profile": "b200 tensor-core quanta",
-                   "tile_quanta": list(net.tiling[:2]), "min_ninst_per_ldata": net.tiling[2], "tiles": nasm.num_ninst, "flops_per_step": flops,
+                   "tile_quanta": list(net.tiling[:2]), "min_ninst_per_ldata": net.tiling[2], "host_graph_tiles": nasm.num_ninst, "flops_per_step": flops,
                    "execution": f"service mode: {len(net.nasms)} tile graphs of batch {batch} in rotation inside one resident scheduler launch per "
                                 "timed block; every step is one complete pass of one graph, input layer's scatter included",
                    "hidden_states": "all materialised" if args.keep_hidden_states else
