@@ -479,7 +479,7 @@ static int build_device_nasm(Engine *e, nasm_t *host_nasm) {
         CUresult r = get_encode_im2col_fn()(&m, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, const_cast<float *>(base), dims, strides, low, up, 32, a_rows, estr,
                                             CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                                             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-        if (r != CUDA_SUCCESS) { ASPEN_ERR("cuTensorMapEncodeIm2col failed (%d)\n", (int)r); return -2; }
+        if (r != CUDA_SUCCESS) return -2;
         maps.push_back(m);
         return (int)maps.size() - 1;
     };
@@ -537,7 +537,7 @@ static int build_device_nasm(Engine *e, nasm_t *host_nasm) {
                 L.amap = add_im2col_map(L.in0, {form.c, L.IW, L.IH, nasm->batch_size}, {L.ld0, (size_t)L.IW * L.ld0, (size_t)L.IH * L.IW * L.ld0}, -(int)L.pad,
                                         (int)L.pad - (int)L.KW + 1, (int)L.pad - (int)L.KH + 1, L.stride, L.stride, L.a_rows);
             }
-            if (L.amap < 0) return -1;
+            if (L.amap < 0) L.a_kind = A_NONE;      // a shape that the driver does not take: fp32 blocks
         } else if (form.kind == A_TMA && (l.type == MATMUL_LAYER || l.type == CONV_LAYER)) {
             add_x_map(L, L.in0, L.H0, W0, (cuuint64_t)L.ld0 * sizeof(float));
         } else if (l.type == FC_LAYER && (L.ld0 == L.IC || L.KH * L.KW == 1)) {
