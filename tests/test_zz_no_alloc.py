@@ -1,8 +1,7 @@
 """aspen_b200_matmul_noalloc: the entry point for callers that may not allocate device memory (plug-ins
 that run inside a fixed memory budget, loops that cannot take the device-wide synchronisation of an
 allocation).  It must give what the regular, allocating API gives for the same matmul layer -- and what
-the CPU oracle gives -- on repeated calls that share its fixed scratch array.  Collected last on purpose:
-the scratch array is process-wide state."""
+the CPU oracle gives -- on repeated calls of different shapes."""
 import os
 
 import numpy as np
@@ -45,7 +44,7 @@ def test_noalloc_matmul_matches_regular_api_on_two_calls_in_a_row(workdir):
     import torch
     L = api.lib()
     rng = np.random.default_rng(7)
-    # second call is smaller and differently shaped: stale descriptors of the first call must not matter
+    # the second call is smaller and differently shaped
     for call, (n, k, m, act, act_name) in enumerate([(300, 192, 260, RELU, "relu"), (130, 64, 72, GELU, "gelu")]):
         x = rng.standard_normal((n, k), dtype=np.float32)
         w = (rng.standard_normal((m, k), dtype=np.float32) / np.sqrt(k)).astype(np.float32)
