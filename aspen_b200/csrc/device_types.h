@@ -66,6 +66,7 @@ struct alignas(32) TileDev {        // a whole sector, one load for the schedule
     unsigned pos_h, pos_w;    // position in the layer's output matrix
     unsigned tile_h, tile_w;  // clipped extents
     unsigned child_off, child_cnt;
+    unsigned need;            // completions of parents that a pass of the tile waits for
 };
 
 // The layer-0 tiles run on the device and turn what the host uploaded into the layer's activation matrix, so a
@@ -115,7 +116,9 @@ struct CtrlDev {
     unsigned long long pipe_ns;    // time budget of in-kernel pipeline waits
     unsigned svc_stop;       // host request: leave once no pass is running or asked for
     unsigned svc_close;      // set by the device: everybody leaves (no error)
-    unsigned ahead;          // a busy CTA lines up a second tile when at least this many ready tiles wait unclaimed (0: never)
+    unsigned ordered;        // the tiles are handed out in a fixed order (scheduler.cuh) instead of as they become ready
+    unsigned ahead;          // a busy CTA lines up a second tile when at least this many ready tiles wait unclaimed (0: never); in a fixed
+                             // order: it claims one when the tile in work has its weights
     unsigned long long idle_ns;    // leave after this long without a pass in progress
 };
 

@@ -187,6 +187,9 @@ struct Engine {
     StatusHost *status_d = nullptr;
     sched::Entry *queue = nullptr;
     unsigned queue_cap = 0;
+    sched::Entry *order = nullptr;    // several graphs in one launch: their tiles in the order they are handed out
+    unsigned order_cap = 0;
+    std::vector<unsigned long long> order_of;   // the images (DeviceNasm::serial) that order is of
     NasmDev *nasms_d = nullptr;
     unsigned nasms_cap = 0;
     std::vector<NasmDev> uploaded;    // what nasms_d holds
@@ -200,7 +203,7 @@ struct Engine {
     std::vector<nasm_t *> svc_pool;   // every graph of the group's rpool that has a device image: what the next launch serves
     unsigned long long idle_ns = 20000000ull;   // the kernel leaves after this long with no pass running
     cudaEvent_t svc_armed_ev = nullptr;
-    unsigned svc_ahead = 32, run_ahead = 0;   // see CtrlDev::ahead: in service mode / in a launch per run
+    unsigned svc_ahead = 32;          // see CtrlDev::ahead
     std::unique_ptr<HostCopy> copy;   // results into pageable memory
     unsigned long long *prof = nullptr;   // per-CTA time accounting, allocated when ASPEN_B200_PROFILE is set
 };
@@ -217,6 +220,10 @@ struct DeviceNasm {
     unsigned *children = nullptr, *dep = nullptr;
     void *wmaps = nullptr;
     NasmDev host;               // the graph's entry in a launch, but for its input
+    unsigned long long serial = 0;      // no two images have the same
+    ClaimOrder claims;
+    std::vector<unsigned> tile_layer;
+    sched::Entry *order = nullptr;      // claims of a launch of this graph alone
     bool round_input = false;   // tensor-core path: the input is rounded to TF32 by the layer-0 tiles
     unsigned *svc_d = nullptr;                               // SVC_* words
     unsigned *svc_done_h = nullptr, *svc_done_d = nullptr;   // mapped: number of the last complete pass
@@ -300,7 +307,6 @@ Engine *engine_create(int device, int precision, unsigned int /*num_dse_hint*/) 
         if (env_u64("ASPEN_B200_IDLE_MS", &v) && v > 0) e->idle_ns = v * 1000000ull;
         if (env_u64("ASPEN_B200_SVC_AHEAD", &v)) e->svc_ahead = (unsigned)v;
         if (env_u64("ASPEN_B200_SERVICE", &v)) e->service = v != 0;      // for programs that cannot call aspen_b200_dse_group_set_service
-        if (env_u64("ASPEN_B200_RUN_AHEAD", &v)) e->run_ahead = (unsigned)v;
         e->copy->prepare(0);
     }
     if (ok && getenv("ASPEN_B200_PROFILE")) {
@@ -328,6 +334,7 @@ void engine_destroy(Engine *e) {
     cudaFree(e->ctrl);
     if (e->status_h) cudaFreeHost((void *)e->status_h);
     cudaFree(e->queue);
+    cudaFree(e->order);
     cudaFree(e->nasms_d);
     cudaFree(e->prof);
     delete e;
@@ -390,7 +397,7 @@ static void fill_layer(const nasm_t *nasm, const DeviceNasm *dn, unsigned i, int
 
 static void free_device_nasm(DeviceNasm *dn) {
     if (!dn) return;
-    cudaFree(dn->arena); cudaFree(dn->layers); cudaFree(dn->tiles); cudaFree(dn->children); cudaFree(dn->dep); cudaFree(dn->wmaps);
+    cudaFree(dn->arena); cudaFree(dn->layers); cudaFree(dn->tiles); cudaFree(dn->children); cudaFree(dn->dep); cudaFree(dn->wmaps); cudaFree(dn->order);
     if (dn->svc_done_h) cudaFreeHost(dn->svc_done_h);
     cudaFree(dn->svc_d);
     cudaFree(dn->in_stage); cudaFree(dn->ids_stage); cudaFree(dn->padded_in);
@@ -736,7 +743,17 @@ static int build_device_nasm(Engine *e, nasm_t *host_nasm) {
             children.push_back(c); children.push_back(tiles[c].layer << 16 | need[c]);
         }
     }
+    for (unsigned t = 0; t < n; t++) tiles[t].need = need[t];
     if (to_device(&dn->tiles, tiles) != 0 || to_device(&dn->children, children) != 0) return -1;
+    std::vector<bool> bypassed(n);
+    dn->tile_layer.resize(n);
+    for (unsigned t = 0; t < n; t++) { dn->tile_layer[t] = tiles[t].layer; bypassed[t] = written_by[tiles[t].layer] != (unsigned)-1; }
+    dn->claims = claim_order(nasm, e->precision, e->n_ctas, kids, need, bypassed);
+    std::vector<sched::Entry> order;
+    for (unsigned t : dn->claims.tile) order.push_back(sched::make_entry(t, 0, tiles[t].layer));
+    if (to_device(&dn->order, order) != 0) return -1;
+    static std::atomic<unsigned long long> serials{0};
+    dn->serial = ++serials;
     CUDA_TRY(cudaMalloc(&dn->dep, std::max<size_t>(n, 1) * sizeof(unsigned)));
     CUDA_TRY(cudaHostAlloc(&dn->svc_done_h, sizeof(unsigned), cudaHostAllocMapped));
     *dn->svc_done_h = 0;
@@ -807,6 +824,36 @@ static NasmDev graph_image(const nasm_t *nasm) {
     return G;
 }
 
+// Several graphs in one launch: all of them progress at the same share of their runs.
+static int merge_orders(Engine *e, const std::vector<nasm_t *> &graphs, unsigned claims) {
+    std::vector<unsigned long long> of;
+    for (const nasm_t *n : graphs) of.push_back(n->dev->serial);
+    if (of == e->order_of) return 0;
+    e->order_of.clear();
+    if (claims > e->order_cap) {
+        cudaFree(e->order);
+        e->order = nullptr;
+        e->order_cap = 0;
+        CUDA_TRY(cudaMalloc(&e->order, (size_t)claims * sizeof(sched::Entry)));
+        e->order_cap = claims;
+    }
+    std::vector<sched::Entry> order;
+    std::vector<size_t> next(graphs.size(), 0);
+    while (order.size() < claims) {
+        size_t g = graphs.size();
+        for (size_t i = 0; i < graphs.size(); i++) {
+            const ClaimOrder &c = graphs[i]->dev->claims;
+            if (next[i] < c.tile.size() && (g == graphs.size() || c.at[next[i]] < graphs[g]->dev->claims.at[next[g]])) g = i;
+        }
+        const unsigned t = graphs[g]->dev->claims.tile[next[g]++];
+        order.push_back(sched::make_entry(t, (unsigned)g, graphs[g]->dev->tile_layer[t]));
+    }
+    // cudaMemcpyAsync from pageable memory returns after the source has been staged
+    CUDA_TRY(cudaMemcpyAsync(e->order, order.data(), order.size() * sizeof(sched::Entry), cudaMemcpyHostToDevice, e->stream));
+    e->order_of = of;
+    return 0;
+}
+
 // `leave`: the kernel ends when the passes owed now are complete.  `chained`: the launch follows others on the stream that
 // complete everything asked for before svc_chain (timing loops).
 static int svc_launch(Engine *e, const std::vector<nasm_t *> &graphs, bool leave, bool chained = false) {
@@ -831,7 +878,16 @@ static int svc_launch(Engine *e, const std::vector<nasm_t *> &graphs, bool leave
         CUDA_TRY(cudaMalloc(&e->nasms_d, graphs.size() * sizeof(NasmDev)));
         e->nasms_cap = (unsigned)graphs.size();
     }
-    if (cap > e->queue_cap) {
+    // A launch that leaves hands its tiles out in a fixed order; service mode's queue takes them as they become ready.
+    const bool ordered = !e->service;
+    sched::Entry *order = nullptr;
+    unsigned claims = 0;
+    if (ordered) {
+        for (const nasm_t *n : graphs) claims += (unsigned)n->dev->claims.tile.size();
+        if (graphs.size() == 1) order = graphs[0]->dev->order;
+        else if (merge_orders(e, graphs, claims) != 0) return -1;
+        else order = e->order;
+    } else if (cap > e->queue_cap) {
         cudaFree(e->queue);
         e->queue = nullptr;
         e->queue_cap = 0;
@@ -847,14 +903,14 @@ static int svc_launch(Engine *e, const std::vector<nasm_t *> &graphs, bool leave
     for (unsigned g0 = 0; g0 < graphs.size(); g0 += sched::ARM_GRAPHS) {
         sched::ArmArgs a;
         a.g0 = g0; a.n = std::min<unsigned>(sched::ARM_GRAPHS, (unsigned)graphs.size() - g0); a.n_nasm = (unsigned)graphs.size();
-        a.cap = cap; a.total = (unsigned)total; a.svc_stop = leave ? 1u : 0u; a.ahead = e->service ? e->svc_ahead : e->run_ahead;
+        a.cap = ordered ? claims : cap; a.total = (unsigned)total; a.svc_stop = leave ? 1u : 0u; a.ahead = ordered ? graphs.size() > 1 : e->svc_ahead; a.ordered = ordered ? 1u : 0u;
         a.stall_ns = e->stall_ns; a.pipe_ns = e->pipe_ns; a.idle_ns = e->idle_ns;
         for (unsigned i = 0; i < a.n; i++) {
             const DeviceNasm *dn = graphs[g0 + i]->dev;
             a.base[i] = chained ? dn->svc_chain : *(volatile unsigned *)dn->svc_done_h;
             a.target[i] = dn->svc_armed;
         }
-        sched::arm_kernel<<<std::min<unsigned>((cap + 255) / 256, 1024), 256, 0, e->stream>>>(e->nasms_d, e->ctrl, e->queue, a);
+        sched::arm_kernel<<<std::min<unsigned>((a.cap + 255) / 256, 1024), 256, 0, e->stream>>>(e->nasms_d, e->ctrl, e->queue, a);
         e->launches++;
     }
     if (e->service) {
@@ -863,9 +919,9 @@ static int svc_launch(Engine *e, const std::vector<nasm_t *> &graphs, bool leave
         CUDA_TRY(cudaStreamWaitEvent(e->io, e->svc_armed_ev, 0));
     }
     if (e->precision == 0)
-        sched::scheduler_kernel<true><<<e->n_ctas, sched::threads<true>(), e->smem_bytes, e->stream>>>(e->nasms_d, e->ctrl, e->queue, e->status_d, e->prof);
+        sched::scheduler_kernel<true><<<e->n_ctas, sched::threads<true>(), e->smem_bytes, e->stream>>>(e->nasms_d, e->ctrl, ordered ? order : e->queue, e->status_d, e->prof);
     else
-        fp32_launch(e->n_ctas, e->smem_bytes, e->stream, e->nasms_d, e->ctrl, e->queue, e->status_d, e->prof);
+        fp32_launch(e->n_ctas, e->smem_bytes, e->stream, e->nasms_d, e->ctrl, ordered ? order : e->queue, e->status_d, e->prof);
     e->launches++;
     CUDA_TRY(cudaGetLastError());
     e->svc_graphs = graphs;

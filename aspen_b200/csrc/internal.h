@@ -180,6 +180,13 @@ struct OperandForm {
 };
 OperandForm operand_form(const aspen_layer_t *l, unsigned seq);
 nasm_t *plan_device_tiles(const nasm_t *nasm, int precision, unsigned int sms, bool served);   // plan.cpp; nullptr: keep the nasm's tiles
+// Order in which a launch hands out the tiles of a graph (plan.cpp): what an idle machine of `workers` SMs would start when.
+struct ClaimOrder {
+    std::vector<unsigned> tile;    // parents before children
+    std::vector<float> at;         // start, as a share of the whole run
+};
+ClaimOrder claim_order(const nasm_t *plan, int precision, unsigned workers, const std::vector<std::vector<unsigned>> &children, const std::vector<unsigned> &need,
+                       const std::vector<bool> &skip);
 nasm_t *own_device_tiles(const nasm_t *nasm);      // plan.cpp: the nasm's tiles, columns a multiple of 16 bytes apart
 int engine_current_device();
 Engine *engine_create(int device, int precision, unsigned int num_dse_hint);

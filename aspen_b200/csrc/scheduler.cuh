@@ -50,7 +50,7 @@ constexpr unsigned PROF_SLOTS = 2 + 2 * PROF_LAYERS + 2;
 
 // A ready tile: low word = local tile id + 1 (0: none), high word = graph << 16 | layer.
 typedef unsigned long long Entry;
-__device__ __forceinline__ Entry make_entry(unsigned tile, unsigned g, unsigned layer) { return (Entry)(tile + 1u) | ((Entry)((g << 16) | layer) << 32); }
+__host__ __device__ __forceinline__ Entry make_entry(unsigned tile, unsigned g, unsigned layer) { return (Entry)(tile + 1u) | ((Entry)((g << 16) | layer) << 32); }
 
 __device__ __forceinline__ unsigned long long global_ns() {
     unsigned long long t;
@@ -186,13 +186,13 @@ static __device__ void end_of_pass(const NasmDev *nasms, unsigned n_nasm, unsign
 // the first of which (g0 = 0) also resets the queue and the control words.
 constexpr unsigned ARM_GRAPHS = 32;
 struct ArmArgs {
-    unsigned g0, n, n_nasm, cap, total, svc_stop, ahead;
+    unsigned g0, n, n_nasm, cap, total, svc_stop, ahead, ordered;
     unsigned long long stall_ns, pipe_ns, idle_ns;
     unsigned base[ARM_GRAPHS], target[ARM_GRAPHS];
 };
 static __global__ void arm_kernel(const NasmDev *nasms, CtrlDev *ctrl, Entry *queue, const ArmArgs a) {
     const unsigned stride = gridDim.x * blockDim.x, t0 = blockIdx.x * blockDim.x + threadIdx.x;
-    if (a.g0 == 0)
+    if (a.g0 == 0 && !a.ordered)
         for (unsigned i = t0; i < a.cap; i += stride) queue[i] = 0u;
     for (unsigned g = 0; g < a.n; g++) {
         const NasmDev &G = nasms[a.g0 + g];
@@ -207,7 +207,7 @@ static __global__ void arm_kernel(const NasmDev *nasms, CtrlDev *ctrl, Entry *qu
     if (t0 == 0 && a.g0 == 0) {
         ctrl->head = 0u; ctrl->tail = 0u; ctrl->done = 0u; ctrl->total = a.total; ctrl->cap = a.cap; ctrl->n_nasm = a.n_nasm;
         ctrl->abort = 0u; ctrl->stop = 0u; ctrl->stall_ns = a.stall_ns; ctrl->pipe_ns = a.pipe_ns;
-        ctrl->svc_stop = a.svc_stop; ctrl->svc_close = 0u; ctrl->idle_ns = a.idle_ns; ctrl->ahead = a.ahead;
+        ctrl->svc_stop = a.svc_stop; ctrl->svc_close = 0u; ctrl->idle_ns = a.idle_ns; ctrl->ahead = a.ahead; ctrl->ordered = a.ordered;
     }
 }
 
@@ -254,30 +254,10 @@ template <bool TENSOR_CORES> __host__ __device__ constexpr unsigned threads() { 
 constexpr unsigned FFMA_BYTES = 96u * 1024u;
 template <bool TENSOR_CORES> __host__ __device__ constexpr unsigned work_bytes() { return TENSOR_CORES ? tc::RING_BYTES + tc::EPI_BYTES : FFMA_BYTES; }
 
-// A role's wait for the next tile.  The scheduler always posts an exit marker eventually (end of
-// run, stop, stall, abort); the time bound only guards against that logic failing.
-__device__ __forceinline__ bool wait_posted(unsigned long long *bar, unsigned parity, CtrlDev *ctrl, StatusHost *status) {
-    #pragma unroll 1
-    for (unsigned spin = 0; spin < 1024u; spin++)
-        if (tc::mbar_try_wait(bar, parity)) return true;
-    const unsigned long long t0 = global_ns(), budget = 2ull * ctrl->stall_ns + 4ull * ctrl->pipe_ns + 1000000000ull;
-    for (unsigned spin = 1;; spin++) {
-        if (tc::mbar_try_wait(bar, parity)) return true;
-        if ((spin & 63u) == 0u) {
-            __nanosleep(64);
-            if (global_ns() - t0 > budget) break;
-        }
-    }
-    if (atomicCAS(&ctrl->abort, 0u, (unsigned)ASPEN_B200_ERR_PIPE) == 0u) {
-        status->info0 = 7; status->info1 = blockIdx.x; status->status = ASPEN_B200_ERR_PIPE;
-        __threadfence_system();
-    }
-    return false;
-}
-
-// Fills a slot with a ready tile and hands it to the roles (whole warp).  The tile's and the layer's descriptors are independent
+// Fills slot k with a tile and hands it to the roles (whole warp).  The tile's and the layer's descriptors are independent
 // loads; both and the graph's addresses are constant while the kernel runs.
-static __device__ __forceinline__ void post(tc::Slot &sl, unsigned long long &posted, const tc::GraphRef &G, Entry entry) {
+static __device__ __forceinline__ void post(tc::Shared *sh, unsigned k, const tc::GraphRef &G, Entry entry) {
+    tc::Slot &sl = sh->slots[k];
     const unsigned lane = threadIdx.x & 31u, g = (unsigned)(entry >> 48), layer = (unsigned)(entry >> 32) & 0xffffu, tile = (unsigned)entry - 1u;
     constexpr unsigned LW = sizeof(LayerDev) / 4, TW = sizeof(TileDev) / 4;
     static_assert(LW == 64 && TW <= 32, "copied in words");
@@ -290,7 +270,15 @@ static __device__ __forceinline__ void post(tc::Slot &sl, unsigned long long &po
     if (lane < TW) reinterpret_cast<unsigned *>(&sl.tile)[lane] = tw;
     if (lane == 0) { sl.live = 1u; sl.nasm = g; sl.maps = G.maps; sl.input = G.input; }
     __syncwarp();
-    if (lane == 0) tc::mbar_arrive(&posted);
+    if (lane == 0) tc::mbar_arrive(&sh->posted[k]);
+}
+static __device__ __forceinline__ void post_ready(tc::Shared *sh, unsigned k) {
+    __syncwarp();
+    if ((threadIdx.x & 31u) == 0) tc::mbar_arrive(&sh->ready[k]);
+}
+// The marker behind the last tile.
+static __device__ __forceinline__ void post_exit(tc::Shared *sh, unsigned k) {
+    if ((threadIdx.x & 31u) == 0) { sh->slots[k].live = 0u; tc::mbar_arrive(&sh->posted[k]); tc::mbar_arrive(&sh->ready[k]); }
 }
 
 static __device__ __noinline__ void scheduler_warp(const NasmDev *nasms, CtrlDev *ctrl, Entry *queue, StatusHost *status, tc::Shared *sh, unsigned long long *my_prof) {
@@ -374,7 +362,8 @@ static __device__ __noinline__ void scheduler_warp(const NasmDev *nasms, CtrlDev
         if (next) {
             const unsigned k = issued % tc::SLOTS;
             const tc::GraphRef G = graph_ref(sh, nasms, (unsigned)(next >> 48));
-            post(sh->slots[k], sh->posted[k], G, next);
+            post(sh, k, G, next);
+            post_ready(sh, k);
             const tc::Slot &sl = sh->slots[k];
             uint2 e = make_uint2(0u, 1u);
             if (lane < sl.tile.child_cnt) e = __ldg(G.children + sl.tile.child_off + lane);
@@ -431,7 +420,152 @@ static __device__ __noinline__ void scheduler_warp(const NasmDev *nasms, CtrlDev
         }
         __nanosleep(20u);
     }
-    if (lane == 0) { sh->slots[issued % tc::SLOTS].live = 0u; tc::mbar_arrive(&sh->posted[issued % tc::SLOTS]); }
+    post_exit(sh, issued % tc::SLOTS);
+}
+
+// A launch in a fixed order.  Every tile of the launch is in `order`, parents before children; a CTA claims the next position,
+// posts that tile at once and waits for its counter itself.  Against the ready queue this takes the counter's answer, the queue's
+// tail, its entry and the descriptors off the way from a tile's last store to its child's first load (what is left: one fence,
+// one reduction, one poll), and a tile's weights stream into the ring while it waits.  What it gives up is the choice among ready
+// tiles: a claimed tile waits for its own parents while another could run.  The order is that of a simulated run
+// (plan.cpp: claim_order), so that a tile's turn comes when its parents are about done.  Device time of a pass, queue and order:
+// CIFAR net x 1 68 and 49 us, BERT 1 x 37 1128 and 878, ResNet-50 x 1 fp32 1126 and 1022, x 32 1541 and 1466, GPT-2 8 x 512 2520
+// and 2461, ResNet-50 + VGG-16 x 16 2132 and 1832.
+// Claims are contiguous and a tile's parents lie before it, so whatever is claimed completes; a CTA asked to stop only
+// claims no more.
+static __device__ __noinline__ void ordered_warp(const NasmDev *nasms, CtrlDev *ctrl, const Entry *order, StatusHost *status, tc::Shared *sh, unsigned long long *my_prof) {
+    const unsigned lane = threadIdx.x & 31u, count = ctrl->cap;
+    const unsigned *watch = lane == 1u ? &ctrl->abort : lane == 2u ? &ctrl->stop : &ctrl->done;
+    const unsigned long long window = ctrl->stall_ns;
+    unsigned issued = 0, running = 0, retired = 0;     // tiles posted / whose parents are complete / completed: at most two apart
+    uint2 edge0 = make_uint2(0u, 1u), edge1 = edge0;   // this lane's first child edge of the tiles in the slots (by parity)
+    enum { NOTHING, TICKET, ENTRY } claim = NOTHING;   // what has been asked for; looked at in a later turn
+    unsigned ticket = 0, need = 0, counted = 0, count_nasm = 0, turn = 0, last_done = 0;
+    const unsigned *dep = nullptr;                     // of the posted tile that waits for its parents
+    Entry entry = 0;
+    const bool ahead = ctrl->ahead != 0u;
+    bool closed = false, out = false, accounting = false, aborted = false;
+    unsigned long long t_progress = __shfl_sync(0xffffffffu, global_ns(), 0), t_mark = t_progress;
+    // the pass's last tile ends it
+    auto account = [&]() {
+        const NasmDev &G = nasms[count_nasm];
+        if (lane == 0 && counted == G.n_exec) {
+            __threadfence_system();
+            *G.completed = ld_relaxed(&G.svc[SVC_BASE]) + 1u;
+            __threadfence_system();
+        }
+        __syncwarp();
+        accounting = false;
+    };
+    while (true) {
+        bool progressed = false;
+        // 1. retire the oldest running tile once every role has finished it
+        if (running > retired) {
+            const unsigned k = retired % tc::SLOTS;
+            unsigned ok = lane == 0 ? (unsigned)tc::mbar_test_wait(&sh->finished[k], (retired / tc::SLOTS) & 1u) : 0u;
+            ok = __shfl_sync(0xffffffffu, ok, 0);
+            if (ok) {
+                __syncwarp();                    // a shuffle orders no memory: what lane 0 has observed holds for the lanes that release it
+                if (my_prof && lane == 0) t_mark = global_ns();
+                const tc::Slot &sl = sh->slots[k];
+                const unsigned g = sl.nasm, cnt = sl.tile.child_cnt;
+                const tc::GraphRef G = graph_ref(sh, nasms, g);
+                uint2 e = (retired & 1u) ? edge1 : edge0;
+                fence_gpu();                     // release: this tile's output
+                for (unsigned idx = lane; idx < cnt; idx += 32u) {
+                    if (idx >= 32u) e = __ldg(G.children + sl.tile.child_off + idx);
+                    asm volatile("red.relaxed.gpu.global.add.u32 [%0], 1;" ::"l"(G.dep + e.x) : "memory");
+                }
+                if (my_prof && lane == 0) my_prof[1] += global_ns() - t_mark;
+                if (accounting) account();
+                // the count of the pass is looked at in a later turn
+                if (lane == 0) {
+                    asm volatile("red.relaxed.gpu.global.add.u32 [%0], 1;" ::"l"(&ctrl->done) : "memory");
+                    counted = atomicAdd(&G.svc[SVC_COUNT], 1u) + 1u;
+                }
+                count_nasm = g;
+                accounting = progressed = true;
+                retired++;
+            }
+        }
+        // 2. the tile that waits for its parents; with nothing else to do the counter is read as fast as it can be
+        if (issued > running) {
+            unsigned v = 0;
+            const bool idle = running == retired;
+            if (lane == 0) v = idle ? ld_acquire(dep) : ld_relaxed(dep);
+            const bool there = __shfl_sync(0xffffffffu, (int)(v - need), 0) >= 0;
+            if (there) {
+                if (!idle) fence_gpu();          // acquire the parents' outputs
+                post_ready(sh, running % tc::SLOTS);
+                running++;
+                progressed = true;
+            }
+        }
+        // 3. claim the next tile
+        bool want = claim == NOTHING && issued == running && issued - retired < 2u && !out && !closed;
+        if (want && issued != retired) {
+            // A busy CTA claims ahead when the tile in work has all its weights, so that the next one's stream in under its epilogue --
+            // but only where several graphs share the launch and work is plenty: alone, the tile it holds back would often be
+            // ready for an idle CTA (ResNet-50 x 32 1466 us a pass without, 1487 with; ResNet-50 and VGG-16 x 16 1995 and 1832).
+            unsigned fed = 0;
+            if (ahead && sh->slots[retired % tc::SLOTS].layer.tc) {
+                if (lane == 0) fed = (unsigned)tc::mbar_test_wait(&sh->fed[retired % tc::SLOTS], (retired / tc::SLOTS) & 1u);
+                fed = __shfl_sync(0xffffffffu, fed, 0);
+            }
+            want = fed != 0u;
+        }
+        if (want) {
+            if (lane == 0) ticket = atomicAdd(&ctrl->head, 1u);
+            claim = TICKET;
+        } else if (claim == TICKET) {
+            ticket = __shfl_sync(0xffffffffu, ticket, 0);
+            out = ticket >= count;
+            claim = out ? NOTHING : ENTRY;
+            if (!out) entry = __ldg(order + ticket);
+        } else if (claim == ENTRY) {
+            const unsigned k = issued % tc::SLOTS;
+            const tc::GraphRef G = graph_ref(sh, nasms, (unsigned)(entry >> 48));
+            post(sh, k, G, entry);
+            const tc::Slot &sl = sh->slots[k];
+            need = sl.tile.need;
+            dep = G.dep + ((unsigned)entry - 1u);
+            uint2 e = make_uint2(0u, 1u);
+            if (lane < sl.tile.child_cnt) e = __ldg(G.children + sl.tile.child_off + lane);
+            if (issued & 1u) edge1 = e; else edge0 = e;
+            issued++;
+            claim = NOTHING;
+        }
+        // 4. completion accounting, behind everything that another tile may be waiting for
+        if (accounting && !progressed) account();
+        if (issued == retired && claim == NOTHING && (out || closed) && !accounting) break;
+        // 5. control words and stall detection
+        if (progressed) continue;
+        if ((++turn & 31u) == 0u) {
+            unsigned word = lane >= 1u && lane <= 3u ? ld_relaxed(watch) : 0u;
+            const unsigned flags = __ballot_sync(0xffffffffu, lane >= 1u && lane <= 2u && word != 0u), done = __shfl_sync(0xffffffffu, word, 3);
+            unsigned long long now = lane == 0 ? global_ns() : 0ull;
+            now = __shfl_sync(0xffffffffu, now, 0);
+            if (flags & 2u) { aborted = true; break; }       // roles leave their tiles unfinished, nothing more will be retired
+            if (flags & 4u) closed = true;
+            if (done != last_done || running > retired) { last_done = done; t_progress = now; }
+            else if (now - t_progress > window) {
+                // nothing running here, nothing completed anywhere for a whole window: the graph cannot progress
+                if (lane == 0 && atomicCAS(&ctrl->abort, 0u, (unsigned)ASPEN_B200_ERR_STALL) == 0u) {
+                    status->info0 = (unsigned)entry - 1u; status->info1 = done; status->status = ASPEN_B200_ERR_STALL;
+                    __threadfence_system();
+                }
+                aborted = true;
+                break;
+            }
+            if (my_prof && lane == 0 && running == retired) my_prof[0] += 1ull;   // idle polls with nothing in flight
+        }
+        if (issued == running) __nanosleep(20u);
+    }
+    if (aborted && issued > running) {                   // the waiting tile is withdrawn
+        if (lane == 0) sh->slots[running % tc::SLOTS].live = 0u;
+        post_ready(sh, running % tc::SLOTS);
+    }
+    post_exit(sh, issued % tc::SLOTS);
 }
 
 // The loops of the one-thread roles, all their state inside: a reference to it would put it into local memory.
@@ -442,16 +576,18 @@ static __device__ __forceinline__ void single_thread_role(unsigned char *smem, t
     unsigned half = 0, acc_uses = 0;
     for (unsigned seq = 0;; seq++) {
         const unsigned k = seq % tc::SLOTS;
-        if (!wait_posted(&sh->posted[k], (seq / tc::SLOTS) & 1u, ctrl, status)) break;
+        const unsigned parity = (seq / tc::SLOTS) & 1u;
+        if (!tc::wait_slot(&sh->posted[k], parity, ctrl, status)) break;
         const tc::Slot &sl = sh->slots[k];
         if (!sl.live) break;
         if (sl.layer.tc) {
             bool ok;
-            if (ROLE == tc::WARP_A) ok = tc::produce_a(sl, ring, r, sh, ctrl, status);
-            else if (ROLE == tc::WARP_B) ok = tc::produce_b(sl, ring, r, sh, ctrl, status);
-            else ok = tc::issue_mma(sl, ring, r, half, acc_uses, sh, ctrl, status);
+            if (ROLE == tc::WARP_A) ok = tc::produce_a(sl, &sh->ready[k], parity, ring, r, sh, ctrl, status);
+            else if (ROLE == tc::WARP_B) ok = tc::produce_b(sl, &sh->ready[k], parity, ring, r, sh, ctrl, status);
+            else ok = tc::wait_ready(sl, &sh->ready[k], parity, ctrl, status) && tc::issue_mma(sl, ring, r, half, acc_uses, sh, ctrl, status);
             if (!ok) break;
         }
+        if (ROLE == tc::WARP_B) tc::mbar_arrive(&sh->fed[k]);
         tc::mbar_arrive(&sh->finished[k]);
     }
     if (*(volatile unsigned *)&ctrl->abort) {
@@ -481,7 +617,7 @@ struct WorkerWarp {
         return t;
     }
     __device__ __forceinline__ bool posted(unsigned seq) {
-        return __all_sync(0xffffffffu, wait_posted(&sh()->posted[seq % tc::SLOTS], (seq / tc::SLOTS) & 1u, ctrl, status));
+        return __all_sync(0xffffffffu, tc::wait_slot(&sh()->ready[seq % tc::SLOTS], (seq / tc::SLOTS) & 1u, ctrl, status));
     }
     __device__ __forceinline__ bool live(unsigned seq) const { return slot(seq).live != 0u; }
     __device__ __forceinline__ bool meets(unsigned seq) const { return slot(seq).layer.meets != 0u; }
@@ -515,7 +651,7 @@ static_assert(128 * ROLE_REGISTERS + 256 * WORKER_REGISTERS <= 384 * 168, "regis
 
 template <bool TENSOR_CORES>
 __global__ void __launch_bounds__(threads<TENSOR_CORES>(), 1)
-scheduler_kernel(const NasmDev *nasms, CtrlDev *ctrl, Entry *queue, StatusHost *status, unsigned long long *prof) {
+scheduler_kernel(const NasmDev *nasms, CtrlDev *ctrl, Entry *queue /* or, ctrl->ordered, the order of the launch */, StatusHost *status, unsigned long long *prof) {
     extern __shared__ __align__(1024) unsigned char smem[];      // stages need 1024-byte alignment for the 128-byte swizzle
     tc::Shared *sh = reinterpret_cast<tc::Shared *>(smem + work_bytes<TENSOR_CORES>());
     const unsigned tid = threadIdx.x, warp = tid >> 5, lane = tid & 31u;
@@ -525,7 +661,7 @@ scheduler_kernel(const NasmDev *nasms, CtrlDev *ctrl, Entry *queue, StatusHost *
         sh->prof_mark = global_ns();
         for (unsigned s = 0; s < tc::MAX_STAGES; s++) { tc::mbar_init(&sh->full[s], 2u); tc::mbar_init(&sh->empty[s], 1u); }
         for (unsigned h = 0; h < 2; h++) { tc::mbar_init(&sh->acc_full[h], 1u); tc::mbar_init(&sh->acc_empty[h], tc::NW / 32u); }
-        for (unsigned k = 0; k < tc::SLOTS; k++) { tc::mbar_init(&sh->posted[k], 1u); tc::mbar_init(&sh->finished[k], tc::NW / 32u + (TENSOR_CORES ? 3u : 0u)); }
+        for (unsigned k = 0; k < tc::SLOTS; k++) { tc::mbar_init(&sh->fed[k], 1u); tc::mbar_init(&sh->posted[k], 1u); tc::mbar_init(&sh->ready[k], 1u); tc::mbar_init(&sh->finished[k], tc::NW / 32u + (TENSOR_CORES ? 3u : 0u)); }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         tc::fence_proxy_async_smem();
     }
@@ -547,7 +683,9 @@ scheduler_kernel(const NasmDev *nasms, CtrlDev *ctrl, Entry *queue, StatusHost *
         else asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(ROLE_REGISTERS));
     }
     if (warp == sched_warp) {
-        scheduler_warp(nasms, ctrl, queue, status, sh, prof ? prof + (size_t)blockIdx.x * PROF_SLOTS : nullptr);
+        unsigned long long *mine = prof ? prof + (size_t)blockIdx.x * PROF_SLOTS : nullptr;
+        if (ctrl->ordered) ordered_warp(nasms, ctrl, queue, status, sh, mine);
+        else scheduler_warp(nasms, ctrl, queue, status, sh, mine);
     } else if (warp >= first_worker) {
         WorkerWarp<TENSOR_CORES> w{ctrl, status, prof};
         worker_loop(w);

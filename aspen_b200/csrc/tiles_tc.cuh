@@ -74,7 +74,9 @@ struct Shared {
     GraphRef graphs[CACHED_GRAPHS];
     unsigned long long full[MAX_STAGES], empty[MAX_STAGES];    // stage filled (both producers) / read by the MMAs
     unsigned long long acc_full[2], acc_empty[2];              // accumulator half complete / read by the workers
-    unsigned long long posted[SLOTS], finished[SLOTS];         // scheduler -> roles / roles -> scheduler
+    unsigned long long posted[SLOTS], finished[SLOTS];         // scheduler -> roles: the slot is filled / roles -> scheduler
+    unsigned long long fed[SLOTS];                             // W producer -> scheduler: the tile's last box is on its way
+    unsigned long long ready[SLOTS];                           // scheduler -> roles: the tile's parents are complete
     unsigned long long prof_mark;                              // time accounting: when the workers' last step ended
     unsigned tmem_base;
     Slot slots[SLOTS];
@@ -147,6 +149,31 @@ __device__ __forceinline__ bool mbar_wait(unsigned long long *bar, unsigned pari
                  "selp.u32 %0, 1, 0, p;\n\t}" : "=r"(ok) : "r"(smem_u32(bar)), "r"(parity) : "memory");
     if (__builtin_expect(ok != 0u, 1)) return true;
     return mbar_wait_slow(bar, parity, ctrl, status, where);
+}
+
+// A role's wait for the next tile (Shared::posted) or for its parents (Shared::ready).  The scheduler always posts an exit marker
+// eventually (end of run, stop, stall, abort); the time bound only guards against that logic failing.
+__device__ __forceinline__ bool wait_slot(unsigned long long *bar, unsigned parity, CtrlDev *ctrl, StatusHost *status) {
+    #pragma unroll 1
+    for (unsigned spin = 0; spin < 1024u; spin++)
+        if (mbar_try_wait(bar, parity)) return true;
+    unsigned long long t0;
+    asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t0));
+    const unsigned long long budget = 2ull * ctrl->stall_ns + 4ull * ctrl->pipe_ns + 1000000000ull;
+    for (unsigned spin = 1;; spin++) {
+        if (mbar_try_wait(bar, parity)) return true;
+        if ((spin & 63u) == 0u) {
+            __nanosleep(64);
+            unsigned long long now;
+            asm volatile("mov.u64 %0, %globaltimer;" : "=l"(now));
+            if (now - t0 > budget) break;
+        }
+    }
+    if (atomicCAS(&ctrl->abort, 0u, (unsigned)ASPEN_B200_ERR_PIPE) == 0u) {
+        status->info0 = 7; status->info1 = blockIdx.x; status->status = ASPEN_B200_ERR_PIPE;
+        __threadfence_system();
+    }
+    return false;
 }
 
 __device__ __forceinline__ void fence_proxy_async_smem() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
@@ -280,14 +307,21 @@ __device__ __forceinline__ bool recut(Ring &r, const LayerDev &L, Shared *sh, Ct
     return true;
 }
 
+// The slot's parents are complete (false: gave up, or the scheduler has withdrawn the tile).
+__device__ __forceinline__ bool wait_ready(const Slot &sl, unsigned long long *ready, unsigned parity, CtrlDev *ctrl, StatusHost *status) {
+    return wait_slot(ready, parity, ctrl, status) && sl.live != 0u;
+}
+
 // ---- X operand producer: one thread ----------------------------------------------------------------------------------
-__device__ __forceinline__ bool produce_a(const Slot &sl, unsigned ring, Ring &r, Shared *sh, CtrlDev *ctrl, StatusHost *status) {
+__device__ __forceinline__ bool produce_a(const Slot &sl, unsigned long long *ready, unsigned ready_parity, unsigned ring, Ring &r, Shared *sh, CtrlDev *ctrl,
+                                          StatusHost *status) {
     const LayerDev &L = sl.layer;
     const Origin g = origin(L, sl.tile);
     const unsigned char *map = sl.maps + (size_t)L.amap * 128;
+    asm volatile("prefetch.tensormap [%0];" ::"l"(map) : "memory");
+    if (!recut(r, L, sh, ctrl, status) || !wait_ready(sl, ready, ready_parity, ctrl, status)) return false;
     // activations were written with ordinary (generic proxy) stores; TMA reads them through the async proxy
     asm volatile("fence.proxy.async.global;" ::: "memory");
-    if (!recut(r, L, sh, ctrl, status)) return false;
     const unsigned kind = L.a_kind, tile_w = sl.tile.tile_w, tile_h = sl.tile.tile_h, per = L.per_stage, chunk_bytes = L.a_rows * 128u;
     if (kind == A_IM2COL) {
         const unsigned pos_w = sl.tile.pos_w, OW = L.OW, hw = L.OH * OW, KW = L.tap_kw, C = L.tap_c, sx = L.tap_sx, sy = L.tap_sy, chunks = L.chunks;
@@ -344,12 +378,20 @@ __device__ __forceinline__ bool produce_a(const Slot &sl, unsigned ring, Ring &r
 }
 
 // ---- W operand producer: one thread ----------------------------------------------------------------------------------
-__device__ __forceinline__ bool produce_b(const Slot &sl, unsigned ring, Ring &r, Shared *sh, CtrlDev *ctrl, StatusHost *status) {
+// Weights depend on no parent: a tile's first stages are filled while it still waits for them.  A stage beyond the ring's is
+// free only after the tile's own MMAs, so its (shorter bounded) wait starts behind the parents'.
+__device__ __forceinline__ bool produce_b(const Slot &sl, unsigned long long *ready, unsigned ready_parity, unsigned ring, Ring &r, Shared *sh, CtrlDev *ctrl,
+                                          StatusHost *status) {
     const LayerDev &L = sl.layer;
     const Origin g = origin(L, sl.tile);
     const unsigned char *map = sl.maps + (size_t)L.wmap * 128;
-    asm volatile("fence.proxy.async.global;" ::: "memory");
     if (!recut(r, L, sh, ctrl, status)) return false;
+    unsigned lead = r.stages;
+    if (L.type == K_ATTENTION_LAYER || L.type == V_ATTENTION_LAYER) {
+        if (!wait_ready(sl, ready, ready_parity, ctrl, status)) return false;
+        asm volatile("fence.proxy.async.global;" ::: "memory");
+        lead = ~0u;
+    }
     const unsigned tile_w = sl.tile.tile_w, tile_h = sl.tile.tile_h, per = L.per_stage, bytes = per * L.b_rows * 128u, b_off = per * L.a_rows * 128u;
     if (L.a_kind == A_HEAD) {
         for (unsigned n0 = 0; n0 < tile_w; n0 += 128u)
@@ -367,6 +409,7 @@ __device__ __forceinline__ bool produce_b(const Slot &sl, unsigned ring, Ring &r
     for (unsigned n0 = 0; n0 < tile_w; n0 += 128u)
         for (unsigned mp = 0; mp < tile_h; mp += BLOCK_ROWS)
             for (unsigned ch = 0, chunks = g.chunks(L, n0); ch < chunks; ch += per) {
+                if (lead-- == 0u && !wait_ready(sl, ready, ready_parity, ctrl, status)) return false;
                 if (!mbar_wait(&sh->empty[r.s], r.parity() ^ 1u, ctrl, status, 9)) return false;
                 mbar_arrive_expect_tx(&sh->full[r.s], bytes);
                 tma_load_3d(ring + r.s * r.stage_bytes + b_off, map, 0, g.by + (int)mp, g.bx + (int)ch, &sh->full[r.s]);

@@ -184,3 +184,30 @@ def test_activations_of_the_tensor_core_epilogue_are_rounded_once(act, workdir):
         assert float(np.abs(want).max()) > 0
         off = np.abs(got.astype(np.float64) - want) / np.spacing(np.abs(want).astype(np.float32))
         assert float(off.max()) <= 1.0, f"layer {layer}: {off.max():.1f} units in the last place at {lin.ravel()[off.argmax()]:.3e}"
+
+
+@pytest.mark.parametrize("precision", [0, 1])
+def test_launches_of_changing_sets_of_graphs(precision, workdir):
+    """A launch's tiles are handed out in an order made for the graphs that owe a pass: one alone, several together, another several."""
+    names = ("tiny_cnn", "tiny_transformer", "custom")
+    dnns = [api.Dnn(*harness.prepare(n, workdir)) for n in names]
+    graphs = [api.Nasm(d, 2, 16 if n == "tiny_transformer" else 0, 8) for d, n in zip(dnns, names)]
+    rpool, group = api.Rpool(), api.DseGroup(0, precision)
+    group.set_rpool(rpool)
+    xs = [harness.make_input(n, (g.ldata_info(0)["W"], g.ldata_info(0)["H"])) for n, g in zip(names, graphs)]
+    alone = {}
+    for owed in ((0,), (1,), (2,), (0, 1, 2), (1, 2), (0, 2), (1, 2), (0,)):
+        for i in owed:
+            rpool.add(graphs[i], xs[i])
+        group.run()
+        for i in owed:
+            group.wait(graphs[i])
+        group.stop()
+        assert group.status() == 0, api.last_error()
+        for i in owed:
+            got = graphs[i].ldata(graphs[i].num_ldata - 1).copy()
+            np.testing.assert_array_equal(got, alone.setdefault(i, got))
+    assert len(alone) == 3 and all(np.abs(v).max() > 0 for v in alone.values())
+    group.close()
+    for o in (*graphs, rpool, *dnns):
+        o.close()

@@ -97,3 +97,11 @@ def test_the_plan_spreads_layers_that_do_not_run_on_the_tensor_cores(batch, seq,
     layers = [(line.split()[0], [int(v) for v in line.split()[1:]]) for line in r.split("\n")[:-1]]
     th, tw, tiles = next(v for t, v in layers if "K_ATTENTION" in t)
     assert tiles >= 148 and th == seq
+
+
+@pytest.mark.parametrize("name,batch,seq,workers", [("tiny_cnn", 3, 0, 148), ("resnet50", 2, 0, 148), ("bert_base", 1, 37, 148), ("tiny_transformer", 2, 16, 1), ("custom", 5, 0, 7)])
+def test_a_launch_hands_out_every_tile_once_behind_its_parents(name, batch, seq, workers, workdir):
+    api.lib()
+    exe = build("claim_order", workdir, f"-L{LIBDIR}", "-laspen_b200", f"-Wl,-rpath,{LIBDIR}")
+    cfg, _ = harness.prepare(name, workdir)
+    passes(exe, cfg, str(batch), str(seq), str(workers))
