@@ -11,16 +11,18 @@
 //     weight row, its lanes stride over k with wide loads, and the dot products with all columns end in a
 //     warp reduction -- every SM pulls weights at once, which no 32-row block shape achieves here.
 //     The line lies at 8: with 16 columns the 32 x 32 blocks below are faster (19.9 against 23.6 us at k = 768, m = 3072).
-//   * larger: the fp32 FMA blocks of gemm_ffma.cuh, shape by `pick_shape`.
-// B200, wall time of a call, launch and wait included (before: the tile queue of the scheduler kernel, set up by a kernel of
-// its own, scalar FMAs from global memory):  1 x 768 x 768 95 -> 17 us, 333 x 770 x 1000 2430 -> 44 us,
-// 4096 x 768 x 3072 4640 -> 467 us (columns x k x rows).
+//   * larger: the fp32 FMA blocks of gemm_ffma.cuh, or the tensor cores over operands split into bf16 parts (gemm_split.cuh), by
+//     `pick_kernel`.
+// B200, wall time of a call, launch and wait included (columns x k x rows):  1 x 768 x 768 17 us;  333 x 770 x 1000 44 us in FMA
+// blocks (45 split);  4096 x 768 x 3072 466 in FMA blocks, 199 split.
 #include "internal.h"
 #include "tiles_simt.cuh"
 #include "gemm_ffma.cuh"
+#include "gemm_split.cuh"
 
 #include <cuda_runtime.h>
 #include <algorithm>
+#include <chrono>
 
 namespace {
 
@@ -117,6 +119,61 @@ __global__ void __launch_bounds__(fmablk::THREADS, 2) matmul_blocks(const Args a
     fmablk::block<S>(smem, threadIdx.x, a.k, lw, lx, BlockBarrier(), fin);
 }
 
+__device__ unsigned split_gave_up;      // a wait of matmul_split ran out (since the host last looked)
+
+template <int VEC>
+struct Operands {
+    Rows<VEC> w, x;
+    __device__ __forceinline__ float4 operator()(bool weight, unsigned row, unsigned k) const { return weight ? w(row, k) : x(row, k); }
+    __device__ __forceinline__ const float *at(bool weight, unsigned row, unsigned k) const { return (weight ? w.base : x.base) + (size_t)row * x.k + k; }
+    __device__ __forceinline__ unsigned ld() const { return x.k; }
+    __device__ __forceinline__ float4 piece(const float *p) const {
+        if (VEC == 4) return __ldg(reinterpret_cast<const float4 *>(p));
+        if (VEC == 2) {
+            const float2 a = __ldg(reinterpret_cast<const float2 *>(p)), b = __ldg(reinterpret_cast<const float2 *>(p + 2));
+            return make_float4(a.x, a.y, b.x, b.y);
+        }
+        return make_float4(__ldg(p), __ldg(p + 1), __ldg(p + 2), __ldg(p + 3));
+    }
+};
+// Bias, the common activations and the store of four outputs; rare activations go over the stored values afterwards, where nothing
+// else is in registers.
+struct FinishPiece {
+    const Args &a;
+    __device__ __forceinline__ bool rare() const { return a.act != NO_ACTIVATION && a.act != LINEAR && a.act != RELU && a.act != GELU; }
+    __device__ __forceinline__ void operator()(unsigned n, unsigned m, const float4 &v) const {
+        if (n >= a.n_cols || m >= a.m) return;
+        float r[4] = {v.x, v.y, v.z, v.w};
+        #pragma unroll
+        for (unsigned j = 0; j < 4; j++) {
+            if (a.bias && m + j < a.m) r[j] += __ldg(a.bias + m + j);
+            if (a.act == RELU) r[j] = r[j] > 0.f ? r[j] : 0.f;
+            else if (a.act == GELU) r[j] = 0.5f * r[j] * (1.f + erff(r[j] * 0.7071067811865475f));
+        }
+        float *o = a.out + (size_t)n * a.m + m;
+        if (a.vec_out && m + 4u <= a.m) *reinterpret_cast<float4 *>(o) = make_float4(r[0], r[1], r[2], r[3]);
+        else
+            #pragma unroll
+            for (unsigned j = 0; j < 4; j++) if (m + j < a.m) o[j] = r[j];
+    }
+    __device__ __forceinline__ void late(unsigned n, unsigned dn, unsigned cn, unsigned m, unsigned cm) const {
+        if (!rare()) return;
+        #pragma unroll 1
+        for (unsigned i = 0; i < cn * cm * 4u; i++) {
+            const unsigned col = n + i / (4u * cm) * dn, row = m + i / 4u % cm * 32u + i % 4u;
+            if (col < a.n_cols && row < a.m) { float *o = a.out + (size_t)col * a.m + row; *o = activate_rare(*o, a.act); }
+        }
+    }
+};
+template <int N, int VEC>
+__global__ void __launch_bounds__(split::THREADS, 1) matmul_split(const Args a) {
+    extern __shared__ __align__(1024) unsigned char smem[];
+    __shared__ split::Shared sh;
+    const Operands<VEC> in{{a.w, a.m, a.k}, {a.x, a.n_cols, a.k}};
+    const FinishPiece out{a};
+    split::blocks<N>(smem, &sh, &split_gave_up, a.n_cols, a.m, a.k, in, out);
+}
+
 // One weight row per warp, N columns (the last ones may be missing).
 template <int N, int VEC>
 __global__ void __launch_bounds__(fmablk::THREADS) matmul_rows(const Args a) {
@@ -151,19 +208,22 @@ __global__ void __launch_bounds__(fmablk::THREADS) matmul_rows(const Args a) {
     if (lane < N && lane < a.n_cols) a.out[(size_t)lane * a.m + m] = act_value(mine + (a.bias ? __ldg(a.bias + m) : 0.f), a.act);
 }
 
-// Shape with the shortest longest SM: blocks are dealt whole, so an SM runs ceil(blocks / SMs) of them, each
-// BM * BN * k FMAs at the shape's share of the FMA rate (one block of k = 3072 alone on its SM: 190, 96 and 30 us).
-unsigned pick_shape(unsigned n_cols, unsigned m, unsigned sms) {
-    static const struct { unsigned bm, bn; float rate; } shapes[] = {{128, 64, 0.80f}, {64, 64, 0.80f}, {32, 32, 0.65f}};
+// What runs a layer of more than 8 columns, by the longest SM: blocks are dealt whole, so an SM runs ceil(blocks / SMs) of them.
+// Measured, us: FMA blocks 3 and their multiply-adds at 163000 a us (32 x 32: 89000; rows that admit only 8- or 4-byte copies take
+// 1.2 or 1.5 times as long), the tensor cores with split operands 16 and per 32 of k 0.16 and 0.69 a block of 64 rows, 0.2 and 0.93
+// of 128.  k = 3072, 4096 columns, m = 3072: 1698 us in FMA blocks, 733 and 510 split; 64 columns: 61 and 82.
+// Splitting is for k >= 256: its error against 64 bits grows with what the accumulator of a 32-deep chunk cuts off, not with k, so that of
+// short sums would be larger than before.  2-norm, N(0, 1) operands, k = 258 / 512 / 770 / 3072: FMA blocks 1.5e-7 / 2.1e-7 / 1.9e-7 /
+// 5.0e-7, split 0.9e-7 / 1.0e-7 / 1.2e-7 / 1.9e-7.
+enum Kernel { FMA_128x64, FMA_64x64, FMA_32x32, SPLIT_128, SPLIT_64 };
+Kernel pick_kernel(unsigned n_cols, unsigned k, unsigned m, unsigned sms, int vec) {
+    auto rounds = [&](unsigned bm, unsigned bn) { return (double)(((unsigned long long)((m + bm - 1) / bm) * ((n_cols + bn - 1) / bn) + sms - 1) / sms); };
+    const double copies = vec == 4 ? 1.0 : vec == 2 ? 1.2 : 1.5, chunks = (k + 31) / 32;
+    const double cost[] = {3 + rounds(128, 64) * 8192.0 * k / 163000 * copies, 3 + rounds(64, 64) * 4096.0 * k / 163000 * copies,
+                           3 + rounds(32, 32) * 1024.0 * k / 89000 * copies, 16 + chunks * (0.2 + 0.93 * rounds(128, 128)), 16 + chunks * (0.16 + 0.69 * rounds(64, 128))};
     unsigned best = 0;
-    float best_cost = 0.f;
-    for (unsigned i = 0; i < 3; i++) {
-        const unsigned bm = shapes[i].bm, bn = shapes[i].bn;
-        const unsigned long long blocks = (unsigned long long)((m + bm - 1) / bm) * ((n_cols + bn - 1) / bn);
-        const float cost = (float)((blocks + sms - 1) / sms) * (float)(bm * bn) / shapes[i].rate;
-        if (i == 0 || cost < best_cost) { best = i; best_cost = cost; }
-    }
-    return best;
+    for (unsigned i = 1; i < (k < 256 ? 3u : 5u); i++) if (cost[i] < cost[best]) best = i;
+    return (Kernel)best;
 }
 
 template <typename S, int VEC>
@@ -171,6 +231,14 @@ void launch_blocks(const Args &a, cudaStream_t stream) {
     // the attribute is per device; asking for it on every call costs a fraction of the launch
     cudaFuncSetAttribute(matmul_blocks<S, VEC>, cudaFuncAttributeMaxDynamicSharedMemorySize, S::SMEM_BYTES);
     matmul_blocks<S, VEC><<<dim3((a.m + S::BM - 1) / S::BM, (a.n_cols + S::BN - 1) / S::BN), fmablk::THREADS, S::SMEM_BYTES, stream>>>(a);
+}
+
+template <int N, int VEC>
+void launch_split(const Args &a, unsigned sms, cudaStream_t stream) {
+    typedef split::Shape<N> S;
+    const unsigned blocks = ((a.m + N - 1) / N) * ((a.n_cols + 127) / 128);
+    cudaFuncSetAttribute(matmul_split<N, VEC>, cudaFuncAttributeMaxDynamicSharedMemorySize, S::SMEM_BYTES);
+    matmul_split<N, VEC><<<std::min(blocks, sms), split::THREADS, S::SMEM_BYTES, stream>>>(a);
 }
 
 template <int VEC>
@@ -183,10 +251,13 @@ void launch(const Args &a, unsigned sms, cudaStream_t stream) {
         else matmul_rows<8, VEC><<<grid, fmablk::THREADS, 0, stream>>>(a);
         return;
     }
-    const unsigned shape = pick_shape(a.n_cols, a.m, sms);
-    if (shape == 0) launch_blocks<fmablk::Large, VEC>(a, stream);
-    else if (shape == 1) launch_blocks<fmablk::Medium, VEC>(a, stream);
-    else launch_blocks<fmablk::Small, VEC>(a, stream);
+    switch (pick_kernel(a.n_cols, a.k, a.m, sms, VEC)) {
+        case FMA_128x64: launch_blocks<fmablk::Large, VEC>(a, stream); break;
+        case FMA_64x64: launch_blocks<fmablk::Medium, VEC>(a, stream); break;
+        case FMA_32x32: launch_blocks<fmablk::Small, VEC>(a, stream); break;
+        case SPLIT_128: launch_split<128, VEC>(a, sms, stream); break;
+        case SPLIT_64: launch_split<64, VEC>(a, sms, stream); break;
+    }
 }
 
 }  // namespace
@@ -210,6 +281,7 @@ extern "C" int aspen_b200_matmul_noalloc(const float *x_dev, const float *w_dev,
     if (err == cudaSuccess) err = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     if (err != cudaSuccess || sms <= 0) { ASPEN_ERR("aspen_b200_matmul_noalloc: no current CUDA device (%s)\n", cudaGetErrorString(err)); return -3; }
     cudaStream_t stream = static_cast<cudaStream_t>(cuda_stream);
+    const auto started = std::chrono::steady_clock::now();
     const Args a{x_dev, w_dev, bias_dev, out_dev, n_cols, k, m, activation, m % 4 == 0 && reinterpret_cast<uintptr_t>(out_dev) % 16 == 0};
     const uintptr_t align = reinterpret_cast<uintptr_t>(x_dev) | reinterpret_cast<uintptr_t>(w_dev);
     if (k % 4 == 0 && align % 16 == 0) launch<4>(a, (unsigned)sms, stream);
@@ -219,5 +291,14 @@ extern "C" int aspen_b200_matmul_noalloc(const float *x_dev, const float *w_dev,
     if (err != cudaSuccess) { ASPEN_ERR("aspen_b200_matmul_noalloc: launch failed: %s\n", cudaGetErrorString(err)); return -3; }
     err = cudaStreamSynchronize(stream);
     if (err != cudaSuccess) { ASPEN_ERR("aspen_b200_matmul_noalloc: %s\n", cudaGetErrorString(err)); return -3; }
+    // a wait that runs out does so after split::LIMIT_NS, so a call that took less has had none
+    if (std::chrono::steady_clock::now() - started > std::chrono::nanoseconds(split::LIMIT_NS / 2)) {
+        unsigned gave_up = 0;
+        const unsigned none = 0;
+        if (cudaMemcpyFromSymbol(&gave_up, split_gave_up, sizeof gave_up) != cudaSuccess || (gave_up && cudaMemcpyToSymbol(split_gave_up, &none, sizeof none) != cudaSuccess) || gave_up) {
+            ASPEN_ERR("aspen_b200_matmul_noalloc: a wait of the kernel ran out\n");
+            return -3;
+        }
+    }
     return 0;
 }

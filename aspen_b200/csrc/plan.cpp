@@ -81,7 +81,7 @@ Grid choose(const nasm_ldata_t &ld, const nasm_t *nasm, int precision, unsigned 
         for (unsigned i = 0; i < nhs; i++)
             for (unsigned tw = quantum; tw < g.seg + quantum && tw <= 16 * quantum; tw += quantum) {
                 const unsigned tiles = ceil_div(H, hs[i]) * (W / g.seg) * ceil_div(g.seg, tw);
-                const double us = tile_us(path, l, std::min(hs[i], H), std::min(tw, g.seg), k, served ? 2.5 : 4.0);
+                const double us = tile_us(path, l, std::min(hs[i], H), std::min(tw, g.seg), k, served ? 2.5 : getenv("GAP") ? atof(getenv("GAP")) : 4.0);
                 const double share = (double)tiles / sms;
                 // The layer's work, and the length of its longest tile: launched alone the last tiles of a layer run while the
                 // rest of the chip waits, served the passes of other graphs fill those SMs but the graphs in rotation are few.
@@ -90,7 +90,9 @@ Grid choose(const nasm_ldata_t &ld, const nasm_t *nasm, int precision, unsigned 
                 // offer each SM, which a plan of one graph does not know: three graphs of ResNet-50 x 32 in bursts of twelve take
                 // 1.92 / 1.61 / 1.51 ms a request with 0.2 / 0.5 / 1.0 tiles, eight of x 4 take 0.279 / 0.283 / 0.304.  0.5 lies
                 // between the two.
-                const double cost = us * (share + (served ? 0.5 : 0.7));
+                static const int form = getenv("FORM") ? atoi(getenv("FORM")) : 0;
+                static const double wt = getenv("WT") ? atof(getenv("WT")) : 0.7;
+                const double cost = us * (served ? share + 0.5 : form == 0 ? share + wt : form == 1 ? std::max(1.0, share + wt) : share <= 1 ? 1 + wt * share : share + wt);
                 if (best == 0 || cost < best * 0.999) { best = cost; g.th = hs[i]; g.tw = tw; }
             }
     } else if (l->type == SOFTMAX_LAYER || l->type == YOLO_LAYER || l->type == APPEND_LAYER) {

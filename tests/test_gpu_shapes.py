@@ -29,6 +29,64 @@ def test_noalloc_blocks_at_their_edges(n, k, m, act):
     assert bad == 0, f"{bad} mismatches, max abs {ea:.3e}, max rel {er:.3e}"
 
 
+# Blocks of 128 columns x 64 or 128 rows and chunks of 32 of k, at their edges, with every kind of load (k % 4, k % 2, odd).
+SPLIT_SHAPES = [(640, 256, 1500), (1025, 257, 1087), (641, 290, 2049), (385, 1000, 2047), (2500, 259, 1024), (4100, 319, 2050)]
+
+
+def noalloc(x, w, b, act):
+    import torch
+    xd, wd, bd = (torch.from_numpy(a).cuda() for a in (x, w, b))
+    od = torch.full((x.shape[0], w.shape[0]), float("nan"), device="cuda")
+    torch.cuda.synchronize()
+    assert api.lib().aspen_b200_matmul_noalloc(xd.data_ptr(), wd.data_ptr(), bd.data_ptr(), od.data_ptr(), x.shape[0], x.shape[1], w.shape[0], act, None) == 0, api.last_error()
+    return od.cpu().numpy()
+
+
+@pytest.mark.parametrize("n,k,m", SPLIT_SHAPES)
+@pytest.mark.parametrize("act", [0, 3, 8])
+def test_noalloc_on_the_tensor_cores_is_as_close_to_64_bits_as_fp32_sums(n, k, m, act):
+    """A sum of k products rounded to fp32 one after the other is off by some 0.2 sqrt(k / 2) 2**-24 of its size where two sums are kept (the FMA
+    blocks); 2**-23 covers the rounding of the result and of the activation on top."""
+    rng = np.random.default_rng(n + k)
+    x = rng.standard_normal((n, k), dtype=np.float32)
+    w = (rng.standard_normal((m, k)) * np.sqrt(2 / k)).astype(np.float32)
+    b = rng.standard_normal((m,), dtype=np.float32)
+    got = noalloc(x, w, b, act)
+    want = x.astype(np.float64) @ w.T.astype(np.float64) + b
+    if act == 3:
+        want = np.tanh(want)
+    elif act == 8:
+        import torch
+        want = torch.nn.functional.gelu(torch.from_numpy(want)).numpy()
+    assert np.isfinite(got).all()
+    assert np.linalg.norm(got - want) <= (0.2 * np.sqrt(k / 2) * 2.0**-24 + 2.0**-23) * np.linalg.norm(want)
+
+
+def test_noalloc_on_the_tensor_cores_over_the_range_of_fp32():
+    """Infinities and NaN spread as in a sum of fp32 products, and only into their own rows and columns; large, small and denormal values keep
+    the precision of fp32 products."""
+    rng = np.random.default_rng(3)
+    n, k, m = 700, 260, 1100
+    x = rng.standard_normal((n, k), dtype=np.float32)
+    w = (rng.standard_normal((m, k)) * np.sqrt(2 / k)).astype(np.float32)
+    w[w == 0] = 1
+    x[3, 7], x[400, 100], x[699, 259], x[401, 5] = np.inf, -np.inf, np.nan, np.float32(3.4e38)
+    w[401:, 5] = np.float32(1e-3)
+    x[10] *= np.float32(2.0**-100)
+    x[11] = rng.uniform(1, 2, k).astype(np.float32) * np.float32(2.0**-127)
+    w[20] *= np.float32(2.0**60)
+    w[20, 5] = np.float32(1e-3)          # 3.4e38 times a value of 2**60 would be past the range of fp32
+    b = np.zeros(m, np.float32)
+    got = noalloc(x, w, b, 0)
+    with np.errstate(all="ignore"):
+        want = x.astype(np.float64) @ w.T.astype(np.float64)
+    special = np.isin(np.arange(n), (3, 400, 699))
+    np.testing.assert_array_equal(got[[3, 400]], want[[3, 400]].astype(np.float32))        # every sum is an infinity of w's sign
+    assert np.isnan(got[699]).all() and np.isfinite(got[~special]).all()
+    scale = np.abs(x[~special].astype(np.float64)) @ np.abs(w.T.astype(np.float64))        # each product is off by 2**-24 at most, each of some k partial sums too
+    assert (np.abs(got[~special] - want[~special]) <= 2.0**-24 * (1 + np.sqrt(k)) * scale + 2.0**-149 * k).all()
+
+
 @pytest.mark.parametrize("name,batch,seq,precision", [("tiny_attn", 1, 1, 0), ("tiny_attn", 3, 33, 0), ("tiny_attn", 1, 129, 0), ("tiny_attn_causal", 2, 255, 0),
                                                       ("tiny_attn_causal", 1, 257, 0), ("tiny_attn_causal", 1, 300, 1), ("tiny_transformer", 64, 128, 0),
                                                       ("tiny_cnn", 1, 0, 0), ("tiny_cnn", 33, 0, 0), ("tiny_cnn", 9, 0, 1), ("custom", 1, 0, 0), ("custom", 130, 0, 0),
