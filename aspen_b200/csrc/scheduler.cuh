@@ -568,27 +568,30 @@ static __device__ __noinline__ void ordered_warp(const NasmDev *nasms, CtrlDev *
     post_exit(sh, issued % tc::SLOTS);
 }
 
-// The loops of the one-thread roles, all their state inside: a reference to it would put it into local memory.
+// The loops of the one-warp roles, all their state inside: a reference to it would put it into local memory.
 template <unsigned ROLE>
-static __device__ __forceinline__ void single_thread_role(unsigned char *smem, tc::Shared *sh, CtrlDev *ctrl, StatusHost *status) {
+static __device__ __forceinline__ void one_warp_role(unsigned char *smem, tc::Shared *sh, CtrlDev *ctrl, StatusHost *status) {
     const unsigned ring = tc::smem_u32(smem);
     tc::Ring r;
     unsigned half = 0, acc_uses = 0;
     for (unsigned seq = 0;; seq++) {
         const unsigned k = seq % tc::SLOTS;
         const unsigned parity = (seq / tc::SLOTS) & 1u;
-        if (!tc::wait_slot(&sh->posted[k], parity, ctrl, status)) break;
+        if (!__all_sync(0xffffffffu, tc::wait_slot(&sh->posted[k], parity, ctrl, status))) break;
         const tc::Slot &sl = sh->slots[k];
-        if (!sl.live) break;
-        if (sl.layer.tc) {
+        if (!tc::uniform(sl.live)) break;
+        if (tc::uniform((unsigned)sl.layer.tc)) {
             bool ok;
             if (ROLE == tc::WARP_A) ok = tc::produce_a(sl, &sh->ready[k], parity, ring, r, sh, ctrl, status);
             else if (ROLE == tc::WARP_B) ok = tc::produce_b(sl, &sh->ready[k], parity, ring, r, sh, ctrl, status);
             else ok = tc::wait_ready(sl, &sh->ready[k], parity, ctrl, status) && tc::issue_mma(sl, ring, r, half, acc_uses, sh, ctrl, status);
             if (!ok) break;
         }
-        if (ROLE == tc::WARP_B) tc::mbar_arrive(&sh->fed[k]);
-        tc::mbar_arrive(&sh->finished[k]);
+        __syncwarp();
+        if ((threadIdx.x & 31u) == 0u) {
+            if (ROLE == tc::WARP_B) tc::mbar_arrive(&sh->fed[k]);
+            tc::mbar_arrive(&sh->finished[k]);
+        }
     }
     if (*(volatile unsigned *)&ctrl->abort) {
         // copies and MMAs of this CTA may still be in flight; they take microseconds
@@ -654,7 +657,7 @@ __global__ void __launch_bounds__(threads<TENSOR_CORES>(), 1)
 scheduler_kernel(const NasmDev *nasms, CtrlDev *ctrl, Entry *queue /* or, ctrl->ordered, the order of the launch */, StatusHost *status, unsigned long long *prof) {
     extern __shared__ __align__(1024) unsigned char smem[];      // stages need 1024-byte alignment for the 128-byte swizzle
     tc::Shared *sh = reinterpret_cast<tc::Shared *>(smem + work_bytes<TENSOR_CORES>());
-    const unsigned tid = threadIdx.x, warp = tid >> 5, lane = tid & 31u;
+    const unsigned tid = threadIdx.x, warp = tc::uniform(tid >> 5);
     constexpr unsigned sched_warp = TENSOR_CORES ? tc::WARP_SCHED : 0u, first_worker = TENSOR_CORES ? tc::WARP_WORK : 1u;
 
     if (tid == 0) {
@@ -689,10 +692,10 @@ scheduler_kernel(const NasmDev *nasms, CtrlDev *ctrl, Entry *queue /* or, ctrl->
     } else if (warp >= first_worker) {
         WorkerWarp<TENSOR_CORES> w{ctrl, status, prof};
         worker_loop(w);
-    } else if (TENSOR_CORES && lane == 0) {
-        if (warp == tc::WARP_A) single_thread_role<tc::WARP_A>(smem, sh, ctrl, status);
-        else if (warp == tc::WARP_B) single_thread_role<tc::WARP_B>(smem, sh, ctrl, status);
-        else single_thread_role<tc::WARP_MMA>(smem, sh, ctrl, status);
+    } else if (TENSOR_CORES) {
+        if (warp == tc::WARP_A) one_warp_role<tc::WARP_A>(smem, sh, ctrl, status);
+        else if (warp == tc::WARP_B) one_warp_role<tc::WARP_B>(smem, sh, ctrl, status);
+        else one_warp_role<tc::WARP_MMA>(smem, sh, ctrl, status);
     }
     __syncwarp();
     if (TENSOR_CORES) tc::tc_fence_before();

@@ -11,18 +11,18 @@
 //
 // Roles.  A tile is a sequence of 128 x (<= 256) blocks, and four kinds of warps walk the same sequence, each at its own pace
 // and across tile boundaries; nothing but mbarriers connects them:
-//     warp A, warp B   one thread each: TMA boxes of the X / W operand into a ring of stages (32 fp32 of k a chunk, up to four chunks
-//                      a stage)
-//     warp MMA         one thread: four tcgen05.mma (k = 8 each) per chunk, accumulators alternate between two halves of TMEM
+//     warp A, warp B   TMA boxes of the X / W operand into a ring of stages (32 fp32 of k a chunk, up to four chunks a stage)
+//     warp MMA         four tcgen05.mma (k = 8 each) per chunk, accumulators alternate between two halves of TMEM
 //     8 worker warps   epilogue: TMEM -> registers -> bias, activation, residual add, softmax -> memory; they also run the
 //                      memory-bound tiles
 // so the operands of the next block (or of the next tile, once the scheduler has posted one) stream in and are multiplied
 // while the previous block is written out.
-// What bounds the k loop.  A one-thread role takes 0.17 us for a wait and a box whatever it holds (a probe that only waits and
-// issues; 0.24 with two boxes, 0.043 a chunk with four chunks in a box), so two threads feed the ring and narrow tiles take several
-// chunks a stage.  A chunk of a 128-column block then takes 0.16 us with 32 or 64 rows, 0.22 with 128 and 0.30 - 0.37 with 256 (all
-// SMs at work, operands in L2; 256 rows is the rate of the measured dense TF32 peak).  The loops below hold no division for the
-// same reason.
+// What bounds the k loop.  The instruction streams of the three issuing warps, for narrow tiles: issued from one lane's own branch a
+// wait and a box take 0.17 us whatever the box holds, since TMA and MMA take their operands from uniform registers and a value of one
+// lane has to be brought there each time.  So the whole warp walks with values that the compiler knows to be uniform, and one lane
+// issues (BERT 1 x 37 875 -> 799 us a pass, ResNet-50 + VGG-16 x 16 1859 -> 1719, ResNet-50 x 32 1465 -> 1398); two warps feed
+// the ring, narrow tiles take several chunks a stage, and the loops hold no division.  A chunk of a block of 256 rows takes
+// 0.30 - 0.37 us (all SMs at work, operands in L2), the rate of the measured dense TF32 peak.
 //
 // Staging.  Both operands are K-major, 32 fp32 (128 bytes) per row and k-chunk, in the 128-byte swizzled shared-memory
 // layout UMMA descriptors and TMA share.  A narrow layer (few tokens, few pixels) stages only the columns it has; the MMA reads
@@ -278,7 +278,7 @@ __device__ __forceinline__ unsigned umma_idesc(unsigned n) {
 struct Origin {
     int ax, ay, bx, by;
     unsigned seen;
-    __device__ __forceinline__ unsigned chunks(const LayerDev &L, unsigned n0) const { return seen ? min(L.chunks, (seen + n0 + 31u) >> 5) : L.chunks; }
+    __device__ __forceinline__ unsigned chunks(unsigned all, unsigned n0) const { return seen ? min(all, (seen + n0 + 31u) >> 5) : all; }
 };
 
 __device__ __forceinline__ Origin origin(const LayerDev &L, const TileDev &T) {
@@ -297,6 +297,18 @@ __device__ __forceinline__ Origin origin(const LayerDev &L, const TileDev &T) {
     return g;
 }
 
+// A value that all lanes of a converged warp hold: the compiler keeps what is computed from it in uniform registers, where the operands of
+// TMA and MMA instructions have to be.
+__device__ __forceinline__ unsigned uniform(unsigned v) { return __shfl_sync(0xffffffffu, v, 0); }
+__device__ __forceinline__ int uniform(int v) { return __shfl_sync(0xffffffffu, v, 0); }
+template <typename T>
+__device__ __forceinline__ const T *uniform(const T *p) { return reinterpret_cast<const T *>(__shfl_sync(0xffffffffu, reinterpret_cast<unsigned long long>(p), 0)); }
+__device__ __forceinline__ Origin uniform(const Origin &g) {
+    Origin u;
+    u.ax = uniform(g.ax); u.ay = uniform(g.ay); u.bx = uniform(g.bx); u.by = uniform(g.by); u.seen = uniform(g.seen);
+    return u;
+}
+
 // Ring position of one role.  `uses` holds, per stage, the parity of the number of times this role has used it.
 struct Ring {
     unsigned s = 0, uses = 0, stage_bytes = 0, stages = 1;
@@ -304,35 +316,44 @@ struct Ring {
     __device__ __forceinline__ unsigned parity() const { return (uses >> s) & 1u; }
 };
 
+// A wait of a whole warp: its lanes give up together.
+__device__ __forceinline__ bool warp_wait(unsigned long long *bar, unsigned parity, CtrlDev *ctrl, StatusHost *status, unsigned where) {
+    return __all_sync(0xffffffffu, mbar_wait(bar, parity, ctrl, status, where));
+}
+
 // Producer side of a change of the ring's cut: every stage must have been read.
 __device__ __forceinline__ bool recut(Ring &r, const LayerDev &L, Shared *sh, CtrlDev *ctrl, StatusHost *status) {
-    if (L.stage_bytes == r.stage_bytes) return true;
+    const unsigned stage_bytes = uniform(L.stage_bytes);
+    if (stage_bytes == r.stage_bytes) return true;
     if (r.stage_bytes)
         for (unsigned i = 0; i < r.stages; i++)
-            if (!mbar_wait(&sh->empty[i], ((r.uses >> i) & 1u) ^ 1u, ctrl, status, 8)) return false;
-    r.s = 0; r.stage_bytes = L.stage_bytes; r.stages = L.stages;
+            if (!warp_wait(&sh->empty[i], ((r.uses >> i) & 1u) ^ 1u, ctrl, status, 8)) return false;
+    r.s = 0; r.stage_bytes = stage_bytes; r.stages = uniform((unsigned)L.stages);
     return true;
 }
 
 // The slot's parents are complete (false: gave up, or the scheduler has withdrawn the tile).
 __device__ __forceinline__ bool wait_ready(const Slot &sl, unsigned long long *ready, unsigned parity, CtrlDev *ctrl, StatusHost *status) {
-    return wait_slot(ready, parity, ctrl, status) && sl.live != 0u;
+    return __all_sync(0xffffffffu, wait_slot(ready, parity, ctrl, status) && sl.live != 0u);
 }
 
-// ---- X operand producer: one thread ----------------------------------------------------------------------------------
+// The three roles below are one warp each: all lanes walk, and one (the same one each time) issues.
+// ---- X operand producer -----------------------------------------------------------------------------------------------
 __device__ __forceinline__ bool produce_a(const Slot &sl, unsigned long long *ready, unsigned ready_parity, unsigned ring, Ring &r, Shared *sh, CtrlDev *ctrl,
                                           StatusHost *status) {
     const LayerDev &L = sl.layer;
-    const Origin g = origin(L, sl.tile);
-    const unsigned char *map = sl.maps + (size_t)L.amap * 128;
-    asm volatile("prefetch.tensormap [%0];" ::"l"(map) : "memory");
+    const Origin g = uniform(origin(L, sl.tile));
+    const unsigned char *map = uniform(sl.maps + (size_t)L.amap * 128);
+    if (elect_one()) asm volatile("prefetch.tensormap [%0];" ::"l"(map) : "memory");
     if (!recut(r, L, sh, ctrl, status) || !wait_ready(sl, ready, ready_parity, ctrl, status)) return false;
     // activations were written with ordinary (generic proxy) stores; TMA reads them through the async proxy
     asm volatile("fence.proxy.async.global;" ::: "memory");
-    const unsigned kind = L.a_kind, tile_w = sl.tile.tile_w, tile_h = sl.tile.tile_h, per = L.per_stage, chunk_bytes = L.a_rows * 128u;
+    const unsigned kind = uniform((unsigned)L.a_kind), tile_w = uniform(sl.tile.tile_w), tile_h = uniform(sl.tile.tile_h), per = uniform((unsigned)L.per_stage),
+                   chunk_bytes = uniform((unsigned)L.a_rows) * 128u;
     if (kind == A_IM2COL) {
-        const unsigned pos_w = sl.tile.pos_w, OW = L.OW, hw = L.OH * OW, KW = L.tap_kw, C = L.tap_c, sx = L.tap_sx, sy = L.tap_sy, chunks = L.chunks;
-        const int pad = (int)L.tap_pad;
+        const unsigned pos_w = uniform(sl.tile.pos_w), OW = uniform(L.OW), hw = uniform(L.OH) * OW, KW = uniform((unsigned)L.tap_kw), C = uniform(L.tap_c),
+                       sx = uniform((unsigned)L.tap_sx), sy = uniform((unsigned)L.tap_sy), chunks = uniform(L.chunks);
+        const int pad = (int)uniform((unsigned)L.tap_pad);
         for (unsigned n0 = 0; n0 < tile_w; n0 += 128u) {
             const unsigned n = pos_w + n0, pn = n / hw, q = n - pn * hw, py = q / OW, px = q - py * OW;      // first output pixel of the block
             const int x0 = (int)(px * sx) - pad, y0 = (int)(py * sy) - pad;
@@ -341,10 +362,11 @@ __device__ __forceinline__ bool produce_a(const Slot &sl, unsigned long long *re
                 for (unsigned ch = 0; ch < chunks; ch += per) {
                     const unsigned count = min(per, chunks - ch);
                     unsigned dst = ring + r.s * r.stage_bytes;
-                    if (!mbar_wait(&sh->empty[r.s], r.parity() ^ 1u, ctrl, status, 2)) return false;
-                    mbar_arrive_expect_tx(&sh->full[r.s], count * chunk_bytes);
+                    if (!warp_wait(&sh->empty[r.s], r.parity() ^ 1u, ctrl, status, 2)) return false;
+                    const bool issue = elect_one();
+                    if (issue) mbar_arrive_expect_tx(&sh->full[r.s], count * chunk_bytes);
                     for (unsigned j = 0; j < count; j++, dst += chunk_bytes) {
-                        tma_load_im2col(dst, map, (int)c, x0, y0, (int)pn, kw, kh, &sh->full[r.s]);
+                        if (issue) tma_load_im2col(dst, map, (int)c, x0, y0, (int)pn, kw, kh, &sh->full[r.s]);
                         c += 32u;
                         if (c == C) { c = 0; if (++kw == KW) { kw = 0; kh++; } }
                     }
@@ -354,16 +376,19 @@ __device__ __forceinline__ bool produce_a(const Slot &sl, unsigned long long *re
         }
         return true;
     }
-    const bool multi = L.a_multi != 0;
+    const bool multi = uniform((unsigned)L.a_multi) != 0u;
+    const unsigned all_chunks = uniform(L.chunks);
     for (unsigned n0 = 0; n0 < tile_w; n0 += 128u) {
-        const unsigned chunks = g.chunks(L, n0);
+        const unsigned chunks = g.chunks(all_chunks, n0);
         const int y = g.ay + (int)n0;
         for (unsigned mp = 0; mp < tile_h; mp += BLOCK_ROWS) {
             if (multi) {
                 for (unsigned ch = 0; ch < chunks; ch += per) {
-                    if (!mbar_wait(&sh->empty[r.s], r.parity() ^ 1u, ctrl, status, 2)) return false;
-                    mbar_arrive_expect_tx(&sh->full[r.s], per * chunk_bytes);
-                    tma_load_3d(ring + r.s * r.stage_bytes, map, 0, y, g.ax + (int)ch, &sh->full[r.s]);
+                    if (!warp_wait(&sh->empty[r.s], r.parity() ^ 1u, ctrl, status, 2)) return false;
+                    if (elect_one()) {
+                        mbar_arrive_expect_tx(&sh->full[r.s], per * chunk_bytes);
+                        tma_load_3d(ring + r.s * r.stage_bytes, map, 0, y, g.ax + (int)ch, &sh->full[r.s]);
+                    }
                     r.step();
                 }
                 continue;
@@ -371,11 +396,13 @@ __device__ __forceinline__ bool produce_a(const Slot &sl, unsigned long long *re
             for (unsigned ch = 0; ch < chunks; ch += per) {
                 const unsigned count = min(per, chunks - ch);
                 unsigned dst = ring + r.s * r.stage_bytes;
-                if (!mbar_wait(&sh->empty[r.s], r.parity() ^ 1u, ctrl, status, 2)) return false;
-                mbar_arrive_expect_tx(&sh->full[r.s], count * chunk_bytes);
-                for (unsigned j = 0; j < count; j++, dst += chunk_bytes) {
-                    if (kind == A_HEAD) tma_load_3d(dst, map, (int)(ch + j) * 32, g.ax, y, &sh->full[r.s]);
-                    else tma_load_2d(dst, map, (g.ax + (int)(ch + j)) * 32, y, &sh->full[r.s]);
+                if (!warp_wait(&sh->empty[r.s], r.parity() ^ 1u, ctrl, status, 2)) return false;
+                if (elect_one()) {
+                    mbar_arrive_expect_tx(&sh->full[r.s], count * chunk_bytes);
+                    for (unsigned j = 0; j < count; j++, dst += chunk_bytes) {
+                        if (kind == A_HEAD) tma_load_3d(dst, map, (int)(ch + j) * 32, g.ax, y, &sh->full[r.s]);
+                        else tma_load_2d(dst, map, (g.ax + (int)(ch + j)) * 32, y, &sh->full[r.s]);
+                    }
                 }
                 r.step();
             }
@@ -384,14 +411,14 @@ __device__ __forceinline__ bool produce_a(const Slot &sl, unsigned long long *re
     return true;
 }
 
-// ---- W operand producer: one thread ----------------------------------------------------------------------------------
+// ---- W operand producer -----------------------------------------------------------------------------------------------
 // Weights depend on no parent: a tile's first stages are filled while it still waits for them.  A stage beyond the ring's is
 // free only after the tile's own MMAs, so its (shorter bounded) wait starts behind the parents'.
 __device__ __forceinline__ bool produce_b(const Slot &sl, unsigned long long *ready, unsigned ready_parity, unsigned ring, Ring &r, Shared *sh, CtrlDev *ctrl,
                                           StatusHost *status) {
     const LayerDev &L = sl.layer;
-    const Origin g = origin(L, sl.tile);
-    const unsigned char *map = sl.maps + (size_t)L.wmap * 128;
+    const Origin g = uniform(origin(L, sl.tile));
+    const unsigned char *map = uniform(sl.maps + (size_t)L.wmap * 128);
     if (!recut(r, L, sh, ctrl, status)) return false;
     unsigned lead = r.stages;
     if (L.type == K_ATTENTION_LAYER || L.type == V_ATTENTION_LAYER) {
@@ -399,61 +426,70 @@ __device__ __forceinline__ bool produce_b(const Slot &sl, unsigned long long *re
         asm volatile("fence.proxy.async.global;" ::: "memory");
         lead = ~0u;
     }
-    const unsigned tile_w = sl.tile.tile_w, tile_h = sl.tile.tile_h, per = L.per_stage, bytes = per * L.b_rows * 128u, b_off = per * L.a_rows * 128u;
+    const unsigned tile_w = uniform(sl.tile.tile_w), tile_h = uniform(sl.tile.tile_h), per = uniform((unsigned)L.per_stage), box = uniform((unsigned)L.b_rows) * 128u,
+                   bytes = per * box, b_off = per * uniform((unsigned)L.a_rows) * 128u, all_chunks = uniform(L.chunks);
     if (L.a_kind == A_HEAD) {
         for (unsigned n0 = 0; n0 < tile_w; n0 += 128u)
             for (unsigned mp = 0; mp < tile_h; mp += BLOCK_ROWS)
-                for (unsigned ch = 0, chunks = L.chunks; ch < chunks; ch += per) {
-                    const unsigned n = min(per, chunks - ch), box = L.b_rows * 128u;
-                    if (!mbar_wait(&sh->empty[r.s], r.parity() ^ 1u, ctrl, status, 9)) return false;
-                    mbar_arrive_expect_tx(&sh->full[r.s], n * box);
-                    for (unsigned j = 0; j < n; j++)
-                        tma_load_3d(ring + r.s * r.stage_bytes + b_off + j * box, map, (int)(ch + j) * 32, g.bx, g.by + (int)mp, &sh->full[r.s]);
+                for (unsigned ch = 0; ch < all_chunks; ch += per) {
+                    const unsigned n = min(per, all_chunks - ch);
+                    if (!warp_wait(&sh->empty[r.s], r.parity() ^ 1u, ctrl, status, 9)) return false;
+                    if (elect_one()) {
+                        mbar_arrive_expect_tx(&sh->full[r.s], n * box);
+                        for (unsigned j = 0; j < n; j++)
+                            tma_load_3d(ring + r.s * r.stage_bytes + b_off + j * box, map, (int)(ch + j) * 32, g.bx, g.by + (int)mp, &sh->full[r.s]);
+                    }
                     r.step();
                 }
         return true;
     }
     for (unsigned n0 = 0; n0 < tile_w; n0 += 128u)
         for (unsigned mp = 0; mp < tile_h; mp += BLOCK_ROWS)
-            for (unsigned ch = 0, chunks = g.chunks(L, n0); ch < chunks; ch += per) {
+            for (unsigned ch = 0, chunks = g.chunks(all_chunks, n0); ch < chunks; ch += per) {
                 if (lead-- == 0u && !wait_ready(sl, ready, ready_parity, ctrl, status)) return false;
-                if (!mbar_wait(&sh->empty[r.s], r.parity() ^ 1u, ctrl, status, 9)) return false;
-                mbar_arrive_expect_tx(&sh->full[r.s], bytes);
-                tma_load_3d(ring + r.s * r.stage_bytes + b_off, map, 0, g.by + (int)mp, g.bx + (int)ch, &sh->full[r.s]);
+                if (!warp_wait(&sh->empty[r.s], r.parity() ^ 1u, ctrl, status, 9)) return false;
+                if (elect_one()) {
+                    mbar_arrive_expect_tx(&sh->full[r.s], bytes);
+                    tma_load_3d(ring + r.s * r.stage_bytes + b_off, map, 0, g.by + (int)mp, g.bx + (int)ch, &sh->full[r.s]);
+                }
                 r.step();
             }
     return true;
 }
 
-// ---- MMA issuer: one thread ------------------------------------------------------------------------------------------
+// ---- MMA issuer -------------------------------------------------------------------------------------------------------
 // `half`: accumulator half of the next block; `acc_uses`: parity of the uses of each half.
 __device__ __forceinline__ bool issue_mma(const Slot &sl, unsigned ring, Ring &r, unsigned &half, unsigned &acc_uses, Shared *sh, CtrlDev *ctrl, StatusHost *status) {
     const LayerDev &L = sl.layer;
-    if (L.stage_bytes != r.stage_bytes) { r.s = 0; r.stage_bytes = L.stage_bytes; r.stages = L.stages; }
-    const unsigned tmem = sh->tmem_base, tile_w = sl.tile.tile_w, tile_h = sl.tile.tile_h, per = L.per_stage;
-    const Origin g = origin(L, sl.tile);
-    const unsigned b_off = per * L.a_rows * 128u, a_step = (L.a_rows * 128u) >> 4, b_step = (L.b_rows * 128u) >> 4;
+    const unsigned stage_bytes = uniform(L.stage_bytes);
+    if (stage_bytes != r.stage_bytes) { r.s = 0; r.stage_bytes = stage_bytes; r.stages = uniform((unsigned)L.stages); }
+    const unsigned tmem = uniform(sh->tmem_base), tile_w = uniform(sl.tile.tile_w), tile_h = uniform(sl.tile.tile_h), per = uniform((unsigned)L.per_stage);
+    const Origin g = uniform(origin(L, sl.tile));
+    const unsigned a_rows = uniform((unsigned)L.a_rows), b_rows = uniform((unsigned)L.b_rows), all_chunks = uniform(L.chunks);
+    const unsigned b_off = per * a_rows * 128u, a_step = (a_rows * 128u) >> 4, b_step = (b_rows * 128u) >> 4;
     for (unsigned n0 = 0; n0 < tile_w; n0 += 128u)
         for (unsigned mp = 0; mp < tile_h; mp += BLOCK_ROWS) {
             const unsigned idesc = umma_idesc((min(BLOCK_ROWS, tile_h - mp) + 15u) & ~15u), d = tmem + half * BLOCK_ROWS;
-            if (!mbar_wait(&sh->acc_empty[half], ((acc_uses >> half) & 1u) ^ 1u, ctrl, status, 6)) return false;
+            if (!warp_wait(&sh->acc_empty[half], ((acc_uses >> half) & 1u) ^ 1u, ctrl, status, 6)) return false;
             acc_uses ^= 1u << half;
             tc_fence_after();
-            for (unsigned ch = 0, chunks = g.chunks(L, n0); ch < chunks; ch += per) {
+            for (unsigned ch = 0, chunks = g.chunks(all_chunks, n0); ch < chunks; ch += per) {
                 const unsigned n = min(per, chunks - ch), sA = ring + r.s * r.stage_bytes;
                 unsigned alow = umma_desc_low(sA), blow = umma_desc_low(sA + b_off);
-                if (!mbar_wait(&sh->full[r.s], r.parity(), ctrl, status, 3)) return false;
+                if (!warp_wait(&sh->full[r.s], r.parity(), ctrl, status, 3)) return false;
                 tc_fence_after();
-                tc_mma_stage(d, alow, blow, idesc, ch);
-                for (unsigned j = 1; j < n; j++) {
-                    alow += a_step;
-                    blow += b_step;
-                    tc_mma_stage(d, alow, blow, idesc, 1u);
+                if (elect_one()) {
+                    tc_mma_stage(d, alow, blow, idesc, ch);
+                    for (unsigned j = 1; j < n; j++) {
+                        alow += a_step;
+                        blow += b_step;
+                        tc_mma_stage(d, alow, blow, idesc, 1u);
+                    }
+                    tc_commit(&sh->empty[r.s]);
+                    if (ch + per >= chunks) tc_commit(&sh->acc_full[half]);
                 }
-                tc_commit(&sh->empty[r.s]);
                 r.step();
             }
-            tc_commit(&sh->acc_full[half]);
             half ^= 1u;
         }
     return true;
