@@ -505,7 +505,7 @@ static int build_device_nasm(Engine *e, nasm_t *host_nasm) {
         const unsigned p0 = nasm->ldata[i].parent_ldata_idx_arr[PARENT_0], p1 = nasm->ldata[i].parent_ldata_idx_arr[PARENT_1];
         const cuuint64_t W0 = p0 != (unsigned)-1 ? nasm->ldata[p0].out_mat_dims[OUT_W] : 0;
         // Operand ring: a W box holds the tile's rows; a stage holds as many chunks as keep the one-thread roles ahead of the MMAs
-        // (0.17 us for a wait and a box, 0.16 us of MMAs a chunk up to 64 rows, 0.22 with 128, 0.3 and more above: tiles_tc.cuh)
+        // (a wait and a box cost the same whatever the box holds: tiles_tc.cuh)
         // while two or more stages fit.
         const unsigned th = nasm->ldata[i].ninst_tile_dims[OUT_H];
         // the epilogue stores 16-byte pieces: a tile has to start on one (a head of ten features does not)

@@ -209,7 +209,7 @@ __global__ void __launch_bounds__(fmablk::THREADS) matmul_rows(const Args a) {
 }
 
 // What runs a layer of more than 8 columns, by the longest SM: blocks are dealt whole, so an SM runs ceil(blocks / SMs) of them.
-// Measured, us: FMA blocks 3 and their multiply-adds at 163000 a us (32 x 32: 89000; rows that admit only 8- or 4-byte copies take
+// Measured, us: FMA blocks 3 and their multiply-adds at 131000 a us (32 x 32: 105000; rows that admit only 8- or 4-byte copies take
 // 1.2 or 1.5 times as long), the tensor cores with split operands 16 and per 32 of k 0.16 and 0.69 a block of 64 rows, 0.2 and 0.93
 // of 128.  k = 3072, 4096 columns, m = 3072: 1698 us in FMA blocks, 733 and 510 split; 64 columns: 61 and 82.
 // Splitting is for k >= 256: its error against 64 bits grows with what the accumulator of a 32-deep chunk cuts off, not with k, so that of
@@ -219,8 +219,8 @@ enum Kernel { FMA_128x64, FMA_64x64, FMA_32x32, SPLIT_128, SPLIT_64 };
 Kernel pick_kernel(unsigned n_cols, unsigned k, unsigned m, unsigned sms, int vec) {
     auto rounds = [&](unsigned bm, unsigned bn) { return (double)(((unsigned long long)((m + bm - 1) / bm) * ((n_cols + bn - 1) / bn) + sms - 1) / sms); };
     const double copies = vec == 4 ? 1.0 : vec == 2 ? 1.2 : 1.5, chunks = (k + 31) / 32;
-    const double cost[] = {3 + rounds(128, 64) * 8192.0 * k / 163000 * copies, 3 + rounds(64, 64) * 4096.0 * k / 163000 * copies,
-                           3 + rounds(32, 32) * 1024.0 * k / 89000 * copies, 16 + chunks * (0.2 + 0.93 * rounds(128, 128)), 16 + chunks * (0.16 + 0.69 * rounds(64, 128))};
+    const double cost[] = {3 + rounds(128, 64) * 8192.0 * k / 131000 * copies, 3 + rounds(64, 64) * 4096.0 * k / 131000 * copies,
+                           3 + rounds(32, 32) * 1024.0 * k / 105000 * copies, 16 + chunks * (0.2 + 0.93 * rounds(128, 128)), 16 + chunks * (0.16 + 0.69 * rounds(64, 128))};
     unsigned best = 0;
     for (unsigned i = 1; i < (k < 256 ? 3u : 5u); i++) if (cost[i] < cost[best]) best = i;
     return (Kernel)best;

@@ -81,18 +81,16 @@ Grid choose(const nasm_ldata_t &ld, const nasm_t *nasm, int precision, unsigned 
         for (unsigned i = 0; i < nhs; i++)
             for (unsigned tw = quantum; tw < g.seg + quantum && tw <= 16 * quantum; tw += quantum) {
                 const unsigned tiles = ceil_div(H, hs[i]) * (W / g.seg) * ceil_div(g.seg, tw);
-                const double us = tile_us(path, l, std::min(hs[i], H), std::min(tw, g.seg), k, served ? 2.5 : getenv("GAP") ? atof(getenv("GAP")) : 4.0);
+                const double us = tile_us(path, l, std::min(hs[i], H), std::min(tw, g.seg), k, 2.5);
                 const double share = (double)tiles / sms;
-                // The layer's work, and the length of its longest tile: launched alone the last tiles of a layer run while the
-                // rest of the chip waits, served the passes of other graphs fill those SMs but the graphs in rotation are few.
-                // (Launched, whole rounds of the SMs instead: GPT-2 8 x 512 2.93 ms, ResNet-50 x 32 1.64; 0.7 / 1.0 / 1.5 tiles:
-                // 2.59 / 2.64 / 3.06 and 1.57 / 1.54 / 1.55.)  Served, the best weight falls with the work that the other graphs
+                // Launched alone a layer of fewer tiles than SMs takes as long as one tile; of a larger one the last tiles run while
+                // half of the chip waits.  (The work and 0.7 tiles whatever the number: ResNet-50 x 3 617 us a pass instead of 570,
+                // x 32 1398 and 1373, BERT 1 x 37 799 and 772.)  Served, the passes of other graphs fill those SMs but the
+                // graphs in rotation are few: the work, and a share of a tile.  There the best weight falls with the work that the other graphs
                 // offer each SM, which a plan of one graph does not know: three graphs of ResNet-50 x 32 in bursts of twelve take
                 // 1.92 / 1.61 / 1.51 ms a request with 0.2 / 0.5 / 1.0 tiles, eight of x 4 take 0.279 / 0.283 / 0.304.  0.5 lies
                 // between the two.
-                static const int form = getenv("FORM") ? atoi(getenv("FORM")) : 0;
-                static const double wt = getenv("WT") ? atof(getenv("WT")) : 0.7;
-                const double cost = us * (served ? share + 0.5 : form == 0 ? share + wt : form == 1 ? std::max(1.0, share + wt) : share <= 1 ? 1 + wt * share : share + wt);
+                const double cost = us * (served ? share + 0.5 : std::max(1.0, share + 0.5));
                 if (best == 0 || cost < best * 0.999) { best = cost; g.th = hs[i]; g.tw = tw; }
             }
     } else if (l->type == SOFTMAX_LAYER || l->type == YOLO_LAYER || l->type == APPEND_LAYER) {
