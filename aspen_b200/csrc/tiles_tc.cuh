@@ -318,7 +318,10 @@ struct Ring {
 
 // A wait of a whole warp: its lanes give up together.
 __device__ __forceinline__ bool warp_wait(unsigned long long *bar, unsigned parity, CtrlDev *ctrl, StatusHost *status, unsigned where) {
-    return __all_sync(0xffffffffu, mbar_wait(bar, parity, ctrl, status, where));
+    #pragma unroll 1
+    for (unsigned tries = 0; tries < 10000u; tries++)
+        if (__all_sync(0xffffffffu, mbar_try_wait(bar, parity))) return true;
+    return __all_sync(0xffffffffu, mbar_wait_slow(bar, parity, ctrl, status, where));
 }
 
 // Producer side of a change of the ring's cut: every stage must have been read.

@@ -247,3 +247,33 @@ def test_fp32_blocks_wait_for_the_tile_before_them(workdir):
         g.close()
         d.close()
     rpool.close()
+
+
+def test_more_graphs_than_a_warp_has_lanes(workdir):
+    """Passes asked for are looked for a lane a graph: with 35 graphs the scan takes a second round."""
+    cfg, wf = harness.prepare("tiny_cnn", workdir)
+    dnn = api.Dnn(cfg, wf)
+    graphs = [api.Nasm(dnn, 1, 0, 4) for _ in range(35)]
+    rpool, group = api.Rpool(), api.DseGroup(0, 0)
+    group.set_rpool(rpool)
+    group.set_service(True)
+    shape = (graphs[0].ldata_info(0)["W"], graphs[0].ldata_info(0)["H"])
+    xs = [np.random.default_rng(i).standard_normal(shape, dtype=np.float32) for i in range(5)]
+    last, seen = graphs[0].num_ldata - 1, {}
+    for turn in range(4):
+        if turn == 0:
+            for i, g in enumerate(graphs):
+                rpool.add(g, xs[i % 5])
+            group.run()
+        for i, g in enumerate(graphs):
+            group.wait(g)
+            got = g.ldata(last).copy()
+            np.testing.assert_array_equal(got, seen.setdefault((i + turn) % 5, got))
+            if turn < 3:
+                rpool.add(g, xs[(i + turn + 1) % 5])
+    group.stop()
+    assert group.status() == 0, api.last_error()
+    assert not any(np.array_equal(seen[0], seen[k]) for k in range(1, 5))
+    group.close()
+    for o in (*graphs, rpool, dnn):
+        o.close()
