@@ -57,7 +57,8 @@ double tile_us(Path path, const aspen_layer_t *l, unsigned th, unsigned tw, unsi
     return gap + (double)ceil_div(th, bm) * ceil_div(tw, bn) * (3.0 + ceil_div(k, kt) * (shape == 2 ? 1.3 : 2.0));
 }
 
-Grid choose(const nasm_ldata_t &ld, const nasm_t *nasm, int precision, unsigned sms, bool served) {
+// `small`: a pass of the graph is less than 100 us of work for the chip.
+Grid choose(const nasm_ldata_t &ld, const nasm_t *nasm, int precision, unsigned sms, bool served, bool small) {
     const aspen_layer_t *l = ld.layer;
     const unsigned *p = l->params;
     const unsigned H = ld.out_mat_dims[OUT_H], W = ld.out_mat_dims[OUT_W];
@@ -81,16 +82,16 @@ Grid choose(const nasm_ldata_t &ld, const nasm_t *nasm, int precision, unsigned 
         for (unsigned i = 0; i < nhs; i++)
             for (unsigned tw = quantum; tw < g.seg + quantum && tw <= 16 * quantum; tw += quantum) {
                 const unsigned tiles = ceil_div(H, hs[i]) * (W / g.seg) * ceil_div(g.seg, tw);
-                const double us = tile_us(path, l, std::min(hs[i], H), std::min(tw, g.seg), k, 2.5);
+                const double us = tile_us(path, l, std::min(hs[i], H), std::min(tw, g.seg), k, served ? 4.0 : 2.5);
                 const double share = (double)tiles / sms;
                 // Launched alone a layer of fewer tiles than SMs takes as long as one tile; of a larger one the last tiles run while
                 // half of the chip waits.  (The work and 0.7 tiles whatever the number: ResNet-50 x 3 617 us a pass instead of 570,
                 // x 32 1398 and 1373, BERT 1 x 37 799 and 772.)  Served, the passes of other graphs fill those SMs but the
-                // graphs in rotation are few: the work, and a share of a tile.  There the best weight falls with the work that the other graphs
-                // offer each SM, which a plan of one graph does not know: three graphs of ResNet-50 x 32 in bursts of twelve take
-                // 1.92 / 1.61 / 1.51 ms a request with 0.2 / 0.5 / 1.0 tiles, eight of x 4 take 0.279 / 0.283 / 0.304.  0.5 lies
-                // between the two.
-                const double cost = us * (served ? share + 0.5 : std::max(1.0, share + 0.5));
+                // graphs in rotation are few: the work, and a share of a tile.  There the best weight falls with the number of
+                // graphs in rotation, which a plan of one graph does not know, but a loop keeps more of them the smaller they are.  In
+                // bursts, 0.3 / 0.4 / 0.5 tiles: 7.11 / 7.24 / 7.59 ms for 32 requests of ResNet-50 x 4 (eight graphs, 40 us of the
+                // tensor cores' work each), 15.8 / 15.1 / 14.9 for 12 of x 32 (three, 320 us); 1.0: 0.304 ms a request of x 4 for 0.283.
+                const double cost = us * (served ? share + (small ? 0.3 : 0.5) : std::max(1.0, share + 0.5));
                 if (best == 0 || cost < best * 0.999) { best = cost; g.th = hs[i]; g.tw = tw; }
             }
     } else if (l->type == SOFTMAX_LAYER || l->type == YOLO_LAYER || l->type == APPEND_LAYER) {
@@ -231,10 +232,12 @@ nasm_t *plan_device_tiles(const nasm_t *nasm, int precision, unsigned sms, bool 
     plan->ldata = nasm->ldata;
     std::vector<Grid> grid(plan->num_ldata);
     unsigned total = 0;
+    double flop = 0;
+    for (const nasm_ldata_t &ld : nasm->ldata) flop += (double)ld.flop_per_output * ld.out_mat_dims[OUT_H] * ld.out_mat_dims[OUT_W];
     for (unsigned i = 0; i < plan->num_ldata; i++) {
         nasm_ldata_t &ld = plan->ldata[i];
         ld.nasm = plan.get();
-        Grid &g = grid[i] = choose(nasm->ldata[i], nasm, precision, sms, served);
+        Grid &g = grid[i] = choose(nasm->ldata[i], nasm, precision, sms, served, flop < 5.4e8 * sms);      // 5.4 TFLOP/s an SM: the measured TF32 peak
         const unsigned H = ld.out_mat_dims[OUT_H], W = ld.out_mat_dims[OUT_W];
         if (H == 0 || W == 0 || W % g.seg != 0) return nullptr;
         g.start = total;
