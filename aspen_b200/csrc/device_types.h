@@ -61,12 +61,19 @@ struct alignas(128) LayerDev {
 };
 static_assert(sizeof(LayerDev) == 256, "two words a lane");
 
-struct alignas(32) TileDev {        // a whole sector, one load for the scheduler
+struct alignas(64) TileDev {        // two sectors, one load for the scheduler
     unsigned layer;
     unsigned pos_h, pos_w;    // position in the layer's output matrix
     unsigned tile_h, tile_w;  // clipped extents
     unsigned child_off, child_cnt;
     unsigned need;            // completions of parents that a pass of the tile waits for
+    // Contractions in the fp32 mode: the values of k that the tile sums.  Where a layer's k is split, `slices` tiles of the same outputs
+    // leave their sums in `part`, [slice][column][rows rounded up to 4], and count at `arrived`; the one that comes last adds them
+    // in order and writes the outputs.
+    unsigned k0, k1;
+    unsigned slice, slices;
+    float *part;
+    unsigned *arrived;
 };
 
 // The layer-0 tiles run on the device and turn what the host uploaded into the layer's activation matrix, so a
@@ -97,6 +104,7 @@ struct NasmDev {
     volatile unsigned *completed;    // mapped host word: number of the last complete pass
     const void *wmaps;               // CUtensorMap[]
     unsigned n_tiles;
+    unsigned n_counters;             // words of dep: a counter per tile, and one per set of tiles with a split k
     unsigned *svc;                   // SVC_* words in device memory
     unsigned n_exec;                 // tiles that complete in one pass (every tile but the ones whose parents write their values)
     unsigned n_input;                // layer-0 tiles (local ids 0 .. n_input-1): the seeds of a pass

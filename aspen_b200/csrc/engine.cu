@@ -668,6 +668,9 @@ static int build_device_nasm(Engine *e, nasm_t *host_nasm) {
     // Tiles, children (CSR).
     const unsigned n = nasm->num_ninst, n_input = nasm->ldata[0].num_ninst;
     std::vector<TileDev> tiles(n);
+    size_t parts = 0;                   // sums of layers whose k is split: floats
+    std::vector<size_t> cells;          // where those of each set of tiles start
+    std::vector<unsigned> cell_of(n);
     std::vector<unsigned> need(n);
     std::vector<std::vector<unsigned>> kids(n);
     bool fused = false;
@@ -678,6 +681,18 @@ static int build_device_nasm(Engine *e, nasm_t *host_nasm) {
         T.layer = (unsigned)(ni.ldata - nasm->ldata.data());
         T.pos_h = ni.out_mat_pos[OUT_H]; T.pos_w = ni.out_mat_pos[OUT_W];
         T.tile_h = ni.tile_dims[OUT_H]; T.tile_w = ni.tile_dims[OUT_W];
+        const LayerDev &L = layers[T.layer];
+        T.slices = ni.ldata->slices;
+        T.slice = T.slices > 1 ? (t - ni.ldata->ninst_start) % T.slices : 0;
+        // whole steps of the fp32 blocks of the tile's shape (tile_gemm_ffma)
+        const unsigned unit = T.tile_w > 32 && T.tile_h > 64 ? 32 : T.tile_w > 32 && T.tile_h > 32 ? 64 : 128, steps = (L.K + unit - 1) / unit;
+        T.k0 = (unsigned)((unsigned long long)steps * T.slice / T.slices) * unit;
+        T.k1 = T.slice + 1 == T.slices ? 0xffffffffu : (unsigned)((unsigned long long)steps * (T.slice + 1) / T.slices) * unit;
+        T.part = nullptr; T.arrived = nullptr;
+        if (T.slices > 1) {
+            if (T.slice == 0) { cells.push_back(parts); parts += (size_t)T.slices * T.tile_w * round_up(T.tile_h, 4); }
+            cell_of[t] = (unsigned)cells.size() - 1;
+        }
         for (unsigned par : ni.parent_ninst_idx)
             if (par >= n || par >= t) { ASPEN_ERR("tile %u lists parent %u that does not precede it\n", t, par); return -1; }
         for (unsigned par : ni.extra_parent_idx)
@@ -720,9 +735,11 @@ static int build_device_nasm(Engine *e, nasm_t *host_nasm) {
                 const unsigned per_col = (Q.out_mat_dims[OUT_H] + qh - 1) / qh;
                 for (unsigned cw = T.pos_w / qw; cw <= (T.pos_w + T.tile_w - 1) / qw; cw++)
                     for (unsigned ch = T.pos_h / qh; ch <= (T.pos_h + T.tile_h - 1) / qh; ch++) {
-                        const unsigned par = Q.ninst_start + cw * per_col + ch;
-                        if (par >= Q.ninst_start + Q.num_ninst || par >= t) { ASPEN_ERR("fused residual: tile %u has no valid producer tile\n", t); return -1; }
-                        reads(par);
+                        for (unsigned s = 0; s < Q.slices; s++) {
+                            const unsigned par = Q.ninst_start + (cw * per_col + ch) * Q.slices + s;
+                            if (par >= Q.ninst_start + Q.num_ninst || par >= t) { ASPEN_ERR("fused residual: tile %u has no valid producer tile\n", t); return -1; }
+                            reads(par);
+                        }
                     }
             }
             std::sort(list.begin(), list.end());
@@ -743,7 +760,16 @@ static int build_device_nasm(Engine *e, nasm_t *host_nasm) {
             children.push_back(c); children.push_back(tiles[c].layer << 16 | need[c]);
         }
     }
-    for (unsigned t = 0; t < n; t++) tiles[t].need = need[t];
+    CUDA_TRY(cudaMalloc(&dn->dep, std::max<size_t>(n + cells.size(), 1) * sizeof(unsigned)));
+    float *part = nullptr;
+    if (parts) {
+        CUDA_TRY(cudaMalloc(&part, parts * sizeof(float)));
+        dn->scratch.push_back(part);
+    }
+    for (unsigned t = 0; t < n; t++) {
+        tiles[t].need = need[t];
+        if (tiles[t].slices > 1) { tiles[t].part = part + cells[cell_of[t]]; tiles[t].arrived = dn->dep + n + cell_of[t]; }
+    }
     if (to_device(&dn->tiles, tiles) != 0 || to_device(&dn->children, children) != 0) return -1;
     std::vector<bool> bypassed(n);
     dn->tile_layer.resize(n);
@@ -754,7 +780,6 @@ static int build_device_nasm(Engine *e, nasm_t *host_nasm) {
     if (to_device(&dn->order, order) != 0) return -1;
     static std::atomic<unsigned long long> serials{0};
     dn->serial = ++serials;
-    CUDA_TRY(cudaMalloc(&dn->dep, std::max<size_t>(n, 1) * sizeof(unsigned)));
     CUDA_TRY(cudaHostAlloc(&dn->svc_done_h, sizeof(unsigned), cudaHostAllocMapped));
     *dn->svc_done_h = 0;
     CUDA_TRY(cudaHostGetDevicePointer(&dn->svc_done_d, dn->svc_done_h, 0));
@@ -769,7 +794,7 @@ static int build_device_nasm(Engine *e, nasm_t *host_nasm) {
     memset(&H, 0, sizeof H);
     H.layers = dn->layers; H.tiles = dn->tiles; H.children = dn->children; H.dep = dn->dep; H.wmaps = dn->wmaps;
     H.completed = dn->svc_done_d; H.svc = dn->svc_d;
-    H.n_tiles = n; H.n_exec = n - n_bypassed; H.n_input = n_input;
+    H.n_tiles = n; H.n_counters = n + (unsigned)cells.size(); H.n_exec = n - n_bypassed; H.n_input = n_input;
     return 0;
 }
 

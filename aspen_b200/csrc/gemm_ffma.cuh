@@ -52,16 +52,17 @@ typedef Shape<64, 32, 4, 2, 1, 2> Tight;      // 24 KB of staging, beside the te
 
 // Loader (one per operand):  void row(int i, unsigned r): row r of the block is this thread's i-th row;
 //     void at(unsigned k): the pieces that follow start at k;  void copy(unsigned dst, int i): stage 4 values of row i.
+// The sums run over k0 (a multiple of 4) .. K - 1; the loaders give zeros from K on.
 // Bar: barrier of the 256 threads.  Out: void operator()(unsigned m, unsigned n, const float *v): outputs m .. m+3 of column n.
 template <typename S, typename LoadW, typename LoadX, typename Bar, typename Out>
-__device__ __forceinline__ void block(unsigned char *smem, unsigned tid, unsigned K, LoadW &loadw, LoadX &loadx, Bar bar, Out &out) {
+__device__ __forceinline__ void block(unsigned char *smem, unsigned tid, unsigned K, LoadW &loadw, LoadX &loadx, Bar bar, Out &out, unsigned k0 = 0) {
     const unsigned group = tid / S::GROUP, gt = tid % S::GROUP;
     // lane bits 0, 3, 4 pick one of 8 groups of 4 output rows, bits 1, 2 one of 4 groups of columns: a quarter warp reads four
     // W rows and two or four X rows at a time (2 % faster than eight and one)
     const unsigned lane = gt & 31u, quad = gt >> 5;
     const unsigned ty = ((lane & 1u) | ((lane >> 2) & 6u)) + 8u * (quad % (S::BM / S::TM / 8)), tx = ((lane >> 1) & 3u) + 4u * (quad / (S::BM / S::TM / 8));
     const unsigned base = (unsigned)__cvta_generic_to_shared(smem);
-    const unsigned srow = tid >> 3, piece = tid & 7u, steps = (K + S::KT - 1) / S::KT;
+    const unsigned srow = tid >> 3, piece = tid & 7u, steps = (K - k0 + S::KT - 1) / S::KT;
 
     #pragma unroll
     for (int i = 0; i < S::RW; i++) loadw.row(i, srow + 32u * i);
@@ -72,7 +73,7 @@ __device__ __forceinline__ void block(unsigned char *smem, unsigned tid, unsigne
             #pragma unroll
             for (int s = 0; s < S::KS; s++) {
                 const unsigned slice = base + (step % S::STAGES) * S::STAGE_BYTES + s * (S::BM + S::BN) * 128;
-                const unsigned k = step * S::KT + s * 32u + piece * 4u;
+                const unsigned k = k0 + step * S::KT + s * 32u + piece * 4u;
                 loadw.at(k);
                 #pragma unroll
                 for (int i = 0; i < S::RW; i++) {

@@ -74,6 +74,7 @@ struct nasm_ldata_t {
     unsigned int out_mat_stride = 0;
     size_t out_mat_mem_size = 0;
     unsigned int ninst_tile_dims[2] = {};
+    unsigned int slices = 1;         // device plan: tiles of the same outputs, each over a part of k; consecutive
     unsigned int ninst_start = 0;
     unsigned int num_ninst = 0;
 };

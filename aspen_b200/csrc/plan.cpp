@@ -23,6 +23,7 @@ struct Grid {
     unsigned seg = 1;              // tiles do not cross multiples of this many columns (a head's or sample's queries)
     unsigned nh = 1, per_seg = 1;  // row tiles; column tiles of a segment
     unsigned start = 0;
+    unsigned ks = 1;               // parts of k, a tile each
 };
 
 bool contraction(LAYER_TYPE t) { return t == CONV_LAYER || t == FC_LAYER || t == MATMUL_LAYER || t == K_ATTENTION_LAYER || t == V_ATTENTION_LAYER; }
@@ -39,7 +40,9 @@ Path path_of(const aspen_layer_t *l, int precision, unsigned seq) { return preci
 // block takes 0.4 us per 32 rows and runs under the next block's main loop.
 // Beside the ring (measured): 64 x 32 blocks, 0.8 us and 1.0 per 32 of k (3 x 3 layers of 48 and 24 channels), 1.6 where operands
 // come value by value (attention with heads of 10); the softmax of scores 1.4 us per 1024.
-double tile_us(Path path, const aspen_layer_t *l, unsigned th, unsigned tw, unsigned k, double gap) {
+// `ks` > 1: one of ks tiles that share k; they write and read their sums and wait for each other's counts, some 3 us.
+double tile_us(Path path, const aspen_layer_t *l, unsigned th, unsigned tw, unsigned k, double gap, unsigned ks = 1) {
+    if (ks > 1) return tile_us(path, l, th, tw, ceil_div(k, ks), gap + 3.0);
     if (path == TENSOR) {
         const unsigned chunks = ceil_div(k, 32), nb = ceil_div(tw, 128) * ceil_div(th, 256), rows = std::min(th, 256u);
         const double loop = chunks * (rows > 128 ? 0.38 : rows > 64 ? 0.28 : 0.19), epi = 0.6 + 0.4 * ceil_div(rows, 32);
@@ -92,7 +95,15 @@ Grid choose(const nasm_ldata_t &ld, const nasm_t *nasm, int precision, unsigned 
                 // bursts, 0.3 / 0.4 / 0.5 tiles: 7.11 / 7.24 / 7.59 ms for 32 requests of ResNet-50 x 4 (eight graphs, 40 us of the
                 // tensor cores' work each), 15.8 / 15.1 / 14.9 for 12 of x 32 (three, 320 us); 1.0: 0.304 ms a request of x 4 for 0.283.
                 const double cost = us * (served ? share + (small ? 0.3 : 0.5) : std::max(1.0, share + 0.5));
-                if (best == 0 || cost < best * 0.999) { best = cost; g.th = hs[i]; g.tw = tw; }
+                if (best == 0 || cost < best * 0.999) { best = cost; g.th = hs[i]; g.tw = tw; g.ks = 1; }
+                // Launched alone in the fp32 mode, a layer that leaves SMs idle shares its k among them: 512 x 49 outputs with k = 4608 are 32
+                // tiles of 48 us, or 128 of 14; ResNet-50 x 1 988 -> 916 us a pass.  (Not on the tensor cores, where a sample's bits
+                // are the same in every batch.)
+                if (!served && !ka && !va && path == FP32)
+                    for (unsigned ks = 2; ks <= 8 && ks * tiles <= sms && k / ks >= 128; ks++) {
+                        const double split = tile_us(path, l, std::min(hs[i], H), std::min(tw, g.seg), k, 2.5, ks);
+                        if (split < best * 0.95) { best = split; g.th = hs[i]; g.tw = tw; g.ks = ks; }
+                    }
             }
     } else if (l->type == SOFTMAX_LAYER || l->type == YOLO_LAYER || l->type == APPEND_LAYER) {
         g.th = ld.ninst_tile_dims[OUT_H]; g.tw = ld.ninst_tile_dims[OUT_W];
@@ -179,7 +190,7 @@ ClaimOrder claim_order(const nasm_t *plan, int precision, unsigned workers, cons
         if (!contraction(l->type)) return 1.0f + 8.0f * th * tw / BYTES_PER_US;
         const unsigned heads = std::max(1u, l->params[NUM_HEAD]);
         const unsigned k = l->type == K_ATTENTION_LAYER ? l->params[NUM_HIDDEN] / heads : l->type == V_ATTENTION_LAYER ? plan->tr_seq_len : layer_contraction_k(l);
-        return (float)tile_us(path_of(l, precision, plan->tr_seq_len), l, th, tw, k, 0);
+        return (float)tile_us(path_of(l, precision, plan->tr_seq_len), l, th, tw, k, 0, ni.ldata->slices);
     };
     float now = 0;
     unsigned idle = workers;
@@ -246,7 +257,8 @@ nasm_t *plan_device_tiles(const nasm_t *nasm, int precision, unsigned sms, bool 
         ld.out_mat_stride = (unsigned)round_up(H, 4);
         ld.out_mat_mem_size = (size_t)ld.out_mat_stride * W * sizeof(float);
         ld.ninst_start = total;
-        ld.num_ninst = g.nh * (W / g.seg) * g.per_seg;
+        ld.slices = g.ks;
+        ld.num_ninst = g.nh * (W / g.seg) * g.per_seg * g.ks;
         total += ld.num_ninst;
     }
     plan->num_ninst = total;
@@ -260,7 +272,7 @@ nasm_t *plan_device_tiles(const nasm_t *nasm, int precision, unsigned sms, bool 
         const unsigned i0 = ld.parent_ldata_idx_arr[PARENT_0], i1 = ld.parent_ldata_idx_arr[PARENT_1];
         for (unsigned t = 0; t < ld.num_ninst; t++) {
             ninst_t &ni = plan->ninst[g.start + t];
-            const unsigned ch = t % g.nh, cw = t / g.nh, seg = cw / g.per_seg, in_seg = (cw % g.per_seg) * g.tw;
+            const unsigned cell = t / g.ks, ch = cell % g.nh, cw = cell / g.nh, seg = cw / g.per_seg, in_seg = (cw % g.per_seg) * g.tw;
             const unsigned h0 = ch * g.th, h1 = std::min(H, h0 + g.th), w0 = seg * g.seg + in_seg, w1 = seg * g.seg + std::min(g.seg, in_seg + g.tw);
             ni.ldata = &ld;
             ni.ninst_idx = g.start + t;
@@ -273,7 +285,8 @@ nasm_t *plan_device_tiles(const nasm_t *nasm, int precision, unsigned sms, bool 
                 r1 = std::min(r1, pl.out_mat_dims[OUT_H]); c1 = std::min(c1, pl.out_mat_dims[OUT_W]);
                 for (unsigned c = c0; c < c1;) {
                     const unsigned s = c / q.seg, k = (c % q.seg) / q.tw, col = s * q.per_seg + k;
-                    for (unsigned r = r0 / q.th; r * q.th < r1; r++) ni.parent_ninst_idx.push_back(q.start + col * q.nh + r);
+                    for (unsigned r = r0 / q.th; r * q.th < r1; r++)
+                        for (unsigned s = 0; s < q.ks; s++) ni.parent_ninst_idx.push_back(q.start + (col * q.nh + r) * q.ks + s);
                     c = s * q.seg + std::min(q.seg, (k + 1) * q.tw);
                 }
             };

@@ -200,7 +200,7 @@ static __global__ void arm_kernel(const NasmDev *nasms, CtrlDev *ctrl, Entry *qu
     for (unsigned g = 0; g < a.n; g++) {
         const NasmDev &G = nasms[a.g0 + g];
         unsigned *dep = G.dep;
-        for (unsigned i = t0, n = G.n_tiles; i < n; i += stride) dep[i] = 0u;
+        for (unsigned i = t0, n = G.n_counters; i < n; i += stride) dep[i] = 0u;
         if (t0 == 0) {
             G.svc[SVC_STARTED] = G.svc[SVC_BASE] = a.base[g];
             G.svc[SVC_TARGET] = a.target[g];
@@ -216,11 +216,13 @@ static __global__ void arm_kernel(const NasmDev *nasms, CtrlDev *ctrl, Entry *qu
 
 // A tile that runs on the worker warps alone; `wt`: worker thread 0 .. tc::NW-1, `scratch`: the shared memory of fp32 blocks.
 template <bool TENSOR_CORES>
-static __device__ __noinline__ void worker_tile(const tc::Slot &sl, unsigned wt, unsigned char *scratch) {
+static __device__ __noinline__ void worker_tile(const tc::Slot &sl, unsigned wt, unsigned char *scratch, unsigned *last) {
     const LayerDev &L = sl.layer;
     const TileDev &T = sl.tile;
     switch (L.type) {
-        case CONV_LAYER: case FC_LAYER: case MATMUL_LAYER: case K_ATTENTION_LAYER: case V_ATTENTION_LAYER: tile_gemm_ffma<!TENSOR_CORES>(L, T, wt, tc::NW, scratch); break;
+        case CONV_LAYER: case FC_LAYER: case MATMUL_LAYER: case K_ATTENTION_LAYER: case V_ATTENTION_LAYER:
+            tile_gemm_ffma<!TENSOR_CORES>(L, T, wt, tc::NW, scratch, last);
+            break;
         case RESIDUAL_LAYER: tile_residual(L, T, wt, tc::NW); break;
         case MAXPOOL_LAYER:
             // whole 16-byte pieces, and every window holds a pixel of the image
@@ -642,7 +644,7 @@ struct WorkerWarp {
         if (prof && wt() == 0) prof[(size_t)blockIdx.x * PROF_SLOTS + PROF_SLOTS - 1] += lap();
         bool ok = true;
         if (TENSOR_CORES && slot(seq).layer.tc) ok = tc::epilogue_tile(slot(seq), half, acc_uses, smem() + tc::RING_BYTES, sh(), ctrl, status);
-        else worker_tile<TENSOR_CORES>(slot(seq), wt(), smem() + (TENSOR_CORES ? tc::RING_BYTES : 0u));
+        else worker_tile<TENSOR_CORES>(slot(seq), wt(), smem() + (TENSOR_CORES ? tc::RING_BYTES : 0u), &sh()->last);
         if (prof && wt() == 0) {
             unsigned long long *mine = prof + (size_t)blockIdx.x * PROF_SLOTS + 2 + slot(seq).tile.layer % PROF_LAYERS;
             mine[0] += lap(); mine[PROF_LAYERS] += 1ull;

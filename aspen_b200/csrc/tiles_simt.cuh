@@ -736,7 +736,13 @@ struct StoreTile {
     __device__ __forceinline__ StoreTile(const LayerDev &L, const TileDev &T, unsigned m, unsigned n)
         : bias(L.type == V_ATTENTION_LAYER || L.type == K_ATTENTION_LAYER ? nullptr : L.bias), out(L.out + (size_t)T.pos_w * L.ldc + T.pos_h), ldc(L.ldc),
           tile_h(T.tile_h), tile_w(T.tile_w), pos_h(T.pos_h), m0(m), n0(n), act(L.type == V_ATTENTION_LAYER ? (int)NO_ACTIVATION : L.act),
-          round(L.round_out != 0 && L.type != K_ATTENTION_LAYER && !late_activation(L)) {}
+          round(L.round_out != 0 && L.type != K_ATTENTION_LAYER && !late_activation(L)) {
+        if (T.slices > 1u) {      // the sums of a part of k, as they are
+            ldc = (T.tile_h + 3u) & ~3u;
+            out = T.part + (size_t)T.slice * tile_w * ldc;
+            bias = nullptr; act = NO_ACTIVATION; round = false;
+        }
+    }
     __device__ __forceinline__ void operator()(unsigned mi, unsigned ni, const float *v) const {
         const unsigned m = m0 + mi, n = n0 + ni;
         if (n >= tile_w || m >= tile_h) return;
@@ -767,10 +773,12 @@ static __device__ __noinline__ void ffma_blocks(const LayerDev &L, const TileDev
             GemmView b = g;
             b.wbase += g.w_transposed ? (size_t)m0 : (size_t)m0 * g.wld;
             if (!g.conv) b.xbase += (size_t)n0 * g.xld;
-            W<S::RW> lw(b, T.tile_h - m0, weights ? L.Kpad : g.K);
+            const unsigned k1 = min(g.K, T.k1);
+            b.K = k1;
+            W<S::RW> lw(b, T.tile_h - m0, T.k1 >= g.K && weights ? L.Kpad : k1);
             X<S::RX> lx(L, b, T.pos_w + n0, T.tile_w - n0);
             StoreTile out(L, T, m0, n0);
-            fmablk::block<S>(scratch, tid, g.K, lw, lx, WorkerBarrier(), out);
+            fmablk::block<S>(scratch, tid, k1, lw, lx, WorkerBarrier(), out, T.k0);
         }
 }
 template <typename S>
@@ -832,12 +840,56 @@ static __device__ __forceinline__ void tile_gemv(const LayerDev &L, const TileDe
     else gemv_columns<8>(L, T, tid, nthr);
 }
 
+// A tile that sums a part of k has stored its sums: whether it is the last one of its set.  All worker threads.
+__device__ __forceinline__ bool arrives_last(const TileDev &T, unsigned tid, unsigned nthr, unsigned *last) {
+    worker_barrier(nthr);
+    if (tid == 0) {
+        asm volatile("fence.acq_rel.gpu;" ::: "memory");        // release: the sums, through the barrier
+        const unsigned before = atomicAdd(T.arrived, 1u);
+        asm volatile("fence.acq_rel.gpu;" ::: "memory");        // acquire: the others'
+        *(volatile unsigned *)last = before % T.slices == T.slices - 1u ? 1u : 0u;
+    }
+    worker_barrier(nthr);
+    return *(volatile unsigned *)last != 0u;
+}
+// The parts' sums added in order (so a run's bits do not depend on which tile came last), bias, activation and store.
+static __device__ __noinline__ void finish_parts(const LayerDev &L, const TileDev &T, unsigned tid, unsigned nthr) {
+    const unsigned tile_h = T.tile_h, h4 = (tile_h + 3u) >> 2, total = T.tile_w * h4, slices = T.slices;
+    const size_t step = (size_t)T.tile_w * h4 * 4u;
+    const float *part = T.part, *bias = L.bias ? L.bias + T.pos_h : nullptr;
+    float *out = L.out + (size_t)T.pos_w * L.ldc + T.pos_h;
+    const size_t ldc = L.ldc;
+    const bool late = late_activation(L), round = L.round_out != 0 && !late, relu = !late && L.act == RELU;
+    for (unsigned i = tid; i < total; i += nthr) {
+        const unsigned n = i / h4, m = (i - n * h4) * 4u;
+        float4 a[8];
+        #pragma unroll
+        for (unsigned s = 0; s < 8; s++) a[s] = ldcg4(part + min(s, slices - 1u) * step + (size_t)i * 4u);
+        float f[4] = {a[0].x, a[0].y, a[0].z, a[0].w};
+        #pragma unroll
+        for (unsigned s = 1; s < 8; s++)
+            if (s < slices) { f[0] += a[s].x; f[1] += a[s].y; f[2] += a[s].z; f[3] += a[s].w; }
+        float *o = out + (size_t)n * ldc + m;
+        #pragma unroll
+        for (unsigned j = 0; j < 4; j++) {
+            if (bias && m + j < tile_h) f[j] += __ldg(bias + m + j);
+            if (relu) f[j] = f[j] > 0.f ? f[j] : 0.f;
+            if (round) f[j] = tf32_round(f[j]);
+        }
+        if (m + 4u <= tile_h && (reinterpret_cast<uintptr_t>(o) & 15u) == 0u) *reinterpret_cast<float4 *>(o) = make_float4(f[0], f[1], f[2], f[3]);
+        else
+            #pragma unroll
+            for (unsigned j = 0; j < 4; j++) if (m + j < tile_h) o[j] = f[j];
+    }
+    if (late) worker_barrier(nthr);
+}
+
 // Tile in fp32 (ref src/tiled_kernels.c:21-490, 784-1038).  FULL: the fp32 mode, 96 KB of staging; the shape of the blocks
 // follows the tile (a shape larger than the tile would compute padding).  Otherwise the few layers of a tensor-core graph without an
 // operand form: scores of heads that are no multiple of four features or of more than 512 keys, values of such heads, convolutions
 // past an im2col map's limits.
 template <bool FULL>
-static __device__ void tile_gemm_ffma(const LayerDev &L, const TileDev &T, unsigned tid, unsigned nthr, unsigned char *scratch) {
+static __device__ void tile_gemm_ffma(const LayerDev &L, const TileDev &T, unsigned tid, unsigned nthr, unsigned char *scratch, unsigned *last) {
     if (L.gemv) { tile_gemv(L, T, tid, nthr); return; }
     const bool pieces = L.a_vec4 != 0 && L.type != V_ATTENTION_LAYER;
     if (!FULL) {
@@ -850,6 +902,10 @@ static __device__ void tile_gemm_ffma(const LayerDev &L, const TileDev &T, unsig
     else if (T.tile_h > 32 && T.tile_w > 32) ffma_shape<fmablk::Medium>(L, T, tid, scratch);
     else ffma_shape<fmablk::Small>(L, T, tid, scratch);
     const unsigned tile_h = T.tile_h, tile_w = T.tile_w;
+    if (T.slices > 1u) {
+        if (!arrives_last(T, tid, nthr, last)) return;
+        finish_parts(L, T, tid, nthr);
+    }
     float *tile = L.out + (size_t)T.pos_w * L.ldc + T.pos_h;
     if (L.type == K_ATTENTION_LAYER) {
         // mask, / sqrt(hd), exp, every column normalised by its sum (no max subtraction, as the reference)

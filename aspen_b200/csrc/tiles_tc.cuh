@@ -79,6 +79,7 @@ struct Shared {
     unsigned long long ready[SLOTS];                           // scheduler -> roles: the tile's parents are complete
     unsigned long long prof_mark;                              // time accounting: when the workers' last step ended
     unsigned tmem_base;
+    unsigned last;                                             // the workers' tile is the last of its set (arrives_last)
     Slot slots[SLOTS];
 };
 static_assert(sizeof(Shared) <= 3072, "Shared must fit beside the ring");

@@ -269,3 +269,30 @@ def test_launches_of_changing_sets_of_graphs(precision, workdir):
     group.close()
     for o in (*graphs, rpool, *dnns):
         o.close()
+
+
+@pytest.mark.parametrize("batch,side,channels,layers", [
+    (1, 7, 64, [(50, 3, 1, 1), (30, 3, 1, 1), (514, 1, 1, 0), (33, 3, 2, 1)]),       # k 576, 450, 30, 4626: rows that are no multiple of four
+    (3, 5, 66, [(64, 5, 1, 2), (130, 3, 1, 1)]),                                     # k 1650, 576; channels that are no multiple of four
+])
+@pytest.mark.parametrize("act", ["relu", "logistic"])
+def test_fp32_layers_whose_k_is_shared_by_several_tiles(batch, side, channels, layers, act, workdir):
+    """Launched alone in the fp32 mode, layers of few tiles split their k; whichever tile comes last adds the sums in the same order, so
+    a run's bits are those of the run before."""
+    text, wl = _conv_net(side, channels, layers, 20)
+    text = text.replace("activation=relu", f"activation={act}")
+    cfg, wf = f"{workdir}/share_{channels}_{act}.cfg", f"{workdir}/share_{channels}_{act}.bin"
+    with open(cfg, "w") as f:
+        f.write(text)
+    ws = weights.make_weights(wl, 47, "he")
+    weights.write_aspen_data(wf, ws)
+    dev = harness.Device(cfg, wf, batch, 0, 20, 1, 1)
+    x = np.random.default_rng(side).standard_normal(dev.input_shape(), dtype=np.float32)
+    assert dev.run(x) == 0, api.last_error()
+    once = [dev.nasm.ldata(i).copy() for i in range(1, dev.nasm.num_ldata)]
+    for _ in range(20):
+        assert dev.run(x) == 0, api.last_error()
+    for i, o in enumerate(once):
+        np.testing.assert_array_equal(dev.nasm.ldata(i + 1), o)
+    layers_match(dev, port.run(text, ws, x, batch, 0), 1)
+    dev.close()
