@@ -1,7 +1,8 @@
 // Persistent device-side dataflow scheduler: the B200 counterpart of the reference's DSE worker
 // loop (dse_schedule, ref src/dse.c:20-108) and ready pool (ref src/rpool.c:390-685).
 //
-// One CTA per SM stays resident for a whole launch.  Its scheduler warp
+// One CTA per SM stays resident for a whole launch.  A launch per run hands its tiles out in a fixed order (`ordered_warp`: claim the
+// next one, wait for its counter); in service mode, where passes of several graphs are at different stages, the scheduler warp
 //   pops a ready tile      (rpool_fetch_ninsts)     ticket = atomicAdd(head); wait for queue[ticket]
 //   lets the CTA run it    (switch on layer type, ref src/dse.c:39-79)
 //   updates the children   (update_children_but_prioritize_dse_target, ref src/dse.c:363-401):
@@ -12,12 +13,11 @@
 // There is no kernel boundary and no barrier between layers: a tile fires as soon as its own
 // parent tiles are complete.
 //
-// Passes.  The host asks for pass number p of a graph by writing p to the graph's SVC_TARGET word.  An idle scheduler
+// Passes.  The host asks for pass number p of a graph by writing p to the graph's SVC_TARGET word.  A scheduler
 // warp that finds an idle graph with target != started claims it (CAS on SVC_IDLE) and pushes its layer-0 tiles; those
 // prepare the input, everything else follows from the dependency counters.  The warp that retires the last tile of a
 // pass writes the pass number to the graph's mapped host word and marks the graph idle.
-//   A launch per run (dse_group_run by default): the passes owed are written before the launch, and the kernel leaves when
-//   none is left.
+//   A launch per run (dse_group_run by default): one pass of each graph that owes one; the kernel leaves when they are complete.
 //   Service mode: the kernel stays resident while the host keeps asking (the counterpart of the reference's DSE threads,
 //   which run from dse_group_run to dse_group_stop and serve whatever rpool_add_nasm brings, ref src/dse.c:20-108,
 //   215-232).  It leaves -- without error -- when no pass is running or asked for and the host has asked it to
