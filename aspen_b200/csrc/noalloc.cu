@@ -12,13 +12,14 @@
 //     warp reduction -- every SM pulls weights at once, which no 32-row block shape achieves here.
 //     The line lies at 8: with 16 columns the 32 x 32 blocks below are faster (19.9 against 23.6 us at k = 768, m = 3072).
 //   * larger: the fp32 FMA blocks of gemm_ffma.cuh, or the tensor cores over operands split into bf16 parts (gemm_split.cuh), by
-//     `pick_kernel`.
+//     `pick_matmul` (matmul_pick.h).
 // B200, wall time of a call, launch and wait included (columns x k x rows):  1 x 768 x 768 17 us;  333 x 770 x 1000 44 us in FMA
 // blocks (45 split);  4096 x 768 x 3072 466 in FMA blocks, 199 split.
 #include "internal.h"
 #include "tiles_simt.cuh"
 #include "gemm_ffma.cuh"
 #include "gemm_split.cuh"
+#include "matmul_pick.h"
 
 #include <cuda_runtime.h>
 #include <algorithm>
@@ -208,24 +209,6 @@ __global__ void __launch_bounds__(fmablk::THREADS) matmul_rows(const Args a) {
     if (lane < N && lane < a.n_cols) a.out[(size_t)lane * a.m + m] = act_value(mine + (a.bias ? __ldg(a.bias + m) : 0.f), a.act);
 }
 
-// What runs a layer of more than 8 columns, by the longest SM: blocks are dealt whole, so an SM runs ceil(blocks / SMs) of them.
-// Measured, us: FMA blocks 3 and their multiply-adds at 131000 a us (32 x 32: 105000; rows that admit only 8- or 4-byte copies take
-// 1.2 or 1.5 times as long), the tensor cores with split operands 16 and per 32 of k 0.16 and 0.69 a block of 64 rows, 0.2 and 0.93
-// of 128.  k = 3072, 4096 columns, m = 3072: 1698 us in FMA blocks, 733 and 510 split; 64 columns: 61 and 82.
-// Splitting is for k >= 256: its error against 64 bits grows with what the accumulator of a 32-deep chunk cuts off, not with k, so that of
-// short sums would be larger than before.  2-norm, N(0, 1) operands, k = 258 / 512 / 770 / 3072: FMA blocks 1.5e-7 / 2.1e-7 / 1.9e-7 /
-// 5.0e-7, split 0.9e-7 / 1.0e-7 / 1.2e-7 / 1.9e-7.
-enum Kernel { FMA_128x64, FMA_64x64, FMA_32x32, SPLIT_128, SPLIT_64 };
-Kernel pick_kernel(unsigned n_cols, unsigned k, unsigned m, unsigned sms, int vec) {
-    auto rounds = [&](unsigned bm, unsigned bn) { return (double)(((unsigned long long)((m + bm - 1) / bm) * ((n_cols + bn - 1) / bn) + sms - 1) / sms); };
-    const double copies = vec == 4 ? 1.0 : vec == 2 ? 1.2 : 1.5, chunks = (k + 31) / 32;
-    const double cost[] = {3 + rounds(128, 64) * 8192.0 * k / 131000 * copies, 3 + rounds(64, 64) * 4096.0 * k / 131000 * copies,
-                           3 + rounds(32, 32) * 1024.0 * k / 105000 * copies, 16 + chunks * (0.2 + 0.93 * rounds(128, 128)), 16 + chunks * (0.16 + 0.69 * rounds(64, 128))};
-    unsigned best = 0;
-    for (unsigned i = 1; i < (k < 256 ? 3u : 5u); i++) if (cost[i] < cost[best]) best = i;
-    return (Kernel)best;
-}
-
 template <typename S, int VEC>
 void launch_blocks(const Args &a, cudaStream_t stream) {
     // the attribute is per device; asking for it on every call costs a fraction of the launch
@@ -251,7 +234,7 @@ void launch(const Args &a, unsigned sms, cudaStream_t stream) {
         else matmul_rows<8, VEC><<<grid, fmablk::THREADS, 0, stream>>>(a);
         return;
     }
-    switch (pick_kernel(a.n_cols, a.k, a.m, sms, VEC)) {
+    switch (pick_matmul(a.n_cols, a.k, a.m, sms, VEC)) {
         case FMA_128x64: launch_blocks<fmablk::Large, VEC>(a, stream); break;
         case FMA_64x64: launch_blocks<fmablk::Medium, VEC>(a, stream); break;
         case FMA_32x32: launch_blocks<fmablk::Small, VEC>(a, stream); break;

@@ -29,30 +29,32 @@ def test_noalloc_blocks_at_their_edges(n, k, m, act):
     assert bad == 0, f"{bad} mismatches, max abs {ea:.3e}, max rel {er:.3e}"
 
 
-# Blocks of 128 columns x 64 or 128 rows and chunks of 32 of k, at their edges, with every kind of load (k % 4, k % 2, odd).
-SPLIT_SHAPES = [(640, 256, 1500), (1025, 257, 1087), (641, 290, 2049), (385, 1000, 2047), (2500, 259, 1024), (4100, 319, 2050)]
+# Blocks of 128 columns x 64 or 128 rows and chunks of 32 of k, at their edges, with every kind of load (k % 4, k % 2, odd), one block an SM
+# and several, and the kernel that runs them (test_native.py).
+SPLIT_SHAPES = [(4100, 256, 2050, "split 128"), (4100, 319, 2050, "split 128"), (1283, 518, 1304, "split 128"), (1283, 516, 1301, "split 128"),
+                (385, 1000, 2047, "split 64"), (385, 1002, 2048, "split 64"), (377, 1001, 2049, "split 64")]
 
 
 def noalloc(x, w, b, act):
     import torch
-    xd, wd, bd = (torch.from_numpy(a).cuda() for a in (x, w, b))
+    xd, wd, bd = (None if a is None else torch.from_numpy(a).cuda() for a in (x, w, b))
     od = torch.full((x.shape[0], w.shape[0]), float("nan"), device="cuda")
     torch.cuda.synchronize()
-    assert api.lib().aspen_b200_matmul_noalloc(xd.data_ptr(), wd.data_ptr(), bd.data_ptr(), od.data_ptr(), x.shape[0], x.shape[1], w.shape[0], act, None) == 0, api.last_error()
+    assert api.lib().aspen_b200_matmul_noalloc(xd.data_ptr(), wd.data_ptr(), None if b is None else bd.data_ptr(), od.data_ptr(), x.shape[0], x.shape[1], w.shape[0], act, None) == 0, api.last_error()
     return od.cpu().numpy()
 
 
-@pytest.mark.parametrize("n,k,m", SPLIT_SHAPES)
-@pytest.mark.parametrize("act", [0, 3, 8])
-def test_noalloc_on_the_tensor_cores_is_as_close_to_64_bits_as_fp32_sums(n, k, m, act):
+@pytest.mark.parametrize("n,k,m,kernel", SPLIT_SHAPES)
+@pytest.mark.parametrize("act,with_bias", [(0, False), (0, True), (3, True), (8, True)])
+def test_noalloc_on_the_tensor_cores_is_as_close_to_64_bits_as_fp32_sums(n, k, m, kernel, act, with_bias):
     """A sum of k products rounded to fp32 one after the other is off by some 0.2 sqrt(k / 2) 2**-24 of its size where two sums are kept (the FMA
     blocks); 2**-23 covers the rounding of the result and of the activation on top."""
     rng = np.random.default_rng(n + k)
     x = rng.standard_normal((n, k), dtype=np.float32)
     w = (rng.standard_normal((m, k)) * np.sqrt(2 / k)).astype(np.float32)
-    b = rng.standard_normal((m,), dtype=np.float32)
+    b = rng.standard_normal((m,), dtype=np.float32) if with_bias else None
     got = noalloc(x, w, b, act)
-    want = x.astype(np.float64) @ w.T.astype(np.float64) + b
+    want = x.astype(np.float64) @ w.T.astype(np.float64) + (b if with_bias else 0)
     if act == 3:
         want = np.tanh(want)
     elif act == 8:
