@@ -4,7 +4,8 @@
 // of which the six up to 2^-16 are kept -- the others are below half a unit of the fp32 product.  The tensor cores multiply bf16 exactly
 // but truncate when they add to an accumulator: a chunk of k = 32 is summed there, smallest products first, and added to the
 // total in registers with rounding to nearest.  Relative error (2-norm, against 64 bits, N(0, 1) operands), FMA blocks and this:
-// see pick_matmul.  Infinities and NaN have no such sum: a tile that meets one is computed again by plain FMAs.
+// see pick_matmul.  Infinities and NaN have no such sum: a block that meets one is
+// computed again by fp32 FMA blocks when the CTA is through with all of its blocks, so that nothing waits for that.
 //
 // What bounds it: shared memory.  A chunk of a 128 x 128 block is 12 MMAs that read 8 KB each, and 49 KB of parts written for them:
 // 1150 cycles at 128 bytes a cycle, against 770 of the tensor pipe.  Hence
@@ -22,7 +23,7 @@
 
 namespace split {
 
-constexpr unsigned THREADS = 640, SPLITTERS = 128, CHUNK = 32, ACCUMULATORS = 4;
+constexpr unsigned THREADS = 640, SPLITTERS = 128, CHUNK = 32, ACCUMULATORS = 4, MAX_BLOCKS = 8192;
 constexpr unsigned long long LIMIT_NS = 2000000000ull;
 
 template <int N>
@@ -37,8 +38,7 @@ struct Shape {
 struct Shared {
     unsigned long long full[4], empty[4];          // stage split / read by the MMAs
     unsigned long long acc_full[ACCUMULATORS], acc_empty[ACCUMULATORS];    // accumulator complete / added to the totals
-    unsigned long long checked[2];                 // all values of the block have been looked at (two blocks in turn)
-    unsigned odd[2];                               // the block has met an infinity or a NaN
+    unsigned odd[MAX_BLOCKS / 32];                 // a bit for each of the CTA's blocks that has met an infinity or a NaN
     unsigned tmem;
 };
 
@@ -101,28 +101,11 @@ __device__ __forceinline__ void tmem_ld16(unsigned taddr, float *v) {
     asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 }
 
-// Rows m0 .. of the columns n0 .. + 31 of a block value by value, by one warp.
-template <typename Load, typename Out>
-static __device__ __noinline__ void again(const Load &load, const Out &out, unsigned n0, unsigned m0, unsigned rows, unsigned K) {
-    const unsigned lane = threadIdx.x & 31u;
-    for (unsigned n = n0 + (lane >> 3); n < n0 + 32u; n += 4u)
-        for (unsigned m = m0 + (lane & 7u) * 4u; m < m0 + rows; m += 32u) {
-            float f[4] = {0.f, 0.f, 0.f, 0.f};
-            #pragma unroll 1
-            for (unsigned k = 0; k < K; k += 4u) {
-                const float4 b = load(false, n, k);
-                #pragma unroll
-                for (unsigned i = 0; i < 4; i++) {
-                    const float4 a = load(true, m + i, k);
-                    f[i] = fmaf(a.x, b.x, f[i]);
-                    if (k + 1u < K) f[i] = fmaf(a.y, b.y, f[i]);
-                    if (k + 2u < K) f[i] = fmaf(a.z, b.z, f[i]);
-                    if (k + 3u < K) f[i] = fmaf(a.w, b.w, f[i]);
-                }
-            }
-            out(n, m, make_float4(f[0], f[1], f[2], f[3]));
-        }
-    out.late(n0 + (lane >> 3), 4u, 8u, m0 + (lane & 7u) * 4u, rows / 32u);
+// Every role is through: the operand stages are free, and what it has stored is seen by the others.
+__device__ __forceinline__ void all_roles_done() {
+    __syncwarp();
+    tc::tc_fence_before();
+    asm volatile("bar.sync 0;" ::: "memory");
 }
 
 // Load: float4 operator()(bool weight, unsigned row, unsigned k): four values of a row of W or X from k on, zeros outside;
@@ -130,9 +113,10 @@ static __device__ __noinline__ void again(const Load &load, const Out &out, unsi
 //       float4 piece(const float *): the four values there.
 // Out:  void operator()(unsigned n, unsigned m, const float4 &v): outputs m .. m + 3 of column n, both possibly outside;
 //       void late(n, dn, cn, m, cm): the same thread's outputs of columns n, n + dn, ... (cn of them), rows m, m + 32, ... (cm) are stored.
-// K > 256: the parts of at most STAGES chunks are ahead of the totals, so that no flag or phase of a block is two blocks ahead.
-template <int N, typename Load, typename Out>
-__device__ __forceinline__ void blocks(unsigned char *smem, Shared *sh, unsigned *gave_up, unsigned cols, unsigned rows, unsigned K, const Load &load, const Out &out) {
+// Again: void operator()(unsigned tid, unsigned n0, unsigned m0): the outputs of a block once more by 256 threads, with infinities and NaN as fp32
+//       sums give them; the operand stages are its shared memory.  At most MAX_BLOCKS blocks in all.
+template <int N, typename Load, typename Out, typename Again>
+__device__ __forceinline__ void blocks(unsigned char *smem, Shared *sh, unsigned *gave_up, unsigned cols, unsigned rows, unsigned K, const Load &load, const Out &out, const Again &again) {
     typedef Shape<N> S;
     const unsigned warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31u;
     const unsigned row_blocks = (rows + N - 1) / N, total = row_blocks * ((cols + 127u) / 128u), chunks = (K + CHUNK - 1) / CHUNK;
@@ -140,10 +124,10 @@ __device__ __forceinline__ void blocks(unsigned char *smem, Shared *sh, unsigned
     if (threadIdx.x == 0) {
         for (int s = 0; s < S::STAGES; s++) { tc::mbar_init(&sh->full[s], SPLITTERS); tc::mbar_init(&sh->empty[s], 1u); }
         for (unsigned h = 0; h < ACCUMULATORS; h++) { tc::mbar_init(&sh->acc_full[h], 1u); tc::mbar_init(&sh->acc_empty[h], 8u); }
-        for (int h = 0; h < 2; h++) { tc::mbar_init(&sh->checked[h], 2u * SPLITTERS); sh->odd[h] = 0u; }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         tc::fence_proxy_async_smem();
     }
+    for (unsigned i = threadIdx.x; i < MAX_BLOCKS / 32; i += THREADS) sh->odd[i] = 0u;
     if (warp == 0) tc::tmem_alloc(&sh->tmem, 512u);
     tc::tc_fence_before();
     __syncthreads();
@@ -188,7 +172,8 @@ __device__ __forceinline__ void blocks(unsigned char *smem, Shared *sh, unsigned
                 do { __nanosleep(1000); asm volatile("mov.u64 %0, %globaltimer;" : "=l"(now)); } while (now - t0 < 2000000ull);
             }
         }
-        __syncwarp();
+        all_roles_done();
+        if (warp == 0) { tc::tc_fence_after(); tc::tmem_dealloc(sh->tmem, 512u); }
     } else if (warp < 12) {
         asm volatile("setmaxnreg.inc.sync.aligned.u32 112;");
         // Two groups of four warps take the chunks in turn: while one splits, the other's loads are on their way.  (One group that asks for
@@ -253,21 +238,24 @@ __device__ __forceinline__ void blocks(unsigned char *smem, Shared *sh, unsigned
             if ((c += 2u) >= chunks) {
                 unsigned c0, c1;
                 unpack(check, c0, c1);
-                if ((c0 | c1) & 0x7fffffffu) *(volatile unsigned *)&sh->odd[block & 1u] = block + 1u;
+                if ((c0 | c1) & 0x7fffffffu) atomicOr(&sh->odd[block / 32u], 1u << (block % 32u));
                 check = 0ull;
-                tc::mbar_arrive(&sh->checked[block & 1u]);
                 block++;
                 c -= chunks;
                 t += gridDim.x;
             }
         }
+        all_roles_done();
+        block = 0;
+        for (unsigned t = blockIdx.x; t < total; t += gridDim.x, block++)
+            if (sh->odd[block / 32u] >> (block % 32u) & 1u) again(threadIdx.x - 128u, t / row_blocks * 128u, t % row_blocks * N);
     } else {
         asm volatile("setmaxnreg.inc.sync.aligned.u32 104;");
         const unsigned q = warp & 3u, first = (warp - 12u) / 4u * (N / 2);        // TMEM lanes 32 q .. + 31: columns; rows first .. + N / 2 - 1
         float *stage = reinterpret_cast<float *>(smem + S::STAGES * S::STAGE_BYTES + (warp - 12u) * 4096u);
-        unsigned it = 0, block = 0;
+        unsigned it = 0;
         bool ok = true;
-        for (unsigned t = blockIdx.x; t < total && ok; t += gridDim.x, block++) {
+        for (unsigned t = blockIdx.x; t < total && ok; t += gridDim.x) {
             const unsigned n0 = t / row_blocks * 128u + q * 32u, m0 = t % row_blocks * N + first;
             float sum[N / 2];
             #pragma unroll
@@ -290,12 +278,7 @@ __device__ __forceinline__ void blocks(unsigned char *smem, Shared *sh, unsigned
                     for (int i = 0; i < 16; i += 2) add2(sum[j + i], sum[j + i + 1], v[i], v[i + 1]);
                 }
             }
-            ok = ok && __all_sync(0xffffffffu, wait(&sh->checked[block & 1u], (block >> 1) & 1u, gave_up));
             if (!ok) break;
-            if (*(volatile unsigned *)&sh->odd[block & 1u] == block + 1u) {
-                again(load, out, n0, m0, N / 2, K);
-                continue;
-            }
             #pragma unroll
             for (int j = 0; j < N / 2; j += 32) {
                 // 32 x 32 outputs through the warp's buffer: then consecutive lanes have consecutive rows
@@ -311,11 +294,8 @@ __device__ __forceinline__ void blocks(unsigned char *smem, Shared *sh, unsigned
             }
             out.late(n0 + (lane >> 3), 4u, 8u, m0 + (lane & 7u) * 4u, N / 64);
         }
+        all_roles_done();
     }
-    __syncwarp();
-    tc::tc_fence_before();
-    __syncthreads();
-    if (warp == 0) { tc::tc_fence_after(); tc::tmem_dealloc(sh->tmem, 512u); }
 }
 
 }  // namespace split

@@ -166,13 +166,34 @@ struct FinishPiece {
         }
     }
 };
+// Outputs of a block of N rows x 128 columns by FMA blocks, 256 threads of the CTA.  64 x 64 with 4 x 4 a thread: the 8 x 4 ones do it in 0.97 of
+// the time, but their registers cost the splitting loop of the same warps spills (4096 x 3072 x 3072: 542 us a call, so 526).
+template <int N, int VEC>
+struct Again {
+    typedef fmablk::Shape<64, 64, 4, 4, 1> S;
+    static_assert(S::SMEM_BYTES <= split::Shape<N>::SMEM_BYTES && 2 * NOALLOC_MAX_TILES <= split::MAX_BLOCKS, "room");
+    struct Barrier { __device__ __forceinline__ void operator()() const { asm volatile("bar.sync 1, 256;" ::: "memory"); } };
+    const Args &a;
+    unsigned char *smem;
+    __device__ __forceinline__ void operator()(unsigned tid, unsigned n0, unsigned m0) const {
+        #pragma unroll 1
+        for (unsigned i = 0; i < N / 32; i++) {
+            const unsigned n = n0 + i % 2u * 64u, m = m0 + i / 2u * 64u;
+            if (n >= a.n_cols || m >= a.m) continue;
+            Stage<VEC, S::RW> lw(a.w + (size_t)m * a.k, a.m - m, a.k);
+            Stage<VEC, S::RX> lx(a.x + (size_t)n * a.k, a.n_cols - n, a.k);
+            Finish fin{a, m, n};
+            fmablk::block<S>(smem, tid, a.k, lw, lx, Barrier(), fin);
+        }
+    }
+};
 template <int N, int VEC>
 __global__ void __launch_bounds__(split::THREADS, 1) matmul_split(const Args a) {
-    extern __shared__ __align__(1024) unsigned char smem[];
+    extern __shared__ __align__(1024) unsigned char split_smem[];
     __shared__ split::Shared sh;
     const Operands<VEC> in{{a.w, a.m, a.k}, {a.x, a.n_cols, a.k}};
     const FinishPiece out{a};
-    split::blocks<N>(smem, &sh, &split_gave_up, a.n_cols, a.m, a.k, in, out);
+    split::blocks<N>(split_smem, &sh, &split_gave_up, a.n_cols, a.m, a.k, in, out, Again<N, VEC>{a, split_smem});
 }
 
 // One weight row per warp, N columns (the last ones may be missing).

@@ -64,6 +64,46 @@ def test_noalloc_on_the_tensor_cores_is_as_close_to_64_bits_as_fp32_sums(n, k, m
     assert np.linalg.norm(got - want) <= (0.2 * np.sqrt(k / 2) * 2.0**-24 + 2.0**-23) * np.linalg.norm(want)
 
 
+@pytest.mark.parametrize("n,k,m,kernel", [(1283, 3072, 1301, "split 128"), (385, 3070, 2047, "split 64")])
+def test_noalloc_blocks_with_infinities_cost_what_fp32_blocks_do(n, k, m, kernel):
+    """One value of each block is an infinity: the SM that had it computes it again in 64 x 64 fp32 blocks, four or two after another, which takes
+    three or four times as long as the tensor cores (value by value 43 and 100 times).  Rounding to nearest is off by 0.42 2**-24 of
+    a value in the root mean square (0.58 2**-24 over the mantissa); two sums of k / 2 products, whose partial sums grow with the square root, end up
+    off by 0.42 sqrt(k) / 2 = 0.3 sqrt(k / 2) units."""
+    import time
+    rng = np.random.default_rng(k)
+    x = rng.standard_normal((n, k), dtype=np.float32)
+    w = (rng.standard_normal((m, k)) * np.sqrt(2 / k)).astype(np.float32)
+
+    def best():
+        t = []
+        for _ in range(5):
+            t0 = time.perf_counter()
+            rc = api.lib().aspen_b200_matmul_noalloc(xd.data_ptr(), wd.data_ptr(), None, od.data_ptr(), n, k, m, 0, None)
+            t.append(time.perf_counter() - t0)
+            assert rc == 0, api.last_error()
+        return min(t)
+
+    import torch
+    xd, wd, od = torch.from_numpy(x).cuda(), torch.from_numpy(w).cuda(), torch.full((n, m), float("nan"), device="cuda")
+    torch.cuda.synchronize()
+    finite = best()
+    rows, cols = np.arange(7, m, 64), np.arange(5, n, 128)
+    w[rows, 3] = np.inf
+    x[cols, 2] = -np.inf
+    xd, wd = torch.from_numpy(x).cuda(), torch.from_numpy(w).cuda()
+    torch.cuda.synchronize()
+    assert best() < 10 * finite
+    got = od.cpu().numpy()
+    with np.errstate(all="ignore"):
+        want = x.astype(np.float64) @ w.T.astype(np.float64)
+    plain = np.ix_(~np.isin(np.arange(n), cols), ~np.isin(np.arange(m), rows))
+    assert np.isfinite(got[plain]).all() and np.linalg.norm(got[plain] - want[plain]) <= (0.3 * np.sqrt(k / 2) * 2.0**-24 + 2.0**-23) * np.linalg.norm(want[plain])
+    other = np.ones((n, m), bool)
+    other[plain] = False
+    np.testing.assert_array_equal(got[other], want[other].astype(np.float32))
+
+
 def test_noalloc_on_the_tensor_cores_over_the_range_of_fp32():
     """Infinities and NaN spread as in a sum of fp32 products, and only into their own rows and columns; large, small and denormal values keep
     the precision of fp32 products."""
