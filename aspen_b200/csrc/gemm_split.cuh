@@ -1,11 +1,14 @@
 // fp32 contraction on the tensor cores: out[n][m] = act(bias[m] + sum_k W[m][k] X[n][k]) with every operand as a sum of three bf16 values.
 //
-// An fp32 value is x = b1 + b2 + b3 exactly (8 bits each, every part the rest rounded to nearest), so W X is nine products of bf16 parts
+// An fp32 value is x = b1 + b2 + b3 (8 bits each), exactly unless |x| < 2^-110, where b3 may need bits below the last of bf16, 2^-133.  W X is
+// nine products of bf16 parts
 // of which the six up to 2^-16 are kept -- the others are below half a unit of the fp32 product.  The tensor cores multiply bf16 exactly
 // but truncate when they add to an accumulator: a chunk of k = 32 is summed there, smallest products first, and added to the
 // total in registers with rounding to nearest.  Relative error (2-norm, against 64 bits, N(0, 1) operands), FMA blocks and this:
-// see pick_matmul.  Infinities and NaN have no such sum: a block that meets one is
-// computed again by fp32 FMA blocks when the CTA is through with all of its blocks, so that nothing waits for that.
+// see pick_matmul.  A block is computed again by fp32 FMA blocks if one of its values has no such sum -- infinities,
+// NaN and values with bits below 2^-133 -- or one of its totals is so small that what the accumulators truncate at the lower end of fp32, up to four
+// units of 2^-149 a chunk, is more than 2^-24 of it (768 products around 2^-130: 2-norm error 1.3e-6, of fp32 sums 5.5e-7).  That is done when the
+// CTA is through with all of its blocks, so that nothing waits for it.  4096 x 768 x 3072: 176 us a call, 900 if every block is marked.
 //
 // What bounds it: shared memory.  A chunk of a 128 x 128 block is 12 MMAs that read 8 KB each, and 49 KB of parts written for them:
 // 1150 cycles at 128 bytes a cycle, against 770 of the tensor pipe.  Hence
@@ -38,7 +41,7 @@ struct Shape {
 struct Shared {
     unsigned long long full[4], empty[4];          // stage split / read by the MMAs
     unsigned long long acc_full[ACCUMULATORS], acc_empty[ACCUMULATORS];    // accumulator complete / added to the totals
-    unsigned odd[MAX_BLOCKS / 32];                 // a bit for each of the CTA's blocks that has met an infinity or a NaN
+    unsigned odd[MAX_BLOCKS / 32];                 // a bit for each of the CTA's blocks that is to be computed again
     unsigned tmem;
 };
 
@@ -74,7 +77,8 @@ __device__ __forceinline__ Pair pack(unsigned x, unsigned y) { Pair p; asm("mov.
 __device__ __forceinline__ void unpack(Pair p, unsigned &x, unsigned &y) { asm("mov.b64 {%0, %1}, %2;" : "=r"(x), "=r"(y) : "l"(p)); }
 __device__ __forceinline__ Pair fma2(Pair a, Pair b, Pair c) { Pair d; asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c)); return d; }
 // The next bf16 part of two values, x's in the low half; what is left of them stays.  The first part is rounded to nearest, so that the
-// rest has either sign; the second is cut off; the third is what is left, eight bits.
+// rest has either sign; the second is cut off; the third is what is left, eight bits: the lower half of its word is zero unless it would need bits
+// below 2^-133, or the value is not finite (or rounds past the range of bf16), which leaves the NaN 0x7fffffff.
 template <int PART>
 __device__ __forceinline__ unsigned take_part(Pair &v) {
     unsigned x, y;
@@ -83,6 +87,8 @@ __device__ __forceinline__ unsigned take_part(Pair &v) {
     if (PART < 2) v = fma2(pack(x & 0xffff0000u, y & 0xffff0000u), pack(-1.f, -1.f), v);
     return __byte_perm(x, y, 0x7632);
 }
+
+__device__ __forceinline__ unsigned either(Pair v) { unsigned x, y; unpack(v, x, y); return x | y; }       // bits of one or the other
 
 __device__ __forceinline__ void add2(float &x, float &y, float a, float b) {
     unsigned long long s, t;
@@ -113,8 +119,8 @@ __device__ __forceinline__ void all_roles_done() {
 //       float4 piece(const float *): the four values there.
 // Out:  void operator()(unsigned n, unsigned m, const float4 &v): outputs m .. m + 3 of column n, both possibly outside;
 //       void late(n, dn, cn, m, cm): the same thread's outputs of columns n, n + dn, ... (cn of them), rows m, m + 32, ... (cm) are stored.
-// Again: void operator()(unsigned tid, unsigned n0, unsigned m0): the outputs of a block once more by 256 threads, with infinities and NaN as fp32
-//       sums give them; the operand stages are its shared memory.  At most MAX_BLOCKS blocks in all.
+// Again: void operator()(unsigned tid, unsigned n0, unsigned m0): the outputs of a block once more by 256 threads, as fp32 sums give them;
+//       the operand stages are its shared memory.  At most MAX_BLOCKS blocks in all.
 template <int N, typename Load, typename Out, typename Again>
 __device__ __forceinline__ void blocks(unsigned char *smem, Shared *sh, unsigned *gave_up, unsigned cols, unsigned rows, unsigned K, const Load &load, const Out &out, const Again &again) {
     typedef Shape<N> S;
@@ -182,7 +188,7 @@ __device__ __forceinline__ void blocks(unsigned char *smem, Shared *sh, unsigned
         const unsigned r0 = (warp & 3u) * 4u + (lane >> 3), k0 = (lane & 7u) * 4u, group = (warp >> 2) - 1u;
         constexpr int G = 4;
         float4 v[S::PIECES];
-        Pair check = 0ull;                            // a NaN once a value was not finite
+        unsigned left = 0;                            // what the third parts could not take, in the lower halves of the words
         unsigned t = blockIdx.x, c = group, s = group, lap = 0, block = 0;
         const size_t step = 16 * (size_t)load.ld();
         auto fetch = [&]() {
@@ -219,11 +225,12 @@ __device__ __forceinline__ void blocks(unsigned char *smem, Shared *sh, unsigned
                 #pragma unroll
                 for (int i = 0; i < G; i++) part[0][i] = make_uint2(take_part<0>(lo[i]), take_part<0>(hi[i]));
                 #pragma unroll
-                for (int i = 0; i < G; i++) { check = fma2(lo[i], 0ull, check); check = fma2(hi[i], 0ull, check); }
-                #pragma unroll
                 for (int i = 0; i < G; i++) part[1][i] = make_uint2(take_part<1>(lo[i]), take_part<1>(hi[i]));
                 #pragma unroll
-                for (int i = 0; i < G; i++) part[2][i] = make_uint2(take_part<2>(lo[i]), take_part<2>(hi[i]));
+                for (int i = 0; i < G; i++) {
+                    part[2][i] = make_uint2(take_part<2>(lo[i]), take_part<2>(hi[i]));
+                    left |= either(lo[i]) | either(hi[i]);
+                }
                 #pragma unroll
                 for (int i = 0; i < G; i++) {
                     const int r = (i0 + i) * 16;
@@ -236,10 +243,8 @@ __device__ __forceinline__ void blocks(unsigned char *smem, Shared *sh, unsigned
             tc::mbar_arrive(&sh->full[s]);
             if ((s += 2u) >= (unsigned)S::STAGES) { s -= S::STAGES; lap++; }
             if ((c += 2u) >= chunks) {
-                unsigned c0, c1;
-                unpack(check, c0, c1);
-                if ((c0 | c1) & 0x7fffffffu) atomicOr(&sh->odd[block / 32u], 1u << (block % 32u));
-                check = 0ull;
+                if (left & 0xffffu) atomicOr(&sh->odd[block / 32u], 1u << (block % 32u));
+                left = 0;
                 block++;
                 c -= chunks;
                 t += gridDim.x;
@@ -253,9 +258,10 @@ __device__ __forceinline__ void blocks(unsigned char *smem, Shared *sh, unsigned
         asm volatile("setmaxnreg.inc.sync.aligned.u32 104;");
         const unsigned q = warp & 3u, first = (warp - 12u) / 4u * (N / 2);        // TMEM lanes 32 q .. + 31: columns; rows first .. + N / 2 - 1
         float *stage = reinterpret_cast<float *>(smem + S::STAGES * S::STAGE_BYTES + (warp - 12u) * 4096u);
-        unsigned it = 0;
+        const float least = (float)chunks * 0x1p-123f;
+        unsigned it = 0, block = 0;
         bool ok = true;
-        for (unsigned t = blockIdx.x; t < total && ok; t += gridDim.x) {
+        for (unsigned t = blockIdx.x; t < total && ok; t += gridDim.x, block++) {
             const unsigned n0 = t / row_blocks * 128u + q * 32u, m0 = t % row_blocks * N + first;
             float sum[N / 2];
             #pragma unroll
@@ -279,6 +285,10 @@ __device__ __forceinline__ void blocks(unsigned char *smem, Shared *sh, unsigned
                 }
             }
             if (!ok) break;
+            bool tiny = false;
+            #pragma unroll
+            for (int i = 0; i < N / 2; i++) tiny = tiny || (fabsf(sum[i]) < least && sum[i] != 0.f);
+            if (tiny) atomicOr(&sh->odd[block / 32u], 1u << (block % 32u));
             #pragma unroll
             for (int j = 0; j < N / 2; j += 32) {
                 // 32 x 32 outputs through the warp's buffer: then consecutive lanes have consecutive rows

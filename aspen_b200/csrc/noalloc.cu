@@ -166,19 +166,21 @@ struct FinishPiece {
         }
     }
 };
-// Outputs of a block of N rows x 128 columns by FMA blocks, 256 threads of the CTA.  64 x 64 with 4 x 4 a thread: the 8 x 4 ones do it in 0.97 of
-// the time, but their registers cost the splitting loop of the same warps spills (4096 x 3072 x 3072: 542 us a call, so 526).
+// Outputs of a block of N rows x 128 columns by FMA blocks, 256 threads of the CTA.  32 x 32 ones, because they have the smallest error (eight
+// partial sums; k = 768, operands around 2^-100: 1.8e-7, as where the layer itself takes them; 64 x 64 with one slice 3.5e-7) and few
+// registers: those of the 8 x 4 shapes cost the splitting loop of the same warps spills (4096 x 3072 x 3072: 542 us a call instead of
+// 523).  4096 x 768 x 3072 with every block marked: 900 us, in 64 x 64 blocks 826.
 template <int N, int VEC>
 struct Again {
-    typedef fmablk::Shape<64, 64, 4, 4, 1> S;
+    typedef fmablk::Small S;
     static_assert(S::SMEM_BYTES <= split::Shape<N>::SMEM_BYTES && 2 * NOALLOC_MAX_TILES <= split::MAX_BLOCKS, "room");
     struct Barrier { __device__ __forceinline__ void operator()() const { asm volatile("bar.sync 1, 256;" ::: "memory"); } };
     const Args &a;
     unsigned char *smem;
     __device__ __forceinline__ void operator()(unsigned tid, unsigned n0, unsigned m0) const {
         #pragma unroll 1
-        for (unsigned i = 0; i < N / 32; i++) {
-            const unsigned n = n0 + i % 2u * 64u, m = m0 + i / 2u * 64u;
+        for (unsigned i = 0; i < N / 8; i++) {
+            const unsigned n = n0 + i % 4u * 32u, m = m0 + i / 4u * 32u;
             if (n >= a.n_cols || m >= a.m) continue;
             Stage<VEC, S::RW> lw(a.w + (size_t)m * a.k, a.m - m, a.k);
             Stage<VEC, S::RX> lx(a.x + (size_t)n * a.k, a.n_cols - n, a.k);

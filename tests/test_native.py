@@ -8,7 +8,7 @@ import pytest
 import harness
 from aspen_b200 import api, cfgs
 
-from test_gpu_shapes import SPLIT_SHAPES
+from test_gpu_shapes import RANGE_SHAPES, SPLIT_SHAPES
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 LIBDIR = os.path.join(os.path.dirname(HERE), "aspen_b200")
@@ -111,7 +111,7 @@ def test_shapes_that_test_the_split_kernels_run_them(workdir):
     """Of the allocation-free matmul, on the 148 SMs of a B200: every instance (block of 128 or 64 rows, 4, 2 or 1 values a load)."""
     exe = build("matmul_pick", workdir)
     seen = set()
-    for n, k, m, kernel in SPLIT_SHAPES:
+    for n, k, m, kernel in SPLIT_SHAPES + RANGE_SHAPES:
         values = next(v for v in (4, 2, 1) if k % v == 0)
         picked = subprocess.run([exe, *(str(v) for v in (n, k, m, 148, values))], capture_output=True, text=True, check=True).stdout
         assert picked == kernel, (n, k, m)
