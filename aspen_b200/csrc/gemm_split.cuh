@@ -20,7 +20,8 @@
 // chunk against 2 x 0.93).  Persistent: a CTA takes every gridDim-th block, and the splitting of the next one goes on under the stores.
 // 4096 x 3072 outputs, k = 3072: 146 TFLOP/s of fp32 products (FMA blocks: 46).
 //
-// Every wait is bounded (LIMIT_NS); a thread that gives up sets `gave_up`, all roles leave and TMEM is freed.
+// Every wait is bounded (LIMIT_NS) and is for another role of the CTA; a thread that gives up sets the CTA's `gave_up`, all roles leave, TMEM is
+// freed, and the call's word `failed` is set.
 #pragma once
 #include "tiles_tc.cuh"
 
@@ -42,6 +43,7 @@ struct Shared {
     unsigned long long full[4], empty[4];          // stage split / read by the MMAs
     unsigned long long acc_full[ACCUMULATORS], acc_empty[ACCUMULATORS];    // accumulator complete / added to the totals
     unsigned odd[MAX_BLOCKS / 32];                 // a bit for each of the CTA's blocks that is to be computed again
+    unsigned gave_up;                              // a wait ran out
     unsigned tmem;
 };
 
@@ -122,12 +124,14 @@ __device__ __forceinline__ void all_roles_done() {
 // Again: void operator()(unsigned tid, unsigned n0, unsigned m0): the outputs of a block once more by 256 threads, as fp32 sums give them;
 //       the operand stages are its shared memory.  At most MAX_BLOCKS blocks in all.
 template <int N, typename Load, typename Out, typename Again>
-__device__ __forceinline__ void blocks(unsigned char *smem, Shared *sh, unsigned *gave_up, unsigned cols, unsigned rows, unsigned K, const Load &load, const Out &out, const Again &again) {
+__device__ __forceinline__ void blocks(unsigned char *smem, Shared *sh, unsigned *failed, unsigned cols, unsigned rows, unsigned K, const Load &load, const Out &out, const Again &again) {
     typedef Shape<N> S;
     const unsigned warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31u;
     const unsigned row_blocks = (rows + N - 1) / N, total = row_blocks * ((cols + 127u) / 128u), chunks = (K + CHUNK - 1) / CHUNK;
     const unsigned base = tc::smem_u32(smem);
+    unsigned *const gave_up = &sh->gave_up;
     if (threadIdx.x == 0) {
+        sh->gave_up = 0u;
         for (int s = 0; s < S::STAGES; s++) { tc::mbar_init(&sh->full[s], SPLITTERS); tc::mbar_init(&sh->empty[s], 1u); }
         for (unsigned h = 0; h < ACCUMULATORS; h++) { tc::mbar_init(&sh->acc_full[h], 1u); tc::mbar_init(&sh->acc_empty[h], 8u); }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -171,15 +175,19 @@ __device__ __forceinline__ void blocks(unsigned char *smem, Shared *sh, unsigned
                     __syncwarp();
                     if (++s == S::STAGES) { s = 0; lap++; }
                 }
-            if (!ok) {
+        }
+        all_roles_done();
+        if (warp == 0) {
+            if (sh->gave_up) {
                 // MMAs may still be in flight; they take microseconds
                 unsigned long long t0, now;
                 asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t0));
                 do { __nanosleep(1000); asm volatile("mov.u64 %0, %globaltimer;" : "=l"(now)); } while (now - t0 < 2000000ull);
+                if (lane == 0) *failed = 1u;
             }
+            tc::tc_fence_after();
+            tc::tmem_dealloc(sh->tmem, 512u);
         }
-        all_roles_done();
-        if (warp == 0) { tc::tc_fence_after(); tc::tmem_dealloc(sh->tmem, 512u); }
     } else if (warp < 12) {
         asm volatile("setmaxnreg.inc.sync.aligned.u32 112;");
         // Two groups of four warps take the chunks in turn: while one splits, the other's loads are on their way.  (One group that asks for
@@ -252,7 +260,7 @@ __device__ __forceinline__ void blocks(unsigned char *smem, Shared *sh, unsigned
         }
         all_roles_done();
         block = 0;
-        for (unsigned t = blockIdx.x; t < total; t += gridDim.x, block++)
+        for (unsigned t = blockIdx.x; t < total && !sh->gave_up; t += gridDim.x, block++)
             if (sh->odd[block / 32u] >> (block % 32u) & 1u) again(threadIdx.x - 128u, t / row_blocks * 128u, t % row_blocks * N);
     } else {
         asm volatile("setmaxnreg.inc.sync.aligned.u32 104;");

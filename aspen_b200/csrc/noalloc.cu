@@ -19,6 +19,7 @@
 #include "tiles_simt.cuh"
 #include "gemm_ffma.cuh"
 #include "gemm_split.cuh"
+#include "call_slots.h"
 #include "matmul_pick.h"
 
 #include <cuda_runtime.h>
@@ -120,7 +121,11 @@ __global__ void __launch_bounds__(fmablk::THREADS, 2) matmul_blocks(const Args a
     fmablk::block<S>(smem, threadIdx.x, a.k, lw, lx, BlockBarrier(), fin);
 }
 
-__device__ unsigned split_gave_up;      // a wait of matmul_split ran out (since the host last looked)
+// A word for each of the calls that run matmul_split at the same time: a wait of that call's kernel ran out.  One word for all would have
+// a call clear another's, and take the failure of another for its own.
+constexpr unsigned CALLS = 1024;
+__device__ unsigned split_failed[CALLS];
+CallSlots<CALLS> call_slots;
 
 template <int VEC>
 struct Operands {
@@ -190,12 +195,12 @@ struct Again {
     }
 };
 template <int N, int VEC>
-__global__ void __launch_bounds__(split::THREADS, 1) matmul_split(const Args a) {
+__global__ void __launch_bounds__(split::THREADS, 1) matmul_split(const Args a, int call) {
     extern __shared__ __align__(1024) unsigned char split_smem[];
     __shared__ split::Shared sh;
     const Operands<VEC> in{{a.w, a.m, a.k}, {a.x, a.n_cols, a.k}};
     const FinishPiece out{a};
-    split::blocks<N>(split_smem, &sh, &split_gave_up, a.n_cols, a.m, a.k, in, out, Again<N, VEC>{a, split_smem});
+    split::blocks<N>(split_smem, &sh, &split_failed[call], a.n_cols, a.m, a.k, in, out, Again<N, VEC>{a, split_smem});
 }
 
 // One weight row per warp, N columns (the last ones may be missing).
@@ -240,15 +245,15 @@ void launch_blocks(const Args &a, cudaStream_t stream) {
 }
 
 template <int N, int VEC>
-void launch_split(const Args &a, unsigned sms, cudaStream_t stream) {
+void launch_split(const Args &a, unsigned sms, int call, cudaStream_t stream) {
     typedef split::Shape<N> S;
     const unsigned blocks = ((a.m + N - 1) / N) * ((a.n_cols + 127) / 128);
     cudaFuncSetAttribute(matmul_split<N, VEC>, cudaFuncAttributeMaxDynamicSharedMemorySize, S::SMEM_BYTES);
-    matmul_split<N, VEC><<<std::min(blocks, sms), split::THREADS, S::SMEM_BYTES, stream>>>(a);
+    matmul_split<N, VEC><<<std::min(blocks, sms), split::THREADS, S::SMEM_BYTES, stream>>>(a, call);
 }
 
 template <int VEC>
-void launch(const Args &a, unsigned sms, cudaStream_t stream) {
+void launch(const Args &a, MatmulKernel kernel, unsigned sms, int call, cudaStream_t stream) {
     if (a.n_cols <= 8) {
         const unsigned grid = (a.m + fmablk::THREADS / 32 - 1) / (fmablk::THREADS / 32);
         if (a.n_cols == 1) matmul_rows<1, VEC><<<grid, fmablk::THREADS, 0, stream>>>(a);
@@ -257,13 +262,32 @@ void launch(const Args &a, unsigned sms, cudaStream_t stream) {
         else matmul_rows<8, VEC><<<grid, fmablk::THREADS, 0, stream>>>(a);
         return;
     }
-    switch (pick_matmul(a.n_cols, a.k, a.m, sms, VEC)) {
+    switch (kernel) {
         case FMA_128x64: launch_blocks<fmablk::Large, VEC>(a, stream); break;
         case FMA_64x64: launch_blocks<fmablk::Medium, VEC>(a, stream); break;
         case FMA_32x32: launch_blocks<fmablk::Small, VEC>(a, stream); break;
-        case SPLIT_128: launch_split<128, VEC>(a, sms, stream); break;
-        case SPLIT_64: launch_split<64, VEC>(a, sms, stream); break;
+        case SPLIT_128: launch_split<128, VEC>(a, sms, call, stream); break;
+        case SPLIT_64: launch_split<64, VEC>(a, sms, call, stream); break;
     }
+}
+
+// Launches and waits.  Whether a wait of the call's kernel ran out is looked at only if the call took long enough for one.
+cudaError_t run(const Args &a, int vec, MatmulKernel kernel, unsigned sms, int call, cudaStream_t stream, bool *failed) {
+    const auto started = std::chrono::steady_clock::now();
+    if (vec == 4) launch<4>(a, kernel, sms, call, stream);
+    else if (vec == 2) launch<2>(a, kernel, sms, call, stream);
+    else launch<1>(a, kernel, sms, call, stream);
+    cudaError_t err = cudaGetLastError();
+    if (err == cudaSuccess) err = cudaStreamSynchronize(stream);
+    if (err != cudaSuccess || call < 0 || std::chrono::steady_clock::now() - started < std::chrono::nanoseconds(split::LIMIT_NS / 2)) return err;
+    unsigned word = 0;
+    const unsigned none = 0;
+    err = cudaMemcpyFromSymbolAsync(&word, split_failed, sizeof word, call * sizeof word, cudaMemcpyDeviceToHost, stream);
+    if (err == cudaSuccess) err = cudaStreamSynchronize(stream);
+    if (err != cudaSuccess || word == 0) return err;
+    *failed = true;
+    err = cudaMemcpyToSymbolAsync(split_failed, &none, sizeof none, call * sizeof none, cudaMemcpyHostToDevice, stream);
+    return err == cudaSuccess ? cudaStreamSynchronize(stream) : err;
 }
 
 }  // namespace
@@ -287,24 +311,17 @@ extern "C" int aspen_b200_matmul_noalloc(const float *x_dev, const float *w_dev,
     if (err == cudaSuccess) err = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     if (err != cudaSuccess || sms <= 0) { ASPEN_ERR("aspen_b200_matmul_noalloc: no current CUDA device (%s)\n", cudaGetErrorString(err)); return -3; }
     cudaStream_t stream = static_cast<cudaStream_t>(cuda_stream);
-    const auto started = std::chrono::steady_clock::now();
     const Args a{x_dev, w_dev, bias_dev, out_dev, n_cols, k, m, activation, m % 4 == 0 && reinterpret_cast<uintptr_t>(out_dev) % 16 == 0};
     const uintptr_t align = reinterpret_cast<uintptr_t>(x_dev) | reinterpret_cast<uintptr_t>(w_dev);
-    if (k % 4 == 0 && align % 16 == 0) launch<4>(a, (unsigned)sms, stream);
-    else if (k % 2 == 0 && align % 8 == 0) launch<2>(a, (unsigned)sms, stream);
-    else launch<1>(a, (unsigned)sms, stream);
-    err = cudaGetLastError();
-    if (err != cudaSuccess) { ASPEN_ERR("aspen_b200_matmul_noalloc: launch failed: %s\n", cudaGetErrorString(err)); return -3; }
-    err = cudaStreamSynchronize(stream);
+    const int vec = k % 4 == 0 && align % 16 == 0 ? 4 : k % 2 == 0 && align % 8 == 0 ? 2 : 1;
+    MatmulKernel kernel = pick_matmul(n_cols, k, m, (unsigned)sms, vec);
+    int call = -1;
+    if (n_cols > 8 && kernel >= SPLIT_128 && (call = call_slots.take()) < 0) kernel = pick_matmul(n_cols, k, m, (unsigned)sms, vec, false);
+    bool failed = false;
+    err = run(a, vec, kernel, (unsigned)sms, call, stream, &failed);
+    // a word that is set and could not be cleared keeps its number
+    if (call >= 0 && !(failed && err != cudaSuccess)) call_slots.give(call);
+    if (failed) { ASPEN_ERR("aspen_b200_matmul_noalloc: a wait of the kernel ran out\n"); return -3; }
     if (err != cudaSuccess) { ASPEN_ERR("aspen_b200_matmul_noalloc: %s\n", cudaGetErrorString(err)); return -3; }
-    // a wait that runs out does so after split::LIMIT_NS, so a call that took less has had none
-    if (std::chrono::steady_clock::now() - started > std::chrono::nanoseconds(split::LIMIT_NS / 2)) {
-        unsigned gave_up = 0;
-        const unsigned none = 0;
-        if (cudaMemcpyFromSymbol(&gave_up, split_gave_up, sizeof gave_up) != cudaSuccess || (gave_up && cudaMemcpyToSymbol(split_gave_up, &none, sizeof none) != cudaSuccess) || gave_up) {
-            ASPEN_ERR("aspen_b200_matmul_noalloc: a wait of the kernel ran out\n");
-            return -3;
-        }
-    }
     return 0;
 }

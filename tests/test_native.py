@@ -117,3 +117,7 @@ def test_shapes_that_test_the_split_kernels_run_them(workdir):
         assert picked == kernel, (n, k, m)
         seen.add((kernel, values))
     assert len(seen) == 6
+
+
+def test_calls_that_run_at_once_have_numbers_of_their_own(workdir):
+    passes(build("call_slots", workdir, "-lpthread"), timeout=60)
