@@ -15,7 +15,7 @@ HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 LIB = os.path.join(HERE, "libaspen_b200.so")
 SOURCES = ["cfg.cpp", "dnn.cpp", "tiler.cpp", "graph.cpp", "plan.cpp", "runtime.cpp", "engine.cu", "fp32.cu", "noalloc.cu"]
-HEADERS = ["internal.h", "device_types.h", "gemm_ffma.cuh", "gemm_split.cuh", "matmul_pick.h", "call_slots.h", "index_div.h", "hostcopy.h", "fp32.h", "tiles_simt.cuh", "tiles_tc.cuh", "worker_loop.h", "scheduler.cuh",
+HEADERS = ["internal.h", "device_types.h", "gemm_ffma.cuh", "gemm_split.cuh", "matmul_pick.h", "call_slots.h", "recent_sets.h", "index_div.h", "hostcopy.h", "fp32.h", "tiles_simt.cuh", "tiles_tc.cuh", "worker_loop.h", "scheduler.cuh",
            os.path.join("..", "..", "include", "aspen_b200.h")]
 NVCC = os.environ.get("NVCC", "/usr/local/cuda/bin/nvcc")
 FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17", "-Xcompiler", "-fPIC",

@@ -121,3 +121,7 @@ def test_shapes_that_test_the_split_kernels_run_them(workdir):
 
 def test_calls_that_run_at_once_have_numbers_of_their_own(workdir):
     passes(build("call_slots", workdir, "-lpthread"), timeout=60)
+
+
+def test_sets_of_graphs_that_are_run_in_turn_are_kept(workdir):
+    passes(build("recent_sets", workdir))
