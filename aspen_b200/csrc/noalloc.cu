@@ -13,8 +13,8 @@
 //     The line lies at 8: with 16 columns the 32 x 32 blocks below are faster (19.9 against 23.6 us at k = 768, m = 3072).
 //   * larger: the fp32 FMA blocks of gemm_ffma.cuh, or the tensor cores over operands split into bf16 parts (gemm_split.cuh), by
 //     `pick_matmul` (matmul_pick.h).
-// B200, wall time of a call, launch and wait included (columns x k x rows):  1 x 768 x 768 17 us;  333 x 770 x 1000 44 us in FMA
-// blocks (45 split);  4096 x 768 x 3072 466 in FMA blocks, 199 split.
+// B200, wall time of a call, launch and wait included (columns x k x rows):  1 x 768 x 768 17 us;  333 x 770 x 1000 39 us split (44 in
+// FMA blocks);  4096 x 768 x 3072 179 split (466 in FMA blocks).
 #include "internal.h"
 #include "tiles_simt.cuh"
 #include "gemm_ffma.cuh"
