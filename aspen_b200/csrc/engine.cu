@@ -506,7 +506,7 @@ static int build_device_nasm(Engine *e, nasm_t *host_nasm) {
         const bool gemm_w = l.type == CONV_LAYER || l.type == FC_LAYER || l.type == MATMUL_LAYER;
         const unsigned p0 = nasm->ldata[i].parent_ldata_idx_arr[PARENT_0], p1 = nasm->ldata[i].parent_ldata_idx_arr[PARENT_1];
         const cuuint64_t W0 = p0 != (unsigned)-1 ? nasm->ldata[p0].out_mat_dims[OUT_W] : 0;
-        // Operand ring: a W box holds the tile's rows; a stage holds as many chunks as keep the one-thread roles ahead of the MMAs
+        // Operand ring: a W box holds the tile's rows; a stage holds as many chunks as keep the issuing warps ahead of the MMAs
         // (a wait and a box cost the same whatever the box holds: tiles_tc.cuh)
         // while two or more stages fit.
         const unsigned th = nasm->ldata[i].ninst_tile_dims[OUT_H];
@@ -737,11 +737,9 @@ static int build_device_nasm(Engine *e, nasm_t *host_nasm) {
                 const unsigned per_col = (Q.out_mat_dims[OUT_H] + qh - 1) / qh;
                 for (unsigned cw = T.pos_w / qw; cw <= (T.pos_w + T.tile_w - 1) / qw; cw++)
                     for (unsigned ch = T.pos_h / qh; ch <= (T.pos_h + T.tile_h - 1) / qh; ch++) {
-                        for (unsigned s = 0; s < Q.slices; s++) {
-                            const unsigned par = Q.ninst_start + (cw * per_col + ch) * Q.slices + s;
-                            if (par >= Q.ninst_start + Q.num_ninst || par >= t) { ASPEN_ERR("fused residual: tile %u has no valid producer tile\n", t); return -1; }
-                            reads(par);
-                        }
+                        const unsigned par = Q.ninst_start + cw * per_col + ch;            // residuals are fused where k is not split
+                        if (par >= Q.ninst_start + Q.num_ninst || par >= t) { ASPEN_ERR("fused residual: tile %u has no valid producer tile\n", t); return -1; }
+                        reads(par);
                     }
             }
             std::sort(list.begin(), list.end());

@@ -852,14 +852,15 @@ __device__ __forceinline__ bool arrives_last(const TileDev &T, unsigned tid, uns
     worker_barrier(nthr);
     return *(volatile unsigned *)last != 0u;
 }
-// The parts' sums added in order (so a run's bits do not depend on which tile came last), bias, activation and store.
+// The parts' sums added in order (so a run's bits do not depend on which tile came last), bias, activation and store.  fp32 mode: nothing is
+// rounded to TF32.
 static __device__ __noinline__ void finish_parts(const LayerDev &L, const TileDev &T, unsigned tid, unsigned nthr) {
     const unsigned tile_h = T.tile_h, h4 = (tile_h + 3u) >> 2, total = T.tile_w * h4, slices = T.slices;
     const size_t step = (size_t)T.tile_w * h4 * 4u;
     const float *part = T.part, *bias = L.bias ? L.bias + T.pos_h : nullptr;
     float *out = L.out + (size_t)T.pos_w * L.ldc + T.pos_h;
     const size_t ldc = L.ldc;
-    const bool late = late_activation(L), round = L.round_out != 0 && !late, relu = !late && L.act == RELU;
+    const bool late = late_activation(L), relu = !late && L.act == RELU;
     for (unsigned i = tid; i < total; i += nthr) {
         const unsigned n = i / h4, m = (i - n * h4) * 4u;
         float4 a[8];
@@ -874,7 +875,6 @@ static __device__ __noinline__ void finish_parts(const LayerDev &L, const TileDe
         for (unsigned j = 0; j < 4; j++) {
             if (bias && m + j < tile_h) f[j] += __ldg(bias + m + j);
             if (relu) f[j] = f[j] > 0.f ? f[j] : 0.f;
-            if (round) f[j] = tf32_round(f[j]);
         }
         if (m + 4u <= tile_h && (reinterpret_cast<uintptr_t>(o) & 15u) == 0u) *reinterpret_cast<float4 *>(o) = make_float4(f[0], f[1], f[2], f[3]);
         else
