@@ -1,14 +1,17 @@
 // fp32 contraction on the tensor cores: out[n][m] = act(bias[m] + sum_k W[m][k] X[n][k]) with every operand as a sum of three bf16 values.
 //
 // An fp32 value is x = b1 + b2 + b3 (8 bits each), exactly unless |x| < 2^-110, where b3 may need bits below the last of bf16, 2^-133.  W X is
-// nine products of bf16 parts
-// of which the six up to 2^-16 are kept -- the others are below half a unit of the fp32 product.  The tensor cores multiply bf16 exactly
-// but truncate when they add to an accumulator: a chunk of k = 32 is summed there, smallest products first, and added to the
-// total in registers with rounding to nearest.  Relative error (2-norm, against 64 bits, N(0, 1) operands), FMA blocks and this:
-// see pick_matmul.  A block is computed again by fp32 FMA blocks if one of its values has no such sum -- infinities,
-// NaN and values with bits below 2^-133 -- or one of its totals is so small that what the accumulators truncate at the lower end of fp32, up to four
-// units of 2^-149 a chunk, is more than 2^-24 of it (768 products around 2^-130: 2-norm error 1.3e-6, of fp32 sums 5.5e-7).  That is done when the
-// CTA is through with all of its blocks, so that nothing waits for it.  4096 x 768 x 3072: 176 us a call, 900 if every block is marked.
+// nine products of bf16 parts of which the six up to 2^-16 are kept -- the others are below half a unit of the fp32 product.  The tensor cores
+// multiply bf16 exactly but truncate when they add to an accumulator: a chunk of k = 32 is summed there, smallest products first, and added to the
+// total in registers with rounding to nearest.  Relative error (2-norm, against 64 bits, N(0, 1) operands), FMA blocks and this: see pick_matmul.
+//
+// A block is computed again by fp32 FMA blocks, so that its outputs are what fp32 sums give,
+//     if one of its values has no such sum: infinities, NaN, values with bits below 2^-133, values that round past the range of bf16;
+//     if a total is an infinity or a NaN: where a product overflows, those of the parts have either sign and leave inf - inf;
+//     if a total is so small that what the accumulators truncate at the lower end of fp32, up to four units of 2^-149 a chunk, is more than 2^-24
+//     of it (768 products around 2^-130: 2-norm error 1.3e-6, of fp32 sums 5.5e-7).
+// That is done when the CTA is through with all of its blocks, so that nothing waits for it.  4096 x 768 x 3072: 176 us a call, 900 if every block
+// is marked.
 //
 // What bounds it: shared memory.  A chunk of a 128 x 128 block is 12 MMAs that read 8 KB each, and 49 KB of parts written for them:
 // 1150 cycles at 128 bytes a cycle, against 770 of the tensor pipe.  Hence
@@ -266,7 +269,6 @@ __device__ __forceinline__ void blocks(unsigned char *smem, Shared *sh, unsigned
         asm volatile("setmaxnreg.inc.sync.aligned.u32 104;");
         const unsigned q = warp & 3u, first = (warp - 12u) / 4u * (N / 2);        // TMEM lanes 32 q .. + 31: columns; rows first .. + N / 2 - 1
         float *stage = reinterpret_cast<float *>(smem + S::STAGES * S::STAGE_BYTES + (warp - 12u) * 4096u);
-        const float least = (float)chunks * 0x1p-123f;
         unsigned it = 0, block = 0;
         bool ok = true;
         for (unsigned t = blockIdx.x; t < total && ok; t += gridDim.x, block++) {
@@ -293,10 +295,16 @@ __device__ __forceinline__ void blocks(unsigned char *smem, Shared *sh, unsigned
                 }
             }
             if (!ok) break;
-            bool tiny = false;
+            // Too small, or not finite (of two magnitudes the larger bits are the larger value).  Outputs past the last row or column hold
+            // another one's values or zeros.
+            const unsigned least = __float_as_uint((float)chunks * 0x1p-123f);
+            unsigned far = 0;
             #pragma unroll
-            for (int i = 0; i < N / 2; i++) tiny = tiny || (fabsf(sum[i]) < least && sum[i] != 0.f);
-            if (tiny) atomicOr(&sh->odd[block / 32u], 1u << (block % 32u));
+            for (int i = 0; i < N / 2; i++) {
+                const unsigned u = __float_as_uint(sum[i]) & 0x7fffffffu;
+                far = max(far, u == 0u ? 0u : u - least);
+            }
+            if (far >= 0x7f800000u - least) atomicOr(&sh->odd[block / 32u], 1u << (block % 32u));
             #pragma unroll
             for (int j = 0; j < N / 2; j += 32) {
                 // 32 x 32 outputs through the warp's buffer: then consecutive lanes have consecutive rows

@@ -142,6 +142,34 @@ def test_noalloc_on_the_tensor_cores_over_the_range_of_fp32(n, k, m, kernel):
             assert off <= (0.3 * np.sqrt(k / 2) * 2.0**-24 + 2.0**-23) * size + 2.0**-150 * np.sqrt(k * (cols.stop - cols.start)), (row, name, off / size)
 
 
+@pytest.mark.parametrize("n,k,m,kernel", RANGE_SHAPES)
+@pytest.mark.parametrize("act", [0, 4])          # 4: ReLU, which makes a zero of a NaN
+def test_noalloc_on_the_tensor_cores_where_finite_operands_overflow(n, k, m, kernel, act):
+    """Sums past the range of fp32 are infinities, also where the products of the operands' parts overflow with either sign; sums within it are
+    right although a product of rounded parts is past it.  Row 5 of x and row 9 of w lie in one block, rows 130 and 300 in others."""
+    rng = np.random.default_rng(n)
+    x = rng.standard_normal((n, k), dtype=np.float32)
+    w = (rng.standard_normal((m, k)) * np.sqrt(2 / k)).astype(np.float32)
+    x[5] = np.float32(1.1e25) * (1 + rng.random(k, dtype=np.float32) / 64)
+    w[9] = np.float32(1.3e25) * (1 + rng.random(k, dtype=np.float32) / 64)          # 1.4e50 a product
+    w[10] = -w[9]
+    x[130], w[200] = 0, 0
+    x[130, 3], w[200, 3] = np.float32(1.9975), np.float32(2.0**127)          # within the range; 2 * 2**127, as the first part rounds, is not
+    x[300], w[201] = 0, 0
+    x[300, ::2] = w[201, ::2] = np.float32(1.8e19)                                    # each product within the range, their sum past it
+    got = noalloc(x, w, None, act)
+    with np.errstate(over="ignore"):
+        want = (x.astype(np.float64) @ w.T.astype(np.float64)).astype(np.float32)
+    if act == 4:
+        want = np.maximum(want, 0)
+    far = np.isinf(want)
+    assert far[5, 9] and far[300, 201] and (far[5, 10] or act == 4) and np.isfinite(want[130, 200]) and want[130, 200] > np.float32(3.3e38)
+    np.testing.assert_array_equal(got[far], want[far])
+    assert np.isfinite(got[~far]).all()
+    scale = np.abs(x.astype(np.float64)) @ np.abs(w.T.astype(np.float64))        # as above
+    assert (np.abs(got[~far].astype(np.float64) - want[~far]) <= (2.0**-24 * (1 + np.sqrt(k)) * scale + 2.0**-149 * k)[~far]).all()
+
+
 @pytest.mark.parametrize("name,batch,seq,precision", [("tiny_attn", 1, 1, 0), ("tiny_attn", 3, 33, 0), ("tiny_attn", 1, 129, 0), ("tiny_attn_causal", 2, 255, 0),
                                                       ("tiny_attn_causal", 1, 257, 0), ("tiny_attn_causal", 1, 300, 1), ("tiny_transformer", 64, 128, 0),
                                                       ("tiny_cnn", 1, 0, 0), ("tiny_cnn", 33, 0, 0), ("tiny_cnn", 9, 0, 1), ("custom", 1, 0, 0), ("custom", 130, 0, 0),
