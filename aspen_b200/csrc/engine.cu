@@ -177,6 +177,12 @@ void engine_release_dnn(aspen_dnn_t *dnn) {
 }
 
 // ---- engine --------------------------------------------------------------------------------
+struct MergedOrder {
+    sched::Entry *tiles = nullptr;
+    unsigned cap = 0;
+};
+static void free_order(MergedOrder &o) { cudaFree(o.tiles); }
+
 struct Engine {
     int device = 0;
     int precision = 0;
@@ -189,9 +195,10 @@ struct Engine {
     StatusHost *status_d = nullptr;
     sched::Entry *queue = nullptr;
     unsigned queue_cap = 0;
-    // Several graphs in one launch (images, by DeviceNasm::serial): their tiles in the order they are handed out.  A program whose launches
-    // take turns between sets finds each set's order: merged for every launch it cost a call of ResNet-50 + VGG-16 x 16 (1770 us) another 100.
-    RecentSets<sched::Entry *, 8> orders;
+    // Several graphs in one launch (images, by DeviceNasm::serial): their tiles in the order they are handed out, 8 bytes each.  A program whose
+    // launches take turns between sets finds each set's order (64: every set of six graphs).  Made anew for every launch it cost a call of
+    // ResNet-50 + VGG-16 x 16 (1770 us) another 100; the CIFAR net in 56 sets of seven graphs, dse_group_run: 45 us with 8 sets kept, 10 with 64.
+    RecentSets<MergedOrder, 64> orders;
     NasmDev *nasms_d = nullptr;
     unsigned nasms_cap = 0;
     std::vector<NasmDev> uploaded;    // what nasms_d holds
@@ -336,7 +343,7 @@ void engine_destroy(Engine *e) {
     cudaFree(e->ctrl);
     if (e->status_h) cudaFreeHost((void *)e->status_h);
     cudaFree(e->queue);
-    e->orders.drop(0, cudaFree);
+    e->orders.drop(0, free_order);
     cudaFree(e->nasms_d);
     cudaFree(e->prof);
     delete e;
@@ -853,7 +860,7 @@ static NasmDev graph_image(const nasm_t *nasm) {
 static sched::Entry *merge_orders(Engine *e, const std::vector<nasm_t *> &graphs, unsigned claims) {
     std::vector<unsigned long long> of;
     for (const nasm_t *n : graphs) of.push_back(n->dev->serial);
-    if (sched::Entry **known = e->orders.find(of)) return *known;
+    if (MergedOrder *known = e->orders.find(of)) return known->tiles;
     std::vector<sched::Entry> order;
     order.reserve(claims);
     typedef std::pair<float, unsigned> Next;                   // start of a graph's next tile; the graph
@@ -870,16 +877,23 @@ static sched::Entry *merge_orders(Engine *e, const std::vector<nasm_t *> &graphs
         order.push_back(sched::make_entry(t, g, graphs[g]->dev->tile_layer[t]));
         push(g);
     }
-    sched::Entry *made = nullptr;
-    if (cudaMalloc(&made, std::max<size_t>(claims, 1) * sizeof(sched::Entry)) != cudaSuccess ||
-        // cudaMemcpyAsync from pageable memory returns after the source has been staged
-        cudaMemcpyAsync(made, order.data(), order.size() * sizeof(sched::Entry), cudaMemcpyHostToDevice, e->stream) != cudaSuccess) {
+    // With more sets than are kept the memory of one that goes is used again: cudaFree would wait for all that runs on the device.  Whatever
+    // launch read it is ahead on the stream.
+    MergedOrder made;
+    e->orders.make_room(made);
+    if (claims > made.cap) {
+        free_order(made);
+        made = MergedOrder();
+        if (cudaMalloc(&made.tiles, (size_t)claims * sizeof(sched::Entry)) == cudaSuccess) made.cap = claims;
+    }
+    // cudaMemcpyAsync from pageable memory returns after the source has been staged
+    if (claims > made.cap || cudaMemcpyAsync(made.tiles, order.data(), order.size() * sizeof(sched::Entry), cudaMemcpyHostToDevice, e->stream) != cudaSuccess) {
         ASPEN_ERR("CUDA error for the order of a launch: %s\n", cudaGetErrorString(cudaGetLastError()));
-        cudaFree(made);
+        free_order(made);
         return nullptr;
     }
-    e->orders.put(of, made, cudaFree);
-    return made;
+    e->orders.put(of, made);
+    return made.tiles;
 }
 
 // `leave`: the kernel ends when the passes owed now are complete.  `chained`: the launch follows others on the stream that
@@ -1114,7 +1128,7 @@ void engine_detach_nasm(nasm_t *nasm) {
     cudaSetDevice(e->device);
     svc_halt(e);
     e->svc_pool.erase(std::remove(e->svc_pool.begin(), e->svc_pool.end(), nasm), e->svc_pool.end());
-    if (dn->serial) e->orders.drop(dn->serial, cudaFree);
+    if (dn->serial) e->orders.drop(dn->serial, free_order);
     free_device_nasm(dn);
     nasm->dev = nullptr;
 }

@@ -18,13 +18,15 @@ public:
             if (sets[i].of == of) { std::rotate(sets.begin(), sets.begin() + i, sets.begin() + i + 1); return &sets[0].made; }
         return nullptr;
     }
-    // `release(T &)` for what has to make room.
-    template <typename F>
-    void put(const Key &of, const T &made, F release) {
-        if (sets.size() == N) { release(sets.back().made); sets.pop_back(); }
-        sets.insert(sets.begin(), Set{of, made});
+    // With N sets kept the one not used for longest goes: true, and what was made for it is the caller's to use again.
+    bool make_room(T &made) {
+        if (sets.size() < N) return false;
+        made = sets.back().made;
+        sets.pop_back();
+        return true;
     }
-    // Sets with this object; all of them if it is 0.
+    void put(const Key &of, const T &made) { sets.insert(sets.begin(), Set{of, made}); }
+    // `release(T &)` for what was made for the sets with this object; all of them if it is 0.
     template <typename F>
     void drop(unsigned long long object, F release) {
         for (size_t i = sets.size(); i-- > 0;)

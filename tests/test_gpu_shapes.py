@@ -228,6 +228,33 @@ def _conv_net(side, channels, layers, out):
     return text + f"[connected]\noutput={out}\nactivation=linear\n", wl
 
 
+def test_launches_of_more_sets_of_graphs_than_are_kept(workdir):
+    """92 sets of seven graphs in turn, without a stop between them: the order of one is written where another's was."""
+    import itertools
+    dnn = api.Dnn(*harness.prepare("custom", workdir))
+    graphs = [api.Nasm(dnn, b, 0, 8) for b in (1, 2, 3, 5, 8, 13, 21)]
+    rpool, group = api.Rpool(), api.DseGroup(0, 0)
+    group.set_rpool(rpool)
+    xs = [harness.make_input("custom", (g.ldata_info(0)["W"], g.ldata_info(0)["H"])) for g in graphs]
+    first = {}
+    for _ in range(2):
+        for owed in itertools.chain(*(itertools.combinations(range(7), r) for r in (7, 2, 3, 4))):
+            for i in owed:
+                rpool.add(graphs[i], xs[i])
+            group.run()
+            for i in owed:
+                group.wait(graphs[i])
+            assert group.status() == 0, api.last_error()
+            for i in owed:
+                got = graphs[i].ldata(graphs[i].num_ldata - 1).copy()
+                np.testing.assert_array_equal(got, first.setdefault(i, got))
+    group.stop()
+    assert len(first) == 7 and all(np.abs(v).max() > 0 for v in first.values())
+    group.close()
+    for o in (*graphs, rpool, dnn):
+        o.close()
+
+
 @pytest.mark.parametrize("batch,side,channels,layers", [
     (3, 30, 3, [(48, 7, 2, 3), (24, 3, 1, 1), (33, 3, 2, 1), (64, 1, 2, 0), (10, 1, 1, 0)]),       # rows of 15 pixels; channels no multiple of 32, or of 4
     (12, 37, 1, [(20, 11, 4, 2), (96, 3, 1, 0), (12, 5, 1, 2)]),                                   # one channel, a window of two chunks a row
