@@ -35,9 +35,12 @@ enum Path { TENSOR, BESIDE_RING, FP32 };      // tensor cores / fp32 blocks in a
 Path path_of(const aspen_layer_t *l, int precision, unsigned seq) { return precision != 0 ? FP32 : operand_form(l, seq).kind != A_NONE ? TENSOR : BESIDE_RING; }
 
 // Estimated microseconds of one tile of th x tw outputs with a k-deep contraction, `gap` of them between two tiles of an SM.
-// Tensor cores: what a 32-deep chunk of a 128-column block takes inside a network, where part of the operands comes from HBM -- 0.38 us
-// with 256 rows, 0.28 with 128 and 0.19 below (0.30 - 0.37, 0.22 and 0.16 with everything in L2: tiles_tc.cuh); the epilogue of a
-// block takes 0.4 us per 32 rows and runs under the next block's main loop.
+// Tensor cores: 0.38 us for a 32-deep chunk of a 128-column block with 256 rows, 0.28 with 128 and 0.19 with 64 or less; the epilogue of a
+// block takes 0.4 us per 32 rows and runs under the next block's main loop.  Measured in launched networks (layers of the same tiles, k = 768
+// and 3072) a chunk takes 0.34, 0.20, 0.17 and, with 32 rows, 0.12 - 0.15 us.  The weights of the narrow ones are larger because a
+// tile's time does not count what more and narrower tiles cost the rest of the chip: with 0.11 in place of 0.19 a pass of GPT-2 8 x 512 takes
+// 3005 us instead of 2390, BERT 16 x 128 1714 for 1484, ResNet-50 x 32 1477 for 1379; with 0.15 2413, 1662 and 1416; with 0.15 and 0.22 (in
+// place of 0.28) 2479, 1473 and 1387.
 // Beside the ring (measured): 64 x 32 blocks, 0.8 us and 1.0 per 32 of k (3 x 3 layers of 48 and 24 channels), 1.6 where operands
 // come value by value (attention with heads of 10); the softmax of scores 1.4 us per 1024.
 // `ks` > 1: one of ks tiles that share k; they write and read their sums and wait for each other's counts, some 3 us.
@@ -60,8 +63,7 @@ double tile_us(Path path, const aspen_layer_t *l, unsigned th, unsigned tw, unsi
     return gap + (double)ceil_div(th, bm) * ceil_div(tw, bn) * (3.0 + ceil_div(k, kt) * (shape == 2 ? 1.3 : 2.0));
 }
 
-// `small`: a pass of the graph is less than 100 us of work for the chip.
-Grid choose(const nasm_ldata_t &ld, const nasm_t *nasm, int precision, unsigned sms, bool served, bool small) {
+Grid choose(const nasm_ldata_t &ld, const nasm_t *nasm, int precision, unsigned sms, bool served) {
     const aspen_layer_t *l = ld.layer;
     const unsigned *p = l->params;
     const unsigned H = ld.out_mat_dims[OUT_H], W = ld.out_mat_dims[OUT_W];
@@ -89,12 +91,15 @@ Grid choose(const nasm_ldata_t &ld, const nasm_t *nasm, int precision, unsigned 
                 const double share = (double)tiles / sms;
                 // Launched alone a layer of fewer tiles than SMs takes as long as one tile; of a larger one the last tiles run while
                 // half of the chip waits.  (The work and 0.7 tiles whatever the number: ResNet-50 x 3 617 us a pass instead of 570,
-                // x 32 1398 and 1373, BERT 1 x 37 799 and 772.)  Served, the passes of other graphs fill those SMs but the
-                // graphs in rotation are few: the work, and a share of a tile.  There the best weight falls with the number of
-                // graphs in rotation, which a plan of one graph does not know, but a loop keeps more of them the smaller they are.  In
-                // bursts, 0.3 / 0.4 / 0.5 tiles: 7.11 / 7.24 / 7.59 ms for 32 requests of ResNet-50 x 4 (eight graphs, 40 us of the
-                // tensor cores' work each), 15.8 / 15.1 / 14.9 for 12 of x 32 (three, 320 us); 1.0: 0.304 ms a request of x 4 for 0.283.
-                const double cost = us * (served ? share + (small ? 0.3 : 0.5) : std::max(1.0, share + 0.5));
+                // x 32 1398 and 1373, BERT 1 x 37 799 and 772.)  Served, the passes of other graphs fill those SMs but the graphs in
+                // rotation are few: the work, and a share of a tile.  What the best share is depends on their number, which a plan of one graph does
+                // not know, and not on their size: up to four graphs prefer 0.5, from six on 0.3.  0.4 is at most 7 % slower than the best of the three
+                // over 35 networks, sizes and numbers, 1.5 % on average (0.3: 11 and 2.9; 0.5: 10 and 1.7; 0.3 for passes of less than 100 us of work
+                // and 0.5 above: 9.5 and 2.2).  Bursts of three or four requests a graph, us with 0.3 / 0.4 / 0.5 tiles: ResNet-50 x 4 with three
+                // graphs 3464 / 3370 / 3164, with four 3776 / 3671 / 3630, six 4463 / 4500 / 4680, eight 6997 / 7129 / 7508; x 16 with four
+                // 10647 / 10329 / 10408, eight 14420 / 14611 / 14748; x 32 with three 15399 / 14673 / 14598, six 20418 / 20417 / 20795; BERT 4 x 128 with
+                // four 9640 / 10061 / 10044, eight 12249 / 13151 / 13232.
+                const double cost = us * (served ? share + 0.4 : std::max(1.0, share + 0.5));
                 if (best == 0 || cost < best * 0.999) { best = cost; g.th = hs[i]; g.tw = tw; g.ks = 1; }
                 // Launched alone in the fp32 mode, a layer that leaves SMs idle shares its k among them: 512 x 49 outputs with k = 4608 are 32
                 // tiles of 48 us, or 128 of 14; ResNet-50 x 1 988 -> 916 us a pass.  (Not on the tensor cores, where a sample's bits
@@ -243,12 +248,10 @@ nasm_t *plan_device_tiles(const nasm_t *nasm, int precision, unsigned sms, bool 
     plan->ldata = nasm->ldata;
     std::vector<Grid> grid(plan->num_ldata);
     unsigned total = 0;
-    double flop = 0;
-    for (const nasm_ldata_t &ld : nasm->ldata) flop += (double)ld.flop_per_output * ld.out_mat_dims[OUT_H] * ld.out_mat_dims[OUT_W];
     for (unsigned i = 0; i < plan->num_ldata; i++) {
         nasm_ldata_t &ld = plan->ldata[i];
         ld.nasm = plan.get();
-        Grid &g = grid[i] = choose(nasm->ldata[i], nasm, precision, sms, served, flop < 5.4e8 * sms);      // 5.4 TFLOP/s an SM: the measured TF32 peak
+        Grid &g = grid[i] = choose(nasm->ldata[i], nasm, precision, sms, served);
         const unsigned H = ld.out_mat_dims[OUT_H], W = ld.out_mat_dims[OUT_W];
         if (H == 0 || W == 0 || W % g.seg != 0) return nullptr;
         g.start = total;
