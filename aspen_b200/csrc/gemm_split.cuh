@@ -2,15 +2,18 @@
 //
 // An fp32 value is x = b1 + b2 + b3 (8 bits each), exactly unless |x| < 2^-110, where b3 may need bits below the last of bf16, 2^-133.  W X is
 // nine products of bf16 parts of which the six up to 2^-16 are kept -- the others are below half a unit of the fp32 product.  The tensor cores
-// multiply bf16 exactly but truncate when they add to an accumulator: a chunk of k = 32 is summed there, smallest products first, and added to the
-// total in registers with rounding to nearest.  Relative error (2-norm, against 64 bits, N(0, 1) operands), FMA blocks and this: see pick_matmul.
+// multiply bf16 exactly but truncate when they add to an accumulator: a chunk of k = 32 is summed there, smallest products first; two chunks are
+// added to each other and then to the total in registers, with rounding to nearest.  Relative error, 2-norm, against 64 bits (k = 256 / 770 /
+// 3072): N(0, 1) operands 0.8 / 1.0 / 1.4e-7, FMA blocks of 64 x 64 1.5 / 2.5 / 5.0, of 32 x 32 1.1 / 1.8 / 3.5; operands of one sign 0.7 / 0.8 /
+// 1.1e-7, FMA blocks of 64 x 64 0.7 / 1.0 / 1.9, of 32 x 32 (eight partial sums) 0.5 / 0.6 / 1.0, the one place where they are closer: what
+// the accumulators cut off is all of one sign there.  (Chunks added to the total one by one: 0.8 / 1.1 / 1.9 and 0.7 / 0.9 / 1.4.)
 //
 // A block is computed again by fp32 FMA blocks, so that its outputs are what fp32 sums give,
 //     if one of its values has no such sum: infinities, NaN, values with bits below 2^-133, values that round past the range of bf16;
 //     if a total is an infinity or a NaN: where a product overflows, those of the parts have either sign and leave inf - inf;
 //     if a total is so small that what the accumulators truncate at the lower end of fp32, up to four units of 2^-149 a chunk, is more than 2^-24
 //     of it (768 products around 2^-130: 2-norm error 1.3e-6, of fp32 sums 5.5e-7).
-// That is done when the CTA is through with all of its blocks, so that nothing waits for it.  4096 x 768 x 3072: 176 us a call, 900 if every block
+// That is done when the CTA is through with all of its blocks, so that nothing waits for it.  4096 x 768 x 3072: 180 us a call, 900 if every block
 // is marked.
 //
 // What bounds it: shared memory.  A chunk of a 128 x 128 block is 12 MMAs that read 8 KB each, and 49 KB of parts written for them:
@@ -18,7 +21,7 @@
 //     warps 4 - 11   read both operands from global memory into registers, split them and store the parts in the 64-byte swizzled K-major
 //                    layout (a raw copy in shared memory would cost another 64 KB a chunk)
 //     warp 0         12 MMAs a chunk, into four accumulators in turn
-//     warps 12 - 19  add a finished accumulator to the totals (each holds 32 columns x N / 2 rows in registers), then bias, activation, stores
+//     warps 12 - 19  add two finished accumulators to the totals (each holds 32 columns x N / 2 rows in registers), then bias, activation, stores
 // N (128 or 64 rows of W a block) is the caller's choice; with 256 the totals leave too few registers for loads in flight (1.84 us a
 // chunk against 2 x 0.93).  Persistent: a CTA takes every gridDim-th block, and the splitting of the next one goes on under the stores.
 // 4096 x 3072 outputs, k = 3072: 146 TFLOP/s of fp32 products (FMA blocks: 46).
@@ -103,13 +106,15 @@ __device__ __forceinline__ void add2(float &x, float &y, float a, float b) {
     asm("mov.b64 {%0, %1}, %2;" : "=f"(x), "=f"(y) : "l"(s));
 }
 
-__device__ __forceinline__ void tmem_ld16(unsigned taddr, float *v) {
+// Eight columns of each of two accumulators.
+__device__ __forceinline__ void tmem_ld8x2(unsigned first, unsigned second, float *v) {
     unsigned *r = reinterpret_cast<unsigned *>(v);
-    asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
-                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
-                   "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
-                 : "r"(taddr) : "memory");
-    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%16];\n\t"
+                 "tcgen05.ld.sync.aligned.32x32b.x8.b32 {%8, %9, %10, %11, %12, %13, %14, %15}, [%17];\n\t"
+                 "tcgen05.wait::ld.sync.aligned;"
+                 : "=&r"(r[0]), "=&r"(r[1]), "=&r"(r[2]), "=&r"(r[3]), "=&r"(r[4]), "=&r"(r[5]), "=&r"(r[6]), "=&r"(r[7]),
+                   "=&r"(r[8]), "=&r"(r[9]), "=&r"(r[10]), "=&r"(r[11]), "=&r"(r[12]), "=&r"(r[13]), "=&r"(r[14]), "=&r"(r[15])
+                 : "r"(first), "r"(second) : "memory");
 }
 
 // Every role is through: the operand stages are free, and what it has stored is seen by the others.
@@ -276,23 +281,30 @@ __device__ __forceinline__ void blocks(unsigned char *smem, Shared *sh, unsigned
             float sum[N / 2];
             #pragma unroll
             for (int i = 0; i < N / 2; i++) sum[i] = 0.f;
-            for (unsigned c = 0; c < chunks; c++, it++) {
-                const unsigned h = it % ACCUMULATORS, from = sh->tmem + h * N + first + (q << 21);
-                ok = __all_sync(0xffffffffu, wait(&sh->acc_full[h], (it / ACCUMULATORS) & 1u, gave_up));
+            for (unsigned c = 0; c < chunks; c += 2u) {
+                // Two chunks are added to each other first: half as many roundings in the size of the totals.
+                const bool two = c + 1u < chunks;
+                const unsigned h0 = it % ACCUMULATORS, h1 = two ? (it + 1u) % ACCUMULATORS : h0, from = sh->tmem + first + (q << 21);
+                ok = wait(&sh->acc_full[h0], (it / ACCUMULATORS) & 1u, gave_up) && (!two || wait(&sh->acc_full[h1], ((it + 1u) / ACCUMULATORS) & 1u, gave_up));
+                ok = __all_sync(0xffffffffu, ok);
                 if (!ok) break;
                 tc::tc_fence_after();
                 #pragma unroll
-                for (int j = 0; j < N / 2; j += 16) {
+                for (int j = 0; j < N / 2; j += 8) {
                     float v[16];
-                    tmem_ld16(from + j, v);
-                    if (j + 16 == N / 2) {
+                    tmem_ld8x2(from + h0 * N + j, from + h1 * N + j, v);
+                    if (j + 8 == N / 2) {
                         tc::tc_fence_before();
                         __syncwarp();
-                        if (lane == 0) tc::mbar_arrive(&sh->acc_empty[h]);
+                        if (lane == 0) { tc::mbar_arrive(&sh->acc_empty[h0]); if (two) tc::mbar_arrive(&sh->acc_empty[h1]); }
                     }
                     #pragma unroll
-                    for (int i = 0; i < 16; i += 2) add2(sum[j + i], sum[j + i + 1], v[i], v[i + 1]);
+                    for (int i = 0; i < 8; i += 2) {
+                        add2(v[i], v[i + 1], two ? v[8 + i] : 0.f, two ? v[9 + i] : 0.f);
+                        add2(sum[j + i], sum[j + i + 1], v[i], v[i + 1]);
+                    }
                 }
+                it += two ? 2u : 1u;
             }
             if (!ok) break;
             // Too small, or not finite (of two magnitudes the larger bits are the larger value).  Outputs past the last row or column hold

@@ -9,9 +9,8 @@
 // On either side of the lines, columns x k x m: 64 x 3072 x 3072 60 us in FMA blocks of 32 x 32 and 81 split by 64; 333 x 770 x 1000 40 and 36;
 // 963 x 392 x 836 39 and 25; 1024 x 768 x 2048 split by 64 54 and by 128 42; 4096 x 3072 x 3072 1696 in FMA blocks of 64 x 64 and 522 split by 128.
 // `split` false: FMA blocks only (so many calls run at once that there is no number for this one: call_slots.h).
-// Splitting is for k >= 256: its error against 64 bits grows with what the accumulator of a 32-deep chunk cuts off, not with k, so that of
-// short sums would be larger than before.  2-norm, N(0, 1) operands, k = 258 / 512 / 770 / 3072: FMA blocks 1.5e-7 / 2.1e-7 / 1.9e-7 /
-// 5.0e-7, split 0.9e-7 / 1.0e-7 / 1.2e-7 / 1.9e-7.
+// Splitting is for k >= 256: its error against 64 bits is mostly what the accumulator of a 32-deep chunk cuts off, whatever k is, so that of
+// short sums would be larger than before.  Both errors: gemm_split.cuh.
 enum MatmulKernel { FMA_128x64, FMA_64x64, FMA_32x32, SPLIT_128, SPLIT_64 };
 inline MatmulKernel pick_matmul(unsigned n_cols, unsigned k, unsigned m, unsigned sms, int vec, bool split = true) {
     auto rounds = [&](unsigned bm, unsigned bn) { return (double)(((unsigned long long)((m + bm - 1) / bm) * ((n_cols + bn - 1) / bn) + sms - 1) / sms); };

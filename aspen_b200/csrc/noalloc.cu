@@ -14,7 +14,7 @@
 //   * larger: the fp32 FMA blocks of gemm_ffma.cuh, or the tensor cores over operands split into bf16 parts (gemm_split.cuh), by
 //     `pick_matmul` (matmul_pick.h).
 // B200, wall time of a call, launch and wait included (columns x k x rows):  1 x 768 x 768 17 us;  333 x 770 x 1000 39 us split (44 in
-// FMA blocks);  4096 x 768 x 3072 179 split (466 in FMA blocks).
+// FMA blocks);  4096 x 768 x 3072 180 split (466 in FMA blocks).
 #include "internal.h"
 #include "tiles_simt.cuh"
 #include "gemm_ffma.cuh"

@@ -65,6 +65,17 @@ def test_noalloc_on_the_tensor_cores_is_as_close_to_64_bits_as_fp32_sums(n, k, m
     assert np.linalg.norm(got - want) <= (0.2 * np.sqrt(k / 2) * 2.0**-24 + 2.0**-23) * np.linalg.norm(want)
 
 
+@pytest.mark.parametrize("n,k,m,kernel", [(1283, 3072, 1301, "split 128"), (385, 3072, 2048, "split 64")])
+def test_noalloc_on_the_tensor_cores_adds_chunks_two_by_two(n, k, m, kernel):
+    """Operands of one sign, whose partial sums grow evenly: k / 64 additions to a total, each off by 0.42 2**-24 of it in the root mean square (see
+    below), come to 0.42 sqrt(k / 64 / 3), and the accumulators of a chunk cut off up to a unit twice, at half the sum and at all of it, 1.1 2**-24
+    together.  (With every chunk added to the total by itself it is 2.4 2**-24, past this bound.)"""
+    rng = np.random.default_rng(k + m)
+    x, w = np.abs(rng.standard_normal((n, k), dtype=np.float32)), np.abs(rng.standard_normal((m, k), dtype=np.float32))
+    got, want = noalloc(x, w, None, 0), x.astype(np.float64) @ w.T.astype(np.float64)
+    assert np.linalg.norm(got - want) <= np.sqrt(0.42**2 * k / 192 + 1.1**2) * 2.0**-24 * np.linalg.norm(want)
+
+
 @pytest.mark.parametrize("n,k,m,kernel", [(1283, 3072, 1301, "split 128"), (385, 3070, 2047, "split 64")])
 def test_noalloc_blocks_with_infinities_cost_what_fp32_blocks_do(n, k, m, kernel):
     """One value of each block is an infinity: the SM that had it computes it again in 32 x 32 fp32 blocks, one after another, which takes
