@@ -256,12 +256,17 @@ void aspen_b200_rpool_add_nasm_tokens(rpool_t *rpool, nasm_t *nasm, const int *t
 void aspen_b200_set_hidden_states(int keep);
 
 /* No counterpart in the reference.  One matmul layer, out[n][m] = act(bias[m] + sum_k w[m][k] * x[n][k])
- * in fp32 FMA arithmetic, in one kernel launch and WITHOUT ALLOCATING ANYTHING.  It is for callers that are not allowed
+ * in fp32 precision, in one kernel launch and WITHOUT ALLOCATING ANYTHING.  Which kernel runs follows from the shape, the pointers'
+ * alignment and the GPU's number of SMs: fp32 FMAs, or, for more than 8 columns and k >= 256 where it is faster, tensor cores over operands split
+ * into three bf16 parts each, added in fp32.  Both are off from 64-bit sums by some units of 2^-24 in the 2-norm; the split form by less, but for
+ * operands that are all of one sign (up to 1.3 times as much as the closest FMA form).  Blocks of outputs with infinities, NaN, overflow or values
+ * at the lower end of fp32 are computed with FMAs there too.  The layer is for callers that are not allowed
  * to call cudaMalloc: plug-ins of a serving runtime that fixes all memory pools at start-up and treats a later
  * allocation as a bug, and loops that cannot afford the device-wide synchronisation an allocation
  * implies.  All pointers are DEVICE pointers the caller owns: x [n_cols][k], w [m][k],
  * bias [m] or NULL, out [n_cols][m], rows contiguous; cuda_stream is a cudaStream_t (NULL = default).
- * No memory besides the caller's buffers is used, so calls on several streams and host threads do not disturb one another.
+ * No device memory besides the caller's buffers is used but a word for each of up to 1024 calls that run at the same time, in an array of the
+ * library (more at once run FMAs), so calls on several streams and host threads do not disturb one another.
  * At most ASPEN_B200_NOALLOC_MAX_TILES blocks of 128 x 128 outputs, i.e. ceil(m/128) * ceil(n_cols/128) <= 4096; a larger
  * call fails with -2 and changes nothing.
  * The call waits for its own work on `cuda_stream` and returns after the work has finished.  Returns 0, -1 bad arguments,
