@@ -13,7 +13,6 @@
 #include <algorithm>
 #include <memory>
 #include <mutex>
-#include <queue>
 #include <sched.h>
 #include <unordered_map>
 
@@ -856,27 +855,16 @@ static NasmDev graph_image(const nasm_t *nasm) {
     return G;
 }
 
-// Several graphs in one launch: all of them progress at the same share of their runs.
+// The order of a launch of several graphs.
 static sched::Entry *merge_orders(Engine *e, const std::vector<nasm_t *> &graphs, unsigned claims) {
     std::vector<unsigned long long> of;
     for (const nasm_t *n : graphs) of.push_back(n->dev->serial);
     if (MergedOrder *known = e->orders.find(of)) return known->tiles;
+    std::vector<const ClaimOrder *> each;
+    for (const nasm_t *n : graphs) each.push_back(&n->dev->claims);
     std::vector<sched::Entry> order;
     order.reserve(claims);
-    typedef std::pair<float, unsigned> Next;                   // start of a graph's next tile; the graph
-    std::priority_queue<Next, std::vector<Next>, std::greater<Next>> next;
-    std::vector<size_t> place(graphs.size(), 0);
-    auto push = [&](unsigned g) {
-        const ClaimOrder &c = graphs[g]->dev->claims;
-        if (place[g] < c.tile.size()) next.push(Next(c.at[place[g]], g));
-    };
-    for (unsigned g = 0; g < graphs.size(); g++) push(g);
-    while (!next.empty()) {
-        const unsigned g = next.top().second, t = graphs[g]->dev->claims.tile[place[g]++];
-        next.pop();
-        order.push_back(sched::make_entry(t, g, graphs[g]->dev->tile_layer[t]));
-        push(g);
-    }
+    for (const Claim &c : merge_claims(each)) order.push_back(sched::make_entry(c.tile, c.graph, graphs[c.graph]->dev->tile_layer[c.tile]));
     // With more sets than are kept the memory of one that goes is used again: cudaFree would wait for all that runs on the device.  Whatever
     // launch read it is ahead on the stream.
     MergedOrder made;

@@ -185,9 +185,13 @@ nasm_t *plan_device_tiles(const nasm_t *nasm, int precision, unsigned int sms, b
 struct ClaimOrder {
     std::vector<unsigned> tile;    // parents before children
     std::vector<float> at;         // start, as a share of the whole run
+    float us = 0;                  // the whole run
+    unsigned runs = 0;             // the tiles behind these have lists that cannot be satisfied
 };
 ClaimOrder claim_order(const nasm_t *plan, int precision, unsigned workers, const std::vector<std::vector<unsigned>> &children, const std::vector<unsigned> &need,
                        const std::vector<bool> &skip);
+struct Claim { unsigned graph, tile; };
+std::vector<Claim> merge_claims(const std::vector<const ClaimOrder *> &graphs);      // one launch of several graphs (plan.cpp)
 nasm_t *own_device_tiles(const nasm_t *nasm);      // plan.cpp: the nasm's tiles, columns a multiple of 16 bytes apart
 int engine_current_device();
 Engine *engine_create(int device, int precision, unsigned int num_dse_hint);

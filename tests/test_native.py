@@ -129,3 +129,8 @@ def test_calls_that_run_at_once_have_numbers_of_their_own(workdir):
 
 def test_sets_of_graphs_that_are_run_in_turn_are_kept(workdir):
     passes(build("recent_sets", workdir))
+
+
+def test_a_launch_of_several_graphs_has_the_small_ones_done_first(workdir):
+    api.lib()
+    passes(build("merge_claims", workdir, f"-L{LIBDIR}", "-laspen_b200", f"-Wl,-rpath,{LIBDIR}"))
