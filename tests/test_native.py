@@ -123,6 +123,13 @@ def test_shapes_that_test_the_split_kernels_run_them(workdir):
     assert len(seen) == 6
 
 
+@pytest.mark.parametrize("n,k,m,values,us", [(446, 167, 2114, 1, (31.6, 37.7)), (727, 178, 1253, 2, (27.6, 31.4)), (395, 23, 2300, 1, (18.9, 25.5)), (3566, 143, 512, 1, (40.6, 56.5)),
+                                             (709, 232, 1421, 4, (36.8, 39.1))])
+def test_short_sums_of_many_outputs_run_in_large_blocks(n, k, m, values, us, workdir):
+    """us: of a call on a B200, in 128 x 64 blocks and in 32 x 32 ones."""
+    assert subprocess.run([build("matmul_pick", workdir), *(str(v) for v in (n, k, m, 148, values))], capture_output=True, text=True, check=True).stdout == "fma 128x64"
+
+
 def test_calls_that_run_at_once_have_numbers_of_their_own(workdir):
     passes(build("call_slots", workdir, "-lpthread"), timeout=60)
 
