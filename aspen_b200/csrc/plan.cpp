@@ -43,9 +43,10 @@ Path path_of(const aspen_layer_t *l, int precision, unsigned seq) { return preci
 // place of 0.28) 2479, 1473 and 1387.
 // Beside the ring (measured): 64 x 32 blocks, 0.8 us and 1.0 per 32 of k (3 x 3 layers of 48 and 24 channels), 1.6 where operands
 // come value by value (attention with heads of 10); the softmax of scores 1.4 us per 1024.
-// `ks` > 1: one of ks tiles that share k; they write and read their sums and wait for each other's counts, some 3 us.
+// `ks` > 1: one of ks tiles that share k; they wait for each other's counts, some 3 us, each writes its sums and the last one reads all of
+// them, 12 KB a us.
 double tile_us(Path path, const aspen_layer_t *l, unsigned th, unsigned tw, unsigned k, double gap, unsigned ks = 1) {
-    if (ks > 1) return tile_us(path, l, th, tw, ceil_div(k, ks), gap + 3.0);
+    if (ks > 1) return tile_us(path, l, th, tw, ceil_div(k, ks), gap + 3.0 + 4.0 * th * tw * (ks + 1) / 12e3);
     if (path == TENSOR) {
         const unsigned chunks = ceil_div(k, 32), nb = ceil_div(tw, 128) * ceil_div(th, 256), rows = std::min(th, 256u);
         const double loop = chunks * (rows > 128 ? 0.38 : rows > 64 ? 0.28 : 0.19), epi = 0.6 + 0.4 * ceil_div(rows, 32);
@@ -102,11 +103,13 @@ Grid choose(const nasm_ldata_t &ld, const nasm_t *nasm, int precision, unsigned 
                 const double cost = us * (served ? share + 0.4 : std::max(1.0, share + 0.5));
                 if (best == 0 || cost < best * 0.999) { best = cost; g.th = hs[i]; g.tw = tw; g.ks = 1; }
                 // Launched alone in the fp32 mode, a layer that leaves SMs idle shares its k among them: 512 x 49 outputs with k = 4608 are 32
-                // tiles of 48 us, or 128 of 14; ResNet-50 x 1 988 -> 916 us a pass.  (Not on the tensor cores, where a sample's bits
-                // are the same in every batch.)
+                // tiles of 48 us, or 128 of 14; ResNet-50 x 1 959 -> 820 us a pass, BERT 1 x 37 1508 -> 1472.  (Not on the tensor cores, where a
+                // sample's bits are the same in every batch.)  The tiles of all parts count as a layer's others do: as if they cost one tile
+                // however full they leave the chip, 256 x 128 tiles in three parts were chosen for 336 of 64 x 64 (BERT 2 x 200 4817 us a pass;
+                // without any sharing 3897, so 3898; 3 x 50 2355, 1953, 1953; VGG-16 x 1 1433, 1352, 1353; ResNet-50 x 3 1578, 1477, 1477).
                 if (!served && !ka && !va && path == FP32)
                     for (unsigned ks = 2; ks <= 8 && ks * tiles <= sms && k / ks >= 128; ks++) {
-                        const double split = tile_us(path, l, std::min(hs[i], H), std::min(tw, g.seg), k, 2.5, ks);
+                        const double split = tile_us(path, l, std::min(hs[i], H), std::min(tw, g.seg), k, 2.5, ks) * std::max(1.0, ks * share + 0.5);
                         if (split < best * 0.95) { best = split; g.th = hs[i]; g.tw = tw; g.ks = ks; }
                     }
             }
