@@ -58,10 +58,13 @@ double tile_us(Path path, const aspen_layer_t *l, unsigned th, unsigned tw, unsi
         return gap + ceil_div(th, 64) * ceil_div(tw, 32) * (0.8 + ceil_div(k, 32) * (pieces ? 1.0 : 1.6)) + softmax;
     }
     // fp32 blocks (gemm_ffma.cuh), shapes as tile_gemm_ffma picks them: some 3 us for filling the pipeline, the reduction and the
-    // stores, then steps of 32, 64 or 128 of k
+    // stores, then steps of 32, 64 or 128 of k.  Attention, measured: scores of 200 keys x 64 queries, k = 64, 33 us; values, staged one by one,
+    // 64 x 64 with k = 50 and 200 17 and 28 us.
     const int shape = th > 64 && tw > 32 ? 0 : th > 32 && tw > 32 ? 1 : 2;
     const unsigned bm = shape == 0 ? 128 : shape == 1 ? 64 : 32, bn = shape == 2 ? 32 : 64, kt = 32u << shape;
-    return gap + (double)ceil_div(th, bm) * ceil_div(tw, bn) * (3.0 + ceil_div(k, kt) * (shape == 2 ? 1.3 : 2.0));
+    const bool ka = l->type == K_ATTENTION_LAYER, va = l->type == V_ATTENTION_LAYER;
+    const double step = (shape == 2 ? 1.3 : 2.0) + (va ? 1.5 : 0), attention = ka ? 6.0 + 1.4 * th * tw / 1024 : va ? 11.0 : 0;
+    return gap + (double)ceil_div(th, bm) * ceil_div(tw, bn) * (3.0 + ceil_div(k, kt) * step) + attention;
 }
 
 Grid choose(const nasm_ldata_t &ld, const nasm_t *nasm, int precision, unsigned sms, bool served) {
@@ -88,7 +91,7 @@ Grid choose(const nasm_ldata_t &ld, const nasm_t *nasm, int precision, unsigned 
         for (unsigned i = 0; i < nhs; i++)
             for (unsigned tw = quantum; tw < g.seg + quantum && tw <= 16 * quantum; tw += quantum) {
                 const unsigned tiles = ceil_div(H, hs[i]) * (W / g.seg) * ceil_div(g.seg, tw);
-                const double us = tile_us(path, l, std::min(hs[i], H), std::min(tw, g.seg), k, served ? 4.0 : 2.5);
+                const double us = tile_us(path, l, std::min(hs[i], H), std::min(tw, g.seg), k, served || path == FP32 ? 4.0 : 2.5);
                 const double share = (double)tiles / sms;
                 // Launched alone a layer of fewer tiles than SMs takes as long as one tile; of a larger one the last tiles run while
                 // half of the chip waits.  (The work and 0.7 tiles whatever the number: ResNet-50 x 3 617 us a pass instead of 570,
@@ -100,13 +103,16 @@ Grid choose(const nasm_ldata_t &ld, const nasm_t *nasm, int precision, unsigned 
                 // graphs 3464 / 3370 / 3164, with four 3776 / 3671 / 3630, six 4463 / 4500 / 4680, eight 6997 / 7129 / 7508; x 16 with four
                 // 10647 / 10329 / 10408, eight 14420 / 14611 / 14748; x 32 with three 15399 / 14673 / 14598, six 20418 / 20417 / 20795; BERT 4 x 128 with
                 // four 9640 / 10061 / 10044, eight 12249 / 13151 / 13232.
-                const double cost = us * (served ? share + 0.4 : std::max(1.0, share + 0.5));
+                // (fp32 mode, launched, us a pass with 0.5 and 2.5 us between two tiles as for the tensor cores, and with 0.3 and 4.0: BERT 4 x 200 6173 and
+                // 5935, 6 x 128 5332 and 5040, 16 x 128 12858 and 12298, VGG-16 x 8 8379 and 8150, ResNet-50 x 4 1697 and 1655, BERT 1 x 37 1474 and 1476.)
+                const double rest = path == FP32 ? 0.3 : 0.5;
+                const double cost = us * (served ? share + 0.4 : std::max(1.0, share + rest));
                 if (best == 0 || cost < best * 0.999) { best = cost; g.th = hs[i]; g.tw = tw; g.ks = 1; }
                 // Launched alone in the fp32 mode, a layer that leaves SMs idle shares its k among them: 512 x 49 outputs with k = 4608 are 32
-                // tiles of 48 us, or 128 of 14; ResNet-50 x 1 959 -> 820 us a pass, BERT 1 x 37 1508 -> 1472.  (Not on the tensor cores, where a
+                // tiles of 48 us, or 128 of 14; ResNet-50 x 1 959 -> 824 us a pass, BERT 1 x 37 1508 -> 1476.  (Not on the tensor cores, where a
                 // sample's bits are the same in every batch.)  The tiles of all parts count as a layer's others do: as if they cost one tile
-                // however full they leave the chip, 256 x 128 tiles in three parts were chosen for 336 of 64 x 64 (BERT 2 x 200 4817 us a pass;
-                // without any sharing 3897, so 3898; 3 x 50 2355, 1953, 1953; VGG-16 x 1 1433, 1352, 1353; ResNet-50 x 3 1578, 1477, 1477).
+                // however full they leave the chip, 256 x 128 tiles in three parts were chosen for 336 of 64 x 64 (BERT 2 x 200 4817 us a pass,
+                // without any sharing 3897, so 3898; 3 x 50 2355, 1953, 1953; ResNet-50 x 3 1578, 1477, 1477).
                 if (!served && !ka && !va && path == FP32)
                     for (unsigned ks = 2; ks <= 8 && ks * tiles <= sms && k / ks >= 128; ks++) {
                         const double split = tile_us(path, l, std::min(hs[i], H), std::min(tw, g.seg), k, 2.5, ks) * std::max(1.0, ks * share + 0.5);
